@@ -62,6 +62,7 @@ struct to_gen_s {
     double* d_results;                   // [RS][8]
     to_csc csc;                          // [RS*C] packed migration matrices
     int* d_counts = nullptr;             // [max_roads] road cell counts (device rasterisation)
+    unsigned* d_bits = nullptr;          // [max_roads][raster_words] the roads' cell bitmaps
     float* d_feat = nullptr;             // [max_roads][16] surrogate features
     // captured generation (opts.graph)
     cudaGraphExec_t exec = nullptr;
@@ -338,7 +339,7 @@ to_status evaluate_direct(to_ctx ctx, to_gen g, int R, const int* cell_off,
     if (!cell_off) {
         // road cells from the segments, on the device
         TO_TRY(to_k::rasterise_roads(ctx, R, seg_off, segs, g->W, g->H, g->xs, g->ys, o->sem,
-                                     g->d_cell_off, g->d_cells, g->max_cells, g->d_counts));
+                                     g->d_cell_off, g->d_cells, g->max_cells, g->d_counts, g->d_bits));
         cell_off = g->d_cell_off;
         cells = g->d_cells;
     }
@@ -454,7 +455,7 @@ to_status evaluate(to_ctx ctx, to_gen g, int R, const int* cell_off,
     to_status st = TO_OK;
     if (!cell_off) {
         st = to_k::rasterise_roads(ctx, R, seg_off, segs, g->W, g->H, g->xs, g->ys, o->sem,
-                                   g->d_cell_off, g->d_cells, g->max_cells, g->d_counts);
+                                   g->d_cell_off, g->d_cells, g->max_cells, g->d_counts, g->d_bits);
         a.cell_off = g->d_cell_off;
         a.cells = g->d_cells;
     }
@@ -582,6 +583,7 @@ to_status to_scene_create(to_ctx ctx, const to_scene* sc, to_gen* out) {
     acc(RS * 5 * 8);
     acc((RS * TO_RESULT_STRIDE + 64) * 8);
     acc((R + 1) * 4);
+    acc(R * to_k::raster_words(g->W, g->H) * 4);
     acc(R * 16 * 4);
     acc(R * g->n_label_types * n * 4);
     const size_t cap = (size_t)NP * 32;
@@ -618,6 +620,7 @@ to_status to_scene_create(to_ctx ctx, const to_scene* sc, to_gen* out) {
     g->d_stats = carve<double>(p, RS * 5);
     g->d_results = carve<double>(p, RS * TO_RESULT_STRIDE + 64);
     g->d_counts = carve<int>(p, R + 1);
+    g->d_bits = carve<unsigned>(p, R * to_k::raster_words(g->W, g->H));
     g->d_feat = carve<float>(p, R * 16);
     g->d_labels = carve<int>(p, R * g->n_label_types * n);
     g->csc.ptr = carve<int>(p, RS * C * (NP + 1));
@@ -928,7 +931,7 @@ to_status to_road_features_d(to_ctx ctx, to_gen g, int R, const int* seg_off,
     cudaSetDevice(ctx->device);
     if (!cell_off) {
         TO_TRY(to_k::rasterise_roads(ctx, R, seg_off, segs, g->W, g->H, g->xs, g->ys, TO_SEM_CORRECTED,
-                                     g->d_cell_off, g->d_cells, g->max_cells, g->d_counts));
+                                     g->d_cell_off, g->d_cells, g->max_cells, g->d_counts, g->d_bits));
         cell_off = g->d_cell_off;
         cells = g->d_cells;
     }

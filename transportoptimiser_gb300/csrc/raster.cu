@@ -7,16 +7,16 @@
 // grid lines x = k xs and y = k ys, the span's points are sorted by (x, y)
 // (ascending when the span runs towards larger x, else descending), equal
 // neighbours are dropped, and each piece between consecutive points lies in
-// the cell (ceil(mid_x / xs), ceil(mid_y / ys)) of its midpoint.  Here a CTA
-// per road has each warp take one span at a time: the lanes write the
-// span's crossings to shared memory, rank them (the same order an
+// the cell (ceil(mid_x / xs), ceil(mid_y / ys)) of its midpoint.  Here a
+// warp takes one span at a time, whatever road it belongs to: the lanes
+// write the span's crossings to shared memory, rank them (the same order an
 // insertion sort gives: a point's rank counts the points before it, ties
-// by position), and mark the midpoint cells of consecutive points in a
-// shared-memory bitmap of the grid; the road's cells leave in ascending
-// order.  The arithmetic is the reference's, operation for operation, in
-// double; `sem` 0 keeps its quirk for the x of a vertical-line crossing
-// (computed from row q of the crossing list, RoadCells.cpp:189-194), 1 uses
-// the crossing's own y.
+// by position), and mark the midpoint cells of consecutive points in the
+// road's bitmap of the grid; a CTA per road then writes the cells in
+// ascending order.  The arithmetic is the reference's, operation for
+// operation, in double; `sem` 0 keeps its quirk for the x of a
+// vertical-line crossing (computed from row q of the crossing list,
+// RoadCells.cpp:189-194), 1 uses the crossing's own y.
 #include "to_internal.cuh"
 #include "to_model.cuh"
 
@@ -38,19 +38,41 @@ struct RasterArgs {
     int* flags;
 };
 
-// marks the cells of road r in the bitmap (W*H bits); scratch: per warp
-// two buffers of kSpanMax points
-__device__ void mark_road(int r, const RasterArgs& a, unsigned* bits, SpanPt* scratch) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    SpanPt* raw = scratch + (size_t)warp * 2 * kSpanMax;
-    SpanPt* srt = raw + kSpanMax;
+// What bounds it: the FP64 pipe (2 lanes a cycle and SM on this part) and,
+// at a few dozen points a span, latency.  So: no rank by comparing every
+// pair of points (n^2 FP64 comparisons a span) - the crossings of the
+// vertical grid lines and those of the horizontal ones each come out in
+// order, so a point's rank is its place in its own list plus a binary
+// search in the other; the pairwise ranks remain for spans where a list is
+// not in order (semantics 0, or rows of equal x); no division by a spacing
+// of 1; spans instead of roads as the unit of work, so that no CTA waits
+// for a road of 64 spans; and each span worked on once - the bitmaps stay
+// in global memory (5 KB a road) between counting and writing.  256 roads
+// of 8-64 points on 200 x 200 cells: 6.0 -> 0.20 ms.
+__global__ void __launch_bounds__(kRasterWarps * 32)
+k_raster_mark(int R, RasterArgs a, unsigned* __restrict__ bitmaps, int nwords) {
+    extern __shared__ __align__(16) unsigned char sm_raster[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    SpanPt* raw = reinterpret_cast<SpanPt*>(sm_raster) + (size_t)warp * kSpanMax;
+    unsigned short* order = reinterpret_cast<unsigned short*>(
+        sm_raster + (size_t)kRasterWarps * kSpanMax * sizeof(SpanPt)) + (size_t)warp * kSpanMax;
     const double xs = a.xs, ys = a.ys;
-    const int g0 = a.seg_off[r], g1 = a.seg_off[r + 1];
-    for (int g = g0 + warp; g < g1; g += nw) {
+    const bool ux = xs == 1.0, uy = ys == 1.0;            // v / 1 is v
+    auto dx = [&](double v) { return ux ? v : v / xs; };
+    auto dy = [&](double v) { return uy ? v : v / ys; };
+    const int g1 = a.seg_off[R];
+    for (int g = a.seg_off[0] + blockIdx.x * kRasterWarps + warp; g < g1;
+         g += gridDim.x * kRasterWarps) {
+        int r = 0, top = R;                               // the span's road
+        while (top - r > 1) {
+            const int mid = (r + top) >> 1;
+            if (a.seg_off[mid] <= g) r = mid; else top = mid;
+        }
+        unsigned* bits = bitmaps + (size_t)r * nwords;
         const double x0 = a.segs[4 * (size_t)g], y0 = a.segs[4 * (size_t)g + 1];
         const double x1 = a.segs[4 * (size_t)g + 2], y1 = a.segs[4 * (size_t)g + 3];
-        const int h = (int)(x1 / xs) - (int)(x0 / xs);
-        const int v = (int)(y1 / ys) - (int)(y0 / ys);
+        const int h = (int)dx(x1) - (int)dx(x0);
+        const int v = (int)dy(y1) - (int)dy(y0);
         const int ah = h < 0 ? -h : h, av = v < 0 ? -v : v, n = ah + av;
         if (n > kSpanMax) {                    // longer than any span inside the grid
             if (lane == 0 && a.flags) atomicExch(a.flags, TO_DEVERR_CELL);
@@ -59,21 +81,19 @@ __device__ void mark_road(int r, const RasterArgs& a, unsigned* bits, SpanPt* sc
         const double m = (y1 - y0) / (x1 - x0), b = y0 - x0 * m;
         const double m2 = (x1 - x0) / (y1 - y0), b2 = x0 - y0 * m2;
         const bool mf = isfinite(m), m2f = isfinite(m2);
+        // first grid line and step of each list
+        const double hx = h > 0 ? floor(dx(x0)) + 1.0
+                                : ceil(dx(x0)) - (fmod(x0, xs) == 0.0 ? 0.0 : 1.0);
+        const double vy = v > 0 ? floor(dy(y0)) + 1.0
+                                : ceil(dy(y0)) - (fmod(y0, ys) == 0.0 ? 0.0 : 1.0);
+        const double hs = h > 0 ? 1.0 : -1.0, vs = v > 0 ? 1.0 : -1.0;
         for (int q = lane; q < ah; q += 32) {
-            double px;
-            if (h > 0) px = xs * (floor(x0 / xs) + (double)(q + 1));
-            else if (fmod(x0, xs) == 0.0) px = xs * (ceil(x0 / xs) - (double)q);
-            else px = xs * (ceil(x0 / xs) - (double)(q + 1));
+            const double px = xs * (hx + hs * (double)q);  // whole numbers: exact
             raw[q].x = px;
             raw[q].y = mf ? m * px + b : y0;
         }
-        for (int q = lane; q < av; q += 32) {
-            double py;
-            if (v > 0) py = ys * (floor(y0 / ys) + (double)(q + 1));
-            else if (fmod(y0, ys) == 0.0) py = ys * (ceil(y0 / ys) - (double)q);
-            else py = ys * (ceil(y0 / ys) - (double)(q + 1));
-            raw[ah + q].y = py;
-        }
+        for (int q = lane; q < av; q += 32) raw[ah + q].y = ys * (vy + vs * (double)q);
+        for (int q = lane; q < n; q += 32) order[q] = (unsigned short)q;
         __syncwarp();
         for (int q = lane; q < av; q += 32) {
             const double src = (a.sem == 0) ? raw[q].y : raw[ah + q].y;
@@ -81,25 +101,49 @@ __device__ void mark_road(int r, const RasterArgs& a, unsigned* bits, SpanPt* sc
         }
         __syncwarp();
         const bool asc = x1 >= x0;
-        for (int i = lane; i < n; i += 32) {
-            const SpanPt pi = raw[i];
-            int rank = 0;
-            for (int j = 0; j < n; ++j) {
-                const SpanPt pj = raw[j];
-                const bool before = asc ? pt_less(pj, pi) : pt_less(pi, pj);
-                const bool tie = !pt_less(pj, pi) && !pt_less(pi, pj);
-                rank += (before || (tie && j < i)) ? 1 : 0;
+        auto before = [&](SpanPt p, SpanPt q) { return asc ? pt_less(p, q) : pt_less(q, p); };
+        // both lists in order?  (not a number is never in order)
+        bool bad = false;
+        for (int q = lane; q < n; q += 32) {
+            const SpanPt p = raw[q];
+            bad = bad || !(p.x == p.x && p.y == p.y) ||
+                  (q + 1 != ah && q + 1 < n && before(raw[q + 1], p));
+        }
+        if (!__any_sync(0xffffffffu, bad)) {
+            for (int i = lane; i < n; i += 32) {
+                const SpanPt pi = raw[i];
+                // points of the other list before this one; equal points keep
+                // their position's order (the first list's come first)
+                const bool first = i < ah;
+                const int base = first ? ah : 0;
+                int lo = 0, hi = first ? av : ah;
+                while (lo < hi) {
+                    const int mid = (lo + hi) >> 1;
+                    const SpanPt pj = raw[base + mid];
+                    if (first ? before(pj, pi) : !before(pi, pj)) lo = mid + 1; else hi = mid;
+                }
+                order[(first ? i : i - ah) + lo] = (unsigned short)i;
             }
-            srt[rank] = pi;
+        } else {
+            for (int i = lane; i < n; i += 32) {
+                const SpanPt pi = raw[i];
+                int rank = 0;
+                for (int j = 0; j < n; ++j) {
+                    const SpanPt pj = raw[j];
+                    const bool tie = !pt_less(pj, pi) && !pt_less(pi, pj);
+                    rank += (before(pj, pi) || (tie && j < i)) ? 1 : 0;
+                }
+                order[rank] = (unsigned short)i;
+            }
         }
         __syncwarp();
         for (int k = lane; k <= n; k += 32) {
             SpanPt pa, pb;
-            if (k == 0) { pa.x = x0; pa.y = y0; } else pa = srt[k - 1];
-            if (k == n) { pb.x = x1; pb.y = y1; } else pb = srt[k];
+            if (k == 0) { pa.x = x0; pa.y = y0; } else pa = raw[order[k - 1]];
+            if (k == n) { pb.x = x1; pb.y = y1; } else pb = raw[order[k]];
             if (pa.x == pb.x && pa.y == pb.y) continue;
-            const double cxd = ceil((0.5 * (pa.x + pb.x) - 0.0) / xs);
-            const double cyd = ceil((0.5 * (pa.y + pb.y) - 0.0) / ys);
+            const double cxd = ceil(dx(0.5 * (pa.x + pb.x) - 0.0));
+            const double cyd = ceil(dy(0.5 * (pa.y + pb.y) - 0.0));
             if (!(cxd >= 0.0 && cxd < (double)a.W && cyd >= 0.0 && cyd < (double)a.H)) continue;
             const int c = (int)cxd + (int)cyd * a.W;
             atomicOr(&bits[c >> 5], 1u << (c & 31));
@@ -108,72 +152,50 @@ __device__ void mark_road(int r, const RasterArgs& a, unsigned* bits, SpanPt* sc
     }
 }
 
-__device__ __forceinline__ SpanPt* span_scratch(unsigned* bits, int nw) {
-    return reinterpret_cast<SpanPt*>(bits + ((nw + 3) & ~3));
-}
-
-__global__ void k_raster_count(int R, RasterArgs ra, int* __restrict__ counts) {
-    extern __shared__ __align__(16) unsigned bits[];
-    __shared__ int s_c;
-    const int r = blockIdx.x;
-    const int W = ra.W, H = ra.H;
-    const int nw = (W * H + 31) >> 5;
-    for (int i = threadIdx.x; i < nw; i += blockDim.x) bits[i] = 0u;
-    if (threadIdx.x == 0) s_c = 0;
-    __syncthreads();
-    mark_road(r, ra, bits, span_scratch(bits, nw));
-    __syncthreads();
+// cells of each road: a warp per road
+__global__ void __launch_bounds__(128)
+k_raster_count(int R, const unsigned* __restrict__ bitmaps, int nwords, int* __restrict__ counts) {
+    const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (r >= R) return;
+    const unsigned* bits = bitmaps + (size_t)r * nwords;
     int c = 0;
-    for (int i = threadIdx.x; i < nw; i += blockDim.x) c += __popc(bits[i]);
-    for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-    if ((threadIdx.x & 31) == 0) atomicAdd(&s_c, c);
-    __syncthreads();
-    if (threadIdx.x == 0) counts[r] = s_c;
+    for (int i = lane; i < nwords; i += 32) c += __popc(bits[i]);
+    c = __reduce_add_sync(0xffffffffu, c);
+    if (lane == 0) counts[r] = c;
 }
 
-// exclusive scan of counts[0..R) into off[0..R] (one CTA)
-__global__ void k_scan_counts(int R, const int* __restrict__ counts, int* __restrict__ off,
-                              int max_cells, int* flags) {
-    __shared__ int s_w[32];
-    const int nt = blockDim.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int carry = 0;
-    for (int b = 0; b < R; b += nt) {
-        const int i = b + threadIdx.x;
-        const int v = i < R ? counts[i] : 0;
-        int x = v;
-        for (int o = 1; o < 32; o <<= 1) {
-            int y = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane >= o) x += y;
-        }
-        if (lane == 31) s_w[warp] = x;
-        __syncthreads();
-        int wb = 0, tot = 0;
-        for (int w = 0; w < (nt >> 5); ++w) { if (w < warp) wb += s_w[w]; tot += s_w[w]; }
-        if (i < R) off[i] = carry + wb + x - v;
-        carry += tot;
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        off[R] = carry;
-        if (carry > max_cells && flags) atomicExch(flags, TO_DEVERR_PATCHES);
-    }
-}
+constexpr int kRasterWriteThreads = 256;
 
-__global__ void k_raster_write(int R, RasterArgs ra, const int* __restrict__ off, int max_cells,
-                               int* __restrict__ cells) {
-    extern __shared__ __align__(16) unsigned bits[];
+// offsets and cells in ascending order, a CTA per road; each adds up the
+// counts of the roads before it (a few hundred)
+__global__ void __launch_bounds__(kRasterWriteThreads)
+k_raster_write(int R, const unsigned* __restrict__ bitmaps, int nwords,
+               const int* __restrict__ counts, int* __restrict__ off, int max_cells,
+               int* __restrict__ cells, int* flags) {
     __shared__ int s_w[32];
+    __shared__ int s_base;
     const int r = blockIdx.x;
-    const int W = ra.W, H = ra.H;
-    const int nw = (W * H + 31) >> 5;
-    for (int i = threadIdx.x; i < nw; i += blockDim.x) bits[i] = 0u;
-    __syncthreads();
-    mark_road(r, ra, bits, span_scratch(bits, nw));
-    __syncthreads();
-    // ascending cell order: each thread takes a contiguous run of words
     const int nt = blockDim.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int chunk = (nw + nt - 1) / nt;
-    const int w0 = threadIdx.x * chunk, w1 = min(nw, w0 + chunk);
+    if (threadIdx.x == 0) s_base = 0;
+    __syncthreads();
+    int before = 0;
+    for (int i = threadIdx.x; i < r; i += nt) before += counts[i];
+    before = __reduce_add_sync(0xffffffffu, before);
+    if (lane == 0 && before) atomicAdd(&s_base, before);
+    __syncthreads();
+    const int base = s_base;
+    if (threadIdx.x == 0) {
+        off[r] = base;
+        if (r == R - 1) {
+            const int total = base + counts[r];
+            off[R] = total;
+            if (total > max_cells && flags) atomicExch(flags, TO_DEVERR_PATCHES);
+        }
+    }
+    // each thread takes a contiguous run of words
+    const unsigned* bits = bitmaps + (size_t)r * nwords;
+    const int chunk = (nwords + nt - 1) / nt;
+    const int w0 = threadIdx.x * chunk, w1 = min(nwords, w0 + chunk);
     int c = 0;
     for (int i = w0; i < w1; ++i) c += __popc(bits[i]);
     int x = c;
@@ -185,7 +207,7 @@ __global__ void k_raster_write(int R, RasterArgs ra, const int* __restrict__ off
     __syncthreads();
     int wb = 0;
     for (int w = 0; w < warp; ++w) wb += s_w[w];
-    int pos = off[r] + wb + x - c;
+    int pos = base + wb + x - c;
     for (int i = w0; i < w1; ++i) {
         unsigned b = bits[i];
         while (b) {
@@ -382,24 +404,31 @@ __global__ void k_road_features(int R, int W, int H, const int* __restrict__ bas
 
 namespace to_k {
 
+size_t raster_words(int W, int H) { return ((size_t)W * H + 31) >> 5; }
+
 to_status rasterise_roads(to_ctx ctx, int R, const int* seg_off, const double* segs, int W, int H,
                           double xs, double ys, int sem, int* cell_off, int* cells, int max_cells,
-                          int* counts_scratch) {
-    const size_t nw = (size_t)((W * H + 31) >> 5);
-    const size_t smem = ((nw + 3) & ~size_t(3)) * sizeof(unsigned) +
-                        (size_t)kRasterWarps * 2 * kSpanMax * sizeof(SpanPt);
-    if (smem > ctx->smem_optin)
+                          int* counts_scratch, unsigned* bits_scratch) {
+    const int nw = (int)raster_words(W, H);
+    const size_t smem = (size_t)kRasterWarps * kSpanMax * (sizeof(SpanPt) + sizeof(unsigned short));
+    // grids past about 780,000 cells stay refused (the entry points' limit)
+    if ((((size_t)nw + 3) & ~size_t(3)) * sizeof(unsigned) + (size_t)131072 > ctx->smem_optin)
         return to_set_error(ctx, TO_ERR_UNSUPPORTED, "grid %d x %d too large to rasterise", W, H);
     if (!(xs > 0.0) || !(ys > 0.0)) return to_set_error(ctx, TO_ERR_INVALID, "grid spacing");
     RasterArgs ra{seg_off, segs, W, H, sem, xs, ys, ctx->d_flags};
-    TO_CUDA(ctx, cudaFuncSetAttribute(k_raster_count, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)smem));
-    TO_CUDA(ctx, cudaFuncSetAttribute(k_raster_write, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    TO_CUDA(ctx, cudaFuncSetAttribute(k_raster_mark, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)smem));
     to_prof_begin(ctx, "rasterise");
-    k_raster_count<<<R, kRasterWarps * 32, smem, ctx->stream>>>(R, ra, counts_scratch);
-    k_scan_counts<<<1, 1024, 0, ctx->stream>>>(R, counts_scratch, cell_off, max_cells, ctx->d_flags);
-    k_raster_write<<<R, kRasterWarps * 32, smem, ctx->stream>>>(R, ra, cell_off, max_cells, cells);
+    TO_CUDA(ctx, cudaMemsetAsync(bits_scratch, 0, (size_t)R * nw * sizeof(unsigned), ctx->stream));
+    // the span count is device data: three CTAs of 72 KB shared memory an SM,
+    // each warp striding over the spans (at most 64 a road are usual)
+    const int sms = ctx->sm_count > 0 ? ctx->sm_count : TO_SM_TARGET;
+    const int blocks = (16 * R < 3 * sms) ? 16 * R : 3 * sms;
+    k_raster_mark<<<blocks, kRasterWarps * 32, smem, ctx->stream>>>(R, ra, bits_scratch, nw);
+    k_raster_count<<<(R + 3) / 4, 128, 0, ctx->stream>>>(R, bits_scratch, nw, counts_scratch);
+    k_raster_write<<<R, kRasterWriteThreads, 0, ctx->stream>>>(R, bits_scratch, nw, counts_scratch,
+                                                              cell_off, max_cells, cells,
+                                                              ctx->d_flags);
     to_prof_end(ctx);
     ctx->launches += 3;
     TO_CUDA(ctx, cudaGetLastError());

@@ -112,7 +112,9 @@ to_status line_segment_intersect(to_ctx ctx, int T, const double* d_xy1, int G,
 // keeps the reference's vertical-crossing quirk)
 to_status rasterise_roads(to_ctx ctx, int R, const int* seg_off, const double* segs, int W,
                           int H, double xs, double ys, int sem, int* cell_off, int* cells,
-                          int max_cells, int* counts_scratch);
+                          int max_cells, int* counts_scratch, unsigned* bits_scratch);
+// words of one road's bitmap (rasterise_roads' bits_scratch holds R of them)
+size_t raster_words(int W, int H);
 to_status road_features(to_ctx ctx, int R, int W, int H, const int* base, const float* popmap,
                         const int* seg_off, const double* segs, const int* cell_off,
                         const int* cells, float* feat);
