@@ -255,16 +255,12 @@ to_status run_choice(to_ctx ctx, to_gen g, const to_mte_args& m, int RS, int cho
 to_status rov_stage(to_ctx ctx, to_gen g, int R, int NE, int road0) {
     to_rov_args a = g->rov;
     a.nr = R; a.PT = R * a.P; a.G = R * a.C;
-    a.lblocks = (a.PT + 1023) / 1024;
     a.np = g->NP; a.ne = NE;
     a.n_patches = g->d_np; a.params = g->d_rov_params; a.init_pops = g->d_ip;
     a.caps = g->d_cp; a.mmm = g->d_mmm; a.road_ids = g->d_road_ids;
     a.stats = g->d_rov_stats;
     k_road_ids<<<(R + 127) / 128, 128, 0, ctx->stream>>>(R, road0, g->d_road_ids);
     TO_LAUNCHED(ctx);
-    // the kNN's per-query search radius starts from last year's; clear it
-    // so that every generation starts the same way
-    TO_CUDA(ctx, cudaMemsetAsync(a.kth, 0, (size_t)a.G * a.Q * sizeof(float), ctx->stream));
     to_csc csc = g->csc;
     if (csc.uent) {
         // every control's packed columns in one list per destination; at most
@@ -733,8 +729,6 @@ to_status to_scene_set_rov(to_ctx ctx, to_gen g, const to_rov_problem* t) {
     if (kmax > TO_KNN_KMAX) return to_set_error(ctx, TO_ERR_UNSUPPORTED, "k %d", kmax);
     const size_t PT = (size_t)NR * P, G = (size_t)NR * C;
     const size_t blk = (size_t)Rr * d + 2 * (size_t)Q;
-    const size_t nacc = (size_t)(d + 1) * (d + 4) / 2;   // sums a query (doubles)
-    const int lblocks = (int)((PT + 1023) / 1024);
     const size_t U1 = (size_t)(U > 0 ? U : 1);
     size_t bytes = 0;
     auto acc = [&](size_t b) { bytes += to_align256(b); };
@@ -742,15 +736,19 @@ to_status to_scene_set_rov(to_ctx ctx, to_gen g, const to_rov_problem* t) {
     acc(NR * 4); acc((size_t)NR * 5 * 8); acc((size_t)S * 8 * 4);
     acc((size_t)Y * PT * 4); acc(U1 * (Y + 1) * PT * 4); acc((size_t)S * (Y + 1) * PT * 4);
     acc((size_t)S * C * Y * PT * 4);
-    acc(G * d * P * 4); acc(G * d * P * 4); acc(G * P * 4); acc(G * 4); acc(G * 4);
-    acc((size_t)NR * d * 4); acc((size_t)NR * d * 4); acc(G * d * P * 4); acc(G * P * 4);
-    acc((size_t)NR * d * Rr * 4);
-    acc(G * (TO_KNN_GCELLS + 1) * 4); acc(G * sizeof(to_knn_grid)); acc(G * Q * 4);
-    acc(G * lblocks * 4); acc(G * d * 2 * 4); acc(4); acc(G * Q * nacc * 8);
-    acc(G * blk * 4);
     acc((size_t)Y * PT * 4); acc((size_t)Y * PT * 4); acc((size_t)Y * PT * 4);
-    acc((size_t)Y * S * PT * 4);
-    acc(G * Q); acc(G * Q * 4); acc(4); acc((size_t)NR * 4);
+    acc((size_t)NR * 4);
+    to_rov_args a;
+    memset(&a, 0, sizeof(a));
+    a.P = P; a.Y = Y; a.S = S; a.C = C; a.U = U; a.R = Rr; a.Q = Q;
+    a.nF = t->n_fuels; a.Cm = t->n_commodities; a.demand_idx = t->demand_idx;
+    a.sem = 1; a.road = 0; a.dt = t->dt; a.rrr = t->rrr;
+    a.unit_cost = t->unit_cost; a.unit_revenue = t->unit_revenue; a.scaling = 2.0f;
+    a.seed = t->seed; a.kmax = kmax; a.algo = 4; a.k_mult = 10;
+    a.touched = 1; a.reg_by_slot = 1; a.flags = ctx->d_flags;
+    to_k::rov_plan(a, NR);
+    acc((size_t)a.slots * G * blk * 4);
+    bytes += to_k::rov_scratch(a, NR, nullptr);
     cudaError_t e = cudaMalloc(&g->rov_buf, bytes);
     if (e != cudaSuccess) {
         g->rov_buf = nullptr;
@@ -761,14 +759,6 @@ to_status to_scene_set_rov(to_ctx ctx, to_gen g, const to_rov_problem* t) {
     TO_CUDA(ctx, cudaMemset(g->rov_buf, 0, bytes));
     g->rov_bytes = bytes;
     char* p = g->rov_buf;
-    to_rov_args a;
-    memset(&a, 0, sizeof(a));
-    a.P = P; a.Y = Y; a.S = S; a.C = C; a.U = U; a.R = Rr; a.Q = Q;
-    a.nF = t->n_fuels; a.Cm = t->n_commodities; a.demand_idx = t->demand_idx;
-    a.sem = 1; a.road = 0; a.dt = t->dt; a.rrr = t->rrr;
-    a.unit_cost = t->unit_cost; a.unit_revenue = t->unit_revenue; a.scaling = 2.0f;
-    a.seed = t->seed; a.kmax = kmax; a.algo = 4; a.k_mult = 10;
-    a.touched = 1; a.reg_one_year = 1; a.flags = ctx->d_flags;
     float* d_flows = carve<float>(p, C);
     float* d_unc = carve<float>(p, 6 * U1);
     float* d_fc = carve<float>(p, 16);
@@ -782,32 +772,12 @@ to_status to_scene_set_rov(to_ctx ctx, to_gen g, const to_rov_problem* t) {
     a.uRes = carve<float>(p, U1 * (Y + 1) * PT);
     a.totalPops = carve<float>(p, (size_t)S * (Y + 1) * PT);
     a.aars = carve<float>(p, (size_t)S * C * Y * PT);
-    a.xraw = carve<float>(p, G * d * P);
-    a.xn = carve<float>(p, G * d * P);
-    a.yv = carve<float>(p, G * P);
-    a.npts = carve<int>(p, G);
-    a.kc = carve<int>(p, G);
-    a.gmin = carve<float>(p, (size_t)NR * d);
-    a.gmax = carve<float>(p, (size_t)NR * d);
-    a.qax = carve<float>(p, (size_t)NR * d * Rr);
-    a.gsx = carve<float>(p, G * d * P);
-    a.gsi = carve<int>(p, G * P);
-    a.gcell = carve<int>(p, G * (TO_KNN_GCELLS + 1));
-    a.ggrid = carve<to_knn_grid>(p, G);
-    a.kth = carve<float>(p, G * Q);
-    a.lcnt = carve<int>(p, G * lblocks);
-    a.lkey = carve<unsigned>(p, G * d * 2);
-    a.knn_next = carve<int>(p, 1);
-    a.knn_acc = carve<double>(p, G * Q * nacc);
-    a.reg = carve<float>(p, G * blk);
     a.condExp = carve<float>(p, (size_t)Y * PT);
     a.optCont = carve<int>(p, (size_t)Y * PT);
     a.unitProfits = carve<float>(p, (size_t)Y * PT);
-    a.adjPops = carve<float>(p, (size_t)Y * S * PT);
-    a.qmark = carve<unsigned char>(p, G * Q);
-    a.qlist = carve<int>(p, G * Q);
-    a.qcount = carve<int>(p, 1);
     a.qroad = carve<unsigned>(p, NR);
+    a.reg = carve<float>(p, (size_t)a.slots * G * blk);
+    to_k::rov_scratch(a, NR, p);
     TO_CUDA(ctx, cudaMemcpy(d_flows, t->flows, C * sizeof(float), cudaMemcpyHostToDevice));
     if (U > 0)
         TO_CUDA(ctx, cudaMemcpy(d_unc, t->uncert, 6 * (size_t)U * sizeof(float),

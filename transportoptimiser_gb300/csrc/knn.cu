@@ -1,4 +1,6 @@
-// knn.cu - k nearest neighbours and multiple local linear regression.
+// knn.cu - k nearest neighbours by a warp per query: the kNN entry point, and
+// the ROV's regressions for roads of very many paths (knn_fit.cu has the
+// others).
 //
 // Reference: knn_cuda_with_indexes::knn (include/gpuCode/
 // knn_cuda_with_indexes.cu:475-618: a P x Q distance matrix, a per-query
@@ -11,11 +13,9 @@
 // or below it is searched among the stored keys (ties at the k-th place
 // broken by index): exactly the set the reference's stable insertion sort
 // returns.  The kNN entry point then sorts them by (squared distance,
-// index), as the reference returns them; the ROV sorts them by index.
-// Groups of at most 320 points keep every key in registers and search the
-// exact-k threshold on them, and their compaction already yields index
-// order, with no sort.  When the search fails (ties keep the count out of
-// the window), a 4 x 8-bit radix select on the same keys takes over.
+// index), as the reference returns them; the ROV sorts them by index.  When
+// the search fails (ties keep the count out of the window), a 4 x 8-bit
+// radix select on the same keys takes over.
 //
 // For the ROV the points of each control are first binned into a uniform
 // cell grid (k_knn_grid, a counting sort), so a threshold pass visits only
@@ -545,32 +545,23 @@ struct GridPass {
     }
 };
 
-// groups of at most this many points keep every key in registers (10 per
-// lane: the generation's groups hold about P/C = 256 points; fewer slots
-// send the larger groups to the cell grid, more cost every query the
-// empty slots) and search the threshold on them, without the cell grid.
-// (Copies of the search for 8 and 9 slots, taken by the smaller groups,
-// made the kernel slower: 40.3 -> 43.7 ms a 256-road generation.)
-constexpr int kRegKeys = 10;
-constexpr int kReg = 32 * kRegKeys;
-
 // Per regression group (road, control): bounding box of the normalised
 // points, a cell grid of about 32n/k cells (at most TO_KNN_GCELLS; a few
 // points per cell, since rows are set up 32 at a time and cost little), and
 // a counting sort of the points into it.  One CTA per group.
-__global__ void __launch_bounds__(1024) k_knn_grid(to_rov_args a) {
+__global__ void __launch_bounds__(1024) k_knn_grid(to_rov_args a, int slot) {
     const int c = blockIdx.x, d = a.S + 1, P = a.P;
-    const int n = a.npts[c], k = a.kc[c];
+    const size_t gs0 = (size_t)slot * a.G + c;
+    const int n = a.npts[gs0], k = a.kc[gs0];
     __shared__ int s_cnt[TO_KNN_GCELLS];
     __shared__ unsigned s_umin[TO_LSM_MAXD], s_umax[TO_LSM_MAXD];
     __shared__ int s_bad;
     __shared__ int s_wsum[32];
     __shared__ to_knn_grid s_g;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const float* xs = a.xn + (size_t)c * d * P;
+    const float* xs = a.xn + gs0 * d * P;
     if (tid < d) { s_umin[tid] = 0xFFFFFFFFu; s_umax[tid] = 0u; }
     if (tid == 0) s_bad = 0;
-    if (c == 0 && tid == 0) *a.knn_next = 0;     // work counter of k_knn_rov
     __syncthreads();
     for (int j = 0; j < d; ++j) {
         float lo = INFINITY, hi = -INFINITY;
@@ -635,8 +626,7 @@ __global__ void __launch_bounds__(1024) k_knn_grid(to_rov_args a) {
         a.ggrid[c] = g;
     }
     __syncthreads();
-    // groups the register search takes need only the box (T0), not the cells
-    if (!s_g.ok || n <= kReg) return;
+    if (!s_g.ok) return;
     int ncell = 1;
     for (int j = 0; j < d; ++j) ncell *= s_g.G[j];
     for (int i = tid; i < ncell; i += blockDim.x) s_cnt[i] = 0;
@@ -690,73 +680,13 @@ __global__ void __launch_bounds__(1024) k_knn_grid(to_rov_args a) {
 // query) items from a counter, so no warp waits on another: items differ a
 // lot in cost (queries outside the point cloud need wide radii).  A query's
 // threshold starts from its k-th distance of the year before, times
-// kSeedGrow (kSeedGrowReg where the keys are in registers).  After the
-// selection every lane accumulates the normal equations of neighbours lane,
-// lane+32, ... of the k nearest in ascending point index; the 32 partials
-// of each sum are added in lane order through shared memory, and the
-// item's sums are stored as doubles at its list position.  k_knn_solve
-// then solves one system per thread (FP64 square-root-free Cholesky,
-// to_lsm_math.h).
+// kSeedGrow.  After the selection every lane accumulates the normal
+// equations of neighbours lane, lane+32, ... of the k nearest in ascending
+// point index; the 32 partials of each sum are added in lane order through
+// shared memory, and the item's sums are stored as doubles at its list
+// position.  k_knn_solve then solves one system per thread (FP64
+// square-root-free Cholesky, to_lsm_math.h).
 constexpr float kSeedGrow = 1.4f;
-// the register search re-counts cheaply: it starts from last year's k-th
-// distance itself (about k keys qualify)
-constexpr float kSeedGrowReg = 1.0f;
-
-// The k nearest of keys held in registers (lane l holds points l, l+32,
-// ...): the threshold moves until exactly k keys are at or below it; where
-// equal keys straddle the k-th place, every key below the tied value is
-// taken and then the lowest-index keys at it - the k smallest by (key,
-// index).  The k points go to ws.sel in ascending point index (the order
-// the regression sums them in).  Returns the k-th smallest key, or -1 when
-// the threshold leaves the finite range (the caller falls back).
-__device__ float reg_select_exact(const float (&key)[kRegKeys], int k, int dim, float T,
-                                  WarpScratch& ws) {
-    const int lane = threadIdx.x & 31;
-    const unsigned lt_mask = (1u << lane) - 1u;
-    const float expo = 2.0f / (float)dim;
-    float lo = -1.0f, hi = -1.0f;
-    bool tie = false;
-    for (int iter = 0;; ++iter) {
-        if (iter == 200 || !(T < INFINITY) || !(T >= 0.0f)) return -1.0f;
-        unsigned mine = 0;
-#pragma unroll
-        for (int u = 0; u < kRegKeys; ++u) mine += (key[u] <= T) ? 1u : 0u;
-        const int cnt = (int)__reduce_add_sync(kFull, mine);
-        if (cnt == k) break;
-        if (!exact_step(cnt, k, expo, T, lo, hi)) { tie = true; break; }
-    }
-    // tie: lo and hi are adjacent floats, fewer than k keys <= lo and more
-    // than k <= hi, so the keys in between all equal hi
-    int need = 0;
-    if (tie) {
-        unsigned below = 0;
-#pragma unroll
-        for (int u = 0; u < kRegKeys; ++u) below += (key[u] < hi) ? 1u : 0u;
-        need = k - (int)__reduce_add_sync(kFull, below);
-    }
-    int pos = 0, eqs = 0;
-    unsigned top = 0;
-#pragma unroll
-    for (int u = 0; u < kRegKeys; ++u) {
-        bool take;
-        if (!tie) {
-            take = key[u] <= T;
-        } else {
-            const bool eq = key[u] == hi;
-            const unsigned me = __ballot_sync(kFull, eq);
-            take = key[u] < hi || (eq && eqs + __popc(me & lt_mask) < need);
-            eqs += __popc(me);
-        }
-        const unsigned m = __ballot_sync(kFull, take);
-        if (take) {
-            ws.sel[pos + __popc(m & lt_mask)] = pack_sel(key[u], lane + 32 * u);
-            top = max(top, __float_as_uint(key[u]));
-        }
-        pos += __popc(m);
-    }
-    __syncwarp();
-    return __uint_as_float(__reduce_max_sync(kFull, top));
-}
 
 // ws.sel[0..k) from (key, index) order into ascending index order: the
 // words swapped, one sort, swapped back
@@ -786,66 +716,55 @@ size_t knn_rov_smem() { return sizeof(WarpScratch) * kWarps; }
 
 template <int D>
 __global__ void __launch_bounds__(kWarps * 32, 4)
-k_knn_rov(to_rov_args a, int t) {
+k_knn_rov(to_rov_args a, int slot) {
     extern __shared__ __align__(16) unsigned char sm_raw[];
     constexpr int M = D + 1, NA = knn_acc_len<D>();
     constexpr int NS = knn_sums<D>();
     const int P = a.P, Q = a.Q;
     const int lane = threadIdx.x & 31;
     WarpScratch& ws = reinterpret_cast<WarpScratch*>(sm_raw)[threadIdx.x >> 5];
-    // (group, query) items, group g = road*C + control: every grid query, or
-    // the year's list of the queries the backward pass reads
-    const int items = a.touched ? *a.qcount : a.G * Q;
-    const bool qpow2 = (Q & (Q - 1)) == 0;
-    const int qshift = qpow2 ? __ffs(Q) - 1 : 0;
-    // two positions of the year's list a request (half the round trips to
-    // the counter) where the list holds at least two items a warp; one
-    // where it is short (a single road), so that no warp waits idle
+    // places of the year's tiles, each the grid queries of one group
+    const int items = a.ntiles[slot] * TO_ROV_TILE;
+    const int2* tiles = a.tiles + (size_t)slot * a.G * ((Q + TO_ROV_TILE - 1) / TO_ROV_TILE);
+    // two places a request (half the round trips to the counter) where there
+    // are at least two a warp; one where the list is short, so that no warp
+    // waits idle
     const int take = (items >= 2 * (int)gridDim.x * kWarps) ? 2 : 1;
     for (;;) {
         int l0 = 0;
-        if (lane == 0) l0 = atomicAdd(a.knn_next, take);
+        if (lane == 0) l0 = atomicAdd(a.ntiles + a.slots + slot, take);
         l0 = __shfl_sync(kFull, l0, 0);
         if (l0 >= items) break;
         for (int li = l0; li < l0 + take && li < items; ++li) {
-            const int item = a.touched ? a.qlist[li] : li;
-            const int c = qpow2 ? (item >> qshift) : item / Q;
-            const int qi = item - c * Q;
-            const int n = a.npts[c], k = a.kc[c];
+            const int2 tile = tiles[li / TO_ROV_TILE];
+            const int c = tile.x, at = tile.y + li % TO_ROV_TILE;
+            const size_t gs0 = (size_t)slot * a.G + c;
+            if (at >= a.gcount[gs0]) continue;
+            const int qi = a.touched ? a.qlist[gs0 * Q + at] : at;
+            const int n = a.npts[gs0], k = a.kc[gs0];
             if (n < 3 || k <= 0) continue;           // k_knn_solve writes 0
-            const float* xs = a.xn + (size_t)c * D * P;
+            const float* xs = a.xn + gs0 * D * P;
             const float* y = a.yv + (size_t)c * P;
-            const float* xr = a.xraw + (size_t)c * D * P;
+            const float* xr = a.xraw + gs0 * D * P;
             const float T0 = a.ggrid[c].T0;
             float* kth_prev = a.kth + (size_t)c * Q;
             const float kp = kth_prev[qi];
             float T = kp > 0.0f ? kp * kSeedGrow : T0;
             float qn[D], xq[D];
-            to_rov_query<D>(a, c / a.C, qi, qn, xq);
+            to_rov_query<D>(a, slot, c / a.C, qi, qn, xq);
             // the k nearest into ws.sel in ascending point index; kth = the k-th
             // smallest distance (squared)
             float kth = -1.0f;
-            if (n <= kReg) {
-                float key[kRegKeys];
-#pragma unroll
-                for (int u = 0; u < kRegKeys; ++u) {
-                    const int i = lane + 32 * u;
-                    key[u] = (i < n) ? sqdist(xs, P, i, D, qn) : INFINITY;
-                }
-                kth = reg_select_exact(key, k, D, kp > 0.0f ? kp * kSeedGrowReg : T0, ws);
+            if (a.ggrid[c].ok) {
+                const to_knn_grid g = a.ggrid[c];
+                GridPass<D> gp{&g, a.gsx + (size_t)c * D * P, a.gsi + (size_t)c * P,
+                               a.gcell + (size_t)c * (TO_KNN_GCELLS + 1), P, qn, &ws, k};
+                kth = threshold_select(k, D, T, ws, gp);
             } else {
-                if (a.ggrid[c].ok) {
-                    // the cell grid, copied only where it is used
-                    const to_knn_grid g = a.ggrid[c];
-                    GridPass<D> gp{&g, a.gsx + (size_t)c * D * P, a.gsi + (size_t)c * P,
-                                   a.gcell + (size_t)c * (TO_KNN_GCELLS + 1), P, qn, &ws, k};
-                    kth = threshold_select(k, D, T, ws, gp);
-                } else {
-                    ScanPass sp{xs, P, n, D, qn, &ws};
-                    kth = threshold_select(k, D, T, ws, sp);
-                }
-                if (kth >= 0.0f) to_index_order(ws, k);
+                ScanPass sp{xs, P, n, D, qn, &ws};
+                kth = threshold_select(k, D, T, ws, sp);
             }
+            if (kth >= 0.0f) to_index_order(ws, k);
             if (kth < 0.0f) {                         // exact radix selection
                 warp_select(xs, P, n, D, qn, k, ws);
                 kth = __uint_as_float((unsigned)(ws.sel[k - 1] >> 32));
@@ -877,7 +796,7 @@ k_knn_rov(to_rov_args a, int t) {
                 to_lsm_acc_add(D, acc, to_lsm_weight_within(dd, h, rh), y[i], xv, xq);
             }
             // the item's NS sums, at its list position
-            double* sa = a.knn_acc + (size_t)li * NS;
+            double* sa = a.knn_acc + ((size_t)c * Q + at) * NS;
             // the normal-equation sums: every lane's partials into shared memory
             // (sum e in row e, lane in column, rows 33 wide), then lane e adds
             // row e's 32 partials in lane order
@@ -905,32 +824,32 @@ k_knn_rov(to_rov_args a, int t) {
     }
 }
 
-// One regression system per thread over the year's list, 128 at a time: a
-// chunk's sums (NS doubles a system, consecutive list positions) are copied
-// to shared memory word by word with consecutive threads on consecutive
-// words (rows padded to an odd stride), then each thread solves its own and
-// writes the intercept at grid query qi of group c (0 where the group has
-// too few points).
+// One regression system per thread, a tile at a time: its sums (NS doubles
+// a system, consecutive list positions) are copied to shared memory word by
+// word with consecutive threads on consecutive words (rows padded to an odd
+// stride), then each thread solves its own and writes the intercept at its
+// grid query (0 where the group has too few points).
 template <int D>
-__global__ void __launch_bounds__(128) k_knn_solve(to_rov_args a, int t) {
+__global__ void __launch_bounds__(TO_ROV_TILE) k_knn_solve(to_rov_args a, int t, int slot) {
     constexpr int NS = knn_sums<D>(), NSP = NS | 1;
-    __shared__ double s[128 * NSP];
-    const int total = a.touched ? *a.qcount : a.G * a.Q;
-    for (int base = blockIdx.x * 128; base < total; base += gridDim.x * 128) {
-        const int cnt = min(128, total - base);
+    __shared__ double s[TO_ROV_TILE * NSP];
+    const int total = a.ntiles[slot], Q = a.Q;
+    const int2* tiles = a.tiles + (size_t)slot * a.G * ((Q + TO_ROV_TILE - 1) / TO_ROV_TILE);
+    for (int ti = blockIdx.x; ti < total; ti += gridDim.x) {
+        const int c = tiles[ti].x, start = tiles[ti].y;
+        const size_t gs0 = (size_t)slot * a.G + c;
+        const int cnt = min(TO_ROV_TILE, a.gcount[gs0] - start);
         __syncthreads();
-        const double* src = a.knn_acc + (size_t)base * NS;
-        for (int q = threadIdx.x; q < cnt * NS; q += 128) {
+        const double* src = a.knn_acc + ((size_t)c * Q + start) * NS;
+        for (int q = threadIdx.x; q < cnt * NS; q += TO_ROV_TILE) {
             const int i = q / NS;
             s[i * NSP + (q - i * NS)] = src[q];
         }
         __syncthreads();
         if ((int)threadIdx.x >= cnt) continue;
-        const int li = base + threadIdx.x;
-        const int item = a.touched ? a.qlist[li] : li;
-        if (item >= a.G * a.Q) continue;
-        const int c = item / a.Q, qi = item - c * a.Q;
-        const int n = a.npts[c], k = a.kc[c];
+        const int at = start + threadIdx.x;
+        const int qi = a.touched ? a.qlist[gs0 * Q + at] : at;
+        const int n = a.npts[gs0], k = a.kc[gs0];
         const float y = (n >= 3 && k > 0) ? to_lsm_solve_compact(D, s + threadIdx.x * NSP) : 0.0f;
         (to_rov_reg_block(a, t, c) + (size_t)a.R * D)[qi] = y;
     }
@@ -976,17 +895,17 @@ to_status launch_knn_rov(to_ctx ctx, const to_rov_args& a, int t) {
     TO_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_knn_rov<D>,
                                                                kWarps * 32, smem));
     if (per_sm < 1) per_sm = 1;
-    const int items = a.G * a.Q;
-    int grid = (ctx->sm_count > 0 ? ctx->sm_count : 152) * per_sm;
-    if (grid > (items + kWarps - 1) / kWarps) grid = (items + kWarps - 1) / kWarps;
+    const int sms = ctx->sm_count > 0 ? ctx->sm_count : TO_SM_TARGET;
+    const int tiles = a.G * ((a.Q + TO_ROV_TILE - 1) / TO_ROV_TILE);
+    int grid = sms * per_sm;
+    if (grid > tiles * (TO_ROV_TILE / kWarps)) grid = tiles * (TO_ROV_TILE / kWarps);
     to_prof_begin(ctx, "knn");
-    k_knn_rov<D><<<grid, kWarps * 32, smem, ctx->stream>>>(a, t);
+    k_knn_rov<D><<<grid, kWarps * 32, smem, ctx->stream>>>(a, t - a.slot0);
     to_prof_end(ctx);
     TO_LAUNCHED(ctx);
     to_prof_begin(ctx, "knn_solve");
-    const int sblocks = (items + 127) / 128;
-    const int smax = (ctx->sm_count > 0 ? ctx->sm_count : 152) * 16;
-    k_knn_solve<D><<<sblocks < smax ? sblocks : smax, 128, 0, ctx->stream>>>(a, t);
+    k_knn_solve<D><<<tiles < sms * 16 ? tiles : sms * 16, TO_ROV_TILE, 0, ctx->stream>>>(
+        a, t, t - a.slot0);
     to_prof_end(ctx);
     TO_LAUNCHED(ctx);
     return TO_OK;
@@ -1000,14 +919,10 @@ size_t knn_smem(int dim, int points) {
 
 namespace to_k {
 
-to_status knn_rov(to_ctx ctx, const to_rov_args& a, int t) {
+to_status knn_rov_grid(to_ctx ctx, const to_rov_args& a, int t) {
     const int d = a.S + 1;
-    if (a.kmax > TO_KNN_KMAX)
-        return to_set_error(ctx, TO_ERR_UNSUPPORTED, "k %d exceeds %d", a.kmax, TO_KNN_KMAX);
-    if (d < 2 || d > TO_LSM_MAXD)
-        return to_set_error(ctx, TO_ERR_UNSUPPORTED, "regression dimension %d", d);
     to_prof_begin(ctx, "knn_grid");
-    k_knn_grid<<<a.G, 1024, 0, ctx->stream>>>(a);
+    k_knn_grid<<<a.G, 1024, 0, ctx->stream>>>(a, t - a.slot0);
     to_prof_end(ctx);
     TO_LAUNCHED(ctx);
     switch (d) {

@@ -14,11 +14,11 @@
 //    for all years and evaluates all controls' migrations from one read of
 //    the populations; the random streams are regenerated from Philox where
 //    they are consumed (nothing of size P*Y*N is stored);
-//  * the reference's serial <<<1,1>>> compaction and min/max kernels become
-//    per-chunk counts, an ordered scatter and a per-road finish over all SMs;
-//  * kNN runs on the device (knn.cu): persistent warps, one query at a time,
-//    the same neighbour set and order as the reference's stable insertion
-//    sort without its P x Q distance matrix or host round trips;
+//  * the reference's serial <<<1,1>>> compaction and min/max kernels become a
+//    CTA per (road, year), all years independent of one another;
+//  * kNN and regressions run on the device (knn_fit.cu): a thread per grid
+//    query, the same neighbour set as the reference's stable insertion sort
+//    without its P x Q distance matrix or host round trips;
 //  * the local linear systems are accumulated in FP32 and solved in FP64
 //    (Cholesky); expectations are reduced in FP64;
 //  * several roads can be valued in one batch: paths are road-major and the
@@ -256,6 +256,22 @@ k_rov_forward(to_rov_args a) {
 }
 
 
+// Unit profits of every path and year: those the regression states hold
+// (profS) and those the decisions use (unitProfits) - the same but for
+// reference semantics, whose two kernels read their process arrays with
+// different strides.  A profit takes a Philox block and a Box-Muller pair,
+// and the states, the query marks and the decisions of a year all use it.
+__global__ void __launch_bounds__(256) k_rov_profit(to_rov_args a) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    const int t = 1 + blockIdx.y, Y = a.Y;
+    if (p >= a.PT) return;
+    const size_t at = (size_t)t * a.PT + p;
+    const float ps = unit_profit(a, p, t, Y + 1, Y + 1);
+    a.profS[at] = ps;
+    if (a.sem != 0) return;                    // profS is unitProfits
+    a.unitProfits[at] = (t == Y - 1) ? unit_profit(a, p, t, Y + 1, Y) : unit_profit(a, p, t, Y, Y);
+}
+
 // terminal year (backwardInduction :2375-2463)
 __global__ void k_rov_terminal(to_rov_args a) {
     int p = blockIdx.x * blockDim.x + threadIdx.x;
@@ -264,55 +280,15 @@ __global__ void k_rov_terminal(to_rov_args a) {
     float state[TO_ROV_MAXC * (TO_LSM_MAXD - 1) + 1];
     for (int c = 0; c < C; ++c)
         for (int s = 0; s < S; ++s) state[c * S + s] = adj_pop(a, p, t, s, c);
-    float prof = unit_profit(a, p, t, a.Y + 1, a.sem == 0 ? a.Y : a.Y + 1);
-    state[S * C] = prof;
+    state[S * C] = a.unitProfits[(size_t)t * a.PT + p];
     float best;
     int bc;
     to_rovd::decide_terminal(a, state, best, bc);
     a.condExp[(size_t)t * a.PT + p] = best;
     a.optCont[(size_t)t * a.PT + p] = bc;
-    a.unitProfits[(size_t)t * a.PT + p] = prof;
-    for (int s = 0; s < S; ++s)
-        a.adjPops[((size_t)t * S + s) * a.PT + p] = state[(C - 1) * S + s];
-}
-
-// Per year: regression states, stable compaction by the year's random
-// control (allocateXYRegressionData :1012-1069), per-control and global
-// min/max (computeStateMinMax :1073-1148), k, normalised points and the
-// axis values of the regression grid.  Points are grouped by (road,
-// control), g = r*C + c.  Launches over chunks of kLsmChunk paths:
-// per-chunk counts by group, then the scatter in path order (earlier
-// chunks of the road + earlier warps + rank among the warp's lanes of the
-// same group) with min/max folded into order-preserving integer keys; then
-// one thread per road for its totals, k, min/max rules and grid axes, and
-// the normalisation across the grid.
-
-constexpr int kLsmChunk = 1024;
-// roads of a batch have at least this many paths, so a chunk touches at
-// most kLsmChunk / kLsmMinPaths + 2 roads
-constexpr int kLsmMinPaths = 128;
-constexpr int kLsmLocal = (kLsmChunk / kLsmMinPaths + 2) * TO_ROV_MAXC;
-
-// the year's regression group of path p: (road, control) when every
-// species' adjusted population clears its threshold (or the control is 0),
-// else -1
-__device__ __forceinline__ int lsm_group(const to_rov_args& a, int p, int t) {
-    if (p >= a.PT) return -1;
-    const int ctl = a.controls[(size_t)t * a.PT + p];
-    const int g = (p / a.P) * a.C + ctl;
-    if (ctl == 0) return g;
-    for (int s = 0; s < a.S; ++s)
-        if (adj_pop(a, p, t, s, a.C - 1) < a.params[8 * s + 3]) return -1;
-    return g;
-}
-
-// first group of chunk b and how many groups it can hold
-__device__ __forceinline__ void lsm_chunk_groups(const to_rov_args& a, int b, int& g0, int& nloc) {
-    const int p0 = b * kLsmChunk;
-    const int p1 = min(p0 + kLsmChunk, a.PT) - 1;
-    const int r0 = p0 / a.P, r1 = p1 / a.P;
-    g0 = r0 * a.C;
-    nloc = (r1 - r0 + 1) * a.C;
+    if (a.adjPops)
+        for (int s = 0; s < S; ++s)
+            a.adjPops[((size_t)t * S + s) * a.PT + p] = state[(C - 1) * S + s];
 }
 
 // order-preserving unsigned key of a float (min/max through integer atomics)
@@ -325,283 +301,323 @@ __device__ __forceinline__ float lsm_unkey(unsigned k) {
     return __uint_as_float(k);
 }
 
-__global__ void __launch_bounds__(kLsmChunk) k_lsm_count(to_rov_args a, int t) {
-    __shared__ int s_cnt[kLsmLocal];
-    const int d = a.S + 1, tid = threadIdx.x, lane = tid & 31;
-    int g0, nloc;
-    lsm_chunk_groups(a, blockIdx.x, g0, nloc);
-    for (int q = tid; q < nloc; q += blockDim.x) s_cnt[q] = 0;
-    if (blockIdx.x == 0)
-        for (int q = tid; q < a.G * d; q += blockDim.x) {
-            a.lkey[2 * q] = 0xFFFFFFFFu;
-            a.lkey[2 * q + 1] = 0u;
-        }
-    __syncthreads();
-    const int grp = lsm_group(a, blockIdx.x * kLsmChunk + tid, t);
-    const unsigned peers = __match_any_sync(0xffffffffu, grp);
-    if (grp >= 0 && lane == __ffs(peers) - 1) atomicAdd(&s_cnt[grp - g0], __popc(peers));
-    __syncthreads();
-    for (int q = tid; q < nloc; q += blockDim.x)
-        a.lcnt[(size_t)(g0 + q) * gridDim.x + blockIdx.x] = s_cnt[q];
-}
+// What the regressions of one (road, year) are fitted on, one CTA each:
+//  1 the regression states of the road's paths, compacted stably by the
+//    year's random control (allocateXYRegressionData :1012-1069; a path
+//    whose species miss their thresholds under another control than 0 is
+//    left out), with their ranges (computeStateMinMax :1073-1148);
+//  2 counts, k, the reference's range rules and the grid axes
+//    (createQueryPoints :1187-1190);
+//  3 the normalised points (SimulateGPU.cu:4591-4603);
+//  4 touched-query mode: k_rov_backward at this year reads control c's
+//    regressions at the 2^d corners of the cell holding the path's own state
+//    for c (to_lsm_interp), for every control valid for the path; exactly
+//    those grid queries are marked in a bitmap;
+//  5 the bitmaps as one ascending query list per group, cut into tiles of
+//    TO_ROV_TILE for k_knn_select.
+// None of it depends on the values of later years, so a launch takes as many
+// years as the scratch holds.  Latency bound (a CTA is a chain of short
+// passes over a few hundred paths), which many CTAs an SM hide: 7.7 -> 1.5 ms
+// a 256-road generation, 3.6 -> 0.22 ms a road of 10,000 paths (six kernels
+// and a cell grid a year before).
+constexpr int kPrepThreads = 512;
+constexpr int kPrepBitmap = 32 * 1024;     // bytes of shared memory for the marks
 
-__global__ void __launch_bounds__(kLsmChunk) k_lsm_scatter(to_rov_args a, int t) {
-    const int P = a.P, S = a.S, C = a.C, d = S + 1, nb = gridDim.x;
-    __shared__ int s_off[kLsmLocal];
-    __shared__ int s_scan[kLsmLocal][32];
-    __shared__ unsigned s_key[kLsmLocal][TO_LSM_MAXD][2];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
-    int g0, nloc;
-    lsm_chunk_groups(a, blockIdx.x, g0, nloc);
-    // chunk offsets: warp q sums group q's counts in the road's earlier chunks
-    for (int q = warp; q < nloc; q += nw) {
-        const int g = g0 + q;
-        const int bfirst = (int)(((size_t)(g / C) * P) / kLsmChunk);
-        int acc = 0;
-        for (int b = bfirst + lane; b < (int)blockIdx.x; b += 32) acc += a.lcnt[(size_t)g * nb + b];
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        if (lane == 0) s_off[q] = acc;
-    }
-    for (int q = tid; q < nloc * 32; q += blockDim.x) s_scan[q >> 5][q & 31] = 0;
-    for (int q = tid; q < nloc * d; q += blockDim.x) {
+__global__ void __launch_bounds__(kPrepThreads) k_lsm_prepare(to_rov_args a) {
+    extern __shared__ unsigned s_bits[];
+    constexpr int NW = kPrepThreads / 32;
+    __shared__ int s_wcnt[NW][TO_ROV_MAXC];
+    __shared__ int s_base[TO_ROV_MAXC];
+    __shared__ unsigned s_key[TO_ROV_MAXC][TO_LSM_MAXD][2];
+    __shared__ float s_mn[TO_ROV_MAXC + 1][TO_LSM_MAXD], s_mx[TO_ROV_MAXC + 1][TO_LSM_MAXD];
+    __shared__ float s_lo[TO_LSM_MAXD], s_hi[TO_LSM_MAXD];      // ends of the raw axes
+    __shared__ int s_scan[NW];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int r = blockIdx.x, slot = blockIdx.y, t = a.slot0 + slot;
+    const int P = a.P, S = a.S, C = a.C, R = a.R, Q = a.Q, d = S + 1, Y = a.Y;
+    const size_t PT = (size_t)a.PT, p_0 = (size_t)r * P;
+    const size_t gs0 = (size_t)slot * a.G + (size_t)r * C;      // first group of the slot's road
+    float* xraw = a.xraw + gs0 * d * P;
+    int* pidx = a.pidx + gs0 * P;
+
+    // 1
+    for (int q = tid; q < C * d; q += kPrepThreads) {
         s_key[q / d][q % d][0] = 0xFFFFFFFFu;
         s_key[q / d][q % d][1] = 0u;
     }
-    __syncthreads();                     // zeroed before any warp adds to them
-    const int p = blockIdx.x * kLsmChunk + tid;
-    const int grp = lsm_group(a, p, t);
-    float xv[TO_LSM_MAXD];
-    if (grp >= 0) {
-        for (int s = 0; s < S; ++s) xv[s] = adj_pop(a, p, t, s, C - 1);
-        xv[S] = unit_profit(a, p, t, a.Y + 1, a.Y + 1);
-    }
-    // lanes of the same group: rank, count and min / max of the states
-    const unsigned peers = __match_any_sync(0xffffffffu, grp);
-    const int before = __popc(peers & ((1u << lane) - 1u));
-    const bool leader = lane == __ffs(peers) - 1;
-    if (grp >= 0) {
-        const int lq = grp - g0;
-        if (leader) s_scan[lq][warp] = __popc(peers);
-        for (int j = 0; j < d; ++j) {
-            const unsigned lo = __reduce_min_sync(peers, lsm_key(xv[j]));
-            const unsigned hi = __reduce_max_sync(peers, lsm_key(xv[j]));
-            if (leader) {
-                atomicMin(&s_key[lq][j][0], lo);
-                atomicMax(&s_key[lq][j][1], hi);
+    if (tid < C) s_base[tid] = 0;
+    for (int p0 = 0; p0 < P; p0 += kPrepThreads) {
+        for (int q = tid; q < NW * C; q += kPrepThreads) s_wcnt[q / C][q % C] = 0;
+        __syncthreads();                     // counts clear, keys set
+        const int pl = p0 + tid;
+        const size_t p = p_0 + pl;
+        int c = -1;
+        float xv[TO_LSM_MAXD];
+        if (pl < P) {
+            c = a.controls[(size_t)t * PT + p];
+            bool ok = true;
+            for (int s = 0; s < S; ++s) {
+                xv[s] = adj_pop(a, (int)p, t, s, C - 1);
+                if (xv[s] < a.params[8 * s + 3]) ok = false;
+            }
+            if (c != 0 && !ok) c = -1;
+            xv[S] = a.profS[(size_t)t * PT + p];
+        }
+        const unsigned peers = __match_any_sync(0xffffffffu, c);
+        const bool leader = lane == __ffs(peers) - 1;
+        if (c >= 0) {
+            if (leader) s_wcnt[warp][c] = __popc(peers);
+            for (int j = 0; j < d; ++j) {
+                const unsigned lo = __reduce_min_sync(peers, lsm_key(xv[j]));
+                const unsigned hi = __reduce_max_sync(peers, lsm_key(xv[j]));
+                if (leader) {
+                    atomicMin(&s_key[c][j][0], lo);
+                    atomicMax(&s_key[c][j][1], hi);
+                }
             }
         }
-    }
-    __syncthreads();
-    if (grp >= 0) {
-        const int lq = grp - g0;
-        int pos = s_off[lq] + before;
-        for (int w = 0; w < warp; ++w) pos += s_scan[lq][w];
-        a.yv[(size_t)grp * P + pos] = a.condExp[(size_t)(t + 1) * a.PT + p];
-        for (int j = 0; j < d; ++j) a.xraw[((size_t)grp * d + j) * P + pos] = xv[j];
-    }
-    for (int q = tid; q < nloc * d; q += blockDim.x) {
-        const int lq = q / d, j = q % d;
-        if (s_key[lq][j][1] != 0u) {     // the chunk holds points of the group
-            const size_t gq = (size_t)(g0 + lq) * d + j;
-            atomicMin(&a.lkey[2 * gq], s_key[lq][j][0]);
-            atomicMax(&a.lkey[2 * gq + 1], s_key[lq][j][1]);
+        __syncthreads();
+        if (c >= 0) {
+            int pos = s_base[c] + __popc(peers & ((1u << lane) - 1u));
+            for (int w = 0; w < warp; ++w) pos += s_wcnt[w][c];
+            pidx[(size_t)c * P + pos] = (int)p;
+            for (int j = 0; j < d; ++j) xraw[((size_t)c * d + j) * P + pos] = xv[j];
         }
+        __syncthreads();
+        if (tid < C) {
+            int n = s_base[tid];
+            for (int w = 0; w < NW; ++w) n += s_wcnt[w][tid];
+            s_base[tid] = n;
+        }
+        __syncthreads();                     // before the next chunk clears the counts
     }
-}
-
-// a warp per road, lanes over its (control, dimension, bin) items: group
-// totals, the reference's min/max rules, the road's combined range, k and
-// the regression grid axes
-constexpr int kStatsWarps = 4;
-
-__global__ void __launch_bounds__(kStatsWarps * 32) k_lsm_stats(to_rov_args a, int t, int nb) {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int r = blockIdx.x * kStatsWarps + w;
-    if (r >= a.nr) return;
-    __shared__ int s_cnt[kStatsWarps][TO_ROV_MAXC];
-    __shared__ float s_mn[kStatsWarps][TO_ROV_MAXC + 1][TO_LSM_MAXD];
-    __shared__ float s_mx[kStatsWarps][TO_ROV_MAXC + 1][TO_LSM_MAXD];
-    const int P = a.P, S = a.S, C = a.C, d = S + 1, R = a.R;
-    const int bfirst = (int)(((size_t)r * P) / kLsmChunk);
-    const int blast = (int)(((size_t)r * P + P - 1) / kLsmChunk);
-    int* cnt = s_cnt[w];
-    float (*mn)[TO_LSM_MAXD] = s_mn[w];
-    float (*mx)[TO_LSM_MAXD] = s_mx[w];
-    for (int c = lane; c < C; c += 32) {
-        const size_t g = (size_t)r * C + c;
-        int n = 0;
-        for (int b = bfirst; b <= blast; ++b) n += a.lcnt[g * nb + b];
-        cnt[c] = n;
-    }
-    __syncwarp();
-    // each control's own ranges (control 0, and any with more than d + 1
+    // 2: each control's own ranges (control 0, and any with more than d + 1
     // points), then the others take control 0's
-    for (int q = lane; q < C * d; q += 32) {
+    for (int q = tid; q < C * d; q += kPrepThreads) {
         const int c = q / d, j = q - c * d;
-        const size_t g = (size_t)r * C + c;
-        if (!((c == 0) || (cnt[c] > d + 1))) continue;
-        if (cnt[c] > 0) {
-            float lo = lsm_unkey(a.lkey[2 * (g * d + j)]);
-            float hi = lsm_unkey(a.lkey[2 * (g * d + j) + 1]);
+        if (!((c == 0) || (s_base[c] > d + 1))) continue;
+        float lo = 0.0f, hi = 0.0f;
+        if (s_base[c] > 0) {
+            lo = lsm_unkey(s_key[c][j][0]);
+            hi = lsm_unkey(s_key[c][j][1]);
             // the reference scans from the first point with
             // "if (xmin > x) ... else if (xmax < x)": plain min and max,
             // except that a first value of -0/+0 keeps its sign when it is
             // the extreme
-            const float first = a.xraw[(g * d + j) * P];
+            const float first = xraw[((size_t)c * d + j) * P];
             if (lo == first) lo = first;
             if (hi == first) hi = first;
-            mn[c][j] = lo; mx[c][j] = hi;
-        } else {
-            mn[c][j] = 0.0f; mx[c][j] = 0.0f;
         }
+        s_mn[c][j] = lo;
+        s_mx[c][j] = hi;
     }
-    __syncwarp();
-    for (int q = lane; q < C * d; q += 32) {
+    __syncthreads();
+    for (int q = tid; q < C * d; q += kPrepThreads) {
         const int c = q / d, j = q - c * d;
-        if ((c == 0) || (cnt[c] > d + 1)) continue;
-        mn[c][j] = mn[0][j]; mx[c][j] = mx[0][j];
+        if ((c == 0) || (s_base[c] > d + 1)) continue;
+        s_mn[c][j] = s_mn[0][j];
+        s_mx[c][j] = s_mx[0][j];
     }
-    __syncwarp();
-    for (int j = lane; j < d; j += 32) {
-        float lo = mn[0][j], hi = mx[0][j];
+    __syncthreads();
+    if (tid < d) {
+        const int j = tid;
+        float lo = s_mn[0][j], hi = s_mx[0][j];
         for (int c = 1; c < C; ++c) {
-            if (lo > mn[c][j]) lo = mn[c][j];
-            if (hi < mx[c][j]) hi = mx[c][j];
+            if (lo > s_mn[c][j]) lo = s_mn[c][j];
+            if (hi < s_mx[c][j]) hi = s_mx[c][j];
         }
-        mn[C][j] = lo; mx[C][j] = hi;
-        a.gmin[(size_t)r * d + j] = lo;
-        a.gmax[(size_t)r * d + j] = hi;
+        s_mn[C][j] = lo;
+        s_mx[C][j] = hi;
+        s_lo[j] = to_lsm_query_axis(0, lo, hi, R);
+        s_hi[j] = to_lsm_query_axis(R - 1, lo, hi, R);
     }
-    __syncwarp();
-    if (a.qax)
-        for (int q = lane; q < d * R; q += 32) {
-            const int j = q / R, di = q - j * R;
-            const float lo = mn[C][j], hi = mx[C][j];
-            a.qax[((size_t)r * d + j) * R + di] =
-                to_lsm_normalise(to_lsm_query_axis(di, lo, hi, R), lo, hi, j == S, a.scaling);
-        }
-    for (int c = lane; c < C; c += 32) {
-        const size_t g = (size_t)r * C + c;
-        const int n = cnt[c];
+    __syncthreads();
+    for (int q = tid; q < d * R; q += kPrepThreads) {
+        const int j = q / R, di = q - j * R;
+        const float lo = s_mn[C][j], hi = s_mx[C][j];
+        const float raw = to_lsm_query_axis(di, lo, hi, R);
+        a.qax[((size_t)slot * a.nr + r) * d * R + q] = to_lsm_normalise(raw, lo, hi, j == S, a.scaling);
+        for (int c = 0; c < C; ++c) to_rov_reg_block(a, t, (size_t)r * C + c)[q] = raw;
+    }
+    if (tid < C) {
+        const int n = s_base[tid];
         int k = 0;
         if (n > 3) {
             k = (int)((double)a.k_mult * (log((double)n) + 1.0));
             if (k > n) k = n;
         }
-        a.npts[g] = n;
-        a.kc[g] = k;
+        a.npts[gs0 + tid] = n;
+        a.kc[gs0 + tid] = k;
     }
-    // axis values of the regression grid (createQueryPoints :1187-1190)
-    for (int q = lane; q < C * d * R; q += 32) {
-        const int c = q / (d * R), jr = q - c * d * R, j = jr / R, di = jr - j * R;
-        float* ax = to_rov_reg_block(a, t, (size_t)r * C + c);
-        ax[(size_t)j * R + di] = to_lsm_query_axis(di, mn[C][j], mx[C][j], R);
+    // 3 (in place unless the raw states are kept: reference semantics)
+    float* xn = a.xn + gs0 * d * P;
+    for (int cj = warp; cj < C * d; cj += NW) {
+        const int c = cj / d, j = cj - c * d, n = s_base[c];
+        const float lo = s_mn[C][j], hi = s_mx[C][j];
+        for (int m = lane; m < n; m += 32)
+            xn[(size_t)cj * P + m] = to_lsm_normalise(xraw[(size_t)cj * P + m], lo, hi, j == S,
+                                                      a.scaling);
     }
-}
-
-// normalised points (host normalisation, SimulateGPU.cu:4591-4603)
-__global__ void __launch_bounds__(256) k_lsm_norm(to_rov_args a) {
-    const int P = a.P, S = a.S, C = a.C, d = S + 1;
-    const size_t total = (size_t)a.G * d * P;
-    for (size_t q = (size_t)blockIdx.x * blockDim.x + threadIdx.x; q < total;
-         q += (size_t)gridDim.x * blockDim.x) {
-        const size_t gj = q / P;
-        const int m = (int)(q - gj * P);
-        const int g = (int)(gj / d), j = (int)(gj - (size_t)g * d);
-        if (m >= a.npts[g]) continue;
-        const size_t r = (size_t)(g / C);
-        a.xn[q] = to_lsm_normalise(a.xraw[q], a.gmin[r * d + j], a.gmax[r * d + j], j == S,
-                                   a.scaling);
+    const int per = (Q + TO_ROV_TILE - 1) / TO_ROV_TILE;
+    int2* tiles = a.tiles + (size_t)slot * a.G * per;
+    if (!a.touched) {
+        // every grid query of every group
+        __shared__ int s_t0;
+        if (tid == 0) s_t0 = atomicAdd(&a.ntiles[slot], C * per);
+        if (tid < C) a.gcount[gs0 + tid] = Q;
+        __syncthreads();
+        for (int q = tid; q < C * per; q += kPrepThreads)
+            tiles[s_t0 + q] = make_int2(r * C + q / per, (q % per) * TO_ROV_TILE);
+        return;
     }
-}
-
-// Touched-query mode, corrected semantics: k_rov_backward at year t reads
-// control c's regression block of the path's road at the 2^d corners of
-// the cell holding the path's own state for c (to_lsm_interp), for every
-// control valid for the path (decide_interior).  Mark exactly those grid
-// queries; k_lsm_list compacts the marks into the year's work list and
-// clears them again.  The reads happen after this year's axes are written
-// (k_lsm_stats), so the corners are the ones the backward pass will read.
-__global__ void __launch_bounds__(256) k_lsm_mark(to_rov_args a, int t) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p == 0) *a.qcount = 0;
-    if (p >= a.PT) return;
-    const int C = a.C, S = a.S, d = S + 1, R = a.R;
-    const int r = p / a.P;
-    float state[TO_ROV_MAXC * (TO_LSM_MAXD - 1) + 1];
-    for (int c = 0; c < C; ++c)
-        for (int s = 0; s < S; ++s) state[c * S + s] = adj_pop(a, p, t, s, c);
-    const int sy = a.Y + 1;
-    const float prof = unit_profit(a, p, t, sy, sy);
+    // 4
+    const int qw = (Q + 31) >> 5;
+    unsigned* bits = a.bmap ? a.bmap + ((size_t)slot * a.nr + r) * C * qw : s_bits;
+    for (int q = tid; q < C * qw; q += kPrepThreads) bits[q] = 0u;
+    __syncthreads();
+    for (int pl = tid; pl < P; pl += kPrepThreads) {
+        const int p = (int)(p_0 + pl);
+        const float prof = a.profS[(size_t)t * PT + p];
+        const int lp = to_lsm_lower_index(prof, s_lo[S], s_hi[S], R);
+        for (int c = 0; c < C; ++c) {
+            bool valid = true;
+            int base = 0;
+            int li[TO_LSM_MAXD];
+            for (int s = 0; s < S; ++s) {
+                const float v = adj_pop(a, p, t, s, c);
+                if (v < threshold(a, s) && c > 0) { valid = false; break; }
+                li[s] = to_lsm_lower_index(v, s_lo[s], s_hi[s], R);
+                base = base * R + li[s];
+            }
+            if (!valid) continue;
+            base = base * R + lp;
+            unsigned* mk = bits + (size_t)c * qw;
+            for (int corner = 0; corner < (1 << S); ++corner) {
+                // the corner's offset; its neighbour along the last dimension
+                // lies one query further
+                int idx = base, mul = R;
+                for (int s = S - 1; s >= 0; --s) {
+                    if ((corner >> (S - 1 - s)) & 1) idx += mul;
+                    mul *= R;
+                }
+                const unsigned b0 = 1u << (idx & 31);
+                if ((idx & 31) < 31) {
+                    atomicOr(&mk[idx >> 5], b0 | (b0 << 1));
+                } else {
+                    atomicOr(&mk[idx >> 5], b0);
+                    atomicOr(&mk[(idx >> 5) + 1], 1u);
+                }
+            }
+        }
+    }
+    __syncthreads();
+    // 5
+    int fitted = 0;
     for (int c = 0; c < C; ++c) {
-        bool valid = true;
-        for (int s = 0; s < S; ++s)
-            if (state[c * S + s] < threshold(a, s) && c > 0) { valid = false; break; }
-        if (!valid) continue;
-        const size_t g = (size_t)r * C + c;
-        const float* rb = to_rov_reg_block(a, t, g);
-        int li[TO_LSM_MAXD];
-        for (int j = 0; j < d; ++j) {
-            const float v = (j < S) ? state[c * S + j] : prof;
-            li[j] = to_lsm_lower_index(v, rb[j * R], rb[j * R + R - 1], R);
+        const unsigned* mk = bits + (size_t)c * qw;
+        const int chunk = (qw + kPrepThreads - 1) / kPrepThreads;
+        const int w0 = tid * chunk, w1 = min(qw, w0 + chunk);
+        int cnt = 0;
+        for (int w = w0; w < w1; ++w) cnt += __popc(mk[w]);
+        int x = cnt;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
         }
-        unsigned char* mk = a.qmark + g * a.Q;
-        for (int corner = 0; corner < (1 << d); ++corner) {
-            int idx = 0;
-            for (int j = 0; j < d; ++j) idx = idx * R + li[j] + ((corner >> (d - 1 - j)) & 1);
-            mk[idx] = 1;
+        if (lane == 31) s_scan[warp] = x;
+        __syncthreads();
+        int pos = x - cnt, total = 0;
+        for (int w = 0; w < NW; ++w) { if (w < warp) pos += s_scan[w]; total += s_scan[w]; }
+        int* list = a.qlist + (gs0 + c) * Q;
+        for (int w = w0; w < w1; ++w)
+            for (unsigned b = mk[w]; b; b &= b - 1) list[pos++] = w * 32 + __ffs(b) - 1;
+        if (tid == 0) {
+            a.gcount[gs0 + c] = total;
+            const int nt = (total + TO_ROV_TILE - 1) / TO_ROV_TILE;
+            const int t0 = nt > 0 ? atomicAdd(&a.ntiles[slot], nt) : 0;
+            for (int i = 0; i < nt; ++i) tiles[t0 + i] = make_int2(r * C + c, i * TO_ROV_TILE);
         }
+        fitted += total;
+        __syncthreads();
     }
+    if (tid == 0 && a.qroad && fitted) atomicAdd(&a.qroad[r], (unsigned)fitted);
 }
 
-// compaction of the year's marks into flat items g*Q + q (any order: each
-// item writes only its own outputs), clearing them for the next year
-__global__ void __launch_bounds__(1024) k_lsm_list(to_rov_args a) {
-    __shared__ int s_w[32];
-    __shared__ int s_base;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const size_t total = (size_t)a.G * a.Q;
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const bool on = i < total && a.qmark[i] != 0;
-    const unsigned b = __ballot_sync(0xffffffffu, on);
-    if (lane == 0) s_w[warp] = __popc(b);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int tot = 0;
-        for (int w = 0; w < nw; ++w) { const int v = s_w[w]; s_w[w] = tot; tot += v; }
-        s_base = tot > 0 ? atomicAdd(a.qcount, tot) : 0;
-    }
-    __syncthreads();
-    if (on) {
-        a.qlist[s_base + s_w[warp] + __popc(b & ((1u << lane) - 1u))] = (int)i;
-        a.qmark[i] = 0;
-    }
-    if (a.qroad && b) {
-        // queries fitted per road (a warp's 32 items mostly share one road)
-        const int road = (int)(i / ((size_t)a.Q * a.C));
-        const unsigned same = __match_any_sync(0xffffffffu, road);
-        if (on && lane == __ffs(same & b) - 1) atomicAdd(&a.qroad[road], (unsigned)__popc(same & b));
-    }
+// the values the year's points regress on, group by group (cell-grid search)
+__global__ void __launch_bounds__(256) k_lsm_values(to_rov_args a, int t, int slot) {
+    const int g = blockIdx.y, m = blockIdx.x * blockDim.x + threadIdx.x;
+    const size_t gs = (size_t)slot * a.G + g;
+    if (m < a.npts[gs])
+        a.yv[(size_t)g * a.P + m] = a.condExp[(size_t)(t + 1) * a.PT + a.pidx[gs * a.P + m]];
 }
 
 }  // namespace
 
 namespace {
 
-// backwardInduction for 0 < t < Y-1 (:2464-2776)
-__global__ void k_rov_backward(to_rov_args a, int t) {
-    int p = blockIdx.x * blockDim.x + threadIdx.x;
+// backwardInduction for 0 < t < Y-1 (:2464-2776), a thread per path.  The
+// interior decision of corrected semantics is unrolled for the number of
+// species: states and corner weights in registers instead of arrays indexed
+// at run time in local memory, the profit read instead of drawn again; and
+// for up to CU controls, whose loads are then all in flight together (a
+// control the path may not take is interpolated too and not looked at).
+// Bound by the latency of the dependent loads (states, axes, 2^d corners;
+// the regressions stay in L2): 47 -> 29 us a year of 196,608 paths of three
+// species, 21 -> 10 us of 10,000 paths of two.
+template <int S, int CU>
+__global__ void __launch_bounds__(128) k_rov_backward(to_rov_args a, int t) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= a.PT) return;
+    const int C = a.C, R = a.R, r = p / a.P;
+    const float prof = a.unitProfits[(size_t)t * a.PT + p];
+    const float disc = 1.0f + a.rrr * a.dt / 100.0f;
+    float tot[S];
+#pragma unroll
+    for (int s = 0; s < S; ++s) tot[s] = a.totalPops[((size_t)s * (a.Y + 1) + t) * a.PT + p];
+    float best = 0.0f;
+    int bc = 0;
+    for (int c0 = 0; c0 < C; c0 += CU) {
+        float pay[CU];
+        bool valid[CU];
+#pragma unroll
+        for (int u = 0; u < CU; ++u) {
+            const int c = c0 + u < C ? c0 + u : C - 1;
+            float st[S];
+            valid[u] = c0 + u < C;
+#pragma unroll
+            for (int s = 0; s < S; ++s) {
+                st[s] = tot[s] * a.aars[(((size_t)s * C + c) * a.Y + t) * a.PT + p];
+                if (st[s] < a.params[8 * s + 3] && c > 0) valid[u] = false;
+            }
+            if (c == C - 1 && a.adjPops)
+#pragma unroll
+                for (int s = 0; s < S; ++s) a.adjPops[((size_t)t * S + s) * a.PT + p] = st[s];
+            const float cur = a.flows[c] * prof;
+            const float v = to_lsm_interp(to_rov_reg_block(a, t, (size_t)r * C + c), R, S, st, prof);
+            double ce = (double)(v / disc);
+            if (ce > 0.0) ce = 0.0;
+            pay[u] = (float)((double)cur + ce);
+        }
+#pragma unroll
+        for (int u = 0; u < CU; ++u)
+            if (valid[u] && (c0 + u == 0 || pay[u] < best)) { best = pay[u]; bc = c0 + u; }
+    }
+    a.condExp[(size_t)t * a.PT + p] = best;
+    a.optCont[(size_t)t * a.PT + p] = bc;
+}
+
+// reference semantics (one species)
+__global__ void __launch_bounds__(128) k_rov_backward_ref(to_rov_args a, int t) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= a.PT) return;
     const int C = a.C, S = a.S;
     float state[TO_ROV_MAXC * (TO_LSM_MAXD - 1) + 1];
     for (int c = 0; c < C; ++c)
         for (int s = 0; s < S; ++s) state[c * S + s] = adj_pop(a, p, t, s, c);
-    for (int s = 0; s < S; ++s)
-        a.adjPops[((size_t)t * S + s) * a.PT + p] = state[(C - 1) * S + s];
-    int sy = (a.sem == 0) ? a.Y : a.Y + 1;
-    float prof = unit_profit(a, p, t, sy, sy);
-    state[S * C] = prof;
-    a.unitProfits[(size_t)t * a.PT + p] = prof;
+    if (a.adjPops)
+        for (int s = 0; s < S; ++s)
+            a.adjPops[((size_t)t * S + s) * a.PT + p] = state[(C - 1) * S + s];
+    state[S * C] = a.unitProfits[(size_t)t * a.PT + p];
     float best;
     int bc;
     to_rovd::decide_interior(a, t, p / a.P, state, best, bc);
@@ -778,43 +794,117 @@ to_status rov_run(to_ctx ctx, to_rov_args a, const to_csc* csc) {
     return rov_backward(ctx, a, pblocks, tpb, nullptr);
 }
 
-to_status rov_backward(to_ctx ctx, const to_rov_args& a, int pblocks, int tpb,
+// bytes of one prepared year, besides the fixed ones
+static size_t slot_bytes(const to_rov_args& a, int max_roads) {
+    const size_t G = (size_t)max_roads * a.C, d = a.S + 1;
+    const size_t per = (a.Q + TO_ROV_TILE - 1) / TO_ROV_TILE;
+    return G * d * a.P * 4 * (a.sem == 0 ? 2 : 1) + G * a.P * 4 + (a.touched ? G * a.Q * 4 : 0) +
+           G * per * 8 + (a.reg_by_slot ? G * ((size_t)a.R * d + 2 * (size_t)a.Q) * 4 : 0);
+}
+
+void rov_plan(to_rov_args& a, int max_roads) {
+    // all years where they fit in half a gigabyte (a road, a small batch); a
+    // 256-road generation takes a few at a time, enough CTAs a launch
+    const auto fit = [&](size_t bytes, size_t most) {
+        const size_t n = ((size_t)512 << 20) / (bytes > 0 ? bytes : 1);
+        return (int)(n < 1 ? 1 : (n > most ? most : n));
+    };
+    a.slots = fit(slot_bytes(a, max_roads), (size_t)a.Y - 2);
+    a.sel_slots = fit(knn_select_bytes(a, max_roads), (size_t)a.slots);
+}
+
+size_t rov_scratch(to_rov_args& a, int max_roads, char* base) {
+    const size_t T = a.slots, NR = max_roads, G = NR * a.C, d = a.S + 1, P = a.P, Q = a.Q;
+    const size_t per = (Q + TO_ROV_TILE - 1) / TO_ROV_TILE, qw = (Q + 31) / 32;
+    size_t off = 0;
+    auto take = [&](size_t b) {
+        char* p = base ? base + off : nullptr;
+        off += to_align256(b);
+        return p;
+    };
+    a.xn = (float*)take(T * G * d * P * 4);
+    a.xraw = a.sem == 0 ? (float*)take(T * G * d * P * 4) : a.xn;
+    a.pidx = (int*)take(T * G * P * 4);
+    a.npts = (int*)take(T * G * 4);
+    a.kc = (int*)take(T * G * 4);
+    a.qax = (float*)take(T * NR * d * a.R * 4);
+    a.qlist = a.touched ? (int*)take(T * G * Q * 4) : nullptr;
+    a.gcount = (int*)take(T * G * 4);
+    a.tiles = (int2*)take(T * G * per * 8);
+    a.ntiles = (int*)take(2 * T * 4);
+    a.bmap = (a.touched && a.C * qw * 4 > (size_t)kPrepBitmap)
+                 ? (unsigned*)take(T * NR * a.C * qw * 4) : nullptr;
+    a.profS = a.sem == 0 ? (float*)take((size_t)a.Y * NR * P * 4) : a.unitProfits;
+    if (a.P <= TO_ROV_SCAN_PATHS) {
+        const size_t tiles = (size_t)a.sel_slots * G * per;
+        a.nbr = (unsigned short*)take(tiles * TO_ROV_TILE * a.kmax * 2);
+        a.kthv = (float*)take(tiles * TO_ROV_TILE * 4);
+    } else {
+        a.yv = (float*)take(G * P * 4);
+        a.gsx = (float*)take(G * d * P * 4);
+        a.gsi = (int*)take(G * P * 4);
+        a.gcell = (int*)take(G * (TO_KNN_GCELLS + 1) * 4);
+        a.ggrid = (to_knn_grid*)take(G * sizeof(to_knn_grid));
+        a.kth = (float*)take(G * Q * 4);
+        a.knn_acc = (double*)take(G * Q * ((d + 1) * (d + 4) / 2) * 8);
+    }
+    return off;
+}
+
+to_status rov_backward(to_ctx ctx, const to_rov_args& args, int pblocks, int tpb,
                        const to_csc* csc) {
+    to_rov_args a = args;
     if (a.algo == 6 && (!csc || !a.popsY || !a.gmY || a.nr != 1))
         return to_set_error(ctx, TO_ERR_UNSUPPORTED, "ALGO6 needs the sparse forward pass, one road");
-    if (a.touched && (a.sem != 1 || a.algo != 4 || !a.qmark || !a.qlist || !a.qcount ||
-                      (size_t)a.G * a.Q > (size_t)0x7fffffff))
+    if (a.touched && (a.sem != 1 || a.algo != 4 || !a.qlist))
         return to_set_error(ctx, TO_ERR_INVALID, "touched-query mode: sem 1, ALGO4, scratch");
-    if (a.touched)
-        TO_CUDA(ctx, cudaMemsetAsync(a.qmark, 0, (size_t)a.G * a.Q, ctx->stream));
+    if (a.slots < 1 || (size_t)a.G * a.Q > (size_t)0x7fffffff)
+        return to_set_error(ctx, TO_ERR_INVALID, "regression scratch: %d years", a.slots);
+    if (a.S < 1 || a.S + 1 > TO_LSM_MAXD)
+        return to_set_error(ctx, TO_ERR_UNSUPPORTED, "%d species", a.S);
+    const bool scan = a.P <= TO_ROV_SCAN_PATHS;
+    // the cell-grid search starts a query from its k-th distance a year
+    // later; cleared so that every valuation starts the same way
+    if (!scan) TO_CUDA(ctx, cudaMemsetAsync(a.kth, 0, (size_t)a.G * a.Q * 4, ctx->stream));
     if (a.qroad) TO_CUDA(ctx, cudaMemsetAsync(a.qroad, 0, (size_t)a.nr * sizeof(unsigned), ctx->stream));
+    to_prof_begin(ctx, "lsm_prepare");
+    k_rov_profit<<<dim3((a.PT + 255) / 256, a.Y - 1), 256, 0, ctx->stream>>>(a);
+    to_prof_end(ctx);
+    TO_LAUNCHED(ctx);
     k_rov_terminal<<<pblocks, tpb, 0, ctx->stream>>>(a);
     TO_LAUNCHED(ctx);
-    if (a.lblocks != (a.PT + kLsmChunk - 1) / kLsmChunk || (a.nr > 1 && a.P < kLsmMinPaths))
-        return to_set_error(ctx, TO_ERR_INVALID, "regression chunks %d", a.lblocks);
-    int fblocks = (int)(((size_t)a.G * (a.S + 1) * a.P + 255) / 256);
-    if (fblocks > 4 * 152) fblocks = 4 * 152;
+    const size_t bits = (a.touched && !a.bmap) ? (size_t)a.C * ((a.Q + 31) / 32) * 4 : 0;
+    TO_CUDA(ctx, cudaFuncSetAttribute(k_lsm_prepare, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      kPrepBitmap));
+    int low = a.Y - 1, sel = a.Y - 1;          // first prepared year, first with neighbours
     for (int t = a.Y - 2; t > 0; --t) {
-        to_prof_begin(ctx, "lsm_prepare");
-        k_lsm_count<<<a.lblocks, kLsmChunk, 0, ctx->stream>>>(a, t);
-        TO_LAUNCHED(ctx);
-        k_lsm_scatter<<<a.lblocks, kLsmChunk, 0, ctx->stream>>>(a, t);
-        TO_LAUNCHED(ctx);
-        k_lsm_stats<<<(a.nr + kStatsWarps - 1) / kStatsWarps, kStatsWarps * 32, 0, ctx->stream>>>(
-            a, t, a.lblocks);
-        TO_LAUNCHED(ctx);
-        k_lsm_norm<<<fblocks, 256, 0, ctx->stream>>>(a);
-        TO_LAUNCHED(ctx);
-        if (a.touched) {
-            k_lsm_mark<<<(a.PT + 255) / 256, 256, 0, ctx->stream>>>(a, t);
-            TO_LAUNCHED(ctx);
-            k_lsm_list<<<(int)(((size_t)a.G * a.Q + 1023) / 1024), 1024, 0, ctx->stream>>>(a);
+        if (t < low) {
+            low = t - a.slots + 1 > 1 ? t - a.slots + 1 : 1;
+            a.slot0 = low;
+            to_prof_begin(ctx, "lsm_prepare");
+            TO_CUDA(ctx, cudaMemsetAsync(a.ntiles, 0, 2 * (size_t)a.slots * sizeof(int), ctx->stream));
+            k_lsm_prepare<<<dim3(a.nr, t - low + 1), kPrepThreads, bits, ctx->stream>>>(a);
+            to_prof_end(ctx);
             TO_LAUNCHED(ctx);
         }
-        to_prof_end(ctx);
-        TO_TRY(knn_rov(ctx, a, t));      // kNN and the local linear regressions
+        if (scan) {
+            if (t < sel) {
+                sel = t - a.sel_slots + 1 > low ? t - a.sel_slots + 1 : low;
+                a.sel0 = sel - low;
+                TO_TRY(knn_rov_select(ctx, a, t - sel + 1));
+            }
+            TO_TRY(knn_rov_fit(ctx, a, t));
+        } else {
+            k_lsm_values<<<dim3((a.P + 255) / 256, a.G), 256, 0, ctx->stream>>>(a, t, t - a.slot0);
+            TO_LAUNCHED(ctx);
+            TO_TRY(knn_rov_grid(ctx, a, t));
+        }
         to_prof_begin(ctx, "rov_backward");
-        k_rov_backward<<<pblocks, tpb, 0, ctx->stream>>>(a, t);
+        if (a.sem == 0) k_rov_backward_ref<<<pblocks, tpb, 0, ctx->stream>>>(a, t);
+        else if (a.S == 1) k_rov_backward<1, 3><<<pblocks, tpb, 0, ctx->stream>>>(a, t);
+        else if (a.S == 2) k_rov_backward<2, 3><<<pblocks, tpb, 0, ctx->stream>>>(a, t);
+        else if (a.S == 3) k_rov_backward<3, 3><<<pblocks, tpb, 0, ctx->stream>>>(a, t);
+        else k_rov_backward<4, 3><<<pblocks, tpb, 0, ctx->stream>>>(a, t);
         to_prof_end(ctx);
         TO_LAUNCHED(ctx);
         // ALGO6: the year's value becomes the realised payoff of each path

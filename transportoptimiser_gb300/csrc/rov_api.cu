@@ -135,8 +135,6 @@ to_status to_simulate_rov_batch(to_ctx ctx, int n_roads, const to_rov_problem* p
     const int kmax = k_rule(P) > 0 ? k_rule(P) : 1;
     if (kmax > TO_KNN_KMAX) return to_set_error(ctx, TO_ERR_UNSUPPORTED, "k %d", kmax);
     const size_t blk = (size_t)R * d + 2 * (size_t)Q;
-    const int lblocks = (PT + 1023) / 1024;
-    const size_t nacc = (size_t)(d + 1) * (d + 4) / 2;   // sums a query (doubles)
     const int cap = NP * 64 < NP * NP ? NP * 64 : NP * NP;
     size_t bytes = 0;
     auto acc = [&](size_t b) { bytes += to_align256(b); };
@@ -145,16 +143,8 @@ to_status to_simulate_rov_batch(to_ctx ctx, int n_roads, const to_rov_problem* p
     acc(C * 4); acc(6 * (size_t)(U > 0 ? U : 1) * 4); acc(16 * 4); acc(16 * 4); acc(16 * 4); acc(16 * 4);
     acc((size_t)Y * PT * 4); acc((size_t)(U > 0 ? U : 1) * (Y + 1) * PT * 4);
     acc((size_t)S * (Y + 1) * PT * 4); acc((size_t)S * C * Y * PT * 4);
-    acc((size_t)G * d * P * 4); acc((size_t)G * d * P * 4); acc((size_t)G * P * 4);
-    acc(G * 4); acc(G * 4); acc((size_t)NR * d * 4); acc((size_t)NR * d * 4);
-    acc((size_t)NR * d * R * 4);
-    acc((size_t)G * d * P * 4); acc((size_t)G * P * 4);
-    acc((size_t)G * (TO_KNN_GCELLS + 1) * 4); acc((size_t)G * sizeof(to_knn_grid));
-    acc((size_t)G * Q * 4);
-    acc((size_t)G * lblocks * 4); acc((size_t)G * d * 2 * 4);
-    acc(4); acc((size_t)G * Q * nacc * 8);
-    acc((size_t)Y * G * blk * 4); acc((size_t)Y * PT * 4); acc((size_t)Y * PT * 4);
-    acc((size_t)Y * PT * 4); acc((size_t)Y * S * PT * 4); acc((size_t)NR * 5 * 8);
+    acc((size_t)Y * PT * 4); acc((size_t)Y * PT * 4); acc((size_t)Y * PT * 4);
+    acc((size_t)Y * S * PT * 4); acc((size_t)NR * 5 * 8);
     acc((size_t)RS * C * (NP + 1) * 4); acc((size_t)RS * C * cap * 2); acc((size_t)RS * C * cap * 4);
     acc((size_t)RS * C * 4);
     // union form of each road-species' C <= 3 matrices
@@ -166,9 +156,8 @@ to_status to_simulate_rov_batch(to_ctx ctx, int n_roads, const to_rov_problem* p
     bool want_reg = false;
     for (int r = 0; r < NR; ++r) want_reg |= results[r].regression != nullptr;
     const bool touched = pr->sem == 1 && algo == 4 && !want_reg;
-    if (touched) { acc((size_t)G * Q); acc((size_t)G * Q * 4); acc(4); }
-    TO_TRY(to_arena_reserve(ctx, bytes + 4096));
-    TO_CUDA(ctx, cudaMemsetAsync(ctx->arena, 0, bytes, ctx->stream));
+    bool want_adj = false;
+    for (int r = 0; r < NR; ++r) want_adj |= results[r].adj_pops != nullptr;
     to_rov_args a;
     memset(&a, 0, sizeof(a));
     a.P = P; a.Y = Y; a.S = S; a.C = C; a.U = U; a.R = R; a.Q = Q;
@@ -178,6 +167,16 @@ to_status to_simulate_rov_batch(to_ctx ctx, int n_roads, const to_rov_problem* p
     a.unit_cost = pr->unit_cost; a.unit_revenue = pr->unit_revenue; a.scaling = 2.0f;
     a.seed = pr->seed; a.np = NP; a.ne = NP; a.kmax = kmax; a.flags = ctx->d_flags;
     a.algo = algo; a.k_mult = algo == 6 ? 3 : 10;
+    a.touched = touched ? 1 : 0;
+    // every year's regressions are kept where the caller wants them or the
+    // re-simulation reads them again
+    a.reg_by_slot = (want_reg || algo == 6) ? 0 : 1;
+    to_k::rov_plan(a, NR);
+    const size_t nreg = (size_t)(a.reg_by_slot ? a.slots : Y) * G * blk;
+    acc(nreg * 4);
+    const size_t lsm = to_k::rov_scratch(a, NR, nullptr);
+    acc(lsm);
+    TO_TRY(to_arena_reserve(ctx, bytes + 4096));
     float* d_mmm = to_arena_take<float>(ctx, mmm.size());
     float* d_ip = to_arena_take<float>(ctx, ip.size());
     float* d_cp = to_arena_take<float>(ctx, cp.size());
@@ -195,30 +194,21 @@ to_status to_simulate_rov_batch(to_ctx ctx, int n_roads, const to_rov_problem* p
     a.uRes = to_arena_take<float>(ctx, (size_t)(U > 0 ? U : 1) * (Y + 1) * PT);
     a.totalPops = to_arena_take<float>(ctx, (size_t)S * (Y + 1) * PT);
     a.aars = to_arena_take<float>(ctx, (size_t)S * C * Y * PT);
-    a.xraw = to_arena_take<float>(ctx, (size_t)G * d * P);
-    a.xn = to_arena_take<float>(ctx, (size_t)G * d * P);
-    a.yv = to_arena_take<float>(ctx, (size_t)G * P);
-    a.npts = to_arena_take<int>(ctx, G);
-    a.kc = to_arena_take<int>(ctx, G);
-    a.gmin = to_arena_take<float>(ctx, (size_t)NR * d);
-    a.gmax = to_arena_take<float>(ctx, (size_t)NR * d);
-    a.qax = to_arena_take<float>(ctx, (size_t)NR * d * R);
-    a.gsx = to_arena_take<float>(ctx, (size_t)G * d * P);
-    a.gsi = to_arena_take<int>(ctx, (size_t)G * P);
-    a.gcell = to_arena_take<int>(ctx, (size_t)G * (TO_KNN_GCELLS + 1));
-    a.ggrid = to_arena_take<to_knn_grid>(ctx, G);
-    a.kth = to_arena_take<float>(ctx, (size_t)G * Q);
-    a.lcnt = to_arena_take<int>(ctx, (size_t)G * lblocks);
-    a.lkey = to_arena_take<unsigned>(ctx, (size_t)G * d * 2);
-    a.lblocks = lblocks;
-    a.knn_next = to_arena_take<int>(ctx, 1);
-    a.knn_acc = to_arena_take<double>(ctx, (size_t)G * Q * nacc);
-    a.reg = to_arena_take<float>(ctx, (size_t)Y * G * blk);
+    a.reg = to_arena_take<float>(ctx, nreg);
     a.condExp = to_arena_take<float>(ctx, (size_t)Y * PT);
     a.optCont = to_arena_take<int>(ctx, (size_t)Y * PT);
     a.unitProfits = to_arena_take<float>(ctx, (size_t)Y * PT);
     a.adjPops = to_arena_take<float>(ctx, (size_t)Y * S * PT);
     a.stats = to_arena_take<double>(ctx, (size_t)NR * 5);
+    char* lsm_base = to_arena_take<char>(ctx, lsm);
+    if (!lsm_base) return to_set_error(ctx, TO_ERR_ALLOC, "arena sizing");
+    to_k::rov_scratch(a, NR, lsm_base);
+    // what no kernel writes and the caller may ask for: year 0 of the profits
+    // and populations, the surfaces of the first and last year
+    TO_CUDA(ctx, cudaMemsetAsync(a.unitProfits, 0, (size_t)PT * 4, ctx->stream));
+    if (want_adj) TO_CUDA(ctx, cudaMemsetAsync(a.adjPops, 0, (size_t)S * PT * 4, ctx->stream));
+    else a.adjPops = nullptr;
+    if (want_reg) TO_CUDA(ctx, cudaMemsetAsync(a.reg, 0, nreg * 4, ctx->stream));
     to_csc csc;
     csc.ptr = to_arena_take<int>(ctx, (size_t)RS * C * (NP + 1));
     csc.idx = to_arena_take<uint16_t>(ctx, (size_t)RS * C * cap);
@@ -237,13 +227,6 @@ to_status to_simulate_rov_batch(to_ctx ctx, int n_roads, const to_rov_problem* p
     if (algo == 6) {
         a.popsY = to_arena_take<float>(ctx, (size_t)Y * S * NP * P);
         a.gmY = to_arena_take<float>(ctx, (size_t)Y * S * P);
-    }
-    if (touched) {
-        a.touched = 1;
-        a.qmark = to_arena_take<unsigned char>(ctx, (size_t)G * Q);
-        a.qlist = to_arena_take<int>(ctx, (size_t)G * Q);
-        a.qcount = to_arena_take<int>(ctx, 1);
-        if (!a.qcount) return to_set_error(ctx, TO_ERR_ALLOC, "arena sizing");
     }
     if (!csc.nnz || (algo == 6 && !a.gmY)) return to_set_error(ctx, TO_ERR_ALLOC, "arena sizing");
     TO_TRY(up(ctx, d_mmm, mmm.data(), mmm.size()));
@@ -323,7 +306,7 @@ to_status to_simulate_rov_batch(to_ctx ctx, int n_roads, const to_rov_problem* p
     };
     TO_TRY(fetch_rows(0, a.condExp, (size_t)Y));
     TO_TRY(fetch_rows(1, a.unitProfits, (size_t)Y));
-    TO_TRY(fetch_rows(2, a.adjPops, (size_t)Y * S));
+    if (want_adj) TO_TRY(fetch_rows(2, a.adjPops, (size_t)Y * S));
     bool want_oc = false;
     for (int r = 0; r < NR; ++r) want_oc |= results[r].opt_cont != nullptr;
     if (want_reg) {

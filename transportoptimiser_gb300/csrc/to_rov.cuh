@@ -47,48 +47,54 @@ struct to_rov_args {
     float* uRes;                      // [U][Y+1][PT]
     float* totalPops;                 // [S][Y+1][PT]
     float* aars;                      // [S][C][Y][PT]
-    // regression scratch (device), per group g = r*C + c
-    float* xraw;                      // [G][d][P] compacted raw states
-    float* xn;                        // [G][d][P] normalised
-    float* yv;                        // [G][P]
-    int* npts;                        // [G]
-    int* kc;                          // [G]
-    float* gmin;                      // [nr][d]
-    float* gmax;                      // [nr][d]
-    float* qax;                       // [nr][d][R] normalised grid axes of the year (may be null)
+    // regression scratch (device).  What a year's regressions are fitted on -
+    // the states, their ranges and the list of grid queries - does not depend
+    // on the values of later years, so it is prepared for up to `slots` years
+    // at a time; slot = t - slot0.  Per slot, per group g = r*C + c:
+    int slots, slot0;
+    int sel0, sel_slots;              // first slot with selected neighbours, how many fit
+    float* xraw;                      // [slots][G][d][P] compacted raw states (sem 0 only, else xn)
+    float* xn;                        // [slots][G][d][P] normalised
+    int* pidx;                        // [slots][G][P] path of the batch behind each point
+    int* npts;                        // [slots][G]
+    int* kc;                          // [slots][G]
+    float* qax;                       // [slots][nr][d][R] normalised grid axes of the year
+    int* qlist;                       // [slots][G][Q] grid queries to fit, ascending (touched mode)
+    int* gcount;                      // [slots][G] how many
+    int2* tiles;                      // [slots][G * ceil(Q / TO_ROV_TILE)] {group, first place in its list}
+    int* ntiles;                      // [slots] tiles; [slots] next tile to work on
+    unsigned short* nbr;              // [sel_slots][tiles][kmax][TO_ROV_TILE] neighbours, ascending
+    float* kthv;                      // [sel_slots][tiles][TO_ROV_TILE] k-th squared distances
+    unsigned* bmap;                   // [slots][nr][C][ceil(Q / 32)] query marks too many for shared memory
+    float* profS;                     // [Y][PT] unit profit of the regression states
+    int k_mult;                       // k = k_mult (ln n + 1): 10 ALGO4, 3 ALGO6
+    int algo;                         // 4 or 6
+    float* popsY;                     // ALGO6: [Y][S][ne][P] patch populations, start of year
+    float* gmY;                       // ALGO6: [Y][S][P] mean growth rate of the year
+    int kmax;
+    // above TO_ROV_SCAN_PATHS paths a road (the cell-grid search, knn.cu)
+    float* yv;                        // [G][P] values of the year after
     float* gsx;                       // [G][d][P] points in cell order
     int* gsi;                         // [G][P] their original indices
     int* gcell;                       // [G][TO_KNN_GCELLS + 1] cell starts
     to_knn_grid* ggrid;               // [G]
     float* kth;                       // [G][Q] k-th squared distance, year before
-    int* lcnt;                        // [G][lblocks] points per group and path chunk
-    unsigned* lkey;                   // [G][d][2] min / max keys of the states
-    int lblocks;                      // path chunks of the compaction
-    int k_mult;                       // k = k_mult (ln n + 1): 10 ALGO4, 3 ALGO6
-    int algo;                         // 4 or 6
-    float* popsY;                     // ALGO6: [Y][S][ne][P] patch populations, start of year
-    float* gmY;                       // ALGO6: [Y][S][P] mean growth rate of the year
-    int* knn_next;                    // work counter of the kNN kernel
-    double* knn_acc;                  // [G*Q][(d+1)(d+4)/2] normal-equation sums per listed query
-    int kmax;
+    double* knn_acc;                  // [G][Q][(d+1)(d+4)/2] normal-equation sums per listed query
     // touched-query mode (corrected semantics, ALGO4, surfaces not
     // returned): a year's regressions are fitted only at the grid queries
     // some path's interpolation reads; the others are never read
     int touched;
-    unsigned char* qmark;             // [G][Q] marks of the current year (kept zero between years)
-    int* qlist;                       // [G*Q] flat items g*Q + q of the marked queries
-    int* qcount;                      // number of entries in qlist
     unsigned* qroad;                  // [nr] queries fitted per road over the years (may be null)
-    // 1: reg holds only the current year's blocks (the regressions of year
-    // t are written and read within year t; nothing returns them)
-    int reg_one_year;
+    // 1: reg holds only the prepared years' blocks, by slot (the regressions of
+    // year t are written and read within year t; nothing returns them)
+    int reg_by_slot;
     int* flags;                       // device error word (plan checks), may be null
     // outputs (device)
-    float* reg;                       // [Y][G][R*d + 2Q]
+    float* reg;                       // [Y or slots][G][R*d + 2Q]
     float* condExp;                   // [Y][PT]
     int* optCont;                     // [Y][PT]
     float* unitProfits;               // [Y][PT]
-    float* adjPops;                   // [Y][S][PT]
+    float* adjPops;                   // [Y][S][PT], or null
     double* stats;                    // [nr][5]: value, control, SD, SE, n
 };
 
@@ -96,19 +102,22 @@ struct to_rov_args {
 // grid values, then Q standard deviations
 __host__ __device__ __forceinline__ float* to_rov_reg_block(const to_rov_args& a, int t, size_t g) {
     const size_t blk = (size_t)a.R * (a.S + 1) + 2 * (size_t)a.Q;
-    return a.reg + ((size_t)(a.reg_one_year ? 0 : t) * a.G + g) * blk;
+    return a.reg + ((size_t)(a.reg_by_slot ? t - a.slot0 : t) * a.G + g) * blk;
 }
 
 // grid query q of the current year: normalised coordinates (for kNN) and
 // the coordinates the regression centres on (createQueryPoints + host
 // normalisation; sem 0 centres on the unit grid, SimulateGPU.cu:2964-2966)
+// grid queries of one group that a CTA fits at a time
+#define TO_ROV_TILE 128
+// paths a road up to which a query scans every point of its group
+#define TO_ROV_SCAN_PATHS 32768
+
 template <int D>
-__device__ __forceinline__ void to_rov_query(const to_rov_args& a, int road, int q, float* qn,
-                                             float* xq) {
+__device__ __forceinline__ void to_rov_query(const to_rov_args& a, int slot, int road, int q,
+                                             float* qn, float* xq) {
     const int R = a.R;
-    const float* lo = a.gmin + (size_t)road * D;
-    const float* hi = a.gmax + (size_t)road * D;
-    const float* ax = a.qax ? a.qax + (size_t)road * D * R : nullptr;
+    const float* ax = a.qax + ((size_t)slot * a.nr + road) * D * R;
     const bool pow2 = (R & (R - 1)) == 0;
     const int lr = pow2 ? __ffs(R) - 1 : 0;           // log2 R
     int rem = q;
@@ -124,11 +133,8 @@ __device__ __forceinline__ void to_rov_query(const to_rov_args& a, int road, int
             rem -= di * div;
             div /= R;
         }
-        // the year's normalised axis values, computed once per road
-        // (k_lsm_stats) with the same operations
-        const float nv = ax ? ax[j * R + di]
-                            : to_lsm_normalise(to_lsm_query_axis(di, lo[j], hi[j], R), lo[j],
-                                               hi[j], j == a.S, a.scaling);
+        // the year's normalised axis values, computed once per road (k_lsm_prepare)
+        const float nv = ax[j * R + di];
         qn[j] = nv;
         xq[j] = (a.sem == 0) ? to_lsm_unit_axis(di, R) : nv;
     }
@@ -138,8 +144,18 @@ struct to_csc;
 namespace to_k {
 // csc: the packed migration matrices for the sparse forward pass, or null
 to_status rov_run(to_ctx ctx, to_rov_args a, const to_csc* csc);
-// kNN + local linear regressions of year t (cell grid, then fused kernel)
-to_status knn_rov(to_ctx ctx, const to_rov_args& a, int t);
+// bytes of regression scratch for a.slots years, and its pointers carved from
+// `base` (null: only the size)
+size_t rov_scratch(to_rov_args& a, int max_roads, char* base);
+// sets the years to prepare and to select neighbours for at a time
+void rov_plan(to_rov_args& a, int max_roads);
+// the k nearest points of every listed grid query of `years` prepared years,
+// from slot a.sel0; then the local linear regressions of one of them
+size_t knn_select_bytes(const to_rov_args& a, int max_roads);
+to_status knn_rov_select(to_ctx ctx, const to_rov_args& a, int years);
+to_status knn_rov_fit(to_ctx ctx, const to_rov_args& a, int t);
+// both for year t by the cell-grid search (groups of very many points)
+to_status knn_rov_grid(to_ctx ctx, const to_rov_args& a, int t);
 // generic kNN: ref dim-major [dim][n], query dim-major [dim][Q]
 to_status knn(to_ctx ctx, const float* ref, int n, const float* query, int Q,
               int dim, int k, float* dist, int* ind);
