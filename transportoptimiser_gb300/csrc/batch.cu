@@ -81,6 +81,7 @@ struct to_gen_s {
     double* d_pen = nullptr;             // [S][3]
     // ROV of every road (to_scene_set_rov)
     bool rov_on = false;
+    bool rov_union = false;              // the last planned generation fits the union form
     to_rov_args rov{};                   // road-independent fields + scratch
     char* rov_buf = nullptr;
     size_t rov_bytes = 0;
@@ -265,8 +266,8 @@ to_status rov_stage(to_ctx ctx, to_gen g, int R, int NE, int road0) {
     if (csc.uent) {
         // every control's packed columns in one list per destination; at most
         // as many entries as the widest packed matrix (nested patterns)
-        csc.ucap_smem = csc.cap_smem;
-        if (to_k::rov_union_smem(NE, g->C, csc.ucap_smem) > ctx->smem_optin) csc.uent = nullptr;
+        csc.ucap_smem = csc.cap_smem + NE;      // and the padding of every list
+        if (!g->rov_union) csc.uent = nullptr;
         else TO_TRY(to_k::union_csc(ctx, g->NP, g->C, g->d_np, R * g->S, csc));
     }
     return to_k::rov_run(ctx, a, &csc);
@@ -375,6 +376,7 @@ to_status evaluate_direct(to_ctx ctx, to_gen g, int R, const int* cell_off,
                       to_k::rov_sparse_smem(NE, g->C, g->csc.cap_smem) > ctx->smem_optin))
         return to_set_error(ctx, TO_ERR_UNSUPPORTED, "the ROV forward pass does not fit %d patches",
                             NE);
+    g->rov_union = to_k::rov_union_smem(NE, g->C, g->csc.cap_smem + NE) <= ctx->smem_optin;
     TO_TRY(grow_end(ctx, g, (size_t)RS * o->mte_paths));
     to_mte_args m = mte_args(ctx, g, o, NE);
     int choice;
@@ -590,7 +592,7 @@ to_status to_scene_create(to_ctx ctx, const to_scene* sc, to_gen* out) {
     // pass's form): the species models' patterns are nested - control c's
     // entries are a subset of the lowest-hazard control's - so a union
     // holds no more entries than that control's packed matrix
-    const size_t ucap = C <= 3 ? cap : 0;
+    const size_t ucap = C <= 3 ? cap + NP : 0;   // and the padding of every list
     if (C <= 3) { acc(RS * ucap * 16); acc(RS * (NP + 1) * 4); acc(RS * 4); }
     if ((e = cudaMalloc(&g->buf, bytes)) != cudaSuccess) return fail(e);
     g->buf_bytes = bytes;
@@ -746,6 +748,8 @@ to_status to_scene_set_rov(to_ctx ctx, to_gen g, const to_rov_problem* t) {
     a.unit_cost = t->unit_cost; a.unit_revenue = t->unit_revenue; a.scaling = 2.0f;
     a.seed = t->seed; a.kmax = kmax; a.algo = 4; a.k_mult = 10;
     a.touched = 1; a.reg_by_slot = 1; a.flags = ctx->d_flags;
+    a.ctas = ctx->sm_count > 0 ? ctx->sm_count : TO_SM_TARGET;
+    a.np = g->NP;
     to_k::rov_plan(a, NR);
     acc((size_t)a.slots * G * blk * 4);
     bytes += to_k::rov_scratch(a, NR, nullptr);

@@ -716,7 +716,7 @@ size_t knn_rov_smem() { return sizeof(WarpScratch) * kWarps; }
 
 template <int D>
 __global__ void __launch_bounds__(kWarps * 32, 4)
-k_knn_rov(to_rov_args a, int slot) {
+k_knn_rov_cells(to_rov_args a, int slot) {
     extern __shared__ __align__(16) unsigned char sm_raw[];
     constexpr int M = D + 1, NA = knn_acc_len<D>();
     constexpr int NS = knn_sums<D>();
@@ -889,10 +889,10 @@ k_knn_generic(const float* ref_g, int n, const float* query, int Q, int dim, int
 template <int D>
 to_status launch_knn_rov(to_ctx ctx, const to_rov_args& a, int t) {
     const size_t smem = knn_rov_smem();
-    TO_CUDA(ctx, cudaFuncSetAttribute(k_knn_rov<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    TO_CUDA(ctx, cudaFuncSetAttribute(k_knn_rov_cells<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)smem));
     int per_sm = 0;
-    TO_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_knn_rov<D>,
+    TO_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_knn_rov_cells<D>,
                                                                kWarps * 32, smem));
     if (per_sm < 1) per_sm = 1;
     const int sms = ctx->sm_count > 0 ? ctx->sm_count : TO_SM_TARGET;
@@ -900,7 +900,7 @@ to_status launch_knn_rov(to_ctx ctx, const to_rov_args& a, int t) {
     int grid = sms * per_sm;
     if (grid > tiles * (TO_ROV_TILE / kWarps)) grid = tiles * (TO_ROV_TILE / kWarps);
     to_prof_begin(ctx, "knn");
-    k_knn_rov<D><<<grid, kWarps * 32, smem, ctx->stream>>>(a, t - a.slot0);
+    k_knn_rov_cells<D><<<grid, kWarps * 32, smem, ctx->stream>>>(a, t - a.slot0);
     to_prof_end(ctx);
     TO_LAUNCHED(ctx);
     to_prof_begin(ctx, "knn_solve");

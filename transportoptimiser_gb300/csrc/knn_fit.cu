@@ -11,7 +11,7 @@
 // ever idles over a short list and the per-query bookkeeping - scans,
 // selections, solves - costs a thread what it used to cost a warp.  The
 // neighbours do not depend on the values of later years, so they are
-// selected (k_knn_select) for as many years at once as fill the GPU:
+// selected (k_knn_rov) for as many years at once as fill the GPU:
 //   1 a histogram of a sample of the squared distances, 8 buckets an octave,
 //     estimates the k-th;
 //   2 a histogram of all of them, 32 buckets an octave around the estimate,
@@ -37,6 +37,7 @@
 // paths, 100,000 queries of about 3,300 points: 4.2 -> 1.2 ms.
 #include <cmath>
 
+#include "to_f2.cuh"
 #include "to_internal.cuh"
 #include "to_lsm_math.h"
 #include "to_rov.cuh"
@@ -52,36 +53,6 @@ constexpr int kSide = 16;                  // most distances in the last bucket
 constexpr unsigned kMark = 0x8000u;        // a listed point of the last bucket
 static_assert(TO_ROV_SCAN_PATHS <= 32768, "point numbers of 15 bits");
 constexpr unsigned kAll = 0xffffffffu;
-
-// two packed floats (low half first), each operation rounded as its scalar
-typedef unsigned long long f2;
-__device__ __forceinline__ f2 pack2(float a, float b) {
-    f2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ void bits2(f2 v, unsigned& a, unsigned& b) {
-    asm("mov.b64 {%0, %1}, %2;" : "=r"(a), "=r"(b) : "l"(v));
-}
-__device__ __forceinline__ f2 add2(f2 a, f2 b) {
-    f2 r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
-    f2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ void unpack2(f2 v, float& a, float& b) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-}
-__device__ __forceinline__ f2 both2(float a) { return pack2(a, a); }
-__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
-    f2 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
 
 // squared distances (as bits) of points i .. i+3 of the tile to the query;
 // nq holds its negated coordinates, each twice
@@ -196,7 +167,7 @@ size_t select_smem(int d, int kmax) {
 
 // blockIdx.y: slot of the year, from a.sel0
 template <int D>
-__global__ void __launch_bounds__(kT, 5) k_knn_select(to_rov_args a) {
+__global__ void __launch_bounds__(kT, 5) k_knn_rov(to_rov_args a) {
     extern __shared__ __align__(16) unsigned char sm_fit[];
     __shared__ int s_tile;
     float* pts = reinterpret_cast<float*>(sm_fit);                    // [D][kPts]
@@ -654,7 +625,7 @@ __global__ void __launch_bounds__(kWide) k_knn_fit_wide(to_rov_args a, int t) {
 template <int D>
 to_status launch_select(to_ctx ctx, const to_rov_args& a, int years) {
     const size_t smem = select_smem(D, a.kmax);
-    const auto k = k_knn_select<D>;
+    const auto k = k_knn_rov<D>;
     TO_CUDA(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int per_sm = 0;
     TO_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kT, smem));

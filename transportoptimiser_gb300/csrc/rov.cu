@@ -314,7 +314,7 @@ __device__ __forceinline__ float lsm_unkey(unsigned k) {
 //    for c (to_lsm_interp), for every control valid for the path; exactly
 //    those grid queries are marked in a bitmap;
 //  5 the bitmaps as one ascending query list per group, cut into tiles of
-//    TO_ROV_TILE for k_knn_select.
+//    TO_ROV_TILE for k_knn_rov.
 // None of it depends on the values of later years, so a launch takes as many
 // years as the scratch holds.  Latency bound (a CTA is a chain of short
 // passes over a few hundred paths), which many CTAs an SM hide: 7.7 -> 1.5 ms
@@ -747,6 +747,7 @@ to_status rov_backward(to_ctx ctx, const to_rov_args& a, int pblocks, int tpb,
 
 to_status rov_run(to_ctx ctx, to_rov_args a, const to_csc* csc) {
     const int P = a.PT;                        // every path of the batch
+    a.rk = to_make_round_keys(a.seed);
     const int tpb = 128;
     const int pblocks = (P + tpb - 1) / tpb;
     to_prof_begin(ctx, "rov_exog");
@@ -835,6 +836,11 @@ size_t rov_scratch(to_rov_args& a, int max_roads, char* base) {
     a.bmap = (a.touched && a.C * qw * 4 > (size_t)kPrepBitmap)
                  ? (unsigned*)take(T * NR * a.C * qw * 4) : nullptr;
     a.profS = a.sem == 0 ? (float*)take((size_t)a.Y * NR * P * 4) : a.unitProfits;
+    a.fwd_next = (int*)take(4);
+    if (a.C <= 3) {
+        a.fwd_part = (f2*)take((size_t)a.ctas * 2 * a.C * (a.np / 4) * 32 * 8);
+        a.fwd_far = (f2*)take((size_t)a.ctas * a.np * 32 * 8);
+    }
     if (a.P <= TO_ROV_SCAN_PATHS) {
         const size_t tiles = (size_t)a.sel_slots * G * per;
         a.nbr = (unsigned short*)take(tiles * TO_ROV_TILE * a.kmax * 2);

@@ -148,7 +148,7 @@ to_status to_simulate_rov_batch(to_ctx ctx, int n_roads, const to_rov_problem* p
     acc((size_t)RS * C * (NP + 1) * 4); acc((size_t)RS * C * cap * 2); acc((size_t)RS * C * cap * 4);
     acc((size_t)RS * C * 4);
     // union form of each road-species' C <= 3 matrices
-    const int ucap = C <= 3 ? (C * cap < NP * NP ? C * cap : NP * NP) : 0;
+    const int ucap = C <= 3 ? (C * cap < NP * NP ? C * cap : NP * NP) + NP : 0;   // lists padded
     if (C <= 3) { acc((size_t)RS * ucap * 16); acc((size_t)RS * (NP + 1) * 4); acc((size_t)RS * 4); }
     if (algo == 6) { acc((size_t)Y * S * NP * P * 4); acc((size_t)Y * S * P * 4); }
     // regressions fitted only where the backward pass reads them, unless
@@ -171,6 +171,7 @@ to_status to_simulate_rov_batch(to_ctx ctx, int n_roads, const to_rov_problem* p
     // every year's regressions are kept where the caller wants them or the
     // re-simulation reads them again
     a.reg_by_slot = (want_reg || algo == 6) ? 0 : 1;
+    a.ctas = ctx->sm_count > 0 ? ctx->sm_count : TO_SM_TARGET;
     to_k::rov_plan(a, NR);
     const size_t nreg = (size_t)(a.reg_by_slot ? a.slots : Y) * G * blk;
     acc(nreg * 4);

@@ -20,6 +20,7 @@
 #include <cstring>
 
 #include "to_internal.cuh"
+#include "to_mbar.cuh"
 #include "to_pop.cuh"
 #include "to_rov.cuh"
 #include "to_rov_dev.cuh"
@@ -312,6 +313,7 @@ __global__ void __launch_bounds__(1024) k_mte_order(int n_rs, int rs0, int C, in
 // CTA; a thread per destination merges its C ascending origin lists (count,
 // CTA scan, write).
 // ---------------------------------------------------------------------------
+constexpr int kNoOrigin = 0xFFFF;                  // a zero term: the row of zeros
 __device__ __forceinline__ int union_step(const int* b, const int* e, const uint16_t* const* ix,
                                           int C, int* pos) {
     int lo = 0x7fffffff;
@@ -357,6 +359,7 @@ k_union_csc(int NP, int C, const int* __restrict__ n_patches, to_csc csc) {
             for (int c = 0; c < C; ++c) if (pos[c] < e[c] && (int)ix[c][pos[c]] == lo) ++pos[c];
             ++n;
         }
+        n = (n + 1) & ~1;                          // an even number, the last a zero term
         up[k] = n;
         cnt += n;
     }
@@ -397,87 +400,126 @@ k_union_csc(int NP, int C, const int* __restrict__ n_patches, to_csc csc) {
             out[q++] = make_int4(lo, __float_as_int(v[0]), __float_as_int(v[1]),
                                  __float_as_int(v[2]));
         }
+        if ((q - up[k]) & 1) out[q] = make_int4(kNoOrigin, 0, 0, 0);
     }
 }
 
 // ---------------------------------------------------------------------------
-// ROV forward paths on the union columns (C <= 3 controls) - grid (ceil(P/32),
-// roads), up to 32 warps.  As k_rov_forward_sparse, but
-//  * each non-zero of destination k is one 16-byte shared load {row byte
-//    offset, value of control 0, 1, 2} that serves every control's
-//    migration (three FMA chains, each in ascending origin order with exact
-//    zero terms where a control has no entry);
-//  * a warp takes the year's groups of four destinations from a shared
-//    counter, widest group first, and writes the new populations to the
-//    second buffer, so that no warp waits at the year's barrier for a fixed
-//    share of wide columns;
-//  * the growth mean's three draws per path are drawn for kGmChunk years at
-//    a time by the whole CTA, and every warp carries the lane's growth mean
-//    forward itself (same expression, same bits) - two barriers a year.
-// The values equal k_rov_forward_sparse's bit for bit: every group's
-// arithmetic and every sum's order is unchanged, only who computes it.
+// ROV forward paths on the union columns (C <= 3 controls), two paths a
+// lane.  Persistent: one CTA an SM, taking 64-path tiles of the roads from a
+// counter.  Bound by instruction issue (and shared-memory latency below it),
+// so the work is laid out for few instructions a path:
+//  * a row of the populations holds two paths a lane, so that an entry of a
+//    destination's list, its address and the loop around it serve both, and
+//    the growth, the sums and the arithmetic of the normals run on packed
+//    pairs (to_f2.cuh);
+//  * the growth normals' Philox blocks share what does not change between
+//    groups, years or paths and read their round keys from the constant bank;
+//  * the year's populations are read from one buffer and written to another,
+//    so a warp takes groups of four destinations from a shared counter,
+//    widest first, and a year has one barrier, split: a warp that is done
+//    arrives, draws the normals of its own first group of the next year and
+//    only then waits (39.1 -> 37.5 ms).  Where two buffers do not fit
+//    beside the lists, the other one is in global memory (it stays in L2)
+//    and copied back after the barrier.  What the year's end needs
+//    summed over the groups - each control's migrated totals, in group order -
+//    goes through a small global scratch (it stays in L2) and is added up
+//    during the next year by whichever warp takes it, like the total of the
+//    populations: no warp waits for a chain of 80 additions.
+// 256 roads, 768 paths, 3 species, 50 years: 50.4 -> 37.5 ms (one path a
+// lane before), 65% of the issue slots, the FMA pipe at about the same.  The values
+// are those of k_rov_forward_sparse bit for bit: every group's arithmetic
+// and every sum's order is unchanged, only who computes it.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(1024, 1)
-k_rov_forward_union(to_rov_args a, to_csc csc) {
-    extern __shared__ __align__(16) unsigned char sm_raw[];
-    const int NE = a.ne, NG = NE >> 2, C = a.C, Y = a.Y, P = a.P;
-    const size_t PT = (size_t)a.PT;
-    const int rd = blockIdx.y;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, W = blockDim.x >> 5;
-    const int path = blockIdx.x * kLanes + lane;
-    const size_t gp = (size_t)rd * P + path;
-    int4* ue = reinterpret_cast<int4*>(sm_raw);                    // [ucap_smem]
-    float* bufA = reinterpret_cast<float*>(ue + csc.ucap_smem);    // [NE][32]
-    float* bufB = bufA + (size_t)NE * kLanes;                      // [NE][32]
-    float* part = bufB + (size_t)NE * kLanes;                      // [C+1][NG][32]
-    float2* capr = reinterpret_cast<float2*>(part + (size_t)(C + 1) * NG * kLanes);  // [NE]
-    float* xs = reinterpret_cast<float*>(capr + NE);               // [kGmChunk][3][32]
-    float* tot = xs + kGmChunk * 3 * kLanes;                       // [32]
-    float* ntot = tot + kLanes;                                    // [32]
-    int* uptr = reinterpret_cast<int*>(ntot + kLanes);             // [NE+1]
-    int* order = uptr + NE + 1;                                    // [NG]
-    int* grab = order + NG;                                        // [2]
-    const uint32_t road = (uint32_t)a.road_ids[rd];
+constexpr int kPairPaths = 64;
 
-    for (int s = 0; s < a.S; ++s) {
-        const int rs = rd * a.S + s;
-        const int N = a.n_patches[rs];
-        const int N4 = (N + 3) & ~3;
-        const int NGr = N4 >> 2;
-        const float* sp = a.params + 8 * s;
-        const float* ip = a.init_pops + (size_t)rs * a.np;
-        const int nu = csc.unnz[rs];
-        if (nu < 0 || nu > csc.ucap_smem || N > NE) {
+// shared memory of one (road, species): with both populations buffers, or
+// with the next year's in global memory
+__host__ __device__ inline size_t pair_bytes(int N4, int nu, bool two) {
+    return (size_t)((nu + 1) & ~1) * 16 + (size_t)(two ? 2 : 1) * (N4 + 1) * kLanes * 8 +
+           (size_t)N4 * 16 + (size_t)kGmChunk * 3 * kPairPaths * 4 + (size_t)2 * kLanes * 8 +
+           (size_t)(N4 + 4 + N4 / 4 + 4) * 4;
+}
+constexpr int kPairStatic = 3072;          // static shared memory and slack
+constexpr int kPairThreads = 1024;         // 512, 640 and 768: 39.9, 39.7 and 40.3 ms where 1024 takes 37.5
+
+template <bool REF>
+__global__ void __launch_bounds__(kPairThreads, 1)
+k_rov_forward_union(to_rov_args a, to_csc csc, int smem) {
+    extern __shared__ __align__(16) unsigned char sm_raw[];
+    __shared__ int s_item, s_grab[2];
+    __shared__ to_bm_tables s_tab;
+    __shared__ __align__(8) uint64_t s_bar;    // end of a year: an arrival a warp
+    const int C = a.C, Y = a.Y, P = a.P, S = a.S;
+    const size_t PT = (size_t)a.PT;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tiles = (P + kPairPaths - 1) / kPairPaths, items = tiles * a.nr * S;
+    const int ngcap = a.np / 4;
+    f2* part = a.fwd_part + (size_t)blockIdx.x * 2 * C * ngcap * kLanes;   // [2][C][ngcap][32]
+    to_bm_load(s_tab);                         // before the barriers below
+    if (tid == 0) to_mbar::init(&s_bar, kPairThreads / 32);
+    uint32_t phase = 0;
+    for (;;) {
+        if (tid == 0) s_item = atomicAdd(a.fwd_next, 1);
+        __syncthreads();
+        const int item = s_item;
+        __syncthreads();                       // read before it is written again
+        if (item >= items) break;
+        const int s = item % S, rd = item / S / tiles, rs = rd * S + s;
+        const int path0 = (item / S - rd * tiles) * kPairPaths + lane, path1 = path0 + kLanes;
+        const bool live0 = path0 < P, live1 = path1 < P;
+        const size_t gp = (size_t)rd * P + path0;
+        const int N = a.n_patches[rs], nu = csc.unnz[rs];
+        const int N4 = (N + 3) & ~3, NGr = N4 >> 2;
+        if (nu < 0 || N > a.ne || pair_bytes(N4, nu, false) > (size_t)smem) {
             // outside the shape this launch was planned for: flag, no result
-            if (threadIdx.x == 0 && a.flags) atomicExch(a.flags, TO_DEVERR_PLAN);
-            if (warp == 0 && path < P)
-                for (int t = 0; t <= Y; ++t)
-                    a.totalPops[((size_t)s * (Y + 1) + t) * PT + gp] = NAN;
+            if (tid == 0 && a.flags) atomicExch(a.flags, TO_DEVERR_PLAN);
+            for (int t = warp; t <= Y; t += blockDim.x >> 5) {
+                float* out = a.totalPops + ((size_t)s * (Y + 1) + t) * PT + gp;
+                if (live0) out[0] = NAN;
+                if (live1) out[kLanes] = NAN;
+            }
             continue;
         }
-        __syncthreads();
-        float* cur = bufA;
-        float* nxt = bufB;
-        for (int q = threadIdx.x; q < NE * kLanes; q += blockDim.x) {
+        const uint32_t road = (uint32_t)a.road_ids[rd];
+        const uint32_t stream_road = TO_STREAM_GROWTH | (road << 8);
+        to_path_stream ps0, ps1;
+        to_stream_path(ps0, (uint32_t)path0);
+        to_stream_path(ps1, (uint32_t)path1);
+        int4* ue = reinterpret_cast<int4*>(sm_raw);                    // [nu]
+        f2* cur = reinterpret_cast<f2*>(ue + ((nu + 1) & ~1));         // [N4 + 1][32], row N4 zero
+        const bool two = pair_bytes(N4, nu, true) <= (size_t)smem;
+        f2* nxt = two ? cur + (size_t)(N4 + 1) * kLanes : cur;         // the same
+        f2* far = a.fwd_far + (size_t)blockIdx.x * a.np * kLanes;      // [N4][32] otherwise
+        float4* capr = reinterpret_cast<float4*>(nxt + (size_t)(N4 + 1) * kLanes);  // [N4]
+        // draws of the growth mean, then [0] the means and [1] the controls
+        float* xs = reinterpret_cast<float*>(capr + N4);               // [kGmChunk][3][64]
+        f2* tot = reinterpret_cast<f2*>(xs + kGmChunk * 3 * kPairPaths);   // [2][32]
+        int* uptr = reinterpret_cast<int*>(tot + 2 * kLanes);          // [N4 + 1]
+        int* order = uptr + N4 + 4;                                    // [NGr]
+        const float* sp = a.params + 8 * s;
+        const float* ip = a.init_pops + (size_t)rs * a.np;
+        for (int q = tid; q < (N4 + 1) * kLanes; q += blockDim.x) {
             const int k = q / kLanes;
-            cur[q] = (k < N) ? ip[k] : 0.0f;
-            nxt[q] = 0.0f;
+            cur[q] = both2(k < N ? ip[k] : 0.0f);
+            if (k == N4) nxt[q] = both2(0.0f);
         }
-        for (int k = threadIdx.x; k < NE; k += blockDim.x) {
-            const float cp = a.caps[(size_t)rs * a.np + k];
-            capr[k] = make_float2(cp, 1.0f / cp);          // capacity, its reciprocal
+        for (int k = tid; k < N4; k += blockDim.x) {
+            const float cp = a.caps[(size_t)rs * a.np + k], nr = -(1.0f / cp);
+            capr[k] = make_float4(cp, cp, nr, nr);     // capacity, minus its reciprocal
         }
-        for (int k = threadIdx.x; k <= NE; k += blockDim.x)
-            uptr[k] = csc.uptr[(size_t)rs * (a.np + 1) + (k <= a.np ? k : a.np)];
-        for (int e = threadIdx.x; e < nu; e += blockDim.x) {
+        for (int k = tid; k <= N4; k += blockDim.x)
+            uptr[k] = csc.uptr[(size_t)rs * (a.np + 1) + k];
+        for (int e = tid; e < nu; e += blockDim.x) {
             int4 v = csc.uent[(size_t)rs * csc.ucap + e];
-            v.x *= kLanes * (int)sizeof(float);                    // origin -> row byte offset
+            // origin -> row byte offset
+            v.x = (v.x == kNoOrigin ? N4 : v.x) * kLanes * (int)sizeof(f2);
             ue[e] = v;
         }
-        if (threadIdx.x < 2) grab[threadIdx.x] = 0;
+        if (tid < 2) s_grab[tid] = 0;
         __syncthreads();
         // the groups in descending order of entries (ties: lower group first)
-        for (int gq = threadIdx.x; gq < NGr; gq += blockDim.x) {
+        for (int gq = tid; gq < NGr; gq += blockDim.x) {
             const int w = uptr[4 * gq + 4] - uptr[4 * gq];
             int rank = 0;
             for (int u = 0; u < NGr; ++u) {
@@ -486,124 +528,228 @@ k_rov_forward_union(to_rov_args a, to_csc csc) {
             }
             order[rank] = gq;
         }
-        if (warp == 0) {
-            float tt = 0.0f;
-            for (int grp = 0; grp < NGr; ++grp) {
-                const float* v = cur + (size_t)grp * 4 * kLanes + lane;
-                tt = tt + grouped4(v[0], v[kLanes], v[2 * kLanes], v[3 * kLanes]);
-            }
-            tot[lane] = tt;
-            if (path < P) a.totalPops[((size_t)s * (Y + 1)) * PT + gp] = tt;
-        }
-        const float jp = (a.sem == 0) ? sp[5] : sp[6];
+        const float jp = REF ? sp[5] : sp[6];
         const float s5 = sp[5] * sp[5];
-        float g = sp[0];                                           // this lane's growth mean
+        const f2 s7 = both2(sp[7]), one = both2(1.0f), mone = both2(-1.0f);
+        float gmean = sp[0];                           // of path `tid` of the tile (tid < 64)
+        f2 z[4];                                       // normals of the group worked on
+        // totals of the populations at the start of year t
+        auto total = [&](int t) {
+            f2 tt = both2(0.0f);
+#pragma unroll 4
+            for (int grp = 0; grp < NGr; ++grp) {
+                const f2* v = cur + (size_t)grp * 4 * kLanes + lane;
+                tt = add2(tt, add2(add2(add2(v[0], v[kLanes]), v[2 * kLanes]), v[3 * kLanes]));
+            }
+            tot[(t & 1) * kLanes + lane] = tt;
+            float t0, t1;
+            unpack2(tt, t0, t1);
+            float* out = a.totalPops + ((size_t)s * (Y + 1) + t) * PT + gp;
+            if (live0) out[0] = t0;
+            if (live1) out[kLanes] = t1;
+        };
+        // control c's share of the animals left after the migration of year t
+        auto at_risk = [&](int t, int c) {
+            const f2* v = part + ((size_t)(t & 1) * C + c) * ngcap * kLanes + lane;
+            f2 tt = both2(0.0f);
+#pragma unroll 8
+            for (int grp = 0; grp < NGr; ++grp) tt = add2(tt, v[(size_t)grp * kLanes]);
+            float t0, t1, p0, p1;
+            unpack2(tt, t0, t1);
+            unpack2(tot[(t & 1) * kLanes + lane], p0, p1);
+            float* out = a.aars + (((size_t)s * C + c) * Y + t) * PT + gp;
+            if (live0) out[0] = t0 / p0;
+            if (live1) out[kLanes] = t1 / p1;
+        };
+        auto normals = [&](int grp) {
+            to_normal4x2(ps0, ps1,
+                         to_stream_group((uint32_t)((s * N4) >> 2) + grp, stream_road, a.rk),
+                         a.rk, s_tab, z);
+        };
+        auto next_year = [&](int t) {
+            to_stream_year(ps0, (uint32_t)t, a.rk);
+            to_stream_year(ps1, (uint32_t)t, a.rk);
+        };
         for (int t = 0; t < Y; ++t) {
             if (t % kGmChunk == 0) {
                 // the next years' growth-mean draws, one thread each
                 const int nc = min(kGmChunk, Y - t);
-                for (int q = threadIdx.x; q < nc * 3 * kLanes; q += blockDim.x) {
-                    const int yy = q / (3 * kLanes), r = q - yy * 3 * kLanes;
-                    const int which = r >> 5, i = r & 31;
-                    const uint32_t pth = (uint32_t)(blockIdx.x * kLanes + i);
+                for (int q = tid; q < nc * 3 * kPairPaths; q += blockDim.x) {
+                    const int yy = q / (3 * kPairPaths), r = q - yy * 3 * kPairPaths;
+                    const int which = r / kPairPaths, i = r - which * kPairPaths;
+                    const uint32_t pth = (uint32_t)(path0 - lane + i);
                     const int ty = t + yy;
                     float v;
                     if (which == 0) {
-                        v = (to_uniform1(a.seed, TO_STREAM_SP_JUMP, road, pth, ty, s) < jp) ? 1.0f
-                                                                                             : 0.0f;
+                        v = (to_uniform1(a.seed, TO_STREAM_SP_JUMP, road, pth, ty, s) < jp)
+                                ? 1.0f : 0.0f;
                     } else if (which == 1) {
                         v = to_normal1(a.seed, TO_STREAM_SP_BROWNIAN, road, pth, ty, s) * sp[2];
                     } else {
-                        const float zj = to_normal1(a.seed, TO_STREAM_SP_JUMPSIZE, road, pth, ty, s);
-                        const float jsz = (a.sem == 0) ? (zj * s5 - s5 / 2.0f)
-                                                       : (zj * sp[5] - s5 / 2.0f);
+                        const float zj =
+                            to_normal1(a.seed, TO_STREAM_SP_JUMPSIZE, road, pth, ty, s);
+                        const float jsz = REF ? (zj * s5 - s5 / 2.0f) : (zj * sp[5] - s5 / 2.0f);
                         v = to_expf(jsz) - 1.0f;
                     }
                     xs[q] = v;
                 }
                 __syncthreads();
-            }
-            {
-                const float* xt = xs + (t % kGmChunk) * 3 * kLanes;
-                const float jump = xt[lane], brown = xt[kLanes + lane], em1 = xt[2 * kLanes + lane];
-                g = g + sp[4] * (sp[1] - g) * a.dt + g * brown + em1 * g * jump;
-            }
-            if (warp == 0 && a.gmY && path < P) a.gmY[((size_t)t * a.S + s) * P + path] = g;
-            const int my_c = (path < P) ? a.controls[(size_t)t * PT + gp] : 0;
-            if (a.popsY) {
-                for (int q = threadIdx.x; q < NE * kLanes; q += blockDim.x) {
-                    const int pth = blockIdx.x * kLanes + (q & (kLanes - 1));
-                    if (pth < P)
-                        a.popsY[(((size_t)t * a.S + s) * NE + (q >> 5)) * P + pth] = cur[q];
+                // the growth means do not depend on the populations: the
+                // years' recursion, a thread a path
+                if (tid < kPairPaths) {
+                    const int pth = path0 - lane + tid;
+                    int ctl[kGmChunk];
+#pragma unroll
+                    for (int yy = 0; yy < kGmChunk; ++yy)
+                        ctl[yy] = (yy < nc && pth < P)
+                                      ? a.controls[(size_t)(t + yy) * PT + (size_t)rd * P + pth] : 0;
+#pragma unroll
+                    for (int yy = 0; yy < kGmChunk; ++yy)
+                        if (yy < nc) {
+                            float* x = xs + yy * 3 * kPairPaths + tid;
+                            gmean = gmean + sp[4] * (sp[1] - gmean) * a.dt + gmean * x[kPairPaths] +
+                                    x[2 * kPairPaths] * gmean * x[0];
+                            x[0] = gmean;
+                            x[kPairPaths] = __int_as_float(ctl[yy]);
+                            if (a.gmY && pth < P)
+                                a.gmY[((size_t)(t + yy) * S + s) * P + pth] = gmean;
+                        }
                 }
+                __syncthreads();
             }
-            const unsigned char* curb = reinterpret_cast<const unsigned char*>(cur) + lane * 4;
-            int* gc = grab + (t & 1);
+            const float* xt = xs + (t % kGmChunk) * 3 * kPairPaths + lane;
+            const float g0 = xt[0], g1 = xt[kLanes];
+            const int c0 = __float_as_int(xt[kPairPaths]), c1 = __float_as_int(xt[kPairPaths + kLanes]);
+            if (a.popsY)
+                for (int q = tid; q < a.ne * kPairPaths; q += blockDim.x) {
+                    const int k = q / kPairPaths, i = q - k * kPairPaths;
+                    const int pth = path0 - lane + i;
+                    if (pth < P)
+                        a.popsY[(((size_t)t * S + s) * a.ne + k) * P + pth] =
+                            k < N4 ? reinterpret_cast<const float*>(
+                                         cur + (size_t)k * kLanes + (i & 31))[i >> 5] : 0.0f;
+                }
+            const f2 g = pack2(g0, g1);
+            const unsigned char* curb = reinterpret_cast<const unsigned char*>(cur + lane);
+            f2* py = part + (size_t)(t & 1) * C * ngcap * kLanes + lane;
+            // the year's work: a group each, then from the counter the totals and
+            // last year's shares, then the other groups
+            if (t == 0) {
+                next_year(0);
+                if (warp < NGr) normals(order[warp]);
+            }
+            const int lead = t ? 1 + C : 1;
+            int* gc = s_grab + (t & 1);
+            bool own = warp < NGr;
             for (;;) {
-                int i = 0;
-                if (lane == 0) i = atomicAdd(gc, 1);
-                i = __shfl_sync(0xffffffffu, i, 0);
-                if (i >= NGr) break;
-                const int grp = order[i];
-                float z[4];
-                to_normal4(a.seed, TO_STREAM_GROWTH, road, path, t,
-                           (uint32_t)((s * N4) >> 2) + grp, z);
-                float m0[4], m1[4], m2[4], np4[4];
+                int grp;
+                if (own) {
+                    grp = order[warp];
+                    own = false;
+                } else {
+                    int i = 0;
+                    if (lane == 0) i = atomicAdd(gc, 1);
+                    i = __shfl_sync(0xffffffffu, i, 0) - lead;
+                    if (i < 0) {
+                        if (i == -1) total(t);
+                        else at_risk(t - 1, -2 - i);
+                        continue;
+                    }
+                    i += kPairThreads / 32;
+                    if (i >= NGr) break;
+                    grp = order[i];
+                    normals(grp);
+                }
                 // the group's column pointers: one 16-byte load and one word
                 const int4 u4 = reinterpret_cast<const int4*>(uptr)[grp];
                 const int ub[5] = {u4.x, u4.y, u4.z, u4.w, uptr[grp * 4 + 4]};
+                f2 m0, m1, m2;             // the group's migrated sums by control
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     const int k = grp * 4 + j;
-                    float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f;
+                    f2 q0 = 0ull, q1 = 0ull, q2 = 0ull;        // migrated, by control
                     const int e1 = ub[j + 1];
-#pragma unroll 4
-                    for (int e = ub[j]; e < e1; ++e) {
-                        const int4 en = ue[e];
-                        const float x = *reinterpret_cast<const float*>(curb + en.x);
-                        a0 = fmaf(x, __int_as_float(en.y), a0);
-                        a1 = fmaf(x, __int_as_float(en.z), a1);
-                        a2 = fmaf(x, __int_as_float(en.w), a2);
+#pragma unroll 2
+                    for (int e = ub[j]; e < e1; e += 2) {      // an even number of terms
+#pragma unroll
+                        for (int u = 0; u < 2; ++u) {
+                            const int4 en = ue[e + u];
+                            const f2 x = *reinterpret_cast<const f2*>(curb + en.x);
+                            q0 = fma2(x, both2(__int_as_float(en.y)), q0);
+                            q1 = fma2(x, both2(__int_as_float(en.z)), q1);
+                            q2 = fma2(x, both2(__int_as_float(en.w)), q2);
+                        }
                     }
-                    m0[j] = a0; m1[j] = a1; m2[j] = a2;
-                    const float mv = (my_c == 0) ? a0 : ((my_c == 1) ? a1 : a2);
-                    const float gr = (a.sem == 0) ? g + z[j] * sp[7] : fmaf(sp[7] * z[j], g, g);
-                    const float2 cr = capr[k];
-                    // the divisions as to_div_rcp: the same bits
-                    const float v = (a.sem == 0)
-                        ? mv * (1.0f + to_div_rcp(to_div_rcp(gr * (cr.x - mv), cr.x, cr.y), 100.0f,
-                                                  0.01f))
-                        : fmaxf(mv * (1.0f + to_div_rcp(gr * (cr.x - mv), cr.x, cr.y)), 0.0f);
-                    nxt[k * kLanes + lane] = v;
-                    np4[j] = v;
+                    float a00, a01, a10, a11, a20, a21;
+                    unpack2(q0, a00, a01);
+                    unpack2(q1, a10, a11);
+                    unpack2(q2, a20, a21);
+                    m0 = j ? add2(m0, q0) : q0;
+                    m1 = j ? add2(m1, q1) : q1;
+                    m2 = j ? add2(m2, q2) : q2;
+                    const f2 mv = pack2(c0 == 0 ? a00 : (c0 == 1 ? a10 : a20),
+                                        c1 == 0 ? a01 : (c1 == 1 ? a11 : a21));
+                    f2 gr;
+                    if (REF) {
+                        // scalar: ptxas joins a packed multiply and add
+                        float z0, z1;
+                        unpack2(z[j], z0, z1);
+                        gr = pack2(g0 + z0 * sp[7], g1 + z1 * sp[7]);
+                    } else {
+                        gr = fma2(mul2(s7, z[j]), g, g);
+                    }
+                    // (gr (cap - mv)) / cap as to_div_rcp, with minus the
+                    // reciprocal: minus the quotient, the same bits
+                    const ulonglong2 cr = *reinterpret_cast<const ulonglong2*>(capr + k);
+                    const f2 x = mul2(gr, fma2(mv, mone, cr.x));
+                    const f2 nq = mul2(x, cr.y);
+                    f2 nd = fma2(fma2(nq, cr.x, x), cr.y, nq);
+                    f2 v;
+                    if (REF) {
+                        // and / 100, the same way
+                        const f2 q = mul2(nd, both2(0.01f));
+                        const f2 r = fma2(neg2(q), both2(100.0f), nd);
+                        nd = fma2(r, both2(0.01f), q);
+                        v = mul2(mv, fma2(nd, mone, one));
+                    } else {
+                        float v0, v1;
+                        unpack2(mul2(mv, fma2(nd, mone, one)), v0, v1);
+                        v = pack2(fmaxf(v0, 0.0f), fmaxf(v1, 0.0f));
+                    }
+                    if (two) nxt[k * kLanes + lane] = v;
+                    else far[k * kLanes + lane] = v;
                 }
-                part[((size_t)0 * NG + grp) * kLanes + lane] = grouped4(m0[0], m0[1], m0[2], m0[3]);
-                if (C > 1)
-                    part[((size_t)1 * NG + grp) * kLanes + lane] = grouped4(m1[0], m1[1], m1[2], m1[3]);
-                if (C > 2)
-                    part[((size_t)2 * NG + grp) * kLanes + lane] = grouped4(m2[0], m2[1], m2[2], m2[3]);
-                part[((size_t)C * NG + grp) * kLanes + lane] = grouped4(np4[0], np4[1], np4[2], np4[3]);
+                py[(size_t)grp * kLanes] = m0;
+                if (C > 1) py[((size_t)ngcap + grp) * kLanes] = m1;
+                if (C > 2) py[((size_t)2 * ngcap + grp) * kLanes] = m2;
             }
-            // last used in the year before; two barriers before the next year
-            if (threadIdx.x == 0) grab[(t + 1) & 1] = 0;
-            __syncthreads();
-            for (int c = warp; c <= C; c += W) {
-                float tt = 0.0f;
-#pragma unroll 8
-                for (int grp = 0; grp < NGr; ++grp)
-                    tt = tt + part[((size_t)c * NG + grp) * kLanes + lane];
-                if (path < P) {
-                    if (c < C) a.aars[(((size_t)s * C + c) * Y + t) * PT + gp] = tt / tot[lane];
-                    else a.totalPops[((size_t)s * (Y + 1) + t + 1) * PT + gp] = tt;
-                }
-                if (c == C) ntot[lane] = tt;
+            // last used in the year before the last barrier
+            if (tid == 0) s_grab[(t + 1) & 1] = 0;
+            // done: while the others finish, the normals of next year's own group
+            __syncwarp();
+            if (lane == 0) to_mbar::arrive(&s_bar);
+            if (t + 1 < Y) {
+                next_year(t + 1);
+                if (warp < NGr) normals(order[warp]);
             }
-            __syncthreads();
-            if (warp == 0) tot[lane] = ntot[lane];
-            float* tmp = cur;
-            cur = nxt;
-            nxt = tmp;
+            if (!to_mbar::wait(&s_bar, phase)) {
+                if (a.flags) atomicExch(a.flags, TO_DEVERR_SPIN);
+                return;
+            }
+            phase ^= 1u;
+            if (two) {
+                f2* tmp = cur;
+                cur = nxt;
+                nxt = tmp;
+            } else {
+#pragma unroll 4
+                for (int q = tid; q < N4 * kLanes; q += blockDim.x) cur[q] = far[q];
+                __syncthreads();
+            }
         }
+        if (warp == 0) total(Y);
+        else if (warp <= C && Y > 0) at_risk(Y - 1, warp - 1);
+        __syncthreads();
     }
 }
 
@@ -1016,12 +1162,8 @@ size_t rov_sparse_smem(int NE, int C, int cap_smem) {
 }
 
 size_t rov_union_smem(int NE, int C, int ucap_smem) {
-    if (NE > 32 * kMaxG * 4 || C > 3) return ~size_t(0);
-    const int NG = NE / 4;
-    return (size_t)ucap_smem * 16 +
-           (size_t)(2 * NE * kLanes + (C + 1) * NG * kLanes + 2 * NE + kGmChunk * 3 * kLanes +
-                    2 * kLanes) * 4 +
-           (size_t)(NE + 1 + NG + 2) * 4 + 16;
+    if (C > 3) return ~size_t(0);
+    return pair_bytes(NE, ucap_smem, false) + kPairStatic;
 }
 
 to_status union_csc(to_ctx ctx, int NP, int C, const int* n_patches, int n_rs, to_csc& csc) {
@@ -1034,16 +1176,15 @@ to_status union_csc(to_ctx ctx, int NP, int C, const int* n_patches, int n_rs, t
 
 to_status rov_forward_sparse(to_ctx ctx, const to_rov_args& a, to_csc csc) {
     if (csc.uent && a.C <= 3) {
-        const size_t smem = rov_union_smem(a.ne, a.C, csc.ucap_smem);
-        if (smem > ctx->smem_optin)
-            return to_set_error(ctx, TO_ERR_UNSUPPORTED, "union ROV needs %zu B", smem);
-        const dim3 blocks((a.P + kLanes - 1) / kLanes, a.nr);
-        const int NG = a.ne / 4;
-        const int warps = NG < 32 ? (NG > 4 ? NG : 4) : 32;
+        // every (road, species) lays its own sizes out in all of the shared
+        // memory, so a plan's margin costs nothing
+        const int smem = (int)ctx->smem_optin - kPairStatic;
+        const int items = (a.P + kPairPaths - 1) / kPairPaths * a.nr * a.S;
+        const auto pair = a.sem == 0 ? k_rov_forward_union<true> : k_rov_forward_union<false>;
+        TO_CUDA(ctx, cudaMemsetAsync(a.fwd_next, 0, sizeof(int), ctx->stream));
+        TO_CUDA(ctx, cudaFuncSetAttribute(pair, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         to_prof_begin(ctx, "rov_forward_sparse");
-        TO_CUDA(ctx, cudaFuncSetAttribute(k_rov_forward_union,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k_rov_forward_union<<<blocks, warps * 32, smem, ctx->stream>>>(a, csc);
+        pair<<<items < a.ctas ? items : a.ctas, kPairThreads, smem, ctx->stream>>>(a, csc, smem);
         to_prof_end(ctx);
         TO_LAUNCHED(ctx);
         return TO_OK;

@@ -1,6 +1,7 @@
 // to_rov.cuh - argument block of the ROV kernels and the kNN / regression
 // launchers shared with the surrogate builders.
 #pragma once
+#include "to_f2.cuh"
 #include "to_internal.cuh"
 #include "to_lsm_math.h"
 
@@ -28,6 +29,11 @@ struct to_rov_args {
     int nF, Cm, demand_idx, sem, road;
     float dt, rrr, unit_cost, unit_revenue, scaling;
     uint64_t seed;
+    to_round_keys rk;                 // of the seed (rov_run)
+    int ctas;                         // resident CTAs of the paired forward pass
+    int* fwd_next;                    // its work counter
+    f2* fwd_part;                     // [ctas][2][C][np / 4][32] its per-group sums
+    f2* fwd_far;                      // [ctas][np][32] next populations of wide models
     int np, ne;                       // stride / effective width of patch arrays
     int tile_paths, l_chunk;          // forward tile (launcher)
     // inputs (device)

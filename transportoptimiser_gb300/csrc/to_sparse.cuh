@@ -14,7 +14,8 @@ struct to_csc {
     // destination k's entries are the origins where any control has a
     // non-zero, ascending, each as {origin, value of control 0, 1, 2} with
     // 0 where a control has none (an exact zero term, so every control's
-    // sums keep their bits)
+    // sums keep their bits), padded to an even number by a zero term of no
+    // origin
     int4* uent;        // [road-species][ucap]
     int* uptr;         // [road-species][NP + 1]
     int* unnz;         // [road-species], -1 when above ucap
