@@ -1,0 +1,56 @@
+"""The population sweeps of the frozen-policy sensitivities where their layout
+changes course, against the FP64 oracle and its central differences: path
+counts around a tile of 64, patch counts around a group of four and where
+the next year's rows no longer fit in shared memory beside the others, years
+around a checkpoint interval of 10, controls no entry or some entries
+distinguish."""
+import numpy as np
+import pytest
+
+from oracle import pyoracle as po
+from transportoptimiser_gb300.adjoint import FrozenPolicy, theta_from_problem
+
+pytestmark = pytest.mark.gpu
+
+
+def _problem(N, nnz, P, Y, C, S, seed):
+    rng = np.random.default_rng(seed)
+    hz = np.linspace(0.0, 0.4, C)
+    species, cross = [], []
+    for s in range(S):
+        x = (rng.integers(0, 3, (N, N)) * (rng.random((N, N)) < 0.6)).astype(np.int32)  # [l][k]
+        m = np.zeros((N, N))
+        for k in range(N):
+            m[k, rng.choice(N, size=min(N, int(rng.integers(0, 2 * nnz + 1))), replace=False)] = 1.0
+        m *= rng.random((N, N)) * 1.5 / max(nnz, 1)
+        mmm = np.stack([m * np.exp(-x.T * h) for h in hz])
+        ip = rng.integers(100, 2500, N).astype(np.float32)
+        species.append(dict(N=N, params=np.array([0.05, 0.06, 0.05, 0, 0.5, 0.1, 0.2, 0.4], np.float32),
+                            init_pops=ip, caps=2 * ip, mmm=mmm.astype(np.float32)))
+        cross.append(x)
+    unc = np.array([[1, 1, 0.1, 0.2, 0, 0], [1, 1, 0.2, 0.35, 0.1, 0.2]], np.float32)
+    pr = dict(n_paths=P, n_years=Y, dim_res=4, dt=1.0, rrr=7.0, unit_cost=0.5, unit_revenue=1.2,
+              seed=9, road=2, sem=1, species=species,
+              flows=np.linspace(0, 100, C).astype(np.float32), uncert=unc.reshape(-1),
+              fuel_costs=np.array([0.3], np.float32), fuel_idx=np.array([0], np.int32),
+              ore_content=np.array([0.8], np.float32), ore_sd=np.array([0.05], np.float32),
+              demand_idx=-1)
+    ctl = rng.integers(0, C, (Y, P)).astype(np.int32)
+    return pr, cross, hz, ctl
+
+
+@pytest.mark.parametrize("N,nnz,P,Y,C,S", [
+    (1, 1, 1, 1, 1, 1), (3, 2, 33, 9, 2, 1), (4, 2, 64, 10, 3, 3), (65, 4, 65, 11, 3, 2),
+    (70, 3, 20, 21, 8, 1), (400, 3, 3, 4, 3, 1), (512, 2, 5, 11, 2, 1)])
+def test_sweeps_match_fp64(ctx, N, nnz, P, Y, C, S):
+    pr, cross, hz, ctl = _problem(N, nnz, P, Y, C, S, N + P)
+    th = theta_from_problem(pr, hz)
+    out, J = FrozenPolicy(pr, ctl, cross, hz, ctx).jacobian(th)
+    np.testing.assert_allclose(out, po.adjoint_forward(pr, ctl, cross, hz, th), rtol=1e-4)
+    for i in range(th.size):
+        h = 1e-4 * max(abs(th[i]), 1.0)
+        d = np.eye(th.size)[i] * h
+        fd = (po.adjoint_forward(pr, ctl, cross, hz, th + d) -
+              po.adjoint_forward(pr, ctl, cross, hz, th - d)) / (2 * h)
+        scale = np.abs(J).max(axis=1)
+        assert np.all(np.abs(J[:, i] - fd) <= 2e-3 * np.abs(fd) + 1e-3 * scale), (i, J[:, i], fd)

@@ -18,17 +18,30 @@
 // crossing hazard h_c (scales entry (k, l) of M_c by exp(-cross_lk dh_c)).
 // Outputs: E[PV], E[E_s].
 //
-// Forward: PV per path (one thread per path) and the population recursion
-// (one lane per path, states [patch][lane] in shared memory) with the
-// states checkpointed every K years.  Backward (vector-Jacobian product):
-// forward tangents for the scalar recursions (OU, growth-rate mean), and a
-// reverse sweep for the patch populations: each K-year segment is
-// recomputed from its checkpoint, then lambda_t = M_c^T (lambda_{t+1} .
+// Forward: PV per path (a thread per path) and the population recursion with
+// the states checkpointed every K years.  Backward (vector-Jacobian
+// product): forward tangents for the scalar recursions (OU, growth-rate
+// mean), and a reverse sweep for the patch populations: each K-year segment
+// is recomputed from its checkpoint, then lambda_t = M_c^T (lambda_{t+1} .
 // dF/dm) with the parameter terms accumulated on the way.  Per-path
 // contributions are averaged in FP64.
+//
+// The population sweeps run a CTA of 16 warps on 64 paths of one species:
+// lane = two paths, packed (to_f2.cuh); the warps take groups of four
+// patches, so that one Philox block serves the four normals it holds; a
+// patch's migration is one list of the patches it exchanges animals with,
+// each entry holding every control's value, of which a lane reads its own
+// control's - one multiply-add a path and entry whatever the number of
+// controls.  The states that other patches read are in shared memory, a
+// segment's states and migrated states in global memory (they stay in L2).
+// Bound by instruction issue and the latency of the lists' loads: two species
+// of 115 patches, 10,000 paths, 50 years: forward 9.1 -> 0.9 ms, a species'
+// reverse sweep 20 -> 2.0 ms (a thread a path over all patches and every
+// control's pairs before).
 #include <cmath>
 #include <vector>
 
+#include "to_f2.cuh"
 #include "to_internal.cuh"
 
 namespace {
@@ -51,15 +64,27 @@ struct AdjArgs {
     const float* params;                // [S][8]
     const float* init_pops;             // [S][NP]
     const float* caps;                  // [S][NP]
-    const int* coo_off;                 // [S*C + 1] entries of matrix (s, c)
-    const int* coo_k;                   // destination
-    const int* coo_l;                   // source
-    const float* coo_v;                 // value at the base hazards
-    const float* coo_x;                 // crossings of the pair
+    // migration lists of every species: patch k's entries [uptr[s][k],
+    // uptr[s][k + 1]) are the patches it receives from, ascending; the
+    // transposed lists those it sends to.  Entry e holds the values of all
+    // controls at the current hazards (k_adj_values) and a zero, which a
+    // control outside 0 .. C - 1 reads: under it nothing migrates
+    const int *uptr, *tptr;             // [S][NP + 1]
+    const int *ul, *tk;                 // [E] the other patch
+    const int* tsrc;                    // [E] the transposed entry's place in the first lists
+    const int4* uchain;                 // [E] first lists: 32 origin, 32 destination, -crossings
+    const float* base_v;                // [E][C + 1] values at the base hazards
+    float *uval, *tval;                 // [E][C + 1]
     const float* base_h;                // [C] hazards the values were built with
+    int E;
+    to_round_keys rk;
     // tape
     float* ckpt;                        // [S][Y/K + 1][NP][P]
-    float* seg;                         // [S][K][NP][P]
+    f2* segx;                           // [S][tiles][K][NP][32] a segment's states
+    f2* segm;                           // [S][tiles][K][NP][32] and migrated states
+    f2* terms;                          // [S][tiles][2][2][NP][32] a year's terms of mu_s and v_s
+    f2* lam;                            // [S][tiles][NP][32] adjoint of a segment's first state
+    f2* rows;                           // [S][tiles][NP][32] rows shared memory has no room for
     float* gtab;                        // [S][Y][P] growth-rate mean used in year t
     float* gdot;                        // [S][Y][P] its derivative in mu_s
     double* pv;                         // [P]
@@ -164,8 +189,11 @@ __global__ void k_adj_pv_grad(AdjArgs a, int ntheta) {
 }
 
 // growth-rate mean of species s in year t (updated before the year's
-// growth) and its derivative in mu_s, for every year
-__device__ void growth_means(const AdjArgs& a, int s, int p) {
+// growth) and its derivative in mu_s, for every year; a thread per (species,
+// path)
+__global__ void __launch_bounds__(128) k_adj_growth(AdjArgs a) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x, s = blockIdx.y;
+    if (p >= a.P) return;
     const float* sp = a.params + 8 * s;
     const float mu = th_mu(a, s);
     float g = sp[0], gd = 0.0f;
@@ -184,161 +212,395 @@ __device__ void growth_means(const AdjArgs& a, int s, int p) {
     }
 }
 
-// migration m = M_c x for the lane's control (branch-free over controls)
-__device__ __forceinline__ void migrate(const AdjArgs& a, int s, int ctl, int N, int TP,
-                                        const float* x, float* m, const float* hscale) {
-    const int lane = threadIdx.x;
-    for (int k = 0; k < N; ++k) m[k * TP + lane] = 0.0f;
-    for (int c = 0; c < a.C; ++c) {
-        const float sel = (ctl == c) ? 1.0f : 0.0f;
-        const float dh = hscale[c];
-        const int e0 = a.coo_off[s * a.C + c], e1 = a.coo_off[s * a.C + c + 1];
-        for (int e = e0; e < e1; ++e) {
-            const int k = a.coo_k[e], l = a.coo_l[e];
-            const float v = a.coo_v[e] * (dh == 0.0f ? 1.0f : to_expf(-a.coo_x[e] * dh)) * sel;
-            m[k * TP + lane] = fmaf(v, x[l * TP + lane], m[k * TP + lane]);
+// the lists' values at the hazards theta holds
+__global__ void __launch_bounds__(256) k_adj_values(AdjArgs a) {
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= a.E) return;
+    const int src = a.tsrc[e];
+    const float x = __int_as_float(a.uchain[e].z), xs = __int_as_float(a.uchain[src].z);
+    const int W = a.C + 1;
+    for (int c = 0; c < W; ++c) {
+        const float dh = c < a.C ? th_h(a, c) - a.base_h[c] : 0.0f;
+        a.uval[(size_t)e * W + c] = a.base_v[(size_t)e * W + c] *
+                                    (dh == 0.0f ? 1.0f : to_expf(x * dh));
+        a.tval[(size_t)e * W + c] = a.base_v[(size_t)src * W + c] *
+                                    (dh == 0.0f ? 1.0f : to_expf(xs * dh));
+    }
+}
+
+constexpr int kAdjThreads = 512, kAdjWarps = kAdjThreads / 32;
+constexpr int kAdjPaths = 64;                  // paths of a CTA, two a lane
+constexpr int kAdjStatic = 3072;               // static shared memory and slack
+
+// what the sweeps of one (tile, species) share
+struct AdjTile {
+    int s, N, N4, p0, p1;                      // species, patches, the lane's paths
+    bool live0, live1;
+    float v;                                   // growth variability
+    const int *up, *tp;                        // list starts
+    const float* cap;
+    to_path_stream ps0, ps1;
+    uint32_t stream_road, group0;
+    const to_bm_tables* tab;
+};
+
+__device__ __forceinline__ AdjTile adj_tile(const AdjArgs& a, const to_bm_tables* tab) {
+    AdjTile q;
+    q.s = blockIdx.y;
+    q.N = a.n_patches[q.s];
+    q.N4 = (q.N + 3) & ~3;
+    q.p0 = blockIdx.x * kAdjPaths + (threadIdx.x & 31);
+    q.p1 = q.p0 + 32;
+    q.live0 = q.p0 < a.P;
+    q.live1 = q.p1 < a.P;
+    q.v = th_v(a, q.s);
+    q.up = a.uptr + (size_t)q.s * (a.NP + 1);
+    q.tp = a.tptr + (size_t)q.s * (a.NP + 1);
+    q.cap = a.caps + (size_t)q.s * a.NP;
+    to_stream_path(q.ps0, (uint32_t)(q.live0 ? q.p0 : 0));
+    to_stream_path(q.ps1, (uint32_t)(q.live1 ? q.p1 : 0));
+    q.stream_road = TO_STREAM_GROWTH | ((uint32_t)a.road << 8);
+    q.group0 = (uint32_t)((q.s * q.N4) >> 2);
+    q.tab = tab;
+    return q;
+}
+
+// the lane's controls (columns of the lists' values) and growth means of
+// year t, and its streams set to that year; paths past the end: nothing
+// migrates, growth of path 0
+struct AdjYear {
+    int c0, c1;
+    f2 g, gd;
+};
+__device__ __forceinline__ AdjYear adj_year(const AdjArgs& a, AdjTile& q, int t) {
+    AdjYear y;
+    const size_t row = (size_t)t * a.P, sr = ((size_t)q.s * a.Y + t) * a.P;
+    const int p0 = q.live0 ? q.p0 : 0, p1 = q.live1 ? q.p1 : 0;
+    y.c0 = q.live0 ? a.controls[row + p0] : a.C;
+    y.c1 = q.live1 ? a.controls[row + p1] : a.C;
+    if ((unsigned)y.c0 > (unsigned)a.C) y.c0 = a.C;
+    if ((unsigned)y.c1 > (unsigned)a.C) y.c1 = a.C;
+    y.g = pack2(a.gtab[sr + p0], a.gtab[sr + p1]);
+    y.gd = pack2(a.gdot[sr + p0], a.gdot[sr + p1]);
+    to_stream_year(q.ps0, (uint32_t)t, a.rk);
+    to_stream_year(q.ps1, (uint32_t)t, a.rk);
+    return y;
+}
+
+__device__ __forceinline__ void adj_normals(const AdjArgs& a, const AdjTile& q, int grp, f2 (&z)[4]) {
+    to_normal4x2(q.ps0, q.ps1, to_stream_group(q.group0 + grp, q.stream_road, a.rk), a.rk, *q.tab, z);
+}
+
+// migrated state of patch k: the values of the lane's controls times the
+// origins' rows
+__device__ __forceinline__ f2 adj_migrated(const AdjArgs& a, const AdjTile& q, int k,
+                                           const AdjYear& y, const f2* rows) {
+    const int W = a.C + 1, e1 = q.up[k + 1];
+    f2 acc = 0ull;
+#pragma unroll 4
+    for (int e = q.up[k]; e < e1; ++e) {
+        const float* v = a.uval + (size_t)e * W;
+        acc = fma2(pack2(v[y.c0], v[y.c1]), rows[a.ul[e] * 32], acc);
+    }
+    return acc;
+}
+
+// minus x / c.  A capacity with a normal reciprocal: multiply by it and
+// correct once, which gives the division's bits for quotients in the normal
+// range; any other capacity: divide.
+struct AdjCap {
+    f2 c, nr;
+    float cap;
+    bool normal;
+};
+__device__ __forceinline__ AdjCap adj_cap(float cap) {
+    AdjCap r;
+    r.cap = cap;
+    r.normal = fabsf(cap) > 1e-30f && fabsf(cap) < 1e30f;
+    r.c = both2(cap);
+    r.nr = both2(-(1.0f / cap));
+    return r;
+}
+__device__ __forceinline__ f2 adj_neg_div(f2 x, const AdjCap& c) {
+    if (c.normal) {
+        const f2 nq = mul2(x, c.nr);
+        return fma2(fma2(nq, c.c, x), c.nr, nq);
+    }
+    float x0, x1;
+    unpack2(x, x0, x1);
+    return neg2(pack2(x0 / c.cap, x1 / c.cap));
+}
+
+// one year forward: the next states from the rows x (to nx), and for the
+// reverse sweep the migrated and next states (own patches' rows only)
+__device__ __forceinline__ void adj_step(const AdjArgs& a, const AdjTile& q, const AdjYear& y,
+                                         const f2* x, f2* nx, f2* segm, f2* segx) {
+    const int lane = threadIdx.x & 31;
+    const f2 v2 = both2(q.v), one = both2(1.0f), mone = both2(-1.0f);
+    for (int grp = threadIdx.x >> 5; grp < q.N4 / 4; grp += kAdjWarps) {
+        f2 z[4];
+        adj_normals(a, q, grp, z);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int k = grp * 4 + j;
+            if (k >= q.N) break;
+            const f2 m = adj_migrated(a, q, k, y, x + lane);
+            const AdjCap c = adj_cap(q.cap[k]);
+            const f2 gr = fma2(mul2(v2, z[j]), y.g, y.g);
+            const f2 nd = adj_neg_div(mul2(gr, fma2(m, mone, c.c)), c);
+            float x0, x1;
+            unpack2(mul2(m, fma2(nd, mone, one)), x0, x1);
+            const f2 r = pack2(fmaxf(x0, 0.0f), fmaxf(x1, 0.0f));
+            nx[k * 32 + lane] = r;
+            if (segm) {
+                segm[k * 32 + lane] = m;
+                segx[k * 32 + lane] = r;
+            }
         }
     }
 }
 
-__device__ __forceinline__ float growth_z(const AdjArgs& a, int s, int N, int p, int t, int k) {
-    const int N4 = (N + 3) & ~3;
-    float z[4];
-    to_normal4(a.seed, TO_STREAM_GROWTH, (uint32_t)a.road, (uint32_t)p, t,
-               (uint32_t)((s * N4) >> 2) + (uint32_t)(k >> 2), z);
-    return z[k & 3];
+// through a year's growth: mu = lambda * dF/dm of a patch, and its terms of
+// the derivatives in the growth variability and mean
+__device__ __forceinline__ f2 adj_through(const AdjTile& q, const AdjYear& y, float cap, f2 z, f2 m,
+                                          f2 l, f2& tv, f2& tm) {
+    const f2 one = both2(1.0f), mone = both2(-1.0f);
+    const AdjCap c = adj_cap(cap);
+    const f2 vz = mul2(both2(q.v), z);
+    const f2 gr = fma2(vz, y.g, y.g);
+    const f2 room = fma2(m, mone, c.c);                                  // cap - m
+    const f2 f = mul2(m, fma2(adj_neg_div(mul2(gr, room), c), mone, one));
+    const f2 dm = fma2(adj_neg_div(mul2(gr, fma2(m, both2(-2.0f), c.c)), c), mone, one);
+    const f2 dg = neg2(adj_neg_div(mul2(m, room), c));
+    // dF = 0 where the growth is cut off at zero
+    float f0, f1, a0, a1, b0, b1, v0, v1;
+    unpack2(f, f0, f1);
+    unpack2(mul2(l, dg), a0, a1);
+    unpack2(mul2(l, dm), b0, b1);
+    unpack2(vz, v0, v1);
+    const f2 lg = pack2(f0 > 0.0f ? a0 : 0.0f, f1 > 0.0f ? a1 : 0.0f);
+    tv = mul2(mul2(lg, y.g), z);
+    // scalar: ptxas joins a packed multiply and add, which rounds once
+    tm = mul2(mul2(lg, pack2(1.0f + v0, 1.0f + v1)), y.gd);
+    return pack2(f0 > 0.0f ? b0 : 0.0f, f1 > 0.0f ? b1 : 0.0f);
 }
 
-// forward population recursion of one path tile; checkpoints every K years
-// into ckpt (and, when seg_from >= 0, the states of years seg_from ..
-// seg_from + K - 1 into seg)
-__device__ void pop_forward(const AdjArgs& a, int s, int TP, float* x, float* m, int t_from,
-                            int t_to, bool write_ckpt, bool write_seg, int seg_from,
-                            const float* hscale) {
-    const int lane = threadIdx.x, p = blockIdx.x * TP + lane;
-    const int N = a.n_patches[s];
-    const bool live = p < a.P;
-    const int pp = live ? p : 0;
-    const float v = th_v(a, s);
-    const float* cp = a.caps + (size_t)s * a.NP;
-    for (int t = t_from; t < t_to; ++t) {
-        if (write_ckpt && t % kCk == 0 && live)
-            for (int k = 0; k < N; ++k)
-                a.ckpt[(((size_t)s * (a.Y / kCk + 1) + t / kCk) * a.NP + k) * a.P + p] = x[k * TP + lane];
-        if (write_seg && live)
-            for (int k = 0; k < N; ++k)
-                a.seg[(((size_t)s * kCk + (t - seg_from)) * a.NP + k) * a.P + p] = x[k * TP + lane];
-        const int ctl = live ? a.controls[(size_t)t * a.P + p] : 0;
-        migrate(a, s, ctl, N, TP, x, m, hscale);
-        const float g = a.gtab[((size_t)s * a.Y + t) * a.P + pp];
-        for (int k = 0; k < N; ++k) {
-            const float z = growth_z(a, s, N, pp, t, k);
-            const float gr = fmaf(v * z, g, g);
-            const float mv = m[k * TP + lane], c = cp[k];
-            x[k * TP + lane] = fmaxf(mv * (1.0f + gr * (c - mv) / c), 0.0f);
-        }
+// The sums over a year's patches and pairs run in the order one thread a
+// path would take - patches ascending; destinations, then origins - in FP32,
+// so that they round alike however the patches are dealt out.  Growth: one
+// warp adds a year's terms while the others work on the next rows.
+__device__ __forceinline__ void adj_growth_chain(const AdjTile& q, const f2* terms, size_t seg, f2* sums) {
+    const int lane = threadIdx.x & 31;
+    f2 gv = sums[lane], gm = sums[32 + lane];
+#pragma unroll 8
+    for (int k = 0; k < q.N; ++k) {
+        gv = add2(gv, terms[k * 32 + lane]);
+        gm = add2(gm, terms[seg + k * 32 + lane]);
     }
+    sums[lane] = gv;
+    sums[32 + lane] = gm;
+}
+// Hazards: a chain over all pairs, a load latency every few of them, but the
+// years are independent - a segment's years are summed at once, a warp each
+// (a year at a time, by one warp beside the others: a sweep of 4.8 ms where
+// this takes 2.0).
+__device__ __forceinline__ f2 adj_hazard_chain(const AdjArgs& a, const AdjTile& q, const AdjYear& y,
+                                               const f2* mu, const f2* xt) {
+    const int lane = threadIdx.x & 31, W = a.C + 1, e1 = q.up[q.N];
+    const float* v0 = a.uval + y.c0;
+    const float* v1 = a.uval + y.c1;
+    f2 acc = 0ull;
+#pragma unroll 4
+    for (int e = q.up[0]; e < e1; ++e) {
+        const int4 u = a.uchain[e];
+        const f2 v = mul2(both2(__int_as_float(u.z)), pack2(v0[(size_t)e * W], v1[(size_t)e * W]));
+        acc = fma2(mul2(v, mu[u.y + lane]), xt[u.x + lane], acc);
+    }
+    return acc;
 }
 
-// forward: end population per path and checkpoints
-__global__ void k_adj_pop_fwd(AdjArgs a, int TP) {
-    extern __shared__ float sm[];
-    const int s = blockIdx.y, lane = threadIdx.x, p = blockIdx.x * TP + lane;
-    const int N = a.n_patches[s];
-    float* x = sm;                   // [N][TP]
-    float* m = x + (size_t)N * TP;   // [N][TP]
-    __shared__ float hscale[8];
-    if (lane < a.C) hscale[lane] = th_h(a, lane) - a.base_h[lane];
-    if (p < a.P) growth_means(a, s, p);
-    const float* ip = a.init_pops + (size_t)s * a.NP;
-    for (int k = 0; k < N; ++k) x[k * TP + lane] = ip[k];
+// the rows a year wrote become the rows the next one reads
+__device__ __forceinline__ void adj_turn(f2*& x, f2*& nx, int n, int two) {
     __syncthreads();
-    pop_forward(a, s, TP, x, m, 0, a.Y, true, false, 0, hscale);
-    if (p < a.P) {
-        double e = 0.0;
-        for (int k = 0; k < N; ++k) e += (double)x[k * TP + lane];
-        a.endp[(size_t)s * a.P + p] = e;
+    if (two) {
+        f2* t = x;
+        x = nx;
+        nx = t;
+    } else {
+        for (int i = threadIdx.x; i < n; i += kAdjThreads) x[i] = nx[i];
+        __syncthreads();
     }
 }
 
-// backward: reverse sweep over the K-year segments
-__global__ void k_adj_pop_bwd(AdjArgs a, int TP, int ntheta) {
-    extern __shared__ float sm[];
-    const int s = blockIdx.y, lane = threadIdx.x, p = blockIdx.x * TP + lane;
+// forward: end population per path and checkpoints.  `two`: shared memory
+// holds both years' rows, else the next year's go through global memory
+__global__ void __launch_bounds__(kAdjThreads, 2) k_adj_pop_fwd(AdjArgs a, int two) {
+    extern __shared__ __align__(16) unsigned char sm_adj[];
+    __shared__ to_bm_tables s_tab;
+    const int tid = threadIdx.x, lane = tid & 31;
+    AdjTile q = adj_tile(a, &s_tab);
+    f2* x = reinterpret_cast<f2*>(sm_adj);                     // [N][32]
+    f2* nx = two ? x + (size_t)q.N * 32
+                 : a.rows + ((size_t)q.s * gridDim.x + blockIdx.x) * a.NP * 32;
+    const float* ip = a.init_pops + (size_t)q.s * a.NP;
+    to_bm_load(s_tab);
+    for (int i = tid; i < q.N * 32; i += kAdjThreads) x[i] = both2(ip[i >> 5]);
+    __syncthreads();
+    for (int t = 0; t < a.Y; ++t) {
+        const AdjYear y = adj_year(a, q, t);
+        if (t % kCk == 0)
+            for (int k = tid >> 5; k < q.N; k += kAdjWarps) {
+                float* o = a.ckpt + (((size_t)q.s * (a.Y / kCk + 1) + t / kCk) * a.NP + k) * a.P;
+                float x0, x1;
+                unpack2(x[k * 32 + lane], x0, x1);
+                if (q.live0) o[q.p0] = x0;
+                if (q.live1) o[q.p1] = x1;
+            }
+        adj_step(a, q, y, x, nx, nullptr, nullptr);
+        adj_turn(x, nx, q.N * 32, two);
+    }
+    if (tid < 32) {
+        double e0 = 0.0, e1 = 0.0;
+#pragma unroll 4
+        for (int k = 0; k < q.N; ++k) {
+            float x0, x1;
+            unpack2(x[k * 32 + lane], x0, x1);
+            e0 += (double)x0;
+            e1 += (double)x1;
+        }
+        if (q.live0) a.endp[(size_t)q.s * a.P + q.p0] = e0;
+        if (q.live1) a.endp[(size_t)q.s * a.P + q.p1] = e1;
+    }
+}
+
+// backward: reverse sweep over the K-year segments.  The rows other patches
+// read are a segment's states while it is recomputed, then mu: a warp turns
+// year t's mu into lambda_t of four patches and that at once into their
+// year t - 1's mu, so a year takes one barrier either way.  In the reverse
+// years warps take groups from a counter, one of them after the growth sums.
+__global__ void __launch_bounds__(kAdjThreads, 2) k_adj_pop_bwd(AdjArgs a, int two, int ntheta) {
+    extern __shared__ __align__(16) unsigned char sm_adj[];
+    __shared__ to_bm_tables s_tab;
+    __shared__ int s_grab[2];
     // the sweep is linear in the species' output weight: a zero weight
     // contributes exactly zero (the per-path gradients start zeroed)
-    if (a.gout[1 + s] == 0.0f) return;
-    const int N = a.n_patches[s];
-    const bool live = p < a.P;
-    const int pp = live ? p : 0;
-    float* x = sm;                       // [N][TP] state
-    float* m = x + (size_t)N * TP;       // [N][TP] migrated state
-    float* lam = m + (size_t)N * TP;     // [N][TP] adjoint of the state
-    __shared__ float hscale[8];
-    if (lane < a.C) hscale[lane] = th_h(a, lane) - a.base_h[lane];
-    __syncthreads();
-    const float v = th_v(a, s);
-    const float* cp = a.caps + (size_t)s * a.NP;
-    const float w = a.gout[1 + s];
-    for (int k = 0; k < N; ++k) lam[k * TP + lane] = w;
-    float g_mu = 0.0f, g_v = 0.0f, g_h[8];
-    for (int c = 0; c < 8; ++c) g_h[c] = 0.0f;
+    const float w = a.gout[1 + blockIdx.y];
+    if (w == 0.0f) return;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, W = a.C + 1;
+    AdjTile q = adj_tile(a, &s_tab);
+    const int NG = q.N4 / 4;
+    const size_t tile = (size_t)q.s * gridDim.x + blockIdx.x, seg = (size_t)a.NP * 32;
+    f2* gsum = reinterpret_cast<f2*>(sm_adj);                      // [2][32] v_s, mu_s
+    float* gh = reinterpret_cast<float*>(gsum + 64);               // [W][64]
+    float* gy = gh + (size_t)W * kAdjPaths;                        // [kCk][64] a year's
+    f2* x = reinterpret_cast<f2*>(gy + kCk * kAdjPaths);           // [N][32]
+    f2* nx = two ? x + (size_t)q.N * 32 : a.rows + tile * seg;     // [N][32]
+    f2* lam = a.lam + tile * seg;
+    f2* segx = a.segx + tile * kCk * seg;
+    f2* segm = a.segm + tile * kCk * seg;      // in the reverse years mu takes a year's place
+    f2* terms = a.terms + tile * 4 * seg;                          // [t & 1][v_s, mu_s][NP][32]
+    if (tid < 64) gsum[tid] = 0ull;
+    for (int i = tid; i < W * kAdjPaths; i += kAdjThreads) gh[i] = 0.0f;
+    if (tid < 2) s_grab[tid] = 0;
+    to_bm_load(s_tab);
+    for (int i = tid; i < q.N * 32; i += kAdjThreads) lam[i] = both2(w);
+    int turn = 0;                                                  // of the counters
     const int nseg = (a.Y + kCk - 1) / kCk;
     for (int sg = nseg - 1; sg >= 0; --sg) {
         const int t0 = sg * kCk, t1 = min(a.Y, t0 + kCk);
-        // recompute the segment's states from its checkpoint
-        for (int k = 0; k < N; ++k)
-            x[k * TP + lane] = live ? a.ckpt[(((size_t)s * (a.Y / kCk + 1) + sg) * a.NP + k) * a.P + p] : 0.0f;
-        pop_forward(a, s, TP, x, m, t0, t1, false, true, t0, hscale);
-        for (int t = t1 - 1; t >= t0; --t) {
-            // state x_t
-            for (int k = 0; k < N; ++k)
-                x[k * TP + lane] = live ? a.seg[(((size_t)s * kCk + (t - t0)) * a.NP + k) * a.P + p] : 0.0f;
-            const int ctl = live ? a.controls[(size_t)t * a.P + p] : 0;
-            migrate(a, s, ctl, N, TP, x, m, hscale);
-            const float g = a.gtab[((size_t)s * a.Y + t) * a.P + pp];
-            const float gd = a.gdot[((size_t)s * a.Y + t) * a.P + pp];
-            // through the growth: mu_t = lambda * dF/dm (kept in m), params
-            for (int k = 0; k < N; ++k) {
-                const float z = growth_z(a, s, N, pp, t, k);
-                const float gr = fmaf(v * z, g, g);
-                const float mv = m[k * TP + lane], c = cp[k];
-                const float f = mv * (1.0f + gr * (c - mv) / c);
-                const float l = lam[k * TP + lane];
-                float dfdm = 0.0f, dfdgr = 0.0f;
-                if (f > 0.0f) {
-                    dfdm = 1.0f + gr * (c - 2.0f * mv) / c;
-                    dfdgr = mv * (c - mv) / c;
-                }
-                const float lg = l * dfdgr;
-                g_v += lg * g * z;
-                g_mu += lg * (1.0f + v * z) * gd;
-                m[k * TP + lane] = l * dfdm;
-            }
-            // hazards and lambda_t = M_c^T mu_t
-            for (int k = 0; k < N; ++k) lam[k * TP + lane] = 0.0f;
-            for (int c = 0; c < a.C; ++c) {
-                const float sel = (ctl == c) ? 1.0f : 0.0f;
-                const float dh = hscale[c];
-                const int e0 = a.coo_off[s * a.C + c], e1 = a.coo_off[s * a.C + c + 1];
-                float gh = 0.0f;
-                for (int e = e0; e < e1; ++e) {
-                    const int k = a.coo_k[e], l = a.coo_l[e];
-                    const float val = a.coo_v[e] * (dh == 0.0f ? 1.0f : to_expf(-a.coo_x[e] * dh)) * sel;
-                    const float mu_k = m[k * TP + lane];
-                    lam[l * TP + lane] = fmaf(val, mu_k, lam[l * TP + lane]);
-                    gh = fmaf(-a.coo_x[e] * val * mu_k, x[l * TP + lane], gh);
-                }
-                g_h[c] += gh;
+        // the segment's states from its checkpoint
+        __syncthreads();
+        for (int k = warp; k < q.N; k += kAdjWarps) {
+            const float* c = a.ckpt + (((size_t)q.s * (a.Y / kCk + 1) + sg) * a.NP + k) * a.P;
+            segx[k * 32 + lane] = x[k * 32 + lane] =
+                pack2(q.live0 ? c[q.p0] : 0.0f, q.live1 ? c[q.p1] : 0.0f);
+        }
+        __syncthreads();
+        for (int t = t0; t < t1 - 1; ++t) {
+            const AdjYear y = adj_year(a, q, t);
+            adj_step(a, q, y, x, nx, segm + (size_t)(t - t0) * seg, segx + (size_t)(t + 1 - t0) * seg);
+            adj_turn(x, nx, q.N * 32, two);
+        }
+        // the last year's mu
+        AdjYear y = adj_year(a, q, t1 - 1);
+        f2* tt = terms + (size_t)((t1 - 1) & 1) * 2 * seg + lane;
+        for (int grp = warp; grp < NG; grp += kAdjWarps) {
+            f2 z[4];
+            adj_normals(a, q, grp, z);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int k = grp * 4 + j;
+                if (k >= q.N) break;
+                const f2 m = adj_migrated(a, q, k, y, x + lane);
+                nx[k * 32 + lane] = segm[(size_t)(t1 - 1 - t0) * seg + k * 32 + lane] =
+                    adj_through(q, y, q.cap[k], z[j], m, lam[k * 32 + lane], tt[k * 32],
+                                tt[seg + k * 32]);
             }
         }
+        adj_turn(x, nx, q.N * 32, two);
+        for (int t = t1 - 1; t >= t0; --t) {
+            // lambda_t = M_c^T mu_t, then year t - 1's growth
+            const int c0 = y.c0, c1 = y.c1;
+            f2* mt = segm + (size_t)(t - 1 - t0) * seg;
+            if (warp == 0) adj_growth_chain(q, terms + (size_t)(t & 1) * 2 * seg, seg, gsum);
+            if (t > t0) y = adj_year(a, q, t - 1);
+            tt = terms + (size_t)((t - 1) & 1) * 2 * seg + lane;
+            int* counter = s_grab + (turn & 1);
+            for (;;) {
+                int grp = 0;
+                if (lane == 0) grp = atomicAdd(counter, 1);
+                grp = __shfl_sync(0xffffffffu, grp, 0);
+                if (grp >= NG) break;
+                f2 z[4] = {0ull, 0ull, 0ull, 0ull};
+                if (t > t0) adj_normals(a, q, grp, z);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int k = grp * 4 + j;
+                    if (k >= q.N) break;
+                    const float* v0 = a.tval + c0;
+                    const float* v1 = a.tval + c1;
+                    f2 l = 0ull;
+                    const int e1 = q.tp[k + 1];
+#pragma unroll 4
+                    for (int e = q.tp[k]; e < e1; ++e)
+                        l = fma2(pack2(v0[(size_t)e * W], v1[(size_t)e * W]), x[a.tk[e] * 32 + lane], l);
+                    if (t > t0)
+                        nx[k * 32 + lane] = mt[k * 32 + lane] =
+                            adj_through(q, y, q.cap[k], z[j], mt[k * 32 + lane], l, tt[k * 32],
+                                        tt[seg + k * 32]);
+                    else
+                        lam[k * 32 + lane] = l;
+                }
+            }
+            ++turn;
+            if (tid == 0) s_grab[turn & 1] = 0;        // last used before the last barrier
+            adj_turn(x, nx, q.N * 32, two);
+        }
+        for (int t = t1 - 1 - warp; t >= t0; t -= kAdjWarps) {
+            const AdjYear h = adj_year(a, q, t);
+            float h0, h1;
+            unpack2(adj_hazard_chain(a, q, h, segm + (size_t)(t - t0) * seg,
+                                     segx + (size_t)(t - t0) * seg), h0, h1);
+            gy[(t - t0) * kAdjPaths + lane] = h0;
+            gy[(t - t0) * kAdjPaths + 32 + lane] = h1;
+        }
+        __syncthreads();
+        if (warp == 0)
+            for (int t = t1 - 1; t >= t0; --t) {
+                const AdjYear h = adj_year(a, q, t);
+                gh[h.c0 * kAdjPaths + lane] += gy[(t - t0) * kAdjPaths + lane];
+                gh[h.c1 * kAdjPaths + 32 + lane] += gy[(t - t0) * kAdjPaths + 32 + lane];
+            }
     }
-    if (live) {
+    __syncthreads();
+    const float* gs = reinterpret_cast<const float*>(gsum);
+    for (int i = tid; i < (2 + a.C) * kAdjPaths; i += kAdjThreads) {
+        const int what = i / kAdjPaths, j = i - what * kAdjPaths, p = blockIdx.x * kAdjPaths + j;
+        if (p >= a.P) continue;
         double* gp = a.gpath + (size_t)p * ntheta;
         // species blocks are disjoint, so each species writes its own entries
-        gp[2 * a.U + s] = (double)g_mu;
-        gp[2 * a.U + a.S + s] = (double)g_v;
-        for (int c = 0; c < a.C; ++c) atomicAdd(&gp[2 * a.U + 2 * a.S + c], (double)g_h[c]);
+        if (what < 2) gp[2 * a.U + (1 - what) * a.S + q.s] = (double)gs[what * 64 + (j & 31) * 2 + (j >> 5)];
+        else atomicAdd(&gp[2 * a.U + 2 * a.S + what - 2], (double)gh[(what - 2) * kAdjPaths + j]);
     }
 }
 
@@ -358,7 +620,10 @@ __global__ void k_col_mean(int P, int ncol, const double* __restrict__ v, double
     }
 }
 
-int tile_paths(int N) { return N <= 128 ? 128 : (N <= 256 ? 64 : 32); }
+size_t adj_fwd_smem(int N, bool two) { return (size_t)(two ? 2 : 1) * N * 32 * 8; }
+size_t adj_bwd_smem(int N, int C, bool two) {
+    return (size_t)(C + 3 + kCk) * kAdjPaths * 4 + adj_fwd_smem(N, two);
+}
 
 }  // namespace
 
@@ -367,6 +632,7 @@ struct to_tape_s {
     to_ctx ctx = nullptr;
     AdjArgs a;
     int ntheta = 0, nout = 0, maxN = 0;
+    bool two_b = false;                 // the reverse sweep's rows fit in shared memory twice
     char* buf = nullptr;
     double* d_out = nullptr;            // [1 + S] forward outputs
     double* d_grad = nullptr;           // [ntheta] backward result
@@ -395,24 +661,54 @@ to_status to_adjoint_forward(to_ctx ctx, const to_adjoint_problem* pr, const dou
         if (N > maxN) maxN = N;
     }
     const int NP = (maxN + 3) & ~3;
-    // COO lists of every (species, control) matrix with the pair's crossings
-    std::vector<int> off(1, 0), kk, ll;
-    std::vector<float> vv, xx;
+    // lists of every species: the pairs with a non-zero value under any
+    // control, by destination and then by origin
+    std::vector<int> uptr((size_t)S * (NP + 1), 0), tptr((size_t)S * (NP + 1), 0), ul, tk, tsrc;
+    std::vector<int4> chain;
+    std::vector<float> vv;
     for (int s = 0; s < S; ++s) {
         const to_rov_species& sp = rp->species[s];
         const int N = sp.n_patches;
-        for (int c = 0; c < C; ++c) {
-            for (int k = 0; k < N; ++k)
-                for (int l = 0; l < N; ++l) {
-                    const float v = sp.mmm[((size_t)c * N + k) * N + l];
-                    if (v == 0.0f) continue;
-                    kk.push_back(k); ll.push_back(l); vv.push_back(v);
-                    xx.push_back((float)pr->crossings[s][(size_t)l * N + k]);
-                }
-            off.push_back((int)kk.size());
+        int* up = &uptr[(size_t)s * (NP + 1)];
+        int* tp = &tptr[(size_t)s * (NP + 1)];
+        const size_t e0 = ul.size();
+        std::vector<int> cnt(N, 0), dest;
+        for (int k = 0; k < N; ++k) {
+            up[k] = (int)ul.size();
+            for (int l = 0; l < N; ++l) {
+                bool any = false;
+                for (int c = 0; c < C && !any; ++c) any = sp.mmm[((size_t)c * N + k) * N + l] != 0.0f;
+                if (!any) continue;
+                ul.push_back(l);
+                dest.push_back(k);
+                ++cnt[l];
+                for (int c = 0; c < C; ++c) vv.push_back(sp.mmm[((size_t)c * N + k) * N + l]);
+                vv.push_back(0.0f);
+                const float nx = -(float)pr->crossings[s][(size_t)l * N + k];
+                int bits;
+                memcpy(&bits, &nx, 4);
+                chain.push_back(make_int4(l * 32, k * 32, bits, 0));
+            }
+        }
+        for (int k = N; k <= NP; ++k) up[k] = (int)ul.size();
+        // transposed: by origin, destinations ascending
+        int at = (int)e0;
+        for (int l = 0; l < N; ++l) { tp[l] = at; at += cnt[l]; }
+        for (int l = N; l <= NP; ++l) tp[l] = at;
+        tk.resize(ul.size());
+        tsrc.resize(ul.size());
+        std::vector<int> next(tp, tp + N);
+        for (size_t e = e0; e < ul.size(); ++e) {
+            const int q = next[ul[e]]++;
+            tk[q] = dest[e - e0];
+            tsrc[q] = (int)e;
         }
     }
-    const size_t nnz = kk.size() > 0 ? kk.size() : 1;
+    const size_t nE = ul.size() > 0 ? ul.size() : 1;
+    const int tiles = (P + kAdjPaths - 1) / kAdjPaths;
+    const size_t rowb = (size_t)S * tiles * NP * 32 * 8;       // rows of every (species, tile)
+    const bool two_f = adj_fwd_smem(maxN, true) + kAdjStatic <= ctx->smem_optin;
+    const bool two_b = adj_bwd_smem(maxN, C, true) + kAdjStatic <= ctx->smem_optin;
     std::vector<int> np(S);
     std::vector<float> prm((size_t)S * 8), ip((size_t)S * NP, 0.0f), cpv((size_t)S * NP, 1.0f);
     for (int s = 0; s < S; ++s) {
@@ -429,9 +725,14 @@ to_status to_adjoint_forward(to_ctx ctx, const to_adjoint_problem* pr, const dou
     auto acc = [&](size_t b) { bytes += to_align256(b); };
     acc(ntheta * 4); acc((size_t)U * 24 + 4); acc(C * 4); acc(64); acc(64); acc(64); acc(64);
     acc((size_t)Y * P * 4); acc(S * 4); acc((size_t)S * 32); acc((size_t)S * NP * 4);
-    acc((size_t)S * NP * 4); acc(off.size() * 4); acc(nnz * 4); acc(nnz * 4); acc(nnz * 4);
-    acc(nnz * 4); acc(C * 4);
-    acc((size_t)S * (Y / kCk + 1) * NP * P * 4); acc((size_t)S * kCk * NP * P * 4);
+    acc((size_t)S * NP * 4); acc(uptr.size() * 4); acc(tptr.size() * 4);
+    for (int q = 0; q < 3; ++q) acc(nE * 4);
+    acc(nE * 16);
+    for (int q = 0; q < 3; ++q) acc(nE * (C + 1) * 4);
+    acc(C * 4);
+    acc((size_t)S * (Y / kCk + 1) * NP * P * 4); acc(rowb * kCk); acc(rowb * kCk);
+    acc(rowb); acc(rowb * 4);
+    if (!two_f || !two_b) acc(rowb);
     acc((size_t)S * Y * P * 4); acc((size_t)S * Y * P * 4); acc((size_t)P * 8);
     acc((size_t)S * P * 8); acc((size_t)P * ntheta * 8); acc(64); acc(256); acc(256);
     to_tape t = new to_tape_s();
@@ -456,12 +757,19 @@ to_status to_adjoint_forward(to_ctx ctx, const to_adjoint_problem* pr, const dou
     float* d_prm = (float*)take((size_t)S * 32);
     float* d_ip = (float*)take((size_t)S * NP * 4);
     float* d_cp = (float*)take((size_t)S * NP * 4);
-    int* d_off = (int*)take(off.size() * 4);
-    int* d_k = (int*)take(nnz * 4); int* d_l = (int*)take(nnz * 4);
-    float* d_v = (float*)take(nnz * 4); float* d_x = (float*)take(nnz * 4);
+    int* d_up = (int*)take(uptr.size() * 4);
+    int* d_tp = (int*)take(tptr.size() * 4);
+    int* d_ul = (int*)take(nE * 4); int* d_tk = (int*)take(nE * 4); int* d_ts = (int*)take(nE * 4);
+    int4* d_ch = (int4*)take(nE * 16);
+    float* d_v = (float*)take(nE * (C + 1) * 4);
+    a.uval = (float*)take(nE * (C + 1) * 4); a.tval = (float*)take(nE * (C + 1) * 4);
     float* d_bh = (float*)take(C * 4);
     a.ckpt = (float*)take((size_t)S * (Y / kCk + 1) * NP * P * 4);
-    a.seg = (float*)take((size_t)S * kCk * NP * P * 4);
+    a.segx = (f2*)take(rowb * kCk);
+    a.segm = (f2*)take(rowb * kCk);
+    a.lam = (f2*)take(rowb);
+    a.terms = (f2*)take(rowb * 4);
+    a.rows = (!two_f || !two_b) ? (f2*)take(rowb) : nullptr;
     a.gtab = (float*)take((size_t)S * Y * P * 4);
     a.gdot = (float*)take((size_t)S * Y * P * 4);
     a.pv = (double*)take((size_t)P * 8);
@@ -473,8 +781,9 @@ to_status to_adjoint_forward(to_ctx ctx, const to_adjoint_problem* pr, const dou
     t->d_grad = (double*)take(256);
     a.theta = d_th; a.uncert = d_unc; a.flows = d_fl; a.fuel_costs = d_fc; a.fuel_idx = d_fi;
     a.ore_content = d_oc; a.ore_sd = d_os; a.controls = d_ctl; a.n_patches = d_np;
-    a.params = d_prm; a.init_pops = d_ip; a.caps = d_cp; a.coo_off = d_off; a.coo_k = d_k;
-    a.coo_l = d_l; a.coo_v = d_v; a.coo_x = d_x; a.base_h = d_bh; a.gout = d_gout;
+    a.params = d_prm; a.init_pops = d_ip; a.caps = d_cp; a.uptr = d_up; a.tptr = d_tp;
+    a.ul = d_ul; a.tk = d_tk; a.tsrc = d_ts; a.base_v = d_v; a.uchain = d_ch; a.base_h = d_bh;
+    a.E = (int)ul.size(); a.gout = d_gout; a.rk = to_make_round_keys(a.seed);
     auto h2d = [&](void* d, const void* h, size_t b) {
         return b ? cudaMemcpyAsync(d, h, b, cudaMemcpyHostToDevice, ctx->stream) : cudaSuccess;
     };
@@ -492,26 +801,30 @@ to_status to_adjoint_forward(to_ctx ctx, const to_adjoint_problem* pr, const dou
     chk(h2d(d_prm, prm.data(), prm.size() * 4));
     chk(h2d(d_ip, ip.data(), ip.size() * 4));
     chk(h2d(d_cp, cpv.data(), cpv.size() * 4));
-    chk(h2d(d_off, off.data(), off.size() * 4));
-    chk(h2d(d_k, kk.data(), kk.size() * 4));
-    chk(h2d(d_l, ll.data(), ll.size() * 4));
+    chk(h2d(d_up, uptr.data(), uptr.size() * 4));
+    chk(h2d(d_tp, tptr.data(), tptr.size() * 4));
+    chk(h2d(d_ul, ul.data(), ul.size() * 4));
+    chk(h2d(d_tk, tk.data(), tk.size() * 4));
+    chk(h2d(d_ts, tsrc.data(), tsrc.size() * 4));
     chk(h2d(d_v, vv.data(), vv.size() * 4));
-    chk(h2d(d_x, xx.data(), xx.size() * 4));
+    chk(h2d(d_ch, chain.data(), chain.size() * 16));
     chk(h2d(d_bh, bh.data(), C * 4));
     if (ce != cudaSuccess) { cudaFree(t->buf); delete t; return to_check_cuda(ctx, ce, "adjoint inputs"); }
-    t->ntheta = ntheta; t->nout = 1 + S; t->maxN = maxN;
+    t->ntheta = ntheta; t->nout = 1 + S; t->maxN = maxN; t->two_b = two_b;
     // forward
     k_adj_pv<<<(P + 127) / 128, 128, 0, ctx->stream>>>(a);
-    const int TP = tile_paths(maxN);
-    const size_t smf = (size_t)2 * maxN * TP * 4;
-    cudaFuncSetAttribute(k_adj_pop_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smf);
+    const size_t smf = adj_fwd_smem(maxN, two_f);
+    cudaFuncSetAttribute(k_adj_pop_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)(ctx->smem_optin - kAdjStatic));
+    if (a.E > 0) k_adj_values<<<(a.E + 255) / 256, 256, 0, ctx->stream>>>(a);
+    k_adj_growth<<<dim3((P + 127) / 128, S), 128, 0, ctx->stream>>>(a);
     to_prof_begin(ctx, "adjoint_forward");
-    k_adj_pop_fwd<<<dim3((P + TP - 1) / TP, S), TP, smf, ctx->stream>>>(a, TP);
+    k_adj_pop_fwd<<<dim3(tiles, S), kAdjThreads, smf, ctx->stream>>>(a, two_f ? 1 : 0);
     to_prof_end(ctx);
     k_col_mean<<<1, 256, 0, ctx->stream>>>(P, 1, a.pv, d_out);
     for (int s = 0; s < S; ++s)
         k_col_mean<<<1, 256, 0, ctx->stream>>>(P, 1, a.endp + (size_t)s * P, d_out + 1 + s);
-    ctx->launches += 3 + S;
+    ctx->launches += 5 + S;
     ce = cudaGetLastError();
     if (ce == cudaSuccess) ce = cudaMemcpyAsync(t->outputs, d_out, (size_t)(1 + S) * 8, cudaMemcpyDeviceToHost, ctx->stream);
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(ctx->stream);
@@ -537,12 +850,12 @@ to_status to_adjoint_backward(to_ctx ctx, to_tape t, const double* grad_outputs,
         k_adj_pv_grad<<<(P + 127) / 128, 128, 0, ctx->stream>>>(a, ntheta);
         TO_LAUNCHED(ctx);
     }
-    const int TP = tile_paths(t->maxN);
-    const size_t smb = (size_t)3 * t->maxN * TP * 4;
+    const size_t smb = adj_bwd_smem(t->maxN, a.C, t->two_b);
     TO_CUDA(ctx, cudaFuncSetAttribute(k_adj_pop_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)smb));
+                                      (int)(ctx->smem_optin - kAdjStatic)));
     to_prof_begin(ctx, "adjoint_backward");
-    k_adj_pop_bwd<<<dim3((P + TP - 1) / TP, S), TP, smb, ctx->stream>>>(a, TP, ntheta);
+    k_adj_pop_bwd<<<dim3((P + kAdjPaths - 1) / kAdjPaths, S), kAdjThreads, smb, ctx->stream>>>(
+        a, t->two_b ? 1 : 0, ntheta);
     to_prof_end(ctx);
     TO_LAUNCHED(ctx);
     std::vector<double> g(ntheta);
