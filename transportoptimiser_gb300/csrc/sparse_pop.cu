@@ -918,158 +918,290 @@ k_rov_forward_sparse(to_rov_args a, to_csc csc) {
 // ALGO6 path re-simulation (optimalForwardPaths :1199-2206, as its comments
 // describe it).  Grid ceil(P/32): a CTA re-simulates 32 paths (lane = path)
 // from year t0 to the horizon with every species together, since each
-// year's control depends on all species' states:
-//   A. all warps: every (species, control) migration of this year's
-//      populations into shared memory (CSC, ascending origins, as forward);
-//   B. warps (s, c): the grouped total and the adjusted population
-//      tot * (total / tot), the forward pass's arithmetic;
-//   C. warp 0: the decision (regression of the year, or the terminal rule
-//      in the last year) and the realised payoff flows[c] * profit,
-//      discounted by (1 + r dt / 100) per year;
-//   D. all warps: growth of the chosen control's migrated populations with
-//      the forward pass's noise and growth mean (stored by it);
-//   E. warps s: the new totals.
+// year's control depends on all species' states.  A warp owns groups of four
+// patches; a year has three barriers:
+//   A. every control's migration of the group's populations into shared
+//      memory (ascending origins, as forward) and the groups' sums; then the
+//      group's growth normals, which need nothing of the decision;
+//   B. warp c, as soon as all warps are through with A's first part: control
+//      c's adjusted populations tot * (total / tot) from the groups' sums in
+//      order, its payoff under the year's regression (the terminal rule in
+//      the last year);
+//   C. the least valid payoff's control, the growth of its migrated
+//      populations with the forward pass's growth mean (stored by it); warp 0
+//      adds flows[c] * profit, discounted by (1 + r dt / 100) per year.
 // The year-t0 value replaces condExp[t0] and the year-t0 control optCont[t0].
+//
+// Bound by latency: the years of a restart follow one another, the restarts
+// too, and ceil(P/32) CTAs seldom fill the GPU.  So the lists are the union
+// ones where they fit (a loop for all controls, its loads in flight
+// together), the payoffs are a warp's each with everything unrolled, and the
+// profits come from the table the regressions use.  2,000 paths, 2 species of
+// 61 patches, 50 years: 24 -> 7.2 us a year of a restart (five barriers, a
+// loop for every control, one warp deciding and drawing the ore's noise again
+// before).
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(1024, 1)
-k_rov_resim_sparse(to_rov_args a, to_csc csc, int t0) {
-    extern __shared__ unsigned char sm_raw[];
-    const int NE = a.ne, NG = NE >> 2, NP = a.np, C = a.C, S = a.S, Y = a.Y, P = a.P;
-    const int SC = S * C;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, W = blockDim.x >> 5;
-    const int path = blockIdx.x * kLanes + lane;
-    float* cur = reinterpret_cast<float*>(sm_raw);                  // [S][NE][32]
-    float* mig = cur + (size_t)S * NE * kLanes;                     // [S][C][NE][32]
-    float* capv = mig + (size_t)SC * NE * kLanes;                   // [S][NE]
-    float* tot = capv + (size_t)S * NE;                             // [S][32]
-    float* adj = tot + (size_t)S * kLanes;                          // [S][C][32]
-    int* ctl = reinterpret_cast<int*>(adj + (size_t)SC * kLanes);   // [32]
-    int* cptr = ctl + kLanes;                                       // [S*C][NE+1]
-    float* cval = reinterpret_cast<float*>(cptr + (size_t)SC * (NE + 1));  // [S*C][cap_smem]
-    uint16_t* cidx = reinterpret_cast<uint16_t*>(cval + (size_t)SC * csc.cap_smem);
-    const uint32_t road = (uint32_t)a.road;
+constexpr int kResimHeld = 4;              // groups of a warp whose normals wait in registers
 
-    for (int q = threadIdx.x; q < S * NE * kLanes; q += blockDim.x) {
+// shared memory: bytes of the lists, [S] reciprocals and groups' sums beside
+// what every layout has
+__host__ __device__ inline size_t resim_bytes(int NE, int S, int C, size_t lists, bool sums) {
+    const size_t rows = (size_t)S * (C + 1) * NE * kLanes * 4;
+    return rows + (size_t)S * NE * 4 + (size_t)C * kLanes * 4 + lists +
+           (sums ? (size_t)S * NE * 4 + (size_t)S * (C + 1) * (NE >> 2) * kLanes * 4 : 0);
+}
+__host__ __device__ inline size_t resim_lists(int NE, int S, int C, int cap_smem) {
+    return (size_t)S * C * ((NE + 1) * 4 + (size_t)cap_smem * 6) + 16;
+}
+
+template <int S>
+__global__ void __launch_bounds__(1024, 1)
+k_rov_resim(to_rov_args a, to_csc csc, int t0, int smem) {
+    extern __shared__ __align__(16) unsigned char sm_raw[];
+    const int NE = a.ne, NG = NE >> 2, NP = a.np, C = a.C, Y = a.Y, P = a.P, R = a.R;
+    const int SC = S * C;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, W = blockDim.x >> 5;
+    const int path = blockIdx.x * kLanes + lane;
+    const bool live = path < P;
+    // the layout: union lists and the groups' sums where they fit, then the
+    // controls' own lists with the sums, then without
+    int nu = 0;
+    bool uni = csc.uent != nullptr;
+    for (int s = 0; s < S && uni; ++s) {
+        nu += csc.unnz[s];
+        if (csc.unnz[s] < 0) uni = false;
+    }
+    const size_t ulists = (size_t)nu * 16 + (size_t)S * (NE + 1) * 4;
+    const size_t clists = resim_lists(NE, S, C, csc.cap_smem);
+    uni = uni && resim_bytes(NE, S, C, ulists, true) <= (size_t)smem;
+    const bool sums = uni || resim_bytes(NE, S, C, clists, true) <= (size_t)smem;
+    unsigned char* at = sm_raw;
+    auto take = [&](size_t bytes) { unsigned char* r = at; at += bytes; return r; };
+    int4* ue = reinterpret_cast<int4*>(uni ? take((size_t)nu * 16) : at);      // [nu]
+    float* cur = reinterpret_cast<float*>(take((size_t)S * NE * kLanes * 4));  // [S][NE][32]
+    float* mig = reinterpret_cast<float*>(take((size_t)SC * NE * kLanes * 4)); // [S][C][NE][32]
+    float* pay = reinterpret_cast<float*>(take((size_t)C * kLanes * 4));       // [C][32]
+    float* capv = reinterpret_cast<float*>(take((size_t)S * NE * 4));          // [S][NE]
+    float *rcap = nullptr, *msum = nullptr, *tsum = nullptr;
+    if (sums) {
+        rcap = reinterpret_cast<float*>(take((size_t)S * NE * 4));             // [S][NE] 1 / capacity
+        msum = reinterpret_cast<float*>(take((size_t)SC * NG * kLanes * 4));   // [S][C][NG][32]
+        tsum = reinterpret_cast<float*>(take((size_t)S * NG * kLanes * 4));    // [S][NG][32]
+    }
+    const int lists = uni ? S : SC;
+    int* cptr = reinterpret_cast<int*>(take((size_t)lists * (NE + 1) * 4));    // [S] or [S][C], [NE + 1]
+    float* cval = reinterpret_cast<float*>(uni ? at : take((size_t)SC * csc.cap_smem * 4));
+    uint16_t* cidx = reinterpret_cast<uint16_t*>(at);                          // [S][C][cap_smem]
+    const uint32_t stream_road = TO_STREAM_GROWTH | ((uint32_t)a.road << 8);
+
+    for (int q = tid; q < S * NE * kLanes; q += blockDim.x) {
         const int sk = q >> 5, pth = blockIdx.x * kLanes + (q & (kLanes - 1));
         const int s = sk / NE, k = sk - s * NE;
         cur[q] = (pth < P) ? a.popsY[(((size_t)t0 * S + s) * NE + k) * P + pth] : 0.0f;
     }
-    for (int q = threadIdx.x; q < S * NE; q += blockDim.x) {
+    for (int q = tid; q < S * NE; q += blockDim.x) {
         const int s = q / NE, k = q - s * NE;
-        capv[q] = a.caps[(size_t)s * NP + k];
+        const float cp = a.caps[(size_t)s * NP + k];
+        capv[q] = cp;
+        if (sums) rcap[q] = 1.0f / cp;
     }
-    for (int m = 0; m < SC; ++m) {
-        const int nnz = csc.nnz[m];
-        for (int k = threadIdx.x; k <= NE; k += blockDim.x)
-            cptr[m * (NE + 1) + k] = csc.ptr[(size_t)m * (NP + 1) + (k <= NP ? k : NP)];
-        for (int e = threadIdx.x; e < nnz; e += blockDim.x) {
-            cval[(size_t)m * csc.cap_smem + e] = csc.val[(size_t)m * csc.cap + e];
-            cidx[(size_t)m * csc.cap_smem + e] = csc.idx[(size_t)m * csc.cap + e];
+    if (uni) {
+        int e0 = 0;
+        for (int s = 0; s < S; ++s) {
+            const int n = csc.unnz[s];
+            for (int k = tid; k <= NE; k += blockDim.x)
+                cptr[s * (NE + 1) + k] = e0 + csc.uptr[(size_t)s * (NP + 1) + (k <= NP ? k : NP)];
+            for (int e = tid; e < n; e += blockDim.x) {
+                int4 v = csc.uent[(size_t)s * csc.ucap + e];
+                if (v.x == kNoOrigin) v.x = 0;      // its values are zero
+                v.x *= kLanes * (int)sizeof(float);
+                ue[e0 + e] = v;
+            }
+            e0 += n;
+        }
+    } else {
+        for (int m = 0; m < SC; ++m) {
+            const int nnz = csc.nnz[m];
+            for (int k = tid; k <= NE; k += blockDim.x)
+                cptr[m * (NE + 1) + k] = csc.ptr[(size_t)m * (NP + 1) + (k <= NP ? k : NP)];
+            for (int e = tid; e < nnz; e += blockDim.x) {
+                cval[(size_t)m * csc.cap_smem + e] = csc.val[(size_t)m * csc.cap + e];
+                cidx[(size_t)m * csc.cap_smem + e] = csc.idx[(size_t)m * csc.cap + e];
+            }
         }
     }
     __syncthreads();
-    for (int s = warp; s < S; s += W) {
-        float tt = 0.0f;
-        for (int grp = 0; grp < NG; ++grp) {
-            const float* v = cur + ((size_t)s * NE + grp * 4) * kLanes + lane;
-            tt = tt + grouped4(v[0], v[kLanes], v[2 * kLanes], v[3 * kLanes]);
+    if (sums) {
+        for (int q = warp; q < S * NG; q += W) {
+            const float* v = cur + (size_t)q * 4 * kLanes + lane;
+            tsum[q * kLanes + lane] = grouped4(v[0], v[kLanes], v[2 * kLanes], v[3 * kLanes]);
         }
-        tot[s * kLanes + lane] = tt;
+        __syncthreads();
     }
+    // total over the groups of rows [NE][32] (or of their sums [NG][32])
+    auto total = [&](const float* rows, const float* gsum) {
+        float tt = 0.0f;
+        if (sums) {
+#pragma unroll 8
+            for (int grp = 0; grp < NG; ++grp) tt = tt + gsum[grp * kLanes + lane];
+        } else {
+#pragma unroll 4
+            for (int grp = 0; grp < NG; ++grp) {
+                const float* v = rows + (size_t)grp * 4 * kLanes + lane;
+                tt = tt + grouped4(v[0], v[kLanes], v[2 * kLanes], v[3 * kLanes]);
+            }
+        }
+        return tt;
+    };
+    auto draw = [&](int u, int q, float (&z)[4]) {
+        const int s = q / NG, grp = q - s * NG, N4 = (a.n_patches[s] + 3) & ~3;
+        to_path_stream ps;
+        to_stream_path(ps, (uint32_t)path);
+        to_stream_year(ps, (uint32_t)u, a.rk);
+        const to_u32x4 w = to_stream_words(
+            ps, to_stream_group((uint32_t)((s * N4) >> 2) + grp, stream_road, a.rk), a.rk);
+        to_box_muller(w.v[0], w.v[1], &z[0], &z[1]);
+        to_box_muller(w.v[2], w.v[3], &z[2], &z[3]);
+    };
     const float disc = 1.0f + a.rrr * a.dt / 100.0f;
     float val = 0.0f, df = 1.0f;        // warp 0: realised value, discount factor
-    int c0 = 0;
+    int first = 0;
     for (int u = t0; u < Y; ++u) {
-        __syncthreads();
-        // A. migrations of every (species, control)
-        for (int s = 0; s < S; ++s) {
+        const bool last = u == Y - 1;
+        // A
+        for (int q = warp; q < S * NG; q += W) {
+            const int s = q / NG, grp = q - s * NG;
             const float* cs = cur + (size_t)s * NE * kLanes + lane;
-            for (int grp = warp; grp < NG; grp += W) {
-                for (int c = 0; c < C; ++c) {
-                    const int m = s * C + c;
-                    const int* cp = cptr + m * (NE + 1);
-                    const float* cv = cval + (size_t)m * csc.cap_smem;
-                    const uint16_t* ci = cidx + (size_t)m * csc.cap_smem;
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const int k = grp * 4 + j;
-                        float acc = 0.0f;
-                        for (int e = cp[k]; e < cp[k + 1]; ++e)
-                            acc = fmaf(cs[(int)ci[e] * kLanes], cv[e], acc);
-                        mig[((size_t)m * NE + k) * kLanes + lane] = acc;
-                    }
-                }
-            }
-        }
-        __syncthreads();
-        // B. adjusted populations tot * (migrated total / tot)
-        for (int m = warp; m < SC; m += W) {
-            const int s = m / C;
-            float tt = 0.0f;
-            for (int grp = 0; grp < NG; ++grp) {
-                const float* v = mig + ((size_t)m * NE + grp * 4) * kLanes + lane;
-                tt = tt + grouped4(v[0], v[kLanes], v[2 * kLanes], v[3 * kLanes]);
-            }
-            const float ts = tot[s * kLanes + lane];
-            adj[m * kLanes + lane] = ts * (tt / ts);
-        }
-        __syncthreads();
-        // C. the decision and the realised payoff
-        if (warp == 0) {
-            int bc = 0;
-            if (path < P) {
-                float state[TO_ROV_MAXC * (TO_LSM_MAXD - 1) + 1];
-                for (int c = 0; c < C; ++c)
-                    for (int s = 0; s < S; ++s) state[c * S + s] = adj[(s * C + c) * kLanes + lane];
-                const float prof = to_rovd::unit_profit(a, path, u, Y + 1, Y + 1);
-                state[S * C] = prof;
-                float best;
-                if (u == Y - 1) to_rovd::decide_terminal(a, state, best, bc);
-                else to_rovd::decide_interior(a, u, 0, state, best, bc);
-                val = val + (a.flows[bc] * prof) * df;
-                df = df / disc;
-            }
-            if (u == t0) c0 = bc;
-            ctl[lane] = bc;
-        }
-        __syncthreads();
-        if (u == Y - 1) break;
-        // D. growth of the chosen control's migrated populations
-        const int cu = ctl[lane];
-        for (int s = 0; s < S; ++s) {
-            const float* sp = a.params + 8 * s;
-            const int N4 = (a.n_patches[s] + 3) & ~3;
-            const float g = (path < P) ? a.gmY[((size_t)u * S + s) * P + path] : 0.0f;
-            for (int grp = warp; grp < NG; grp += W) {
-                float z[4];
-                to_normal4(a.seed, TO_STREAM_GROWTH, road, path, u,
-                           (uint32_t)((s * N4) >> 2) + grp, z);
+            float* mg = mig + ((size_t)s * C * NE + grp * 4) * kLanes + lane;
+            if (uni) {
+                const int* up = cptr + s * (NE + 1) + grp * 4;
+                float g0 = 0.0f, g1 = 0.0f, g2 = 0.0f;
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    const int k = grp * 4 + j;
-                    const float mv = mig[(((size_t)s * C + cu) * NE + k) * kLanes + lane];
-                    const float gr = (a.sem == 0) ? g + z[j] * sp[7] : fmaf(sp[7] * z[j], g, g);
-                    const float cpk = capv[s * NE + k];
-                    cur[((size_t)s * NE + k) * kLanes + lane] =
-                        (a.sem == 0) ? mv * (1.0f + gr * (cpk - mv) / cpk / 100.0f)
-                                     : fmaxf(mv * (1.0f + gr * (cpk - mv) / cpk), 0.0f);
+                    float q0 = 0.0f, q1 = 0.0f, q2 = 0.0f;
+                    const int e1 = up[j + 1];
+#pragma unroll 2
+                    for (int e = up[j]; e < e1; e += 2) {      // an even number of terms
+#pragma unroll
+                        for (int w = 0; w < 2; ++w) {
+                            const int4 en = ue[e + w];
+                            const float x = *reinterpret_cast<const float*>(
+                                reinterpret_cast<const unsigned char*>(cs) + en.x);
+                            q0 = fmaf(x, __int_as_float(en.y), q0);
+                            q1 = fmaf(x, __int_as_float(en.z), q1);
+                            q2 = fmaf(x, __int_as_float(en.w), q2);
+                        }
+                    }
+                    mg[j * kLanes] = q0;
+                    if (C > 1) mg[(size_t)(NE + j) * kLanes] = q1;
+                    if (C > 2) mg[(size_t)(2 * NE + j) * kLanes] = q2;
+                    g0 = j ? g0 + q0 : q0;
+                    g1 = j ? g1 + q1 : q1;
+                    g2 = j ? g2 + q2 : q2;
+                }
+                float* o = msum + ((size_t)s * C * NG + grp) * kLanes + lane;
+                o[0] = g0;
+                if (C > 1) o[(size_t)NG * kLanes] = g1;
+                if (C > 2) o[(size_t)2 * NG * kLanes] = g2;
+            } else {
+                for (int c = 0; c < C; ++c) {
+                    const int m = s * C + c;
+                    const int* cp = cptr + m * (NE + 1) + grp * 4;
+                    const float* cv = cval + (size_t)m * csc.cap_smem;
+                    const uint16_t* ci = cidx + (size_t)m * csc.cap_smem;
+                    float gs = 0.0f;
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        float acc = 0.0f;
+#pragma unroll 4
+                        for (int e = cp[j]; e < cp[j + 1]; ++e)
+                            acc = fmaf(cs[(int)ci[e] * kLanes], cv[e], acc);
+                        mg[((size_t)c * NE + j) * kLanes] = acc;
+                        gs = j ? gs + acc : acc;
+                    }
+                    if (sums) msum[((size_t)m * NG + grp) * kLanes + lane] = gs;
                 }
             }
         }
         __syncthreads();
-        // E. totals of the new populations
-        for (int s = warp; s < S; s += W) {
-            float tt = 0.0f;
-            for (int grp = 0; grp < NG; ++grp) {
-                const float* v = cur + ((size_t)s * NE + grp * 4) * kLanes + lane;
-                tt = tt + grouped4(v[0], v[kLanes], v[2 * kLanes], v[3 * kLanes]);
+        const float prof = live ? a.profS[(size_t)u * P + path] : 0.0f;
+        // B
+        for (int c = warp; c < C; c += W) {
+            float st[S];
+            bool valid = true;
+#pragma unroll
+            for (int s = 0; s < S; ++s) {
+                const int m = s * C + c;
+                const float ts = total(cur + (size_t)s * NE * kLanes, tsum + (size_t)s * NG * kLanes);
+                const float tt = total(mig + (size_t)m * NE * kLanes, msum + (size_t)m * NG * kLanes);
+                st[s] = ts * (tt / ts);
+                if (st[s] < to_rovd::threshold(a, s) && c > 0) valid = false;
             }
-            tot[s * kLanes + lane] = tt;
+            float r = INFINITY;                    // an invalid control's
+            if (valid && live) {
+                const float now = a.flows[c] * prof;
+                if (last) {
+                    r = now > 0.0f ? 0.0f : now;
+                } else {
+                    const float v = to_lsm_interp(to_rov_reg_block(a, u, c), R, S, st, prof);
+                    double ce = (double)(v / disc);
+                    if (ce > 0.0) ce = 0.0;
+                    r = (float)((double)now + ce);
+                }
+            }
+            pay[c * kLanes + lane] = r;
         }
+        float z[kResimHeld][4];
+        if (!last) {
+#pragma unroll
+            for (int i = 0; i < kResimHeld; ++i)
+                if (warp + i * W < S * NG) draw(u, warp + i * W, z[i]);
+        }
+        __syncthreads();
+        // C
+        int cu = 0;
+        {
+            float best = pay[lane];
+            for (int c = 1; c < C; ++c) {
+                const float r = pay[c * kLanes + lane];
+                if (r < best) { best = r; cu = c; }
+            }
+        }
+        if (u == t0) first = cu;
+        if (warp == 0 && live) {
+            val = val + (a.flows[cu] * prof) * df;
+            df = df / disc;
+        }
+        if (last) break;
+        auto grow = [&](int q, const float (&zz)[4]) {
+            const int s = q / NG, grp = q - s * NG;
+            const float s7 = a.params[8 * s + 7];
+            const float g = live ? a.gmY[((size_t)u * S + s) * P + path] : 0.0f;
+            const float* mg = mig + (((size_t)s * C + cu) * NE + grp * 4) * kLanes + lane;
+            float* o = cur + ((size_t)s * NE + grp * 4) * kLanes + lane;
+            float v[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float mv = mg[j * kLanes], cpk = capv[s * NE + grp * 4 + j];
+                const float gr = fmaf(s7 * zz[j], g, g), x = gr * (cpk - mv);
+                const float d = sums ? to_div_rcp(x, cpk, rcap[s * NE + grp * 4 + j]) : x / cpk;
+                v[j] = fmaxf(mv * (1.0f + d), 0.0f);
+                o[j * kLanes] = v[j];
+            }
+            if (sums) tsum[q * kLanes + lane] = grouped4(v[0], v[1], v[2], v[3]);
+        };
+#pragma unroll
+        for (int i = 0; i < kResimHeld; ++i)
+            if (warp + i * W < S * NG) grow(warp + i * W, z[i]);
+        for (int q = warp + kResimHeld * W; q < S * NG; q += W) {
+            draw(u, q, z[0]);
+            grow(q, z[0]);
+        }
+        __syncthreads();
     }
-    if (warp == 0 && path < P) {
+    if (warp == 0 && live) {
         a.condExp[(size_t)t0 * P + path] = val;
-        a.optCont[(size_t)t0 * P + path] = c0;
+        a.optCont[(size_t)t0 * P + path] = first;
     }
 }
 
@@ -1212,21 +1344,18 @@ to_status rov_forward_sparse(to_ctx ctx, const to_rov_args& a, to_csc csc) {
 }
 
 
-size_t rov_resim_smem(int NE, int S, int C, int cap_smem) {
-    const size_t SC = (size_t)S * C;
-    return ((size_t)S * NE * kLanes + SC * NE * kLanes + (size_t)S * NE + (size_t)S * kLanes +
-            SC * kLanes) * 4 + kLanes * 4 + SC * (NE + 1) * 4 + SC * cap_smem * 6 + 16;
-}
-
 to_status rov_resim_sparse(to_ctx ctx, const to_rov_args& a, to_csc csc, int t0) {
-    const size_t smem = rov_resim_smem(a.ne, a.S, a.C, csc.cap_smem);
-    if (smem > ctx->smem_optin)
-        return to_set_error(ctx, TO_ERR_UNSUPPORTED, "ALGO6 re-simulation needs %zu B", smem);
+    // the smallest layout has to fit; the kernel takes the best one that does
+    const size_t least = resim_bytes(a.ne, a.S, a.C, resim_lists(a.ne, a.S, a.C, csc.cap_smem), false);
+    const size_t limit = ctx->smem_optin;
+    if (least > limit)
+        return to_set_error(ctx, TO_ERR_UNSUPPORTED, "ALGO6 re-simulation needs %zu B", least);
+    const auto kern = a.S == 1 ? k_rov_resim<1> : a.S == 2 ? k_rov_resim<2> : a.S == 3 ? k_rov_resim<3>
+                                                                                       : k_rov_resim<4>;
     const int blocks = (a.P + kLanes - 1) / kLanes;
     to_prof_begin(ctx, "rov_resim");
-    TO_CUDA(ctx, cudaFuncSetAttribute(k_rov_resim_sparse,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_rov_resim_sparse<<<blocks, 1024, smem, ctx->stream>>>(a, csc, t0);
+    TO_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit));
+    kern<<<blocks, 1024, limit, ctx->stream>>>(a, csc, t0, (int)limit);
     to_prof_end(ctx);
     TO_LAUNCHED(ctx);
     return TO_OK;
