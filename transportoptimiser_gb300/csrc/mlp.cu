@@ -5,8 +5,9 @@
 // learned alternative used for GA screening, with the plain Monte Carlo as
 // the fallback and the measure of its error.
 //
-// One CTA owns a tile of 128 rows (TMEM lane = row) and runs the whole
-// forward and, for training, the whole backward pass on it:
+// A CTA of 16 warps owns a tile of 128 rows (TMEM lane = row, a warp a
+// quarter of its 32 rows' columns) and runs the whole forward and, for
+// training, the whole backward pass on it:
 //   F1  H1 = X W1^T            tcgen05 kind::f16, M=128 N=128 K=16
 //   F2  H2 = H1 W2^T           M=128 N=128 K=128
 //   L3  Y = H2 W3^T + b3       SIMT (3 outputs)
@@ -14,12 +15,19 @@
 //   G2  dW2 = dH2^T H1         M=128 (units) N=128 K=128 (rows)
 //   G1  dW1 = dH1^T X          M=128 N=16 K=128
 // Operands are BF16 in shared memory (K-major core-matrix tiles written by
-// the threads, transposed copies where a GEMM contracts over rows),
-// accumulators FP32 in TMEM.  Rounding points (every value that feeds an
-// MMA is rounded to BF16 once; biases, ReLU, layer 3 and all reductions in
-// FP32) are restated by the oracle.  Each tile writes its gradient partial;
-// k_mlp_adam sums the partials in tile order (deterministic) and applies
-// Adam to the FP32 master parameters.
+// the threads; where a GEMM contracts over rows, a tile's core matrices are
+// transposed by ldmatrix / stmatrix), accumulators FP32 in TMEM.  Rounding
+// points (every value that feeds an MMA is rounded to BF16 once; biases,
+// ReLU, layer 3 and all reductions in FP32) are restated by the oracle.
+// Each tile writes its gradient partial; the partials are summed in tile
+// order (deterministic) and Adam is applied to the FP32 master parameters.
+//
+// Training is a chain of small steps (512 rows are four tiles), bound by the
+// latency of what follows what within a step: the FP32 sums over 128 units or
+// rows keep their order, so that a parameter's trajectory does not depend on
+// the thread count, and are a thread each; an epoch is one launch whose CTAs
+// meet twice a step.  20,000 rows, batches of 512, four epochs: 10.2 -> 4.2 ms,
+// 65 -> 25 us a step (three launches a step and four warps a tile before).
 #include <cuda_bf16.h>
 
 #include <cmath>
@@ -42,15 +50,18 @@ constexpr int KB_IN = IN * 2, KB_HID = HID * 2;      // K bytes per row of the b
 constexpr int S_X = 0;                               // X   [128 rows][16]
 constexpr int S_W1 = S_X + 128 * KB_IN;              // W1  [128 units][16]
 constexpr int S_XT = S_W1 + 128 * KB_IN;             // X^T [16][128 rows]
-constexpr int S_A = S_XT + IN * KB_HID;              // H1 [row][unit] -> dH2 [row][unit] -> dH1^T [unit][row]
-constexpr int S_B = S_A + 128 * KB_HID;              // W2 [out][in] -> H2 (row-major bf16)
+constexpr int S_A = S_XT + IN * KB_HID;              // H1 [row][unit] -> dH2 -> dH1
+constexpr int S_B = S_A + 128 * KB_HID;              // W2 [out][in]
 constexpr int S_W2T = S_B + 128 * KB_HID;            // W2^T [in][out]
 constexpr int S_H1T = S_W2T + 128 * KB_HID;          // H1^T [unit][row]
-constexpr int S_D2T = S_H1T + 128 * KB_HID;          // dH2^T [unit][row]
-constexpr int S_F = S_D2T + 128 * KB_HID;            // fp32: W3, b1, b2, b3, dY, loss
+constexpr int S_D2T = S_H1T + 128 * KB_HID;          // dH2^T [unit][row] -> dH1^T
+constexpr int H2_ROW = HID / 2 + 1;                  // words of a row of H2: no bank conflicts
+constexpr int S_H2 = S_D2T + 128 * KB_HID;           // H2 bf16 [row][H2_ROW words]
+constexpr int S_F = S_H2 + 128 * H2_ROW * 4;         // fp32: W3, b1, b2, b3, dY, squared errors
 constexpr int F_W3 = 0, F_B1 = F_W3 + OUT * HID, F_B2 = F_B1 + HID, F_B3 = F_B2 + HID,
-              F_DY = F_B3 + 4, F_L = F_DY + 128 * OUT, F_END = F_L + 128;
+              F_DY = F_B3 + 4, F_L = F_DY + 128 * OUT, F_END = F_L + 128 * OUT;
 constexpr int SMEM_BYTES = S_F + F_END * 4;
+constexpr int NT = 512;                              // threads of a tile
 
 constexpr uint32_t SBO_IN = KB_IN * 8, SBO_HID = KB_HID * 8, LBO = 128;
 
@@ -60,9 +71,6 @@ __device__ __forceinline__ unsigned short bfbits(float x) {
 }
 __device__ __forceinline__ void st_bf16(unsigned char* base, uint32_t off, float x) {
     *reinterpret_cast<unsigned short*>(base + off) = bfbits(x);
-}
-__device__ __forceinline__ float ld_bf16(const unsigned char* base, uint32_t off) {
-    return __bfloat162float(__ushort_as_bfloat16(*reinterpret_cast<const unsigned short*>(base + off)));
 }
 // 8 consecutive K elements of one row as one 16-byte store
 __device__ __forceinline__ void st_bf16x8(unsigned char* base, uint32_t off, const float* v) {
@@ -99,223 +107,404 @@ __device__ __forceinline__ void publish_smem() {
     to_tc::fence_after_sync();
 }
 
-// rows: optional row index list (training order); t/part/loss only when BWD
-template <bool BWD>
-__global__ void __launch_bounds__(128, 1)
-k_mlp(const float* __restrict__ params, int n, const int* __restrict__ rows,
-      const float* __restrict__ x, const float* __restrict__ t, float inv_count,
-      float* __restrict__ y_out, float* __restrict__ part, double* __restrict__ loss_part,
-      int* __restrict__ err) {
-    extern __shared__ __align__(1024) unsigned char sm[];
-    __shared__ __align__(8) uint64_t mbar;
-    __shared__ uint32_t tslot;
-    float* f = reinterpret_cast<float*>(sm + S_F);
-    const int tid = threadIdx.x, warp = tid >> 5;
-    const int r0 = blockIdx.x * 128;
-    const int gr = r0 + tid;
+// the 32 x 32 block at (r0, c0) of a 128 x 128 tile, transposed into dst: a
+// core matrix at a time, four per instruction; the warp wrote it itself
+__device__ __forceinline__ void transpose_block(const unsigned char* src, unsigned char* dst, int r0,
+                                                int c0) {
+    const int lane = threadIdx.x & 31, cg = (c0 >> 3) + (lane >> 3), in = (lane & 7) * 16;
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int rg = (r0 >> 3) + i;
+        uint32_t m[4];
+        to_tc::ldsm_x4_t(src + rg * (KB_HID * 8) + cg * 128 + in, m);
+        to_tc::stsm_x4(dst + cg * (KB_HID * 8) + rg * 128 + in, m);
+    }
+}
+
+// sum of row u of a [128][128] bf16 tile, K ascending
+__device__ __forceinline__ float row_sum(const unsigned char* tile, int u) {
+    const unsigned char* row = tile + (u >> 3) * (KB_HID * 8) + (u & 7) * 16;
+    float s = 0.0f;
+#pragma unroll 4
+    for (int c = 0; c < 16; ++c) {
+        const uint4 q = *reinterpret_cast<const uint4*>(row + c * 128);
+        const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            s = s + __uint_as_float(w[j] << 16);
+            s = s + __uint_as_float(w[j] & 0xFFFF0000u);
+        }
+    }
+    return s;
+}
+
+// a thread's share of a tile's inputs: half a row of x, one target
+struct MlpRows {
+    float x[8], t;
+};
+__device__ __forceinline__ MlpRows load_rows(int r0, int n, const int* __restrict__ rows,
+                                             const float* __restrict__ x,
+                                             const float* __restrict__ t) {
+    const int row = threadIdx.x & 127, which = threadIdx.x >> 7, gr = r0 + row;
     const bool valid = gr < n;
-    const int src = valid ? (rows ? rows[gr] : gr) : 0;
+    const size_t src = valid ? (rows ? rows[gr] : gr) : 0;
+    MlpRows r;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) r.x[k] = valid && which < 2 ? x[src * IN + which * 8 + k] : 0.0f;
+    r.t = valid && t && which < OUT ? t[src * OUT + which] : 0.0f;
+    return r;
+}
+
+// What a CTA keeps across its tiles.
+struct MlpCta {
+    unsigned char* sm;
+    uint64_t* mbar;
+    uint32_t tmem, phase;
+    bool ok;                                   // no MMA wait has expired
+};
+
+// One tile: rows r0 .. r0 + 127 of n.  Parameters are read past L1 (another
+// CTA may have written them).  gp, loss only when BWD.
+template <bool BWD>
+__device__ __forceinline__ void mlp_tile(MlpCta& k, const float* params, int r0, int n,
+                                         const MlpRows& in, float inv_count, float* y_out, float* gp,
+                                         double* loss) {
+    unsigned char* sm = k.sm;
+    float* f = reinterpret_cast<float*>(sm + S_F);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int wr = warp & 3, cq = (warp >> 2) * 32;         // 32 rows and 32 columns of the warp
+    const int row = wr * 32 + lane;
+    const int j128 = tid & 127, which = tid >> 7;           // one of 128, and of four
+    bool ok = k.ok;
 
     // ---- stage parameters (bf16 operand tiles, fp32 for the SIMT parts)
-    for (int e = tid; e < HID * IN; e += 128) {
-        int o = e / IN, k = e - o * IN;
-        st_bf16(sm + S_W1, to_tc::kmaj_off(o, k, KB_IN, 2), params[OFF_W1 + e]);
-    }
-    for (int e = tid; e < HID * HID; e += 128) {
-        int o = e / HID, i = e - o * HID;
-        float w = params[OFF_W2 + e];
-        st_bf16(sm + S_B, to_tc::kmaj_off(o, i, KB_HID, 2), w);
-        if (BWD) st_bf16(sm + S_W2T, to_tc::kmaj_off(i, o, KB_HID, 2), w);
-    }
-    for (int e = tid; e < OUT * HID; e += 128) f[F_W3 + e] = bf(params[OFF_W3 + e]);
-    f[F_B1 + tid] = params[OFF_B1 + tid];
-    f[F_B2 + tid] = params[OFF_B2 + tid];
-    if (tid < OUT) f[F_B3 + tid] = params[OFF_B3 + tid];
-    {
-        float xv[IN];
+    if (tid < 256) {
+        float v[8];
 #pragma unroll
-        for (int k = 0; k < IN; ++k) xv[k] = valid ? x[(size_t)src * IN + k] : 0.0f;
-        st_bf16x8(sm + S_X, to_tc::kmaj_off(tid, 0, KB_IN, 2), xv);
-        st_bf16x8(sm + S_X, to_tc::kmaj_off(tid, 8, KB_IN, 2), xv + 8);
+        for (int j = 0; j < 8; ++j) v[j] = __ldcg(params + OFF_W1 + j128 * IN + which * 8 + j);
+        st_bf16x8(sm + S_W1, to_tc::kmaj_off(j128, which * 8, KB_IN, 2), v);
+    }
+#pragma unroll
+    for (int i = 0; i < 2048 / NT; ++i) {
+        const int e = tid + i * NT, o = (e & 7) | ((e >> 7) << 3), c = ((e >> 3) & 15) * 8;
+        float v[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = __ldcg(params + OFF_W2 + o * HID + c + j);
+        st_bf16x8(sm + S_B, to_tc::kmaj_off(o, c, KB_HID, 2), v);
+    }
+    if (BWD)
+#pragma unroll
+        for (int i = 0; i < 2048 / NT; ++i) {
+            const int o = (which + i * (NT / 128)) * 8;
+            float v[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[j] = __ldcg(params + OFF_W2 + (o + j) * HID + j128);
+            st_bf16x8(sm + S_W2T, to_tc::kmaj_off(j128, o, KB_HID, 2), v);
+        }
+    if (tid < OUT * HID) f[F_W3 + tid] = bf(__ldcg(params + OFF_W3 + tid));
+    else f[F_B1 + j128] = __ldcg(params + OFF_B1 + j128);
+    if (tid < HID) f[F_B2 + tid] = __ldcg(params + OFF_B2 + tid);
+    else if (tid < HID + OUT) f[F_B3 + tid - HID] = __ldcg(params + OFF_B3 + tid - HID);
+    if (tid < 256) {
+        st_bf16x8(sm + S_X, to_tc::kmaj_off(j128, which * 8, KB_IN, 2), in.x);
         if (BWD)
 #pragma unroll
-            for (int k = 0; k < IN; ++k) st_bf16(sm + S_XT, to_tc::kmaj_off(k, tid, KB_HID, 2), xv[k]);
+            for (int j = 0; j < 8; ++j)
+                st_bf16(sm + S_XT, to_tc::kmaj_off(which * 8 + j, j128, KB_HID, 2), in.x[j]);
     }
-    if (tid == 0) to_tc::mbar_init(&mbar, 1);
-    if (warp == 0) to_tc::tmem_alloc<256>(&tslot);
     publish_smem();
-    const uint32_t tmem = tslot;
-    const uint32_t T0 = tmem, T1 = tmem + 128;     // two 128-column accumulators
-    uint32_t phase = 0;
-    bool ok = true;
+    const uint32_t T0 = k.tmem, T1 = k.tmem + 128;          // two 128-column accumulators
 
     // ---- F1
-    if (tid == 0) {
+    if (ok && tid == 0) {
         mma_chain(T0, sm + S_X, SBO_IN, sm + S_W1, SBO_IN, to_tc::idesc(1, 128, HID), 1);
-        to_tc::commit(&mbar);
+        to_tc::commit(k.mbar);
     }
-    ok = wait_mma(&mbar, phase);
-    uint32_t mask1[4] = {0, 0, 0, 0};
+    if (ok) ok = wait_mma(k.mbar, k.phase);
+    uint32_t mask1 = 0, mask2 = 0;
     if (ok) {
-        for (int c0 = 0; c0 < HID; c0 += 16) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int c0 = cq + h * 16;
             float v[16];
-            to_tc::tmem_ld16(to_tc::lane_addr(T0, warp, c0), v);
+            to_tc::tmem_ld16(to_tc::lane_addr(T0, wr, c0), v);
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
-                float a = v[j] + f[F_B1 + c0 + j];
-                if (a > 0.0f) mask1[(c0 + j) >> 5] |= 1u << ((c0 + j) & 31);
+                const float a = v[j] + f[F_B1 + c0 + j];
+                if (a > 0.0f) mask1 |= 1u << (h * 16 + j);
                 v[j] = a > 0.0f ? a : 0.0f;
             }
-            st_bf16x8(sm + S_A, to_tc::kmaj_off(tid, c0, KB_HID, 2), v);
-            st_bf16x8(sm + S_A, to_tc::kmaj_off(tid, c0 + 8, KB_HID, 2), v + 8);
-            if (BWD)
-#pragma unroll
-                for (int j = 0; j < 16; ++j)
-                    st_bf16(sm + S_H1T, to_tc::kmaj_off(c0 + j, tid, KB_HID, 2), v[j]);
+            st_bf16x8(sm + S_A, to_tc::kmaj_off(row, c0, KB_HID, 2), v);
+            st_bf16x8(sm + S_A, to_tc::kmaj_off(row, c0 + 8, KB_HID, 2), v + 8);
         }
+        if (BWD) transpose_block(sm + S_A, sm + S_H1T, wr * 32, cq);
     }
     publish_smem();
 
     // ---- F2
     if (ok && tid == 0) {
         mma_chain(T1, sm + S_A, SBO_HID, sm + S_B, SBO_HID, to_tc::idesc(1, 128, HID), HID / 16);
-        to_tc::commit(&mbar);
+        to_tc::commit(k.mbar);
     }
-    if (ok) ok = wait_mma(&mbar, phase);
-
-    // ---- layer 3 (SIMT) on bf16 H2; H2 kept row-major in S_B for dW3
-    float y[OUT] = {0.0f, 0.0f, 0.0f};
-    unsigned short* h2s = reinterpret_cast<unsigned short*>(sm + S_B);
+    if (ok) ok = wait_mma(k.mbar, k.phase);
+    uint32_t* h2 = reinterpret_cast<uint32_t*>(sm + S_H2);
     if (ok) {
-        for (int c0 = 0; c0 < HID; c0 += 16) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int c0 = cq + h * 16;
             float v[16];
-            to_tc::tmem_ld16(to_tc::lane_addr(T1, warp, c0), v);
+            to_tc::tmem_ld16(to_tc::lane_addr(T1, wr, c0), v);
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
-                const int o = c0 + j;
-                float a = v[j] + f[F_B2 + o];
-                float h = bf(a > 0.0f ? a : 0.0f);
-                if (BWD) h2s[tid * HID + o] = bfbits(h);
-#pragma unroll
-                for (int q = 0; q < OUT; ++q) y[q] = y[q] + h * f[F_W3 + q * HID + o];
+                const float a = v[j] + f[F_B2 + c0 + j];
+                if (a > 0.0f) mask2 |= 1u << (h * 16 + j);
+                v[j] = a > 0.0f ? a : 0.0f;
             }
-        }
 #pragma unroll
-        for (int q = 0; q < OUT; ++q) y[q] = y[q] + f[F_B3 + q];
+            for (int j = 0; j < 16; j += 2)
+                h2[row * H2_ROW + ((c0 + j) >> 1)] = bfbits(v[j]) | ((uint32_t)bfbits(v[j + 1]) << 16);
+        }
+    }
+    __syncthreads();
+
+    // ---- layer 3 (SIMT) on bf16 H2: a thread a (row, output)
+    if (tid < 128 * OUT) {
+        float y = 0.0f;
+        if (ok) {
+            const float* w = f + F_W3 + which * HID;
+#pragma unroll 8
+            for (int o = 0; o < HID / 2; ++o) {
+                const uint32_t u = h2[j128 * H2_ROW + o];
+                y = y + __uint_as_float(u << 16) * w[2 * o];
+                y = y + __uint_as_float(u & 0xFFFF0000u) * w[2 * o + 1];
+            }
+            y = y + f[F_B3 + which];
+        }
+        const bool valid = r0 + j128 < n;
+        if (!BWD) {
+            if (ok && valid) y_out[(size_t)(r0 + j128) * OUT + which] = y;
+        } else {
+            const float d = valid ? y - in.t : 0.0f;
+            f[F_L + which * 128 + j128] = d * d;
+            f[F_DY + j128 * OUT + which] = 2.0f * d * inv_count;
+        }
     }
     if (!BWD) {
-        if (ok && valid)
-            for (int q = 0; q < OUT; ++q) y_out[(size_t)gr * OUT + q] = y[q];
+        k.ok = ok;
+        return;
+    }
+    __syncthreads();
+    // ---- dH2 = (dY W3) * relu'(a2)
+    if (ok) {
+        const float dy0 = f[F_DY + row * OUT + 0], dy1 = f[F_DY + row * OUT + 1],
+                    dy2 = f[F_DY + row * OUT + 2];
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+            const int c0 = cq + h * 8;
+            float v[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const int o = c0 + j;
+                const float g = (dy0 * f[F_W3 + o] + dy1 * f[F_W3 + HID + o]) + dy2 * f[F_W3 + 2 * HID + o];
+                v[j] = (mask2 >> (h * 8 + j)) & 1u ? g : 0.0f;
+            }
+            st_bf16x8(sm + S_A, to_tc::kmaj_off(row, c0, KB_HID, 2), v);
+        }
+        transpose_block(sm + S_A, sm + S_D2T, wr * 32, cq);
+    }
+    publish_smem();
+    // ---- B2 (dH1 pre-mask) into T0, G2 (dW2) into T1
+    if (ok && tid == 0) {
+        mma_chain(T0, sm + S_A, SBO_HID, sm + S_W2T, SBO_HID, to_tc::idesc(1, 128, HID), HID / 16);
+        mma_chain(T1, sm + S_D2T, SBO_HID, sm + S_H1T, SBO_HID, to_tc::idesc(1, 128, HID), HID / 16);
+        to_tc::commit(k.mbar);
+    }
+    // meanwhile: dW3, db2 (rows summed in order, a thread a sum), the loss
+    if (which < OUT) {
+        const uint32_t* hc = h2 + (j128 >> 1);
+        const int sh = (j128 & 1) ? 0 : 16;
+        float g = 0.0f;
+#pragma unroll 8
+        for (int r = 0; r < 128; ++r)
+            g = g + f[F_DY + r * OUT + which] * __uint_as_float((hc[r * H2_ROW] << sh) & 0xFFFF0000u);
+        gp[OFF_W3 + which * HID + j128] = g;
     } else {
-        // ---- loss gradient
-        float l = 0.0f;
+        gp[OFF_B2 + j128] = row_sum(sm + S_D2T, j128);
+    }
+    if (warp == NT / 32 - 1) {
+        double s = 0.0;
 #pragma unroll
-        for (int q = 0; q < OUT; ++q) {
-            float d = valid ? y[q] - t[(size_t)src * OUT + q] : 0.0f;
-            l = l + d * d;
-            f[F_DY + tid * OUT + q] = 2.0f * d * inv_count;
+        for (int i = 0; i < 4; ++i) {
+            const float* q = f + F_L + lane + 32 * i;
+            s += (double)((q[0] + q[128]) + q[256]);
         }
-        f[F_L + tid] = l;
-        to_tc::fence_before_sync();
-        __syncthreads();
-        to_tc::fence_after_sync();
-        if (tid == 0) {
-            double s = 0.0;
-            for (int i = 0; i < 128; ++i) s += (double)f[F_L + i];
-            loss_part[blockIdx.x] = s;
-        }
-        // ---- dH2 = (dY W3) * relu'(a2)
-        const float dy0 = f[F_DY + tid * OUT + 0], dy1 = f[F_DY + tid * OUT + 1],
-                    dy2 = f[F_DY + tid * OUT + 2];
-        if (ok) {
-            for (int c0 = 0; c0 < HID; c0 += 16) {
-                float v[16];
-                to_tc::tmem_ld16(to_tc::lane_addr(T1, warp, c0), v);
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (lane == 0) *loss = s;
+    }
+    if (ok) ok = wait_mma(k.mbar, k.phase);
+    if (ok) {
+        // dH1 = B2 * relu'(a1), transposed for G1; dW2 rows out
+        float4* dst = reinterpret_cast<float4*>(gp + OFF_W2 + (size_t)row * HID + cq);
 #pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    const int o = c0 + j;
-                    float a = v[j] + f[F_B2 + o];
-                    float g = (dy0 * f[F_W3 + o] + dy1 * f[F_W3 + HID + o]) + dy2 * f[F_W3 + 2 * HID + o];
-                    v[j] = a > 0.0f ? g : 0.0f;
-                }
-                st_bf16x8(sm + S_A, to_tc::kmaj_off(tid, c0, KB_HID, 2), v);
-                st_bf16x8(sm + S_A, to_tc::kmaj_off(tid, c0 + 8, KB_HID, 2), v + 8);
-#pragma unroll
-                for (int j = 0; j < 16; ++j)
-                    st_bf16(sm + S_D2T, to_tc::kmaj_off(c0 + j, tid, KB_HID, 2), v[j]);
-            }
-        }
-        publish_smem();
-        // ---- B2 (dH1 pre-mask) into T0, G2 (dW2) into T1
-        if (ok && tid == 0) {
-            mma_chain(T0, sm + S_A, SBO_HID, sm + S_W2T, SBO_HID, to_tc::idesc(1, 128, HID), HID / 16);
-            mma_chain(T1, sm + S_D2T, SBO_HID, sm + S_H1T, SBO_HID, to_tc::idesc(1, 128, HID), HID / 16);
-            to_tc::commit(&mbar);
-        }
-        // meanwhile: dW3, db3, db2 (rows summed in order)
-        float* gp = part + (size_t)blockIdx.x * PSTRIDE;
-        {
-            const int o = tid;
-            float g0 = 0.0f, g1 = 0.0f, g2 = 0.0f, gb2 = 0.0f;
-            for (int r = 0; r < 128; ++r) {
-                float h = __bfloat162float(__ushort_as_bfloat16(h2s[r * HID + o]));
-                g0 = g0 + f[F_DY + r * OUT + 0] * h;
-                g1 = g1 + f[F_DY + r * OUT + 1] * h;
-                g2 = g2 + f[F_DY + r * OUT + 2] * h;
-                gb2 = gb2 + ld_bf16(sm + S_A, to_tc::kmaj_off(r, o, KB_HID, 2));
-            }
-            gp[OFF_W3 + o] = g0;
-            gp[OFF_W3 + HID + o] = g1;
-            gp[OFF_W3 + 2 * HID + o] = g2;
-            gp[OFF_B2 + o] = gb2;
-            if (tid < OUT) {
-                float s = 0.0f;
-                for (int r = 0; r < 128; ++r) s = s + f[F_DY + r * OUT + tid];
-                gp[OFF_B3 + tid] = s;
-            }
-        }
-        if (ok) ok = wait_mma(&mbar, phase);
-        if (ok) {
-            // dH1 = B2 * relu'(a1), stored transposed for G1; dW2 rows out
-            for (int c0 = 0; c0 < HID; c0 += 16) {
-                float v[16];
-                to_tc::tmem_ld16(to_tc::lane_addr(T0, warp, c0), v);
-#pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    const int i = c0 + j;
-                    float g = ((mask1[i >> 5] >> (i & 31)) & 1u) ? v[j] : 0.0f;
-                    st_bf16(sm + S_A, to_tc::kmaj_off(i, tid, KB_HID, 2), g);
-                }
-                to_tc::tmem_ld16(to_tc::lane_addr(T1, warp, c0), v);
-                float4* dst = reinterpret_cast<float4*>(gp + OFF_W2 + (size_t)tid * HID + c0);
-#pragma unroll
-                for (int j = 0; j < 4; ++j) dst[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-            }
-        }
-        publish_smem();
-        // ---- G1 (dW1) into T0
-        if (ok && tid == 0) {
-            mma_chain(T0, sm + S_A, SBO_HID, sm + S_XT, SBO_HID, to_tc::idesc(1, 128, IN), HID / 16);
-            to_tc::commit(&mbar);
-        }
-        {
-            float s = 0.0f;
-            for (int r = 0; r < 128; ++r) s = s + ld_bf16(sm + S_A, to_tc::kmaj_off(tid, r, KB_HID, 2));
-            gp[OFF_B1 + tid] = s;
-        }
-        if (ok) ok = wait_mma(&mbar, phase);
-        if (ok) {
+        for (int h = 0; h < 2; ++h) {
+            const int c0 = cq + h * 16;
             float v[16];
-            to_tc::tmem_ld16(to_tc::lane_addr(T0, warp, 0), v);
-            float4* dst = reinterpret_cast<float4*>(gp + OFF_W1 + (size_t)tid * IN);
+            to_tc::tmem_ld16(to_tc::lane_addr(T0, wr, c0), v);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) dst[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+            for (int j = 0; j < 16; ++j) v[j] = (mask1 >> (h * 16 + j)) & 1u ? v[j] : 0.0f;
+            st_bf16x8(sm + S_A, to_tc::kmaj_off(row, c0, KB_HID, 2), v);
+            st_bf16x8(sm + S_A, to_tc::kmaj_off(row, c0 + 8, KB_HID, 2), v + 8);
+        }
+        transpose_block(sm + S_A, sm + S_D2T, wr * 32, cq);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            float v[16];
+            to_tc::tmem_ld16(to_tc::lane_addr(T1, wr, cq + h * 16), v);
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                dst[h * 4 + j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
         }
     }
-    if (!ok && tid == 0) atomicExch(err, TO_DEVERR_SPIN);
+    publish_smem();
+    // ---- G1 (dW1) into T0
+    if (ok && tid == 0) {
+        mma_chain(T0, sm + S_D2T, SBO_HID, sm + S_XT, SBO_HID, to_tc::idesc(1, 128, IN), HID / 16);
+        to_tc::commit(k.mbar);
+    }
+    if (which == 0) {
+        gp[OFF_B1 + j128] = row_sum(sm + S_D2T, j128);
+    } else if (tid >= 128 && tid < 128 + OUT) {
+        float s = 0.0f;
+#pragma unroll 8
+        for (int r = 0; r < 128; ++r) s = s + f[F_DY + r * OUT + (tid - 128)];
+        gp[OFF_B3 + tid - 128] = s;
+    }
+    if (ok) ok = wait_mma(k.mbar, k.phase);
+    if (ok && warp < 4) {
+        float v[16];
+        to_tc::tmem_ld16(to_tc::lane_addr(T0, warp, 0), v);
+        float4* dst = reinterpret_cast<float4*>(gp + OFF_W1 + (size_t)row * IN);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) dst[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+    }
+    k.ok = ok;
+}
+
+__device__ __forceinline__ MlpCta mlp_enter(unsigned char* sm, uint64_t* mbar, uint32_t* tslot) {
+    if (threadIdx.x == 0) to_tc::mbar_init(mbar, 1);
+    if (threadIdx.x < 32) to_tc::tmem_alloc<256>(tslot);
+    publish_smem();
+    MlpCta k;
+    k.sm = sm; k.mbar = mbar; k.tmem = *tslot; k.phase = 0; k.ok = true;
+    return k;
+}
+__device__ __forceinline__ void mlp_leave(const MlpCta& k, int* err) {
+    if (!k.ok && threadIdx.x == 0) atomicExch(err, TO_DEVERR_SPIN);
     to_tc::fence_before_sync();
     __syncthreads();
-    if (warp == 0) to_tc::tmem_free<256>(tmem);
+    if (threadIdx.x < 32) to_tc::tmem_free<256>(k.tmem);
+}
+
+// rows: optional row index list (training order); t/part/loss only when BWD
+template <bool BWD>
+__global__ void __launch_bounds__(NT, 1)
+k_mlp(const float* params, int n, const int* __restrict__ rows, const float* __restrict__ x,
+      const float* __restrict__ t, float inv_count, float* __restrict__ y_out,
+      float* __restrict__ part, double* __restrict__ loss_part, int* __restrict__ err) {
+    extern __shared__ __align__(1024) unsigned char sm_mlp[];
+    __shared__ __align__(8) uint64_t mbar;
+    __shared__ uint32_t tslot;
+    const int r0 = blockIdx.x * 128;
+    const MlpRows in = load_rows(r0, n, rows, x, BWD ? t : nullptr);
+    MlpCta k = mlp_enter(sm_mlp, &mbar, &tslot);
+    mlp_tile<BWD>(k, params, r0, n, in, inv_count, y_out,
+                  BWD ? part + (size_t)blockIdx.x * PSTRIDE : nullptr,
+                  BWD ? loss_part + blockIdx.x : nullptr);
+    mlp_leave(k, err);
+}
+
+// All CTAs of a cooperative launch: their writes before are seen after.
+// False (everywhere) when the others do not come within a second.
+__device__ __forceinline__ bool grid_meet(unsigned* counter, unsigned& target) {
+    target += gridDim.x;
+    __syncthreads();
+    bool ok = true;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        atomicAdd(counter, 1u);
+        uint64_t t0 = to_tc::now_ns();
+        while ((int)(to_tc::ld_acquire(counter) - target) < 0)
+            if (to_tc::now_ns() - t0 > 1000000000ull) { ok = false; break; }
+        __threadfence();
+    }
+    return !__syncthreads_or(!ok);
+}
+
+// Adam's state and constants
+struct MlpAdam {
+    float *params, *m, *v;                     // [PSTRIDE]
+    const float2* corr;                        // bias corrections of each step
+    float lr, b1, b2, eps;
+};
+__device__ __forceinline__ void adam_update(const MlpAdam& a, float g, float& m, float& v, float& p,
+                                            float c1, float c2) {
+    m = a.b1 * m + (1.0f - a.b1) * g;
+    v = a.b2 * v + (1.0f - a.b2) * g * g;
+    p = p - a.lr * (m / c1) / (sqrtf(v / c2) + a.eps);
+}
+
+// One epoch in one cooperative launch: a step's tiles a CTA each, then the
+// gradient sums and Adam spread over all CTAs.  The next step's rows are
+// fetched before the CTAs meet.
+__global__ void __launch_bounds__(NT, 1)
+k_mlp_epoch(MlpAdam ad, int n, int batch, const int* __restrict__ rows, const float* __restrict__ x,
+            const float* __restrict__ t, float* part, double* loss_part, double* loss,
+            unsigned* counter, int* __restrict__ err) {
+    extern __shared__ __align__(1024) unsigned char sm_mlp[];
+    __shared__ __align__(8) uint64_t mbar;
+    __shared__ uint32_t tslot;
+    const int r0 = blockIdx.x * 128, tid = threadIdx.x;
+    MlpRows in = load_rows(r0, min(batch, n), rows, x, t);
+    MlpCta k = mlp_enter(sm_mlp, &mbar, &tslot);
+    unsigned target = 0;
+    int step = 0;
+    for (int s0 = 0; s0 < n; s0 += batch, ++step) {
+        const int bs = min(batch, n - s0), tiles = (bs + 127) / 128;
+        if ((int)blockIdx.x < tiles)
+            mlp_tile<true>(k, ad.params, r0, bs, in, 1.0f / (3.0f * (float)bs), nullptr,
+                           part + (size_t)blockIdx.x * PSTRIDE, loss_part + blockIdx.x);
+        if (s0 + batch < n) in = load_rows(r0, min(batch, n - s0 - batch), rows + s0 + batch, x, t);
+        to_tc::fence_before_sync();
+        if (!grid_meet(counter, target)) { k.ok = false; break; }
+        to_tc::fence_after_sync();
+        const float2 c = ad.corr[step];
+        for (int q = blockIdx.x * NT + tid; q < PSTRIDE / 4; q += gridDim.x * NT) {
+            float4 g = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            float4 m = __ldcg(reinterpret_cast<const float4*>(ad.m) + q);
+            float4 v = __ldcg(reinterpret_cast<const float4*>(ad.v) + q);
+            float4 p = __ldcg(reinterpret_cast<const float4*>(ad.params) + q);
+#pragma unroll 4
+            for (int i = 0; i < tiles; ++i) {
+                const float4 d = __ldcg(reinterpret_cast<const float4*>(part + (size_t)i * PSTRIDE) + q);
+                g.x = g.x + d.x; g.y = g.y + d.y; g.z = g.z + d.z; g.w = g.w + d.w;
+            }
+            adam_update(ad, g.x, m.x, v.x, p.x, c.x, c.y);
+            adam_update(ad, g.y, m.y, v.y, p.y, c.x, c.y);
+            adam_update(ad, g.z, m.z, v.z, p.z, c.x, c.y);
+            adam_update(ad, g.w, m.w, v.w, p.w, c.x, c.y);
+            reinterpret_cast<float4*>(ad.m)[q] = m;
+            reinterpret_cast<float4*>(ad.v)[q] = v;
+            reinterpret_cast<float4*>(ad.params)[q] = p;
+        }
+        if (blockIdx.x == 0 && tid == 0) {
+            double s = 0.0;
+            for (int i = 0; i < tiles; ++i) s += __ldcg(loss_part + i);
+            *loss += s;
+        }
+        if (!grid_meet(counter, target)) { k.ok = false; break; }
+    }
+    mlp_leave(k, err);
 }
 
 // grad = sum of tile partials (tile order); optional Adam update
@@ -356,7 +545,7 @@ to_status launch_mlp(to_ctx ctx, const float* params, int n, const int* rows, co
     }
     const int tiles = (n + 127) / 128;
     to_prof_begin(ctx, BWD ? "mlp_fwd_bwd" : "mlp_fwd");
-    k_mlp<BWD><<<tiles, 128, SMEM_BYTES, ctx->stream>>>(params, n, rows, x, t, inv_count, y, part,
+    k_mlp<BWD><<<tiles, NT, SMEM_BYTES, ctx->stream>>>(params, n, rows, x, t, inv_count, y, part,
                                                          lp, ctx->d_flags);
     to_prof_end(ctx);
     TO_LAUNCHED(ctx);
@@ -370,6 +559,37 @@ namespace to_k {
 to_status mlp_forward(to_ctx ctx, const float* d_params, int n, const float* d_x, float* d_y) {
     if (n <= 0) return TO_OK;
     return launch_mlp<false>(ctx, d_params, n, nullptr, d_x, nullptr, 0.0f, d_y, nullptr, nullptr);
+}
+
+// one epoch over n rows in the order d_rows; false in *done (and nothing
+// launched) when the CTAs of a step's tiles cannot all be resident
+to_status mlp_epoch(to_ctx ctx, const MlpAdam& ad, int n, int batch, const int* d_rows,
+                    const float* d_x, const float* d_t, float* d_part, double* d_lp, double* d_loss,
+                    unsigned* d_counter, bool* done) {
+    *done = false;
+    const int tiles = (batch + 127) / 128, sms = ctx->sm_count > 0 ? ctx->sm_count : TO_SM_TARGET;
+    if (tiles > sms) return TO_OK;
+    int grid = (PSTRIDE / 4 + NT - 1) / NT;    // Adam: four parameters a thread
+    if (grid > sms) grid = sms;
+    if (grid < tiles) grid = tiles;
+    TO_CUDA(ctx, cudaFuncSetAttribute(k_mlp_epoch, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      SMEM_BYTES));
+    TO_CUDA(ctx, cudaMemsetAsync(d_counter, 0, sizeof(unsigned), ctx->stream));
+    to_prof_begin(ctx, "mlp_fwd_bwd");
+    MlpAdam a = ad;
+    int* err = ctx->d_flags;
+    void* args[] = {&a, &n, &batch, &d_rows, &d_x, &d_t, &d_part, &d_lp, &d_loss, &d_counter, &err};
+    const cudaError_t e = cudaLaunchCooperativeKernel((const void*)k_mlp_epoch, dim3(grid), dim3(NT),
+                                                      args, SMEM_BYTES, ctx->stream);
+    to_prof_end(ctx);
+    if (e == cudaErrorCooperativeLaunchTooLarge) {
+        cudaGetLastError();
+        return TO_OK;
+    }
+    TO_CUDA(ctx, e);
+    TO_LAUNCHED(ctx);
+    *done = true;
+    return TO_OK;
 }
 
 size_t mlp_part_floats(int n) { return (size_t)((n + 127) / 128) * PSTRIDE; }
@@ -501,37 +721,57 @@ to_status to_mlp_train(to_ctx ctx, float* params, int n, const float* x, const f
     if (batch > n) batch = n;
     const int tiles = (batch + 127) / 128;
     const size_t ep = epochs > 0 ? epochs : 1;
-    const size_t bytes = to_align256((size_t)NPARAM * 4) * 3 + to_align256((size_t)n * IN * 4) +
+    const size_t spe = ((size_t)n + batch - 1) / batch;        // steps an epoch
+    const size_t bytes = to_align256((size_t)PSTRIDE * 4) * 3 + to_align256((size_t)n * IN * 4) +
                          to_align256((size_t)n * OUT * 4) + to_align256(ep * n * 4) +
                          to_align256(to_k::mlp_part_floats(batch) * 4) + to_align256((size_t)tiles * 8) +
-                         to_align256(ep * 8);
+                         to_align256(ep * 8) + to_align256(ep * spe * 8) + 256;
     TO_TRY(to_arena_reserve(ctx, bytes + 2048));
-    float* d_p = to_arena_take<float>(ctx, NPARAM);
-    float* d_m = to_arena_take<float>(ctx, NPARAM);
-    float* d_v = to_arena_take<float>(ctx, NPARAM);
+    MlpAdam ad;
+    float* d_p = ad.params = to_arena_take<float>(ctx, PSTRIDE);
+    float* d_m = ad.m = to_arena_take<float>(ctx, PSTRIDE);
+    float* d_v = ad.v = to_arena_take<float>(ctx, PSTRIDE);
     float* d_x = to_arena_take<float>(ctx, (size_t)n * IN);
     float* d_t = to_arena_take<float>(ctx, (size_t)n * OUT);
     int* d_rows = to_arena_take<int>(ctx, ep * n);
     float* d_part = to_arena_take<float>(ctx, to_k::mlp_part_floats(batch));
     double* d_lp = to_arena_take<double>(ctx, tiles);
     double* d_loss = to_arena_take<double>(ctx, ep);
-    std::vector<int> rows(ep * n);
+    float2* d_corr = to_arena_take<float2>(ctx, ep * spe);
+    unsigned* d_counter = to_arena_take<unsigned>(ctx, 1);
+    if (!d_counter) return to_set_error(ctx, TO_ERR_ALLOC, "arena sizing");
+    ad.lr = lr; ad.b1 = 0.9f; ad.b2 = 0.999f; ad.eps = 1e-8f;
+    std::vector<int> rows((size_t)n);
+    std::vector<float2> corr(ep * spe);
+    for (size_t i = 0; i < corr.size(); ++i)
+        corr[i] = make_float2(1.0f - powf(ad.b1, (float)(i + 1)), 1.0f - powf(ad.b2, (float)(i + 1)));
     uint64_t st = seed;
-    for (size_t e = 0; e < ep; ++e) shuffle_rows(rows.data() + e * n, n, st);
     TO_CUDA(ctx, cudaMemcpyAsync(d_p, params, (size_t)NPARAM * 4, cudaMemcpyHostToDevice, ctx->stream));
-    TO_CUDA(ctx, cudaMemsetAsync(d_m, 0, (size_t)NPARAM * 4, ctx->stream));
-    TO_CUDA(ctx, cudaMemsetAsync(d_v, 0, (size_t)NPARAM * 4, ctx->stream));
+    TO_CUDA(ctx, cudaMemsetAsync(d_m, 0, (size_t)PSTRIDE * 4, ctx->stream));
+    TO_CUDA(ctx, cudaMemsetAsync(d_v, 0, (size_t)PSTRIDE * 4, ctx->stream));
     TO_CUDA(ctx, cudaMemcpyAsync(d_x, x, (size_t)n * IN * 4, cudaMemcpyHostToDevice, ctx->stream));
     TO_CUDA(ctx, cudaMemcpyAsync(d_t, t, (size_t)n * OUT * 4, cudaMemcpyHostToDevice, ctx->stream));
-    TO_CUDA(ctx, cudaMemcpyAsync(d_rows, rows.data(), ep * n * 4, cudaMemcpyHostToDevice, ctx->stream));
+    TO_CUDA(ctx, cudaMemcpyAsync(d_corr, corr.data(), corr.size() * sizeof(float2),
+                                 cudaMemcpyHostToDevice, ctx->stream));
     TO_CUDA(ctx, cudaMemsetAsync(d_loss, 0, ep * 8, ctx->stream));
     int step = 0;
     for (int e = 0; e < epochs; ++e) {
+        // an epoch's order is drawn while the GPU works on the one before
+        int* d_order = d_rows + (size_t)e * n;
+        shuffle_rows(rows.data(), n, st);
+        TO_CUDA(ctx, cudaMemcpyAsync(d_order, rows.data(), (size_t)n * 4, cudaMemcpyHostToDevice,
+                                     ctx->stream));
+        ad.corr = d_corr + (size_t)e * spe;
+        bool done = false;
+        TO_TRY(to_k::mlp_epoch(ctx, ad, n, batch, d_order, d_x, d_t, d_part, d_lp, d_loss + e,
+                               d_counter, &done));
+        if (done) continue;
+        step = (int)(e * spe);
         for (int s0 = 0; s0 < n; s0 += batch) {
             const int bs = n - s0 < batch ? n - s0 : batch;
             ++step;
-            TO_TRY(to_k::mlp_grad(ctx, d_p, bs, d_rows + (size_t)e * n + s0, d_x, d_t, d_part, d_lp,
-                                  nullptr, d_p, d_m, d_v, lr, step));
+            TO_TRY(to_k::mlp_grad(ctx, d_p, bs, d_order + s0, d_x, d_t, d_part, d_lp, nullptr, d_p,
+                                  d_m, d_v, lr, step));
             TO_TRY(to_k::mlp_sum_loss(ctx, (bs + 127) / 128, d_lp, d_loss + e));
         }
     }
