@@ -537,7 +537,9 @@ to_status to_simulate_mte(to_ctx ctx, const to_mte_problem* prob,
                    to_align256(prm.size() * 4) + to_align256((size_t)S * 4) +
                    to_align256((size_t)S * P * 4) + to_align256((size_t)S * 5 * 8) +
                    to_align256((size_t)S * (NP + 1) * 4) + to_align256((size_t)S * cap * 2) +
-                   to_align256((size_t)S * cap * 4) + to_align256((size_t)S * 4);
+                   to_align256((size_t)S * cap * 4) + to_align256((size_t)S * 4) +
+                   to_align256((size_t)(S + 1) * 4) +
+                   to_align256(to_k::mte_far_count(ctx, NP) * sizeof(f2));
     TO_TRY(to_arena_reserve(ctx, bytes));
     to_mte_args a;
     memset(&a, 0, sizeof(a));
@@ -555,6 +557,8 @@ to_status to_simulate_mte(to_ctx ctx, const to_mte_problem* prob,
     csc.nnz = to_arena_take<int>(ctx, S);
     csc.cap = cap;
     csc.cap_smem = 0;
+    a.order_buf = to_arena_take<int>(ctx, (size_t)S + 1);
+    a.far_buf = to_arena_take<f2>(ctx, to_k::mte_far_count(ctx, NP));
     TO_TRY(h2d(ctx, d_mmm, mmm.data(), mmm.size()));
     TO_TRY(h2d(ctx, d_ip, ip.data(), ip.size()));
     TO_TRY(h2d(ctx, d_cp, cp.data(), cp.size()));

@@ -96,215 +96,31 @@ __device__ __forceinline__ float grouped4(float a, float b, float c, float d) {
     return ((a + b) + c) + d;
 }
 
-// ---------------------------------------------------------------------------
-// MTE (mteKernel :595-717) - grid (ceil(P/PW), RS), the (road, species) of
-// grid row y taken from a.order when it is set (widest first, k_mte_order).
-// A warp's groups of four destinations are dealt in snake order over the
-// groups sorted by entries (warp w takes ranks w, 2W-1-w, 2W+w), at most
-// MAXG a warp; the next year's populations wait in registers until every
-// warp has read this year's, so one shared buffer suffices.  The growth
-// mean's draws are made kGmChunk years at a time by the whole CTA, and
-// every warp carries its lanes' growth means itself.  The values do not
-// depend on which warp computes a group.
-// ---------------------------------------------------------------------------
 constexpr int kMaxG = 4;
 constexpr int kGmChunk = 16;
-
-template <int MAXG, int PPL>
-__global__ void __launch_bounds__(1024, 1)
-k_mte_sparse(to_mte_args a, to_csc csc) {
-    // PPL paths per lane: lane owns paths lane + 32 i; every non-zero read
-    // from shared memory serves all of them
-    constexpr int PW = kLanes * PPL;                           // paths per CTA
-    extern __shared__ __align__(16) unsigned char sm_raw[];
-    const int NE = a.npe, NG = NE >> 2, NP = a.npad;
-    const int rs = a.rs0 + (a.order ? a.order[blockIdx.y] : (int)blockIdx.y);
-    const int road = rs / a.S, sp = rs - road * a.S;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, W = blockDim.x >> 5;
-    const int mtx = rs * a.C + a.c_use;
-    const int nnz = csc.nnz[mtx];
-    if (nnz < 0 || nnz > csc.cap_smem || a.n_patches[rs] > NE) {
-        // outside the shape this launch was planned for: flag, no result
-        if (threadIdx.x == 0 && a.flags) atomicExch(a.flags, TO_DEVERR_PLAN);
-        const int p = blockIdx.x * PW + (int)threadIdx.x;
-        if (threadIdx.x < PW && p < a.n_paths) a.end_pops[(size_t)rs * a.n_paths + p] = NAN;
-        return;
-    }
-    int2* cent = reinterpret_cast<int2*>(sm_raw);              // [cap_smem] (row byte offset, value)
-    float* cur = reinterpret_cast<float*>(cent + csc.cap_smem);// [NE][PW]
-    float* part = cur + (size_t)NE * PW;                       // [NG][PW]
-    float2* capr = reinterpret_cast<float2*>(part + (size_t)NG * PW);  // [NE] capacity, 1/capacity
-    float* xs = reinterpret_cast<float*>(capr + NE);           // [kGmChunk][3][PW] draws
-    int* cptr = reinterpret_cast<int*>(xs + kGmChunk * 3 * PW);// [NE+1]
-    int* order = cptr + NE + 1;                                // [NG] groups, widest first
-
-    const int N = a.n_patches[rs];
-    const int N4 = (N + 3) & ~3;
-    // groups of this (road, species); the launch is shaped for the widest
-    // model, and the groups past N4 would only ever hold zeros (no
-    // non-zeros reach them, the growth of 0 is 0) so they are not visited.
-    // Their totals are +0, which leaves a sum that started at +0 unchanged.
-    const int NGr = N4 >> 2;
-    const float* ip = a.init_pops + (size_t)rs * NP;
-    const float* sp8 = a.params + 8 * sp;
-    const float p0 = sp8[0], p1 = sp8[1], p2 = sp8[2], p4 = sp8[4], p5 = sp8[5],
-                p6 = sp8[6], p7 = sp8[7];
-    const float sj2 = p5 * p5;
-    const uint32_t road_id = (uint32_t)(a.road0 + road);
-    const int path0 = blockIdx.x * PW + lane;
-
-    for (int q = threadIdx.x; q < NE * PW; q += blockDim.x) {
-        int k = q / PW;
-        cur[q] = (k < N) ? ip[k] : 0.0f;
-    }
-    for (int k = threadIdx.x; k < NE; k += blockDim.x) {
-        const float cp = a.caps[(size_t)rs * NP + k];
-        capr[k] = make_float2(cp, 1.0f / cp);
-    }
-    for (int k = threadIdx.x; k <= NE; k += blockDim.x)
-        cptr[k] = csc.ptr[(size_t)mtx * (NP + 1) + (k <= NP ? k : NP)];
-    for (int e = threadIdx.x; e < nnz; e += blockDim.x) {
-        const int l = csc.idx[(size_t)mtx * csc.cap + e];
-        cent[e] = make_int2(l * PW * (int)sizeof(float),
-                            __float_as_int(csc.val[(size_t)mtx * csc.cap + e]));
-    }
-    __syncthreads();
-    for (int gq = threadIdx.x; gq < NGr; gq += blockDim.x) {
-        const int w = cptr[4 * gq + 4] - cptr[4 * gq];
-        int rank = 0;
-        for (int u = 0; u < NGr; ++u) {
-            const int wu = cptr[4 * u + 4] - cptr[4 * u];
-            rank += (wu > w) || (wu == w && u < gq);
-        }
-        order[rank] = gq;
-    }
-    float g[PPL];
-#pragma unroll
-    for (int i = 0; i < PPL; ++i) g[i] = p0;
-
-    for (int t = 0; t < a.n_years; ++t) {
-        if (t % kGmChunk == 0) {
-            // the next years' growth-mean draws, one thread each: jump
-            // indicator, Brownian term, jump factor minus one
-            const int nc = min(kGmChunk, a.n_years - t);
-            for (int q = threadIdx.x; q < nc * 3 * PW; q += blockDim.x) {
-                const int yy = q / (3 * PW), r = q - yy * 3 * PW;
-                const int which = r / PW, i = r - which * PW;
-                const uint32_t path = (uint32_t)(blockIdx.x * PW + i);
-                const int ty = t + yy;
-                float v;
-                if (which == 0) {
-                    v = (to_uniform1(a.seed, TO_STREAM_SP_JUMP, road_id, path, ty, sp) < p6) ? 1.0f
-                                                                                              : 0.0f;
-                } else if (which == 1) {
-                    v = to_normal1(a.seed, TO_STREAM_SP_BROWNIAN, road_id, path, ty, sp) * p2;
-                } else {
-                    const float zj = to_normal1(a.seed, TO_STREAM_SP_JUMPSIZE, road_id, path, ty, sp);
-                    const float jsz = (a.sem == 0) ? (zj * sj2 - sj2 / 2.0f) : (zj * p5 - sj2 / 2.0f);
-                    v = to_expf(jsz) - 1.0f;
-                }
-                xs[q] = v;
-            }
-            __syncthreads();
-        }
-        const float* xt = xs + (t % kGmChunk) * 3 * PW;
-#pragma unroll
-        for (int i = 0; i < PPL; ++i) {
-            const int pi = lane + kLanes * i;
-            const float jump = xt[pi], brown = xt[PW + pi], em1 = xt[2 * PW + pi];
-            g[i] = g[i] + p4 * (p1 - g[i]) * a.dt + g[i] * brown + em1 * g[i] * jump;
-        }
-        const bool last = (t == a.n_years - 1);
-        float nv[MAXG][4][PPL];
-#pragma unroll
-        for (int gi = 0; gi < MAXG; ++gi) {
-            const int slot = gi * W + ((gi & 1) ? W - 1 - warp : warp);
-            if (slot < NGr) {
-                const int grp = order[slot];
-                float z[PPL][4];
-#pragma unroll
-                for (int i = 0; i < PPL; ++i)
-                    to_normal4(a.seed, TO_STREAM_GROWTH, road_id, (uint32_t)(path0 + kLanes * i), t,
-                               (uint32_t)((sp * N4) >> 2) + grp, z[i]);
-                float msum[PPL];            // grouped4 of the migrated values, in order
-                // the group's column pointers: one 16-byte load and one word
-                const int4 c4 = reinterpret_cast<const int4*>(cptr)[grp];
-                const int cb[5] = {c4.x, c4.y, c4.z, c4.w, cptr[grp * 4 + 4]};
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const int k = grp * 4 + j;
-                    float acc[PPL];
-#pragma unroll
-                    for (int i = 0; i < PPL; ++i) acc[i] = 0.0f;
-                    const int e1 = cb[j + 1];
-#pragma unroll 2
-                    for (int e = cb[j]; e < e1; ++e) {
-                        const int2 ce = cent[e];
-                        const float* row = reinterpret_cast<const float*>(
-                            reinterpret_cast<const unsigned char*>(cur) + ce.x) + lane;
-                        const float v = __int_as_float(ce.y);
-#pragma unroll
-                        for (int i = 0; i < PPL; ++i) acc[i] = fmaf(row[kLanes * i], v, acc[i]);
-                    }
-                    const float2 cr = capr[k];
-#pragma unroll
-                    for (int i = 0; i < PPL; ++i) {
-                        msum[i] = (j == 0) ? acc[i] : msum[i] + acc[i];
-                        float gr = fmaf(p7 * z[i][j], g[i], g[i]);
-                        // the division as to_div_rcp: the same bits
-                        nv[gi][j][i] = acc[i] * (1.0f + to_div_rcp(gr * (cr.x - acc[i]), cr.x, cr.y));
-                    }
-                }
-                if (last)
-#pragma unroll
-                    for (int i = 0; i < PPL; ++i)
-                        part[grp * PW + lane + kLanes * i] = msum[i];
-            }
-        }
-        __syncthreads();
-#pragma unroll
-        for (int gi = 0; gi < MAXG; ++gi) {
-            const int slot = gi * W + ((gi & 1) ? W - 1 - warp : warp);
-            if (slot < NGr) {
-                const int grp = order[slot];
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-#pragma unroll
-                    for (int i = 0; i < PPL; ++i)
-                        cur[(grp * 4 + j) * PW + lane + kLanes * i] = nv[gi][j][i];
-            }
-        }
-        __syncthreads();
-    }
-    for (int i = threadIdx.x; i < PW; i += blockDim.x) {
-        const int path = blockIdx.x * PW + i;
-        if (path >= a.n_paths) continue;
-        float e = 0.0f;
-        if (a.n_years > 0 && a.sem == 0) {
-            for (int grp = 0; grp < NGr; ++grp) e = e + part[grp * PW + i];
-        } else {
-            for (int grp = 0; grp < NGr; ++grp) {
-                const float* v = cur + (size_t)grp * 4 * PW + i;
-                e = e + grouped4(v[0], v[PW], v[2 * PW], v[3 * PW]);
-            }
-        }
-        a.end_pops[(size_t)rs * a.n_paths + path] = e;
-    }
-}
 
 // The launch order of the MTE's (road, species): by descending packed
 // entries of the used control (ties by index), so the widest models start
 // first and the last wave holds the narrow ones.  One CTA.
 __global__ void __launch_bounds__(1024) k_mte_order(int n_rs, int rs0, int C, int c_use,
                                                     const int* __restrict__ nnz, int* order) {
-    for (int i = threadIdx.x; i < n_rs; i += blockDim.x) {
-        const int w = nnz[(size_t)(rs0 + i) * C + c_use];
+    __shared__ int s_w[1024];
+    for (int i0 = 0; i0 < n_rs; i0 += 1024) {
+        const int i = i0 + threadIdx.x;
+        const int w = i < n_rs ? nnz[(size_t)(rs0 + i) * C + c_use] : 0;
         int rank = 0;
-        for (int j = 0; j < n_rs; ++j) {
-            const int wj = nnz[(size_t)(rs0 + j) * C + c_use];
-            rank += (wj > w) || (wj == w && j < i);
+        for (int j0 = 0; j0 < n_rs; j0 += 1024) {
+            const int nj = min(1024, n_rs - j0);
+            __syncthreads();
+            if ((int)threadIdx.x < nj) s_w[threadIdx.x] = nnz[(size_t)(rs0 + j0 + threadIdx.x) * C + c_use];
+            __syncthreads();
+#pragma unroll 8
+            for (int j = 0; j < nj; ++j) {
+                const int wj = s_w[j];
+                rank += (wj > w) || (wj == w && j0 + j < i);
+            }
         }
-        order[rank] = i;
+        if (i < n_rs) order[rank] = i;
     }
 }
 
@@ -749,6 +565,339 @@ k_rov_forward_union(to_rov_args a, to_csc csc, int smem) {
         }
         if (warp == 0) total(Y);
         else if (warp <= C && Y > 0) at_risk(Y - 1, warp - 1);
+        __syncthreads();
+    }
+}
+
+// ---------------------------------------------------------------------------
+// MTE (mteKernel :595-717).  Persistent, the layout of k_rov_forward_union:
+// tiles of 64 paths (two a lane, packed) or 32 from a counter, the (road,
+// species) widest first (k_mte_order), a warp's own group of four
+// destinations and then others from a counter, one split barrier a year with
+// the next year's normals drawn behind it.  Bound by instruction issue (67%
+// of the slots, 725 instructions a group of 64 paths before the lists were
+// laid out by steps), and by a year's latency where there are few tiles.  So
+// a group's four lists run together: a step holds two entries of each
+// destination, the short ones padded by zero terms from a row of zeros, so
+// that there is one loop a group and eight gathers in flight.
+// 40,000 paths, 2 species of 115 patches, 50 years: 1.93 -> 1.50 ms (one CTA
+// an SM with the next year's values in registers and two barriers a year
+// before); 256 roads of 3 species, 64 paths: 2.86 -> 2.57 ms.
+// The values do not depend on which warp computes a group.
+// ---------------------------------------------------------------------------
+// a lane's paths and the arithmetic on them: two (packed) or one
+template <class V> struct to_lane;
+template <> struct to_lane<f2> {
+    static constexpr int paths = 2;
+    struct __align__(16) cap { f2 v, nr; };        // capacity, minus its reciprocal
+    to_path_stream ps0, ps1;
+    __device__ __forceinline__ void path(uint32_t p) {
+        to_stream_path(ps0, p);
+        to_stream_path(ps1, p + kLanes);
+    }
+    __device__ __forceinline__ void year(uint32_t t, const to_round_keys& rk) {
+        to_stream_year(ps0, t, rk);
+        to_stream_year(ps1, t, rk);
+    }
+    __device__ __forceinline__ void normals(const to_group_stream& g, const to_round_keys& rk,
+                                            const to_bm_tables& tab, f2 (&z)[4]) const {
+        to_normal4x2(ps0, ps1, g, rk, tab, z);
+    }
+    static __device__ __forceinline__ f2 load(const float* x) { return pack2(x[0], x[kLanes]); }
+    static __device__ __forceinline__ f2 all(float v) { return both2(v); }
+    static __device__ __forceinline__ f2 add(f2 a, f2 b) { return add2(a, b); }
+    static __device__ __forceinline__ f2 mul(f2 a, f2 b) { return mul2(a, b); }
+    static __device__ __forceinline__ f2 fma(f2 a, f2 b, f2 c) { return fma2(a, b, c); }
+    static __device__ __forceinline__ void store(float* out, int live, f2 v) {
+        float v0, v1;
+        unpack2(v, v0, v1);
+        if (live > 0) out[0] = v0;
+        if (live > kLanes) out[kLanes] = v1;
+    }
+};
+template <> struct to_lane<float> {
+    static constexpr int paths = 1;
+    struct __align__(8) cap { float v, nr; };
+    to_path_stream ps;
+    __device__ __forceinline__ void path(uint32_t p) { to_stream_path(ps, p); }
+    __device__ __forceinline__ void year(uint32_t t, const to_round_keys& rk) {
+        to_stream_year(ps, t, rk);
+    }
+    __device__ __forceinline__ void normals(const to_group_stream& g, const to_round_keys& rk,
+                                            const to_bm_tables& tab, float (&z)[4]) const {
+        const to_u32x4 w = to_stream_words(ps, g, rk);
+        f2 c, s;                                   // of both Box-Muller pairs
+        to_box_muller2(w.v[0], w.v[1], w.v[2], w.v[3], tab, c, s);
+        unpack2(c, z[0], z[2]);
+        unpack2(s, z[1], z[3]);
+    }
+    static __device__ __forceinline__ float load(const float* x) { return x[0]; }
+    static __device__ __forceinline__ float all(float v) { return v; }
+    static __device__ __forceinline__ float add(float a, float b) { return a + b; }
+    static __device__ __forceinline__ float mul(float a, float b) { return a * b; }
+    static __device__ __forceinline__ float fma(float a, float b, float c) { return fmaf(a, b, c); }
+    static __device__ __forceinline__ void store(float* out, int live, float v) {
+        if (live > 0) out[0] = v;
+    }
+};
+
+// shared memory of one (road, species) of N4 destinations: its lists (`list`
+// steps, 0 if they stay in global memory) and one or two population buffers
+__host__ __device__ inline size_t mte_bytes(int N4, int list, bool two, int paths) {
+    return (size_t)kGmChunk * 3 * kLanes * paths * 4 + (size_t)N4 * 8 * paths +
+           (size_t)((N4 + 4 + 2 * (N4 / 4 + 1) + 3) & ~3) * 4 +
+           (size_t)(two ? 2 : 1) * (N4 + 1) * kLanes * 4 * paths + (size_t)list * 64;
+}
+
+template <class V>
+__global__ void __launch_bounds__(kPairThreads, 1)
+k_mte_sparse(to_mte_args a, to_csc csc, to_round_keys rk, int n_rs, int smem, bool far_ok) {
+    using L = to_lane<V>;
+    constexpr int PW = kLanes * L::paths;      // paths of a tile
+    extern __shared__ __align__(16) unsigned char sm_raw[];
+    __shared__ int s_item, s_steps, s_grab[2];
+    __shared__ to_bm_tables s_tab;
+    __shared__ __align__(8) uint64_t s_bar;    // end of a year: an arrival a warp
+    const int Y = a.n_years, P = a.n_paths, NP = a.npad;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, W = blockDim.x >> 5;
+    const int tiles = (P + PW - 1) / PW, items = tiles * n_rs;
+    int* next = a.order_buf + n_rs;
+    to_bm_load(s_tab);                         // before the barriers below
+    if (tid == 0) to_mbar::init(&s_bar, W);
+    uint32_t phase = 0;
+    for (;;) {
+        if (tid == 0) s_item = atomicAdd(next, 1);
+        __syncthreads();
+        const int item = s_item;
+        __syncthreads();                       // read before it is written again
+        if (item >= items) break;
+        const int rq = item / tiles, rs = a.rs0 + (a.order ? a.order[rq] : rq);
+        const int road = rs / a.S, s = rs - road * a.S;
+        const int path0 = (item - rq * tiles) * PW + lane;
+        const int mtx = rs * a.C + a.c_use;
+        const int N = a.n_patches[rs], nnz = csc.nnz[mtx];
+        const int N4 = (N + 3) & ~3, NGr = N4 >> 2;
+        if (nnz < 0 || N > a.npe || mte_bytes(N4, 0, !far_ok, L::paths) > (size_t)smem) {
+            // outside the shape this launch was planned for: flag, no result
+            if (tid == 0 && a.flags) atomicExch(a.flags, TO_DEVERR_PLAN);
+            if (warp == 0) L::store(a.end_pops + (size_t)rs * P + path0, P - path0, L::all(NAN));
+            continue;
+        }
+        const uint32_t road_id = (uint32_t)(a.road0 + road);
+        const uint32_t stream_road = TO_STREAM_GROWTH | (road_id << 8);
+        L lp;
+        lp.path((uint32_t)path0);
+        const float* sp = a.params + 8 * s;
+        const float* ip = a.init_pops + (size_t)rs * NP;
+        const int* gptr = csc.ptr + (size_t)mtx * (NP + 1);
+        const uint16_t* gidx = csc.idx + (size_t)mtx * csc.cap;
+        const float* gval = csc.val + (size_t)mtx * csc.cap;
+
+        // draws of the growth mean, then [0] the means
+        float* xs = reinterpret_cast<float*>(sm_raw);                  // [kGmChunk][3][PW]
+        auto* capr = reinterpret_cast<typename L::cap*>(xs + kGmChunk * 3 * PW);   // [N4]
+        int* cptr = reinterpret_cast<int*>(capr + N4);                 // [N4 + 1]
+        int* order = cptr + N4 + 4;                                    // [NGr]
+        int* start = order + NGr + 1;                                  // [NGr + 1] first step
+        V* cur = reinterpret_cast<V*>(cptr + ((N4 + 4 + 2 * (NGr + 1) + 3) & ~3));
+        for (int k = tid; k < N4; k += blockDim.x) {
+            const float cp = a.caps[(size_t)rs * NP + k];
+            capr[k].v = L::all(cp);
+            capr[k].nr = L::all(-(1.0f / cp));
+        }
+        for (int k = tid; k <= N4; k += blockDim.x) cptr[k] = gptr[k];
+        for (int q = tid; q < (N4 + 1) * kLanes; q += blockDim.x) {    // row N4 stays zero
+            const int k = q / kLanes;
+            cur[q] = L::all(k < N ? ip[k] : 0.0f);
+        }
+        if (tid < 2) s_grab[tid] = 0;
+        __syncthreads();
+        // the groups in descending order of entries (ties: lower group first)
+        for (int gq = tid; gq < NGr; gq += blockDim.x) {
+            const int w = cptr[4 * gq + 4] - cptr[4 * gq];
+            int rank = 0;
+            for (int u = 0; u < NGr; ++u) {
+                const int wu = cptr[4 * u + 4] - cptr[4 * u];
+                rank += (wu > w) || (wu == w && u < gq);
+            }
+            order[rank] = gq;
+        }
+        if (warp == W - 1) {                   // the groups' first steps, 32 groups a scan
+            int base = 0;
+            for (int g0 = 0; g0 < NGr; g0 += 32) {
+                const int gq = g0 + lane;
+                int n = 0;
+                if (gq < NGr)
+                    for (int j = 0; j < 4; ++j) n = max(n, cptr[4 * gq + j + 1] - cptr[4 * gq + j]);
+                n = (n + 1) >> 1;
+                int x = n;
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int y = __shfl_up_sync(0xffffffffu, x, o);
+                    if (lane >= o) x += y;
+                }
+                if (gq < NGr) start[gq] = base + x - n;
+                base += __shfl_sync(0xffffffffu, x, 31);
+            }
+            if (lane == 0) start[NGr] = s_steps = base;
+        }
+        __syncthreads();
+        const int list = s_steps;
+        bool two = true, near = true;
+        if (mte_bytes(N4, list, true, L::paths) > (size_t)smem) {
+            two = !far_ok;
+            near = far_ok && mte_bytes(N4, list, false, L::paths) <= (size_t)smem;
+        }
+        V* nxt = two ? cur + (size_t)(N4 + 1) * kLanes : cur;
+        V* far = reinterpret_cast<V*>(a.far_buf) + (size_t)blockIdx.x * a.npe * kLanes;
+        int4* ent = reinterpret_cast<int4*>(nxt + (size_t)(N4 + 1) * kLanes);
+        if (two)
+            for (int q = tid; q < kLanes; q += blockDim.x) nxt[(size_t)N4 * kLanes + q] = L::all(0.0f);
+        if (near)
+            for (int gq = warp; gq < NGr; gq += W) {
+                const int s0 = start[gq], n8 = (start[gq + 1] - s0) * 8;
+                int2* en = reinterpret_cast<int2*>(ent + (size_t)s0 * 4);
+                for (int q = lane; q < n8; q += 32) {  // [step][destination][2]
+                    const int j = (q >> 1) & 3, e = cptr[4 * gq + j] + 2 * (q >> 3) + (q & 1);
+                    en[q] = e < cptr[4 * gq + j + 1]
+                                ? make_int2(gidx[e] * kLanes * (int)sizeof(V), __float_as_int(gval[e]))
+                                : make_int2(N4 * kLanes * (int)sizeof(V), 0);
+                }
+            }
+        const float s5 = sp[5] * sp[5];
+        // a species without jumps: their indicator is 0 and their factor
+        // finite, so that their term is 0 whatever is drawn
+        const bool jumps = sp[6] > 0.0f || !(fabsf(sp[5]) <= 1.0f);
+        const V s7 = L::all(sp[7]), one = L::all(1.0f), mone = L::all(-1.0f);
+        float gmean = sp[0];                           // of path `tid` of the tile (tid < PW)
+        V z[4];                                        // normals of the group worked on
+        auto normals = [&](int grp) {
+            lp.normals(to_stream_group((uint32_t)((s * N4) >> 2) + grp, stream_road, rk), rk, s_tab, z);
+        };
+        for (int t = 0; t < Y; ++t) {
+            if (t % kGmChunk == 0) {
+                // the next years' growth-mean draws, one thread each
+                const int nc = min(kGmChunk, Y - t);
+                for (int q = tid; q < nc * 3 * PW; q += blockDim.x) {
+                    const int yy = q / (3 * PW), r = q - yy * 3 * PW;
+                    const int which = r / PW, i = r - which * PW;
+                    const uint32_t pth = (uint32_t)(path0 - lane + i);
+                    const int ty = t + yy;
+                    float v = 0.0f;
+                    if (which == 1) {
+                        v = to_normal1(a.seed, TO_STREAM_SP_BROWNIAN, road_id, pth, ty, s) * sp[2];
+                    } else if (jumps) {
+                        if (which == 0) {
+                            v = (to_uniform1(a.seed, TO_STREAM_SP_JUMP, road_id, pth, ty, s) < sp[6])
+                                    ? 1.0f : 0.0f;
+                        } else {
+                            const float zj =
+                                to_normal1(a.seed, TO_STREAM_SP_JUMPSIZE, road_id, pth, ty, s);
+                            const float jsz =
+                                (a.sem == 0) ? (zj * s5 - s5 / 2.0f) : (zj * sp[5] - s5 / 2.0f);
+                            v = to_expf(jsz) - 1.0f;
+                        }
+                    }
+                    xs[q] = v;
+                }
+                __syncthreads();
+                // the growth means do not depend on the populations: the
+                // years' recursion, a thread a path
+                if (tid < PW)
+#pragma unroll 4
+                    for (int yy = 0; yy < nc; ++yy) {
+                        float* x = xs + yy * 3 * PW + tid;
+                        gmean = gmean + sp[4] * (sp[1] - gmean) * a.dt + gmean * x[PW] +
+                                x[2 * PW] * gmean * x[0];
+                        x[0] = gmean;
+                    }
+                __syncthreads();
+            }
+            const V g = L::load(xs + (t % kGmChunk) * 3 * PW + lane);
+            const unsigned char* curb = reinterpret_cast<const unsigned char*>(cur + lane);
+            V* dst = (two ? nxt : far) + lane;
+            const bool migrated = a.sem == 0 && t == Y - 1;    // what the end population sums
+            if (t == 0) {
+                lp.year(0u, rk);
+                if (warp < NGr) normals(order[warp]);
+            }
+            // a group a warp, the rest from the counter
+            int* gc = s_grab + (t & 1);
+            for (int i = warp; i < NGr;) {
+                const int grp = order[i];
+                if (i != warp) normals(grp);
+                V q[4] = {};                           // migrated
+                if (near) {
+                    const int4* en = ent + (size_t)start[grp] * 4;
+                    for (const int4* e1 = ent + (size_t)start[grp + 1] * 4; en < e1; en += 4) {
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            const int4 e = en[j];
+                            q[j] = L::fma(*reinterpret_cast<const V*>(curb + e.x),
+                                          L::all(__int_as_float(e.y)), q[j]);
+                            q[j] = L::fma(*reinterpret_cast<const V*>(curb + e.z),
+                                          L::all(__int_as_float(e.w)), q[j]);
+                        }
+                    }
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        for (int e = cptr[grp * 4 + j]; e < cptr[grp * 4 + j + 1]; ++e)
+                            q[j] = L::fma(cur[gidx[e] * kLanes + lane], L::all(gval[e]), q[j]);
+                }
+                if (migrated)
+                    dst[(size_t)grp * 4 * kLanes] = L::add(L::add(L::add(q[0], q[1]), q[2]), q[3]);
+                else
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const int k = grp * 4 + j;
+                        const V gr = L::fma(L::mul(s7, z[j]), g, g);
+                        // (gr (cap - q)) / cap as to_div_rcp, with minus the
+                        // reciprocal: minus the quotient, the same bits
+                        const typename L::cap cr = capr[k];
+                        const V x = L::mul(gr, L::fma(q[j], mone, cr.v));
+                        const V nq = L::mul(x, cr.nr);
+                        const V nd = L::fma(L::fma(nq, cr.v, x), cr.nr, nq);
+                        dst[k * kLanes] = L::mul(q[j], L::fma(nd, mone, one));
+                    }
+                if (lane == 0) i = atomicAdd(gc, 1);
+                i = __shfl_sync(0xffffffffu, i, 0) + W;
+            }
+            // last used in the year before the last barrier
+            if (tid == 0) s_grab[(t + 1) & 1] = 0;
+            // done: while the others finish, the normals of next year's own group
+            __syncwarp();
+            if (lane == 0) to_mbar::arrive(&s_bar);
+            if (t + 1 < Y) {
+                lp.year((uint32_t)(t + 1), rk);
+                if (warp < NGr) normals(order[warp]);
+            }
+            if (!to_mbar::wait(&s_bar, phase)) {
+                if (a.flags) atomicExch(a.flags, TO_DEVERR_SPIN);
+                return;
+            }
+            phase ^= 1u;
+            if (two) {
+                V* tmp = cur;
+                cur = nxt;
+                nxt = tmp;
+            } else {
+#pragma unroll 4
+                for (int q = tid; q < N4 * kLanes; q += blockDim.x) cur[q] = far[q];
+                __syncthreads();
+            }
+        }
+        if (warp == 0) {
+            const bool migrated = a.sem == 0 && Y > 0;
+            V tt = L::all(0.0f);
+#pragma unroll 4
+            for (int grp = 0; grp < NGr; ++grp) {
+                const V* v = cur + (size_t)grp * 4 * kLanes + lane;
+                tt = L::add(tt, migrated ? v[0]
+                                         : L::add(L::add(L::add(v[0], v[kLanes]), v[2 * kLanes]),
+                                                  v[3 * kLanes]));
+            }
+            L::store(a.end_pops + (size_t)rs * P + path0, P - path0, tt);
+        }
         __syncthreads();
     }
 }
@@ -1220,22 +1369,15 @@ to_status pack_csc(to_ctx ctx, const float* mmm, int NP, int C, const int* n_pat
     return TO_OK;
 }
 
-// paths per lane of the MTE kernel: two when the tile fits (every non-zero
-// read then serves two paths), else one
-static int mte_ppl(int NE, int cap_smem, size_t smem_cap);
-
-size_t mte_sparse_smem_ppl(int NE, int cap_smem, int ppl) {
-    const int maxg = ppl == 1 ? kMaxG : 3;      // 32 warps of maxg groups of four
-    if (NE > 32 * maxg * 4) return ~size_t(0);
-    const int NG = NE / 4, PW = kLanes * ppl;
-    return (size_t)cap_smem * 8 + (size_t)(NE * PW + NG * PW + 2 * NE + kGmChunk * 3 * PW) * 4 +
+size_t mte_sparse_smem(int NE, int cap_smem) {
+    if (NE > 32 * kMaxG * 4) return ~size_t(0);  // 32 warps of kMaxG groups of four
+    const int NG = NE / 4;
+    return (size_t)cap_smem * 8 + (size_t)(NE * kLanes + NG * kLanes + 2 * NE + kGmChunk * 3 * kLanes) * 4 +
            (size_t)(NE + 1 + NG) * 4 + 16;
 }
 
-size_t mte_sparse_smem(int NE, int cap_smem) { return mte_sparse_smem_ppl(NE, cap_smem, 1); }
-
-static int mte_ppl(int NE, int cap_smem, size_t smem_cap) {
-    return mte_sparse_smem_ppl(NE, cap_smem, 2) <= smem_cap ? 2 : 1;
+size_t mte_far_count(to_ctx ctx, int NP) {
+    return (size_t)ctx->sm_count * (NP < 32 * kMaxG * 4 ? NP : 32 * kMaxG * 4) * kLanes;
 }
 
 // warps per CTA: enough that no warp owns more than kMaxG groups of four
@@ -1251,36 +1393,45 @@ static int warps_for(int NE, int min_warps) {
 to_status mte_sparse(to_ctx ctx, to_mte_args a, int n_rs, to_csc csc) {
     if (a.npe <= 0) a.npe = a.npad;
     if (!a.flags) a.flags = ctx->d_flags;
-    const int NE = a.npe;
+    const int NE = a.npe, NE4 = (NE + 3) & ~3;
     if (csc.cap_smem & 1)       // the 8-byte entries must leave the column pointers 16-byte aligned
         return to_set_error(ctx, TO_ERR_INVALID, "packed capacity %d is odd", csc.cap_smem);
-    const int ppl = (a.n_paths > kLanes) ? mte_ppl(NE, csc.cap_smem, ctx->smem_optin) : 1;
-    size_t smem = mte_sparse_smem_ppl(NE, csc.cap_smem, ppl);
+    size_t smem = mte_sparse_smem(NE, csc.cap_smem);
     if (smem > ctx->smem_optin)
         return to_set_error(ctx, TO_ERR_UNSUPPORTED, "sparse MTE needs %zu B", smem);
-    int warps = warps_for(NE, 4);
-    if ((NE / 4 + warps - 1) / warps > kMaxG)
-        return to_set_error(ctx, TO_ERR_UNSUPPORTED, "patches %d", NE);
-    const int PW = kLanes * ppl;
-    dim3 grid((a.n_paths + PW - 1) / PW, n_rs);
-    if (a.order_buf && n_rs > 1) {
+    if (n_rs > 1) {
         k_mte_order<<<1, 1024, 0, ctx->stream>>>(n_rs, a.rs0, a.C, a.c_use, csc.nnz, a.order_buf);
         TO_LAUNCHED(ctx);
         a.order = a.order_buf;
     }
+    const size_t limit = ctx->smem_optin - kPairStatic;
+    // One path a lane where two would use at most half the SMs (200 patches,
+    // 1,000 paths, 2 species: 0.43 against 0.53 ms a call; with 94 tiles of
+    // 64 paths on 152 SMs 0.43 against 0.39).
+    const int pairs = (a.n_paths + 2 * kLanes - 1) / (2 * kLanes) * n_rs;
+    const int paths = a.n_paths <= kLanes || 2 * pairs <= ctx->sm_count ? 1 : 2;
+    const int items = (a.n_paths + paths * kLanes - 1) / (paths * kLanes) * n_rs;
+    // Up to four CTAs an SM, of 32 warps together, where there are tiles for
+    // them and their lists and both buffers fit: few groups leave many warps
+    // of a wide CTA idle, and one CTA's barrier hides behind another's work
+    // (40,000 paths, 2 species of 20 / 40 / 115 patches, one CTA an SM: 1.23
+    // / 1.34 / 2.18 ms a call, four (115: two): 0.73 / 1.00 / 1.93; eight no
+    // better).  The lists' padding is taken as half their entries here; a
+    // model whose lists need more reads them from global memory.
+    int c = (items + ctx->sm_count - 1) / ctx->sm_count;
+    if (c > 4) c = 4;
+    auto share = [&](int n) { return n == 1 ? limit : (limit + 1024) / n - 1024 - kPairStatic; };
+    while (c > 1 && mte_bytes(NE4, csc.cap_smem * 3 / 16 + 8, true, paths) > share(c)) --c;
+    const size_t each = share(c);
+    int W = 32 / c < NE4 / 4 ? 32 / c : NE4 / 4;
+    if (W < 2) W = 2;
+    const int ctas = c * ctx->sm_count;
+    const auto kern = paths == 2 ? k_mte_sparse<f2> : k_mte_sparse<float>;
+    TO_CUDA(ctx, cudaMemsetAsync(a.order_buf + n_rs, 0, sizeof(int), ctx->stream));
+    TO_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)each));
     to_prof_begin(ctx, "mte_sparse");
-    if (ppl == 2) {
-        // 32 warps of at most three groups (NE <= 384): a shorter chain of
-        // groups per warp between the year's barriers than 24 warps of four,
-        // and within 64 registers a thread
-        TO_CUDA(ctx, cudaFuncSetAttribute(k_mte_sparse<3, 2>,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k_mte_sparse<3, 2><<<grid, 1024, smem, ctx->stream>>>(a, csc);
-    } else {
-        TO_CUDA(ctx, cudaFuncSetAttribute(k_mte_sparse<kMaxG, 1>,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k_mte_sparse<kMaxG, 1><<<grid, warps * 32, smem, ctx->stream>>>(a, csc);
-    }
+    kern<<<items < ctas ? items : ctas, W * 32, each, ctx->stream>>>(
+        a, csc, to_make_round_keys(a.seed), n_rs, (int)each, c == 1);
     to_prof_end(ctx);
     TO_LAUNCHED(ctx);
     return TO_OK;

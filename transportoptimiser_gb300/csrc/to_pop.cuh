@@ -1,5 +1,6 @@
 // to_pop.cuh - argument blocks of the population Monte Carlo kernels.
 #pragma once
+#include "to_f2.cuh"
 #include "to_internal.cuh"
 
 struct to_mte_args {
@@ -20,8 +21,9 @@ struct to_mte_args {
     float* end_pops;             // [RS][P]
     int* flags;                  // device error word (plan checks), may be null
     const int* order;            // [n_rs] launch order of the (road, species), or null
-    int* order_buf;              // scratch for it ([n_rs] ints), or null: the
-                                 // sparse launcher then orders widest first
+    int* order_buf;              // scratch of the sparse kernels: that order, widest
+                                 // first, and a work counter ([n_rs + 1])
+    f2* far_buf;                 // scratch of the sparse kernels ([mte_far_count])
     int fault_wait;              // test hook (to_ctx_inject_fault): the tensor-core
                                  // kernel's first wait, on a barrier nothing arrives
                                  // at, runs out at once

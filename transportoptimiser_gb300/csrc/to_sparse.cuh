@@ -30,6 +30,8 @@ namespace to_k {
 to_status pack_csc(to_ctx ctx, const float* mmm, int NP, int C, const int* n_patches,
                    int n_rs, to_csc& csc, int rs0 = 0);
 size_t mte_sparse_smem(int NE, int cap_smem);
+// pairs of floats in to_mte_args::far_buf for patch arrays of stride NP
+size_t mte_far_count(to_ctx ctx, int NP);
 size_t rov_sparse_smem(int NE, int C, int cap_smem);
 // the union form of every (road, species)'s C <= 3 packed matrices
 to_status union_csc(to_ctx ctx, int NP, int C, const int* n_patches, int n_rs, to_csc& csc);
