@@ -408,13 +408,26 @@ to_status to_species_model(to_ctx ctx, const to_species_in* in,
     hs.lambda_mean = in->lambda_mean; hs.lambda_sd = in->lambda_sd;
     hs.lambda_mult = in->lambda_mult; hs.hab_pref_mult = in->hab_pref_mult;
     size_t n = (size_t)W * H;
-    size_t bytes = to_align256(n * 4) * 2 + to_align256(sizeof(hs)) +
-                   to_align256((size_t)(in->G > 0 ? in->G : 1) * 32) + 256 * 4 +
+    // habitable types, first appearance: labelled a CTA each (none where the
+    // patch pass on them does not fit the blocks: one CTA then labels type
+    // by type)
+    int types[TO_MAX_HAB], T = 0;
+    const bool by_type = ((size_t)TO_MAX_HAB * a.xres * a.yres + NM + 65) * sizeof(int) <= ctx->smem_optin;
+    for (int h = 0; h < in->n_hab && by_type; ++h) {
+        const int t = in->habs[h].type;
+        if (t == 3 || t == 4) continue;
+        bool seen = false;
+        for (int q = 0; q < T; ++q) seen |= types[q] == t;
+        if (!seen) types[T++] = t;
+    }
+    const size_t nn = (size_t)NM * NM;
+    size_t bytes = to_align256(n * 4) * 2 + to_align256(sizeof(hs)) + to_align256(T * n * 4) +
+                   to_align256((size_t)(in->G > 0 ? in->G : 1) * 32) + 256 * 5 +
                    to_align256((size_t)NM * 8) * 5 + to_align256((size_t)NM * 4) +
-                   to_align256((size_t)NM * NM * 4) * 2 +
-                   to_align256((size_t)NM * NM * 8) * 2 +
-                   to_align256((size_t)NM * NM * 2) +
-                   to_align256((size_t)C * NM * NM * 8) +
+                   to_align256(nn * 4) + to_align256(nn * 8) + to_align256(nn * 2) +
+                   (out->trans ? to_align256(nn * 8) : 0) +
+                   (out->surv ? to_align256((size_t)C * nn * 8) : 0) +
+                   (out->mmm ? to_align256((size_t)C * nn * 4) : 0) +
                    to_align256((size_t)C * NP * NP * 4) + to_align256((size_t)NP * 4) * 2 +
                    to_align256((size_t)C * 8) + 4096;
     TO_TRY(to_arena_reserve(ctx, bytes));
@@ -432,11 +445,13 @@ to_status to_species_model(to_ctx ctx, const to_species_in* in,
     a.cy = to_arena_take<double>(ctx, NM);
     a.type = to_arena_take<int>(ctx, NM);
     a.crossings_scratch = to_arena_take<int>(ctx, (size_t)NM * NM);
-    a.crossings_out = to_arena_take<int>(ctx, (size_t)NM * NM);
     a.trans_scratch = to_arena_take<double>(ctx, (size_t)NM * NM);
     a.trans_dest = to_arena_take<uint16_t>(ctx, (size_t)NM * NM);
-    a.trans = to_arena_take<double>(ctx, (size_t)NM * NM);
-    a.surv = to_arena_take<double>(ctx, (size_t)C * NM * NM);
+    a.trans = out->trans ? to_arena_take<double>(ctx, nn) : nullptr;
+    a.surv = out->surv ? to_arena_take<double>(ctx, (size_t)C * nn) : nullptr;
+    float* d_mm = out->mmm ? to_arena_take<float>(ctx, (size_t)C * nn) : nullptr;
+    int* d_types = to_arena_take<int>(ctx, TO_MAX_HAB);
+    a.labels = to_arena_take<int>(ctx, T * n);
     a.mmm = to_arena_take<float>(ctx, (size_t)C * NP * NP);
     a.init_pops = to_arena_take<float>(ctx, NP);
     a.caps = to_arena_take<float>(ctx, NP);
@@ -457,7 +472,14 @@ to_status to_species_model(to_ctx ctx, const to_species_in* in,
     a.hab_map = d_hab; a.cell_off = nullptr; a.cells = nullptr; a.pop_map = d_pop;
     a.species = d_sp; a.segs = d_road; a.seg_off = d_G;
     a.n_patches = d_np; a.n_transitions = d_nt; a.d_flags = ctx->d_flags;
+    if (T > 0) TO_TRY(h2d(ctx, d_types, types, T));
+    a.n_label_types = T;
+    a.label_types = d_types;
+    a.zeroed = true;
+    TO_CUDA(ctx, cudaMemsetAsync(a.mmm, 0, (size_t)C * NP * NP * sizeof(float), ctx->stream));
+    if (a.trans) TO_CUDA(ctx, cudaMemsetAsync(a.trans, 0, nn * sizeof(double), ctx->stream));
     TO_TRY(to_k::species_model(ctx, a, 1));
+    TO_TRY(to_k::species_dense(ctx, a, d_mm));
     int N = 0, nt = 0;
     TO_TRY(d2h(ctx, &N, d_np, 1));
     TO_TRY(d2h(ctx, &nt, d_nt, 1));
@@ -471,24 +493,13 @@ to_status to_species_model(to_ctx ctx, const to_species_in* in,
     TO_TRY(d2h(ctx, out->cx, a.cx, N));
     TO_TRY(d2h(ctx, out->cy, a.cy, N));
     TO_TRY(d2h(ctx, out->type, a.type, N));
-    std::vector<int> cr;
-    std::vector<double> tr, sv;
-    std::vector<float> mm;
-    if (out->crossings) { cr.resize((size_t)NM * NM); TO_TRY(d2h(ctx, cr.data(), a.crossings_out, cr.size())); }
-    if (out->trans) { tr.resize((size_t)NM * NM); TO_TRY(d2h(ctx, tr.data(), a.trans, tr.size())); }
-    if (out->surv) { sv.resize((size_t)C * NM * NM); TO_TRY(d2h(ctx, sv.data(), a.surv, sv.size())); }
-    if (out->mmm) { mm.resize((size_t)C * NP * NP); TO_TRY(d2h(ctx, mm.data(), a.mmm, mm.size())); }
+    const size_t NN = (size_t)N * N;
+    if (out->crossings) TO_TRY(d2h(ctx, out->crossings, a.crossings_scratch, NN));
+    if (out->trans) TO_TRY(d2h(ctx, out->trans, a.trans, NN));
+    if (out->surv) TO_TRY(d2h(ctx, out->surv, a.surv, C * NN));
+    if (out->mmm) TO_TRY(d2h(ctx, out->mmm, d_mm, C * NN));
     if (out->iar) TO_TRY(d2h(ctx, out->iar, a.iar, (size_t)C));
     TO_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    for (int i = 0; i < N; ++i)
-        for (int j = 0; j < N; ++j) {
-            if (out->crossings) out->crossings[(size_t)i * N + j] = cr[(size_t)i * NM + j];
-            if (out->trans) out->trans[(size_t)i * N + j] = tr[(size_t)i * NM + j];
-            for (int c = 0; c < C; ++c) {
-                if (out->surv) out->surv[((size_t)c * N + i) * N + j] = sv[((size_t)c * NM + i) * NM + j];
-                if (out->mmm) out->mmm[((size_t)c * N + i) * N + j] = mm[((size_t)c * NP + i) * NP + j];
-            }
-        }
     return TO_OK;
 }
 

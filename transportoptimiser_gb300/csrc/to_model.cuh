@@ -37,12 +37,12 @@ struct to_model_args {
     double *area, *cap, *pop, *cx, *cy;   // [RS][NM]
     int* type;                   // [RS][NM]
     int* crossings_scratch;      // [RS][NM*NM] (N*N packed)
-    int* crossings_out;          // optional [RS][NM][NM]
     double* trans_scratch;       // [RS][NM][NM]
     uint16_t* trans_dest;        // [RS][NM][NM] in-range destinations per origin row
-    double* trans;               // optional [RS][NM][NM]
-    double* surv;                // optional [RS][C][NM][NM]
+    double* trans;               // optional, one road: [N][N], zeroed by the caller
+    double* surv;                // optional, one road: [C][N][N] (species_dense)
     float* mmm;                  // [RS][C][NP][NP] destination-major
+    bool zeroed;                 // the caller zeroed mmm
     // csc_ptr non-null: the migration matrices go straight into the packed
     // form (what k_pack_csc makes of the dense ones) and the dense [C][NP][NP]
     // block of each (road, species) is only scratch, never zeroed
@@ -65,4 +65,7 @@ struct to_model_args {
 
 namespace to_k {
 to_status species_model(to_ctx ctx, const to_model_args& a, int n_rs);
+// after it, one road's survival probabilities (a.surv) and its migration
+// matrices without their padding ([C][N][N])
+to_status species_dense(to_ctx ctx, const to_model_args& a, float* mm);
 }

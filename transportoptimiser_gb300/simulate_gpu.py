@@ -104,8 +104,9 @@ def createSpeciesModel(hab_map, pop_map, W, H, res, habitats, road_colmajor, G, 
     Cn = len(hz)
     b = dict(area=np.zeros(NM), cap=np.zeros(NM), pop=np.zeros(NM), cx=np.zeros(NM),
              cy=np.zeros(NM), type=np.zeros(NM, np.int32))
-    big = dict(crossings=np.zeros(NM * NM, np.int32), trans=np.zeros(NM * NM),
-               surv=np.zeros(Cn * NM * NM), mmm=np.zeros(Cn * NM * NM, np.float32))
+    # room for max_patches; only the N patches' entries are ever touched
+    big = dict(crossings=np.empty(NM * NM, np.int32), trans=np.empty(NM * NM),
+               surv=np.empty(Cn * NM * NM), mmm=np.empty(Cn * NM * NM, np.float32))
     out = _capi.SpeciesOut()
     out.max_patches = NM
     for k in ("area", "cap", "pop", "cx", "cy"):
@@ -123,10 +124,10 @@ def createSpeciesModel(hab_map, pop_map, W, H, res, habitats, road_colmajor, G, 
     res_ = {k: v[:N].copy() for k, v in b.items()}
     res_["N"] = N
     res_["n_transitions"] = out.n_transitions
-    res_["crossings"] = big["crossings"][:N * N].reshape(N, N).copy()
-    res_["trans"] = big["trans"][:N * N].reshape(N, N).copy()
-    res_["surv"] = big["surv"][:Cn * N * N].reshape(Cn, N, N).copy()
-    res_["mmm"] = big["mmm"][:Cn * N * N].reshape(Cn, N, N).copy()
+    res_["crossings"] = big["crossings"][:N * N].reshape(N, N)
+    res_["trans"] = big["trans"][:N * N].reshape(N, N)
+    res_["surv"] = big["surv"][:Cn * N * N].reshape(Cn, N, N)
+    res_["mmm"] = big["mmm"][:Cn * N * N].reshape(Cn, N, N)
     res_["init_pops"] = res_["pop"].astype(np.float32)
     res_["caps"] = res_["cap"].astype(np.float32)
     res_["iar"] = iar
