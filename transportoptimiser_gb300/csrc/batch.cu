@@ -294,10 +294,25 @@ to_status tail(to_ctx ctx, to_gen g, const to_mte_args& m, int RS, int choice,
 
 // Autotuner: time each feasible migration kernel once on this generation
 // (CUDA events on the context stream) and keep the fastest for the shape.
+uint64_t tune_key(const to_mte_args& m, int RS, int NE, bool sparse_ok) {
+    return mix(mix(mix(mix(0, 0), (uint64_t)NE), (uint64_t)m.n_paths),
+               mix((uint64_t)RS, (uint64_t)m.n_years * 2 + (sparse_ok ? 1 : 0)));
+}
+
+// the sparse kernel taken without a trial
+void tuned_record(to_ctx ctx, const to_mte_args& m, int RS, int NE) {
+    to_ctx_s::tune_entry te;
+    te.key = mix(tune_key(m, RS, NE, true), 1);      // not a trial's
+    for (const auto& e : ctx->tune)
+        if (e.key == te.key) return;
+    te.kind = 0; te.ne = NE; te.paths = m.n_paths; te.n_rs = RS; te.choice = CH_SPARSE;
+    te.ms[0] = te.ms[1] = te.ms[2] = -1.0f;
+    ctx->tune.push_back(te);
+}
+
 to_status tuned_choice(to_ctx ctx, to_gen g, const to_mte_args& m, int RS, int NE,
                        bool sparse_ok, bool tc_ok, int* choice) {
-    const uint64_t key = mix(mix(mix(mix(0, 0), (uint64_t)NE), (uint64_t)m.n_paths),
-                             mix((uint64_t)RS, (uint64_t)m.n_years * 2 + (sparse_ok ? 1 : 0)));
+    const uint64_t key = tune_key(m, RS, NE, sparse_ok);
     for (const auto& e : ctx->tune)
         if (e.key == key && e.kind == 0) { *choice = e.choice; return TO_OK; }
     to_ctx_s::tune_entry te;
@@ -344,21 +359,20 @@ to_status evaluate_direct(to_ctx ctx, to_gen g, int R, const int* cell_off,
     }
     to_model_args a;
     model_args(g, R, cell_off, cells, seg_off, segs, o, ctx, a);
-    // sparse migration asked for: the model kernel writes the packed
-    // matrices itself (the tuner's dense candidates need the dense form)
-    // (the ROV stage reads the packed matrices of every control, so a scene
-    // with a ROV always takes them from the model and runs the sparse kernel)
-    const bool packed = (o->migration == TO_MIG_SPARSE_FP32) || g->rov_on;
-    if (packed) csc_direct(g, a);
+    // The model kernel writes the packed matrices itself wherever the sparse
+    // kernel may run.  The dense form is made only if a dense kernel is asked
+    // for or has to be timed (the ROV stage reads the packed matrices of
+    // every control, so a scene with a ROV always runs the sparse kernel).
+    const bool try_sparse = (o->migration == TO_MIG_AUTO || o->migration == TO_MIG_SPARSE_FP32 ||
+                             g->rov_on);
+    bool dense = !try_sparse;
+    if (try_sparse) csc_direct(g, a);
     TO_TRY(to_k::species_model(ctx, a, RS));
     // the widest species model decides the tile shape of the path kernel
     int* d_max = reinterpret_cast<int*>(g->d_results + (size_t)g->max_roads * S * TO_RESULT_STRIDE);
     k_max_int<<<1, 1024, 0, ctx->stream>>>(RS, g->d_np, d_max);
     TO_LAUNCHED(ctx);
-    const bool try_sparse = (o->migration == TO_MIG_AUTO || o->migration == TO_MIG_SPARSE_FP32 ||
-                             g->rov_on);
     if (try_sparse) {
-        if (!packed) TO_TRY(to_k::pack_csc(ctx, g->d_mmm, NP, g->C, g->d_np, RS, g->csc));
         k_min_max_int<<<1, 1024, 0, ctx->stream>>>(RS * g->C, g->csc.nnz, d_max + 1);
         TO_LAUNCHED(ctx);
     }
@@ -385,11 +399,23 @@ to_status evaluate_direct(to_ctx ctx, to_gen g, int R, const int* cell_off,
     if (o->migration == TO_MIG_SPARSE_FP32 || g->rov_on) choice = CH_SPARSE;
     else if (o->migration == TO_MIG_TC_3XTF32) choice = CH_TC;
     else if (o->migration == TO_MIG_SIMT_FP32) choice = CH_SIMT;
-    else TO_TRY(tuned_choice(ctx, g, m, RS, NE, sparse_ok, NE <= 512, &choice));
+    else if (sparse_ok && (long)mm[2] * 10 <= (long)NE * NE) {
+        // No trial where no matrix has a tenth of its entries: the sparse
+        // kernel's time grows with the entries, the dense kernels' does not
+        // (256 roads at 2.5%: 2.6 against 30.6 ms; they meet above 20%), and
+        // the trial would take a hundred milliseconds and the dense matrices.
+        choice = CH_SPARSE;
+        tuned_record(ctx, m, RS, NE);
+    } else {
+        a.csc_ptr = nullptr;
+        TO_TRY(to_k::species_model(ctx, a, RS));
+        dense = true;
+        TO_TRY(tuned_choice(ctx, g, m, RS, NE, sparse_ok, NE <= 512, &choice));
+    }
     TO_TRY(tail(ctx, g, m, RS, choice, d_results_out));
     if (plan) { plan[0] = NE; plan[1] = g->csc.cap_smem; plan[2] = choice; }
     g->last_R = R; g->last_paths = o->mte_paths;
-    g->last_dense = !packed; g->last_csc = try_sparse;
+    g->last_dense = dense; g->last_csc = try_sparse;
     return TO_OK;
 }
 

@@ -571,10 +571,11 @@ k_species_patches_lab(to_model_args a) {
 // CTAs share an SM and the FP64-bound transition rows of one overlap the
 // integer work of the other.
 __global__ void __launch_bounds__(512, 2)
-k_species_links(to_model_args a) {
+k_species_links(to_model_args a, int rows) {     // rows of s_sum
     extern __shared__ __align__(16) unsigned char sml[];
     __shared__ int s_last, s_cnt, s_npair;
     __shared__ int s_tmp[33];
+    __shared__ double s_init;
     const int rs = a.rs0 + blockIdx.x;
     const int road = rs / a.S, sp = rs - road * a.S;
     const to_model_species& S = a.species[sp];
@@ -605,8 +606,8 @@ k_species_links(to_model_args a) {
     float* sgf = cyf + NM;                                      // [4][SC]
     double* s_attr = reinterpret_cast<double*>(sgf + 4 * SC);   // [TO_MAX_HAB]
     double* s_surv = s_attr + TO_MAX_HAB;                       // [C][SC+1]
-    double* s_sum = s_surv + a.C * (SC + 1);                    // [NM] row sums
-    int* s_off = reinterpret_cast<int*>(s_sum + NM);            // [NM+1] row offsets
+    double* s_sum = s_surv + a.C * (SC + 1);                    // [rows][NM] row sums
+    int* s_off = reinterpret_cast<int*>(s_sum + (size_t)rows * NM); // [NM+1] row offsets
     const double lda = S.lambda_mult * S.lambda_sd + S.lambda_mean;
     for (int k = threadIdx.x; k < N; k += blockDim.x) { cxf[k] = (float)cx[k]; cyf[k] = (float)cy[k]; }
     if (seg_tab)
@@ -830,24 +831,34 @@ k_species_links(to_model_args a) {
         // computeAAR / computeInitialAAR, SpeciesRoadPatches.cpp:453-490):
         // 1 - sum_i pop_i sum_j trans(i,j) surv_c(i,j) / sum_i pop_i, each
         // row over its listed destinations ascending, rows ascending
-        __syncthreads();
-        for (int c = 0; c < a.C; ++c) {
-            for (int i = threadIdx.x; i < N; i += blockDim.x) {
+        // The rows of as many controls as there is room for at once, then a
+        // warp a control adds up: the sums are chains of FP64 additions, slow
+        // ones on this part.
+        if (warp == nwarp - 1 && lane == 0) {
+            double init = 0.0;
+#pragma unroll 8
+            for (int i = 0; i < N; ++i) init += popd[i];
+            s_init = init;
+        }
+        for (int c0 = 0; c0 < a.C; c0 += rows) {
+            const int nc = min(rows, a.C - c0);
+            __syncthreads();
+            for (int q = threadIdx.x; q < nc * N; q += blockDim.x) {
+                const int c = q / N, i = q - c * N;
                 const double* rowv = wv + (size_t)i * NM;
                 const uint16_t* rowj = dj + (size_t)i * NM;
                 const int n = s_off[i + 1] - s_off[i];
                 double acc = 0.0;
-                for (int q = 0; q < n; ++q)
-                    acc += rowv[q] * surv_of(c, cross[(size_t)i * N + rowj[q]]);
-                s_sum[i] = popd[i] * acc;
+                for (int k = 0; k < n; ++k)
+                    acc += rowv[k] * surv_of(c0 + c, cross[(size_t)i * N + rowj[k]]);
+                s_sum[c * NM + i] = popd[i] * acc;
             }
             __syncthreads();
-            if (threadIdx.x == 0) {
-                double tot = 0.0, init = 0.0;
-                for (int i = 0; i < N; ++i) { tot += s_sum[i]; init += popd[i]; }
-                a.iar[(size_t)rs * a.C + c] = 1.0 - tot / init;
+            if (warp < nc && lane == 0) {
+                double tot = 0.0;
+                for (int i = 0; i < N; ++i) tot += s_sum[warp * NM + i];
+                a.iar[(size_t)rs * a.C + c0 + warp] = 1.0 - tot / s_init;
             }
-            __syncthreads();
         }
     }
     if (direct) {
@@ -990,11 +1001,14 @@ to_status species_model(to_ctx ctx, const to_model_args& a, int n_rs) {
     TO_CUDA(ctx, cudaFuncSetAttribute(k_species_patches,
                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     // links: float centroids, segment and survival tables
-    const size_t smem2 = (size_t)2 * a.max_patches * sizeof(float) +
+    int rows = 0;
+    size_t smem2 = (size_t)2 * a.max_patches * sizeof(float) +
                          (size_t)4 * TO_SURV_TABLE_SEGS * sizeof(float) +
                          (size_t)(TO_MAX_HAB + a.C * (TO_SURV_TABLE_SEGS + 1)) * sizeof(double) +
-                         (size_t)a.max_patches * sizeof(double) +
-                         (size_t)(a.max_patches + 1) * sizeof(int);
+                   (size_t)(a.max_patches + 1) * sizeof(int);
+    // row sums of every control where two CTAs an SM still fit
+    do smem2 += (size_t)a.max_patches * sizeof(double);
+    while (++rows < (a.iar ? a.C : 1) && smem2 + a.max_patches * sizeof(double) <= 100 * 1024);
     if (smem2 > ctx->smem_optin || a.max_patches > 65535)
         return to_set_error(ctx, TO_ERR_UNSUPPORTED, "%d patches exceed shared memory",
                             a.max_patches);
@@ -1028,7 +1042,7 @@ to_status species_model(to_ctx ctx, const to_model_args& a, int n_rs) {
         TO_LAUNCHED(ctx);
     }
     to_prof_begin(ctx, "species_links");
-    k_species_links<<<n_rs, 512, smem2, ctx->stream>>>(a);
+    k_species_links<<<n_rs, 512, smem2, ctx->stream>>>(a, rows);
     to_prof_end(ctx);
     TO_LAUNCHED(ctx);
     return TO_OK;
