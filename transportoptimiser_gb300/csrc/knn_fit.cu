@@ -461,7 +461,8 @@ __device__ __forceinline__ PairArgs<D> pair_args(const to_rov_args& a, int slot,
     return c;
 }
 
-// the group's points and their values into shared memory [D + 1][np]
+// the group's points and their values into shared memory [D + 1][np]; all but
+// the values, the year before's result, ahead of the wait for that year
 template <int D>
 __device__ __forceinline__ void load_points(const to_rov_args& a, int slot, int t, int g, int np,
                                             float* pts) {
@@ -474,8 +475,12 @@ __device__ __forceinline__ void load_points(const to_rov_args& a, int slot, int 
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
 #pragma unroll
         for (int j = 0; j < D; ++j) pts[j * np + i] = xs[(size_t)j * P + i];
-        pts[D * np + i] = ynext[path[i]];
+        pts[D * np + i] = __int_as_float(path[i]);
     }
+    to_pdl_wait();
+#pragma unroll 4
+    for (int i = threadIdx.x; i < n; i += blockDim.x)
+        pts[D * np + i] = ynext[__float_as_int(pts[D * np + i])];
 }
 
 // shared memory of the fit: a tile's neighbour lists and, of groups small
@@ -498,6 +503,8 @@ __global__ void __launch_bounds__(kT, 4) k_knn_fit(to_rov_args a, int t) {
     float* pts = reinterpret_cast<float*>(sm_fit + (size_t)a.kmax * kT * 2);   // [D + 1][np]
     const int ntiles = a.ntiles[slot], tcap = a.G * ((Q + kT - 1) / kT);
     const int2* tiles = a.tiles + (size_t)slot * tcap;
+    to_pdl_next();
+    if (blockIdx.x >= ntiles) to_pdl_wait();
     for (int ti = blockIdx.x; ti < ntiles; ti += gridDim.x) {
         const int g = tiles[ti].x, start = tiles[ti].y;
         const size_t gs = (size_t)slot * a.G + g;
@@ -507,6 +514,7 @@ __global__ void __launch_bounds__(kT, 4) k_knn_fit(to_rov_args a, int t) {
         const int qi = a.touched ? a.qlist[gs * Q + at] : at;
         float* out = to_rov_reg_block(a, t, g) + (size_t)a.R * D;
         if (n < 3 || k <= 0) {                 // too few points
+            to_pdl_wait();
             if (live) out[qi] = 0.0f;
             continue;
         }
@@ -519,6 +527,7 @@ __global__ void __launch_bounds__(kT, 4) k_knn_fit(to_rov_args a, int t) {
             for (int i = tid; i < k * (kT / 8); i += kT) dst[i] = src[i];
         }
         if (n <= np) load_points<D>(a, slot, t, g, np, pts);
+        else to_pdl_wait();
         __syncthreads();
         if (!live) continue;
         PairArgs<D> pc = pair_args<D>(a, slot, t, g, qi, a.kthv[tg * kT + tid]);
@@ -570,17 +579,23 @@ __global__ void __launch_bounds__(kWide) k_knn_fit_wide(to_rov_args a, int t) {
     unsigned short* lists = reinterpret_cast<unsigned short*>(pts + (D + 1) * np);  // [kmax][kW]
     const int nsub = a.ntiles[slot] * SUB, tcap = a.G * ((Q + kT - 1) / kT);
     const int2* tiles = a.tiles + (size_t)slot * tcap;
+    to_pdl_next();
+    if (blockIdx.x >= nsub) to_pdl_wait();
     for (int si = blockIdx.x; si < nsub; si += gridDim.x) {
         const int ti = si / SUB, q0 = si % SUB * kW;
         const int g = tiles[ti].x, start = tiles[ti].y + q0;
         const size_t gs = (size_t)slot * a.G + g;
         const int n = a.npts[gs], k = a.kc[gs], cnt = a.gcount[gs] - start;
-        if (cnt <= 0) continue;
+        if (cnt <= 0) {
+            to_pdl_wait();
+            continue;
+        }
         const bool live = lane < cnt;
         const int at = live ? start + lane : start;
         const int qi = a.touched ? a.qlist[gs * Q + at] : at;
         float* out = to_rov_reg_block(a, t, g) + (size_t)a.R * D;
         if (n < 3 || k <= 0) {                 // too few points
+            to_pdl_wait();
             if (live && warp == 0) out[qi] = 0.0f;
             continue;
         }
@@ -590,6 +605,7 @@ __global__ void __launch_bounds__(kWide) k_knn_fit_wide(to_rov_args a, int t) {
             reinterpret_cast<uint4*>(lists)[i] = reinterpret_cast<const uint4*>(
                 a.nbr + (tg * a.kmax + (i >> 2)) * kT + q0)[i & 3];
         if (n <= np) load_points<D>(a, slot, t, g, np, pts);
+        else to_pdl_wait();
         __syncthreads();
         PairArgs<D> pc = pair_args<D>(a, slot, t, g, qi, live ? a.kthv[tg * kT + q0 + lane] : 1.0f);
         pc.nb = lists + lane;
@@ -653,7 +669,8 @@ to_status launch_fit(to_ctx ctx, const to_rov_args& a, int t) {
     TO_CUDA(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     to_prof_begin(ctx, "knn_solve");
     const int units = wide ? tiles * (kT / kW) : tiles;
-    k<<<units < 16 * sms ? units : 16 * sms, wide ? kWide : kT, smem, ctx->stream>>>(a, t);
+    TO_CUDA(ctx, to_pdl_launch(k, units < 16 * sms ? units : 16 * sms, wide ? kWide : kT, smem,
+                               ctx->stream, a, t));
     to_prof_end(ctx);
     TO_LAUNCHED(ctx);
     return TO_OK;
