@@ -239,8 +239,10 @@ class TransOptError(RuntimeError):
 def ptr(a: np.ndarray | None, ctype):
     if a is None:
         return None
-    assert a.flags["C_CONTIGUOUS"], "array must be C-contiguous"
-    return a.ctypes.data_as(C.POINTER(ctype))
+    assert a.flags.c_contiguous, "array must be C-contiguous"
+    p = C.cast(a.ctypes.data, C.POINTER(ctype))
+    p._arr = a                  # the pointer keeps its array
+    return p
 
 
 class Context:

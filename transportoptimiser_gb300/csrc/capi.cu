@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "to_grid.h"
+#include "to_host.h"
 #include "to_internal.cuh"
 #include "to_model.cuh"
 #include "to_pop.cuh"
@@ -528,7 +529,8 @@ to_status to_simulate_mte(to_ctx ctx, const to_mte_problem* prob,
     }
     if (maxN > 1020) return to_set_error(ctx, TO_ERR_UNSUPPORTED, "%d patches", maxN);
     const int NP = (maxN + 3) & ~3;
-    std::vector<float> mmm((size_t)S * NP * NP, 0.0f), ip((size_t)S * NP, 0.0f),
+    const size_t n_mmm = (size_t)S * NP * NP;
+    std::vector<float> ip((size_t)S * NP, 0.0f),
         cp((size_t)S * NP, 1.0f), prm((size_t)S * 8);
     std::vector<int> np(S);
     for (int s = 0; s < S; ++s) {
@@ -538,13 +540,11 @@ to_status to_simulate_mte(to_ctx ctx, const to_mte_problem* prob,
         for (int k = 0; k < N; ++k) {
             ip[(size_t)s * NP + k] = sp.init_pops[k];
             cp[(size_t)s * NP + k] = sp.caps[k];
-            for (int l = 0; l < N; ++l)
-                mmm[((size_t)s * NP + k) * NP + l] = sp.mmm[(size_t)k * N + l];
         }
         for (int q = 0; q < 8; ++q) prm[(size_t)s * 8 + q] = sp.params[q];
     }
     const int cap = NP * 64 < NP * NP ? NP * 64 : NP * NP;
-    size_t bytes = to_align256(mmm.size() * 4) + 2 * to_align256(ip.size() * 4) +
+    size_t bytes = to_align256(n_mmm * 4) + 2 * to_align256(ip.size() * 4) +
                    to_align256(prm.size() * 4) + to_align256((size_t)S * 4) +
                    to_align256((size_t)S * P * 4) + to_align256((size_t)S * 5 * 8) +
                    to_align256((size_t)S * (NP + 1) * 4) + to_align256((size_t)S * cap * 2) +
@@ -554,7 +554,7 @@ to_status to_simulate_mte(to_ctx ctx, const to_mte_problem* prob,
     TO_TRY(to_arena_reserve(ctx, bytes));
     to_mte_args a;
     memset(&a, 0, sizeof(a));
-    float* d_mmm = to_arena_take<float>(ctx, mmm.size());
+    float* d_mmm = to_arena_take<float>(ctx, n_mmm);
     float* d_ip = to_arena_take<float>(ctx, ip.size());
     float* d_cp = to_arena_take<float>(ctx, cp.size());
     float* d_prm = to_arena_take<float>(ctx, prm.size());
@@ -570,7 +570,9 @@ to_status to_simulate_mte(to_ctx ctx, const to_mte_problem* prob,
     csc.cap_smem = 0;
     a.order_buf = to_arena_take<int>(ctx, (size_t)S + 1);
     a.far_buf = to_arena_take<f2>(ctx, to_k::mte_far_count(ctx, NP));
-    TO_TRY(h2d(ctx, d_mmm, mmm.data(), mmm.size()));
+    TO_TRY(to_upload_matrices(ctx, d_mmm, S, NP, [=](size_t s) {
+        return std::make_pair(prob->species[s].mmm, prob->species[s].n_patches);
+    }));
     TO_TRY(h2d(ctx, d_ip, ip.data(), ip.size()));
     TO_TRY(h2d(ctx, d_cp, cp.data(), cp.size()));
     TO_TRY(h2d(ctx, d_prm, prm.data(), prm.size()));
@@ -602,15 +604,12 @@ to_status to_simulate_mte(to_ctx ctx, const to_mte_problem* prob,
         TO_TRY(to_k::mte_simt(ctx, a, S));
     }
     TO_TRY(to_k::mte_stats(ctx, a, S, d_stats));
-    std::vector<float> ef((size_t)S * P);
     std::vector<double> st((size_t)S * 5);
-    TO_TRY(d2h(ctx, ef.data(), d_end, ef.size()));
+    TO_TRY(to_download_parts(ctx, d_end, 1, 1, (size_t)S * P, [=](size_t) { return end_pops; }));
     TO_TRY(d2h(ctx, st.data(), d_stats, st.size()));
     TO_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     // a bounded wait that ran out (tensor-core kernel) or a plan check
     TO_TRY(to_check_device_flags(ctx));
-    if (end_pops)
-        for (size_t i = 0; i < ef.size(); ++i) end_pops[i] = (double)ef[i];
     if (stats)
         for (int s = 0; s < S; ++s) {
             stats[s].mean = st[5 * s];

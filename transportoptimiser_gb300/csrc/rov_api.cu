@@ -4,6 +4,7 @@
 #include <cstring>
 #include <vector>
 
+#include "to_host.h"
 #include "to_internal.cuh"
 #include "to_rov.cuh"
 #include "to_sparse.cuh"
@@ -113,7 +114,7 @@ to_status to_simulate_rov_batch(to_ctx ctx, int n_roads, const to_rov_problem* p
         if (!std::isfinite(pr->uncert[i])) return to_set_error(ctx, TO_ERR_NONFINITE, "uncert %d", i);
     const int NP = (maxN + 3) & ~3;
     if (NP > 1020) return to_set_error(ctx, TO_ERR_UNSUPPORTED, "%d patches", maxN);
-    std::vector<float> mmm((size_t)RS * C * NP * NP, 0.0f), ip((size_t)RS * NP, 0.0f),
+    std::vector<float> ip((size_t)RS * NP, 0.0f),
         cp((size_t)RS * NP, 1.0f), prm((size_t)S * 8);
     std::vector<int> np(RS), rid(NR);
     for (int r = 0; r < NR; ++r) {
@@ -124,21 +125,17 @@ to_status to_simulate_rov_batch(to_ctx ctx, int n_roads, const to_rov_problem* p
             int N = sp.n_patches;
             np[rs] = N;
             for (int k = 0; k < N; ++k) { ip[rs * NP + k] = sp.init_pops[k]; cp[rs * NP + k] = sp.caps[k]; }
-            for (int c = 0; c < C; ++c)
-                for (int k = 0; k < N; ++k)
-                    for (int l = 0; l < N; ++l)
-                        mmm[((rs * C + c) * NP + k) * NP + l] = sp.mmm[((size_t)c * N + k) * N + l];
         }
     }
     for (int s = 0; s < S; ++s)
         for (int q = 0; q < 8; ++q) prm[(size_t)s * 8 + q] = pr->species[s].params[q];
     const int kmax = k_rule(P) > 0 ? k_rule(P) : 1;
     if (kmax > TO_KNN_KMAX) return to_set_error(ctx, TO_ERR_UNSUPPORTED, "k %d", kmax);
-    const size_t blk = (size_t)R * d + 2 * (size_t)Q;
+    const size_t blk = (size_t)R * d + 2 * (size_t)Q, n_mmm = (size_t)RS * C * NP * NP;
     const int cap = NP * 64 < NP * NP ? NP * 64 : NP * NP;
     size_t bytes = 0;
     auto acc = [&](size_t b) { bytes += to_align256(b); };
-    acc(mmm.size() * 4); acc(ip.size() * 4); acc(cp.size() * 4); acc(prm.size() * 4); acc(RS * 4);
+    acc(n_mmm * 4); acc(ip.size() * 4); acc(cp.size() * 4); acc(prm.size() * 4); acc(RS * 4);
     acc(NR * 4);
     acc(C * 4); acc(6 * (size_t)(U > 0 ? U : 1) * 4); acc(16 * 4); acc(16 * 4); acc(16 * 4); acc(16 * 4);
     acc((size_t)Y * PT * 4); acc((size_t)(U > 0 ? U : 1) * (Y + 1) * PT * 4);
@@ -178,7 +175,7 @@ to_status to_simulate_rov_batch(to_ctx ctx, int n_roads, const to_rov_problem* p
     const size_t lsm = to_k::rov_scratch(a, NR, nullptr);
     acc(lsm);
     TO_TRY(to_arena_reserve(ctx, bytes + 4096));
-    float* d_mmm = to_arena_take<float>(ctx, mmm.size());
+    float* d_mmm = to_arena_take<float>(ctx, n_mmm);
     float* d_ip = to_arena_take<float>(ctx, ip.size());
     float* d_cp = to_arena_take<float>(ctx, cp.size());
     float* d_prm = to_arena_take<float>(ctx, prm.size());
@@ -230,7 +227,11 @@ to_status to_simulate_rov_batch(to_ctx ctx, int n_roads, const to_rov_problem* p
         a.gmY = to_arena_take<float>(ctx, (size_t)Y * S * P);
     }
     if (!csc.nnz || (algo == 6 && !a.gmY)) return to_set_error(ctx, TO_ERR_ALLOC, "arena sizing");
-    TO_TRY(up(ctx, d_mmm, mmm.data(), mmm.size()));
+    TO_TRY(to_upload_matrices(ctx, d_mmm, (size_t)RS * C, NP, [=](size_t i) {
+        const size_t rs = i / C, c = i % C;
+        const to_rov_species& sp = prs[rs / S].species[rs % S];
+        return std::make_pair(sp.mmm + c * sp.n_patches * sp.n_patches, sp.n_patches);
+    }));
     TO_TRY(up(ctx, d_ip, ip.data(), ip.size()));
     TO_TRY(up(ctx, d_cp, cp.data(), cp.size()));
     TO_TRY(up(ctx, d_prm, prm.data(), prm.size()));
@@ -282,58 +283,16 @@ to_status to_simulate_rov_batch(to_ctx ctx, int n_roads, const to_rov_problem* p
     TO_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     TO_TRY(to_check_device_flags(ctx));
     // road-major device arrays -> each road's [Y][P] (or [Y][S][P]) output
-    std::vector<float> f;
-    std::vector<int> iv;
-    auto fetch_rows = [&](int which, const float* dptr, size_t rows) -> to_status {
-        bool any = false;
-        for (int r = 0; r < NR; ++r) {
-            double* o = which == 0 ? results[r].cond_exp
-                      : which == 1 ? results[r].unit_profits : results[r].adj_pops;
-            any |= o != nullptr;
-        }
-        if (!any) return TO_OK;
-        f.resize(rows * PT);
-        TO_TRY(down(ctx, f.data(), dptr, rows * PT));
-        TO_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-        for (int r = 0; r < NR; ++r) {
-            double* o = which == 0 ? results[r].cond_exp
-                      : which == 1 ? results[r].unit_profits : results[r].adj_pops;
-            if (!o) continue;
-            for (size_t row = 0; row < rows; ++row)
-                for (int p = 0; p < P; ++p)
-                    o[row * P + p] = (double)f[row * PT + (size_t)r * P + p];
-        }
-        return TO_OK;
-    };
-    TO_TRY(fetch_rows(0, a.condExp, (size_t)Y));
-    TO_TRY(fetch_rows(1, a.unitProfits, (size_t)Y));
-    if (want_adj) TO_TRY(fetch_rows(2, a.adjPops, (size_t)Y * S));
-    bool want_oc = false;
-    for (int r = 0; r < NR; ++r) want_oc |= results[r].opt_cont != nullptr;
-    if (want_reg) {
-        f.resize((size_t)Y * G * blk);
-        TO_TRY(down(ctx, f.data(), a.reg, (size_t)Y * G * blk));
-        TO_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-        for (int r = 0; r < NR; ++r) {
-            double* o = results[r].regression;
-            if (!o) continue;
-            for (int t = 0; t < Y; ++t)
-                for (size_t q = 0; q < (size_t)C * blk; ++q)
-                    o[((size_t)t * C) * blk + q] = (double)f[((size_t)t * G + (size_t)r * C) * blk + q];
-        }
-    }
-    if (want_oc) {
-        iv.resize((size_t)Y * PT);
-        TO_TRY(down(ctx, iv.data(), a.optCont, (size_t)Y * PT));
-        TO_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-        for (int r = 0; r < NR; ++r) {
-            int* o = results[r].opt_cont;
-            if (!o) continue;
-            for (int t = 0; t < Y; ++t)
-                for (int p = 0; p < P; ++p) o[(size_t)t * P + p] = iv[(size_t)t * PT + (size_t)r * P + p];
-        }
-    }
-    TO_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    TO_TRY(to_download_parts(ctx, a.condExp, Y, NR, P, [=](size_t r) { return results[r].cond_exp; }));
+    TO_TRY(to_download_parts(ctx, a.unitProfits, Y, NR, P,
+                             [=](size_t r) { return results[r].unit_profits; }));
+    if (want_adj)
+        TO_TRY(to_download_parts(ctx, a.adjPops, (size_t)Y * S, NR, P,
+                                 [=](size_t r) { return results[r].adj_pops; }));
+    if (want_reg)
+        TO_TRY(to_download_parts(ctx, a.reg, Y, NR, C * blk,
+                                 [=](size_t r) { return results[r].regression; }));
+    TO_TRY(to_download_parts(ctx, a.optCont, Y, NR, P, [=](size_t r) { return results[r].opt_cont; }));
     for (int r = 0; r < NR; ++r) {
         const double* sr = st.data() + 5 * (size_t)r;
         results[r].value = sr[0];

@@ -154,7 +154,7 @@ def simulateMTECUDA(species_models, params, n_paths, n_years, dt=1.0, seed=0, ro
         sps[s] = _capi.MteSpecies(int(m["N"]), ptr(prm, C.c_float), ptr(ip, C.c_float),
                                   ptr(cp, C.c_float), ptr(mm, C.c_float))
     prob = _capi.MteProblem(S, n_paths, n_years, dt, seed, road, sem, migration, sps)
-    end = np.zeros(S * n_paths, np.float64)
+    end = np.empty(S * n_paths, np.float64)
     st = (_capi.MteStats * S)()
     ctx.check(ctx.lib.to_simulate_mte(ctx.handle, C.byref(prob), ptr(end, C.c_double), st),
               "to_simulate_mte")
@@ -222,11 +222,11 @@ def simulateROVCUDA(problem: dict, want=("cond_exp", "opt_cont", "unit_profits",
     pr, keep = rov_ctypes(problem, migration)
     d = S + 1
     out = {}
-    if "cond_exp" in want: out["cond_exp"] = np.zeros(Y * P)
-    if "opt_cont" in want: out["opt_cont"] = np.zeros(Y * P, np.int32)
-    if "unit_profits" in want: out["unit_profits"] = np.zeros(Y * P)
-    if "adj_pops" in want: out["adj_pops"] = np.zeros(Y * S * P)
-    if "regression" in want: out["regression"] = np.zeros(Y * Cn * (R * d + 2 * R ** d))
+    if "cond_exp" in want: out["cond_exp"] = np.empty(Y * P)
+    if "opt_cont" in want: out["opt_cont"] = np.empty(Y * P, np.int32)
+    if "unit_profits" in want: out["unit_profits"] = np.empty(Y * P)
+    if "adj_pops" in want: out["adj_pops"] = np.empty(Y * S * P)
+    if "regression" in want: out["regression"] = np.empty(Y * Cn * (R * d + 2 * R ** d))
     r = _capi.RovResult()
     r.cond_exp = ptr(out.get("cond_exp"), C.c_double)
     r.opt_cont = ptr(out.get("opt_cont"), C.c_int)
@@ -260,11 +260,11 @@ def simulateROVCUDA_batch(problems, want=("cond_exp", "opt_cont", "regression"),
         prs[i] = pr
         d = S + 1
         out = {}
-        if "cond_exp" in want: out["cond_exp"] = np.zeros(Y * P)
-        if "opt_cont" in want: out["opt_cont"] = np.zeros(Y * P, np.int32)
-        if "unit_profits" in want: out["unit_profits"] = np.zeros(Y * P)
-        if "adj_pops" in want: out["adj_pops"] = np.zeros(Y * S * P)
-        if "regression" in want: out["regression"] = np.zeros(Y * Cn * (R * d + 2 * R ** d))
+        if "cond_exp" in want: out["cond_exp"] = np.empty(Y * P)
+        if "opt_cont" in want: out["opt_cont"] = np.empty(Y * P, np.int32)
+        if "unit_profits" in want: out["unit_profits"] = np.empty(Y * P)
+        if "adj_pops" in want: out["adj_pops"] = np.empty(Y * S * P)
+        if "regression" in want: out["regression"] = np.empty(Y * Cn * (R * d + 2 * R ** d))
         r = ress[i]
         r.cond_exp = ptr(out.get("cond_exp"), C.c_double)
         r.opt_cont = ptr(out.get("opt_cont"), C.c_int)
