@@ -636,9 +636,7 @@ __global__ void __launch_bounds__(128) k_rov_backward(to_rov_args a, int t) {
             const int c = c0 + u < C ? c0 + u : C - 1;
             const float cur = a.flows[c] * prof;
             const float v = to_lsm_interp(to_rov_reg_block(a, t, (size_t)r * C + c), R, S, st[u], prof);
-            double ce = (double)(v / disc);
-            if (ce > 0.0) ce = 0.0;
-            pay[u] = (float)((double)cur + ce);
+            pay[u] = to_rovd::payoff(cur, v / disc);
         }
 #pragma unroll
         for (int u = 0; u < CU; ++u)

@@ -82,6 +82,14 @@ __device__ __forceinline__ void decide_terminal(const to_rov_args& a, const floa
     }
 }
 
+// A control's payoff: this year's plus the discounted value, capped at zero.
+// Summed in FP32: the reference's sum in double rounded to float is the same
+// value, since 53 bits are two more than twice 24 (S. Figueroa, "When is
+// double rounding innocuous?", 1995), and FP64 is slow on this part.
+__device__ __forceinline__ float payoff(float now, float later) {
+    return now + (later > 0.0f ? 0.0f : later);
+}
+
 // Interior-year decision (backwardInduction :2464-2776): current payoff plus
 // the discounted regression value of year t (capped at zero), least wins;
 // road r's regressions.
@@ -101,9 +109,7 @@ __device__ __forceinline__ void decide_interior(const to_rov_args& a, int t, int
             const float* rb = to_rov_reg_block(a, t, (size_t)r * C + c);
             float v = (a.sem == 0) ? to_lsm_interp_ref(rb, R, S, C, state)
                                    : to_lsm_interp(rb, R, S, state + c * S, state[S * C]);
-            double ce = (double)(v / disc);
-            if (ce > 0.0) ce = 0.0;
-            pay = (float)((double)cur + ce);
+            pay = payoff(cur, v / disc);
         }
         if (c == 0) { best = pay; continue; }
         if (!valid) continue;
