@@ -1065,7 +1065,7 @@ k_rov_forward_sparse(to_rov_args a, to_csc csc) {
 
 // ---------------------------------------------------------------------------
 // ALGO6 path re-simulation (optimalForwardPaths :1199-2206, as its comments
-// describe it).  Grid ceil(P/32): a CTA re-simulates 32 paths (lane = path)
+// describe it).  A CTA re-simulates a tile of 32 or 16 paths (lane = path)
 // from year t0 to the horizon with every species together, since each
 // year's control depends on all species' states.  A warp owns groups of four
 // patches; a year has three barriers:
@@ -1082,69 +1082,79 @@ k_rov_forward_sparse(to_rov_args a, to_csc csc) {
 // The year-t0 value replaces condExp[t0] and the year-t0 control optCont[t0].
 //
 // Bound by latency: the years of a restart follow one another, the restarts
-// too, and ceil(P/32) CTAs seldom fill the GPU.  So the lists are the union
+// too, and the tiles seldom fill the GPU.  So the lists are the union
 // ones where they fit (a loop for all controls, its loads in flight
 // together), the payoffs are a warp's each with everything unrolled, and the
 // profits come from the table the regressions use.  2,000 paths, 2 species of
 // 61 patches, 50 years: 24 -> 7.2 us a year of a restart (five barriers, a
 // loop for every control, one warp deciding and drawing the ore's noise again
-// before).
+// before), then 4.6: what a year runs through exceeded the instruction cache,
+// so one layout is one kernel, one group's normals wait instead of four (8.1
+// against 9.7 ms a valuation) and nothing divides by a run-time count; half a
+// warp a group spreads 2,000 paths over 125 SMs instead of 63.  The lists
+// side by side, or the next year's regressions fetched ahead, cost more in
+// code than they hid (8.1 -> 8.6 ms).
 // ---------------------------------------------------------------------------
-constexpr int kResimHeld = 4;              // groups of a warp whose normals wait in registers
 
 // shared memory: bytes of the lists, [S] reciprocals and groups' sums beside
 // what every layout has
-__host__ __device__ inline size_t resim_bytes(int NE, int S, int C, size_t lists, bool sums) {
-    const size_t rows = (size_t)S * (C + 1) * NE * kLanes * 4;
-    return rows + (size_t)S * NE * 4 + (size_t)C * kLanes * 4 + lists +
-           (sums ? (size_t)S * NE * 4 + (size_t)S * (C + 1) * (NE >> 2) * kLanes * 4 : 0);
+__host__ __device__ inline size_t resim_bytes(int NE, int S, int C, size_t lists, bool sums, int tp) {
+    const size_t rows = (size_t)S * (C + 1) * NE * tp * 4;
+    return rows + (size_t)S * NE * 4 + (size_t)C * tp * 4 + lists +
+           (sums ? (size_t)S * NE * 4 + (size_t)S * (C + 1) * (NE >> 2) * tp * 4 : 0);
 }
 __host__ __device__ inline size_t resim_lists(int NE, int S, int C, int cap_smem) {
     return (size_t)S * C * ((NE + 1) * 4 + (size_t)cap_smem * 6) + 16;
 }
 
-template <int S>
+// TP paths a tile: 32, a warp a group, or 16, half a warp a group ("warp"
+// below).  UNI: union lists, the groups' sums and the tables of the normals
+// all fit; the other layouts are a kernel of their own, since what the years
+// run through has to stay in the instruction cache.
+template <int S, int TP, bool UNI>
 __global__ void __launch_bounds__(1024, 1)
 k_rov_resim(to_rov_args a, to_csc csc, int t0, int smem) {
     extern __shared__ __align__(16) unsigned char sm_raw[];
     const int NE = a.ne, NG = NE >> 2, NP = a.np, C = a.C, Y = a.Y, P = a.P, R = a.R;
     const int SC = S * C;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, W = blockDim.x >> 5;
-    const int path = blockIdx.x * kLanes + lane;
+    const int tid = threadIdx.x, lane = tid % TP, warp = tid / TP, W = blockDim.x / TP;
+    const int path = blockIdx.x * TP + lane;
     const bool live = path < P;
-    // the layout: union lists and the groups' sums where they fit, then the
-    // controls' own lists with the sums, then without
+    // the layout: union lists and the groups' sums, or the controls' own
+    // lists, with the sums where they fit
     int nu = 0;
-    bool uni = csc.uent != nullptr;
-    for (int s = 0; s < S && uni; ++s) {
-        nu += csc.unnz[s];
-        if (csc.unnz[s] < 0) uni = false;
-    }
-    const size_t ulists = (size_t)nu * 16 + (size_t)S * (NE + 1) * 4;
+    if (UNI)
+        for (int s = 0; s < S; ++s) nu += csc.unnz[s];
     const size_t clists = resim_lists(NE, S, C, csc.cap_smem);
-    uni = uni && resim_bytes(NE, S, C, ulists, true) <= (size_t)smem;
-    const bool sums = uni || resim_bytes(NE, S, C, clists, true) <= (size_t)smem;
+    constexpr bool uni = UNI;
+    const bool sums = UNI || resim_bytes(NE, S, C, clists, true, TP) <= (size_t)smem;
     unsigned char* at = sm_raw;
     auto take = [&](size_t bytes) { unsigned char* r = at; at += bytes; return r; };
     int4* ue = reinterpret_cast<int4*>(uni ? take((size_t)nu * 16) : at);      // [nu]
-    float* cur = reinterpret_cast<float*>(take((size_t)S * NE * kLanes * 4));  // [S][NE][32]
-    float* mig = reinterpret_cast<float*>(take((size_t)SC * NE * kLanes * 4)); // [S][C][NE][32]
-    float* pay = reinterpret_cast<float*>(take((size_t)C * kLanes * 4));       // [C][32]
+    float* cur = reinterpret_cast<float*>(take((size_t)S * NE * TP * 4));  // [S][NE][32]
+    float* mig = reinterpret_cast<float*>(take((size_t)SC * NE * TP * 4)); // [S][C][NE][32]
+    float* pay = reinterpret_cast<float*>(take((size_t)C * TP * 4));       // [C][32]
     float* capv = reinterpret_cast<float*>(take((size_t)S * NE * 4));          // [S][NE]
     float *rcap = nullptr, *msum = nullptr, *tsum = nullptr;
     if (sums) {
         rcap = reinterpret_cast<float*>(take((size_t)S * NE * 4));             // [S][NE] 1 / capacity
-        msum = reinterpret_cast<float*>(take((size_t)SC * NG * kLanes * 4));   // [S][C][NG][32]
-        tsum = reinterpret_cast<float*>(take((size_t)S * NG * kLanes * 4));    // [S][NG][32]
+        msum = reinterpret_cast<float*>(take((size_t)SC * NG * TP * 4));   // [S][C][NG][32]
+        tsum = reinterpret_cast<float*>(take((size_t)S * NG * TP * 4));    // [S][NG][32]
     }
     const int lists = uni ? S : SC;
     int* cptr = reinterpret_cast<int*>(take((size_t)lists * (NE + 1) * 4));    // [S] or [S][C], [NE + 1]
     float* cval = reinterpret_cast<float*>(uni ? at : take((size_t)SC * csc.cap_smem * 4));
     uint16_t* cidx = reinterpret_cast<uint16_t*>(at);                          // [S][C][cap_smem]
+    to_bm_tables* tab = nullptr;
+    if (UNI) {
+        at = sm_raw + (((size_t)(at - sm_raw) + 15) & ~(size_t)15);
+        tab = reinterpret_cast<to_bm_tables*>(take(sizeof(to_bm_tables)));
+        to_bm_load(*tab);
+    }
     const uint32_t stream_road = TO_STREAM_GROWTH | ((uint32_t)a.road << 8);
 
-    for (int q = tid; q < S * NE * kLanes; q += blockDim.x) {
-        const int sk = q >> 5, pth = blockIdx.x * kLanes + (q & (kLanes - 1));
+    for (int q = tid; q < S * NE * TP; q += blockDim.x) {
+        const int sk = q / TP, pth = blockIdx.x * TP + (q & (TP - 1));
         const int s = sk / NE, k = sk - s * NE;
         cur[q] = (pth < P) ? a.popsY[(((size_t)t0 * S + s) * NE + k) * P + pth] : 0.0f;
     }
@@ -1163,7 +1173,7 @@ k_rov_resim(to_rov_args a, to_csc csc, int t0, int smem) {
             for (int e = tid; e < n; e += blockDim.x) {
                 int4 v = csc.uent[(size_t)s * csc.ucap + e];
                 if (v.x == kNoOrigin) v.x = 0;      // its values are zero
-                v.x *= kLanes * (int)sizeof(float);
+                v.x *= TP * (int)sizeof(float);
                 ue[e0 + e] = v;
             }
             e0 += n;
@@ -1182,46 +1192,68 @@ k_rov_resim(to_rov_args a, to_csc csc, int t0, int smem) {
     __syncthreads();
     if (sums) {
         for (int q = warp; q < S * NG; q += W) {
-            const float* v = cur + (size_t)q * 4 * kLanes + lane;
-            tsum[q * kLanes + lane] = grouped4(v[0], v[kLanes], v[2 * kLanes], v[3 * kLanes]);
+            const float* v = cur + (size_t)q * 4 * TP + lane;
+            tsum[q * TP + lane] = grouped4(v[0], v[TP], v[2 * TP], v[3 * TP]);
         }
         __syncthreads();
     }
-    // total over the groups of rows [NE][32] (or of their sums [NG][32])
-    auto total = [&](const float* rows, const float* gsum) {
-        float tt = 0.0f;
+    // the warp's first group, whose normals and growth mean wait in registers
+    // (one only: code for more costs more than it hides)
+    const bool own = warp < S * NG;
+    const int spec = own ? warp / NG : 0;
+    to_path_stream ps;
+    to_stream_path(ps, (uint32_t)path);
+    // totals over the groups of every species before (ts) and after (tt)
+    // control c's migration: 2 S chains side by side
+    auto totals = [&](int c, float (&ts)[S], float (&tt)[S]) {
+#pragma unroll
+        for (int s = 0; s < S; ++s) ts[s] = tt[s] = 0.0f;
         if (sums) {
-#pragma unroll 8
-            for (int grp = 0; grp < NG; ++grp) tt = tt + gsum[grp * kLanes + lane];
-        } else {
 #pragma unroll 4
-            for (int grp = 0; grp < NG; ++grp) {
-                const float* v = rows + (size_t)grp * 4 * kLanes + lane;
-                tt = tt + grouped4(v[0], v[kLanes], v[2 * kLanes], v[3 * kLanes]);
-            }
+            for (int grp = 0; grp < NG; ++grp)
+#pragma unroll
+                for (int s = 0; s < S; ++s) {
+                    ts[s] = ts[s] + tsum[((size_t)s * NG + grp) * TP + lane];
+                    tt[s] = tt[s] + msum[((size_t)(s * C + c) * NG + grp) * TP + lane];
+                }
+        } else {
+            for (int grp = 0; grp < NG; ++grp)
+#pragma unroll
+                for (int s = 0; s < S; ++s) {
+                    const float* v = cur + ((size_t)s * NE + grp * 4) * TP + lane;
+                    ts[s] = ts[s] + grouped4(v[0], v[TP], v[2 * TP], v[3 * TP]);
+                    v = mig + ((size_t)(s * C + c) * NE + grp * 4) * TP + lane;
+                    tt[s] = tt[s] + grouped4(v[0], v[TP], v[2 * TP], v[3 * TP]);
+                }
         }
-        return tt;
     };
-    auto draw = [&](int u, int q, float (&z)[4]) {
-        const int s = q / NG, grp = q - s * NG, N4 = (a.n_patches[s] + 3) & ~3;
-        to_path_stream ps;
-        to_stream_path(ps, (uint32_t)path);
-        to_stream_year(ps, (uint32_t)u, a.rk);
+    auto draw = [&](int s, int q, float (&z)[4]) {
+        const int grp = q - s * NG, N4 = (a.n_patches[s] + 3) & ~3;
         const to_u32x4 w = to_stream_words(
             ps, to_stream_group((uint32_t)((s * N4) >> 2) + grp, stream_road, a.rk), a.rk);
-        to_box_muller(w.v[0], w.v[1], &z[0], &z[1]);
-        to_box_muller(w.v[2], w.v[3], &z[2], &z[3]);
+        if (UNI) {
+            f2 cs, sn;                             // of both Box-Muller pairs
+            to_box_muller2(w.v[0], w.v[1], w.v[2], w.v[3], *tab, cs, sn);
+            unpack2(cs, z[0], z[2]);
+            unpack2(sn, z[1], z[3]);
+        } else {
+            to_box_muller(w.v[0], w.v[1], &z[0], &z[1]);
+            to_box_muller(w.v[2], w.v[3], &z[2], &z[3]);
+        }
     };
     const float disc = 1.0f + a.rrr * a.dt / 100.0f;
     float val = 0.0f, df = 1.0f;        // warp 0: realised value, discount factor
     int first = 0;
     for (int u = t0; u < Y; ++u) {
         const bool last = u == Y - 1;
+        // what the year reads from global memory, requested ahead of its use
+        const float prof = live ? a.profS[(size_t)u * P + path] : 0.0f;
+        const float gm = live && own ? a.gmY[((size_t)u * S + spec) * P + path] : 0.0f;
         // A
-        for (int q = warp; q < S * NG; q += W) {
-            const int s = q / NG, grp = q - s * NG;
-            const float* cs = cur + (size_t)s * NE * kLanes + lane;
-            float* mg = mig + ((size_t)s * C * NE + grp * 4) * kLanes + lane;
+        for (int q = warp, i = 0; q < S * NG; q += W, ++i) {
+            const int s = i == 0 ? spec : q / NG, grp = q - s * NG;
+            const float* cs = cur + (size_t)s * NE * TP + lane;
+            float* mg = mig + ((size_t)s * C * NE + grp * 4) * TP + lane;
             if (uni) {
                 const int* up = cptr + s * (NE + 1) + grp * 4;
                 float g0 = 0.0f, g1 = 0.0f, g2 = 0.0f;
@@ -1241,17 +1273,17 @@ k_rov_resim(to_rov_args a, to_csc csc, int t0, int smem) {
                             q2 = fmaf(x, __int_as_float(en.w), q2);
                         }
                     }
-                    mg[j * kLanes] = q0;
-                    if (C > 1) mg[(size_t)(NE + j) * kLanes] = q1;
-                    if (C > 2) mg[(size_t)(2 * NE + j) * kLanes] = q2;
+                    mg[j * TP] = q0;
+                    if (C > 1) mg[(size_t)(NE + j) * TP] = q1;
+                    if (C > 2) mg[(size_t)(2 * NE + j) * TP] = q2;
                     g0 = j ? g0 + q0 : q0;
                     g1 = j ? g1 + q1 : q1;
                     g2 = j ? g2 + q2 : q2;
                 }
-                float* o = msum + ((size_t)s * C * NG + grp) * kLanes + lane;
+                float* o = msum + ((size_t)s * C * NG + grp) * TP + lane;
                 o[0] = g0;
-                if (C > 1) o[(size_t)NG * kLanes] = g1;
-                if (C > 2) o[(size_t)2 * NG * kLanes] = g2;
+                if (C > 1) o[(size_t)NG * TP] = g1;
+                if (C > 2) o[(size_t)2 * NG * TP] = g2;
             } else {
                 for (int c = 0; c < C; ++c) {
                     const int m = s * C + c;
@@ -1264,26 +1296,23 @@ k_rov_resim(to_rov_args a, to_csc csc, int t0, int smem) {
                         float acc = 0.0f;
 #pragma unroll 4
                         for (int e = cp[j]; e < cp[j + 1]; ++e)
-                            acc = fmaf(cs[(int)ci[e] * kLanes], cv[e], acc);
-                        mg[((size_t)c * NE + j) * kLanes] = acc;
+                            acc = fmaf(cs[(int)ci[e] * TP], cv[e], acc);
+                        mg[((size_t)c * NE + j) * TP] = acc;
                         gs = j ? gs + acc : acc;
                     }
-                    if (sums) msum[((size_t)m * NG + grp) * kLanes + lane] = gs;
+                    if (sums) msum[((size_t)m * NG + grp) * TP + lane] = gs;
                 }
             }
         }
         __syncthreads();
-        const float prof = live ? a.profS[(size_t)u * P + path] : 0.0f;
         // B
         for (int c = warp; c < C; c += W) {
-            float st[S];
+            float st[S], ts[S], tt[S];
             bool valid = true;
+            totals(c, ts, tt);
 #pragma unroll
             for (int s = 0; s < S; ++s) {
-                const int m = s * C + c;
-                const float ts = total(cur + (size_t)s * NE * kLanes, tsum + (size_t)s * NG * kLanes);
-                const float tt = total(mig + (size_t)m * NE * kLanes, msum + (size_t)m * NG * kLanes);
-                st[s] = ts * (tt / ts);
+                st[s] = ts[s] * (tt[s] / ts[s]);
                 if (st[s] < to_rovd::threshold(a, s) && c > 0) valid = false;
             }
             float r = INFINITY;                    // an invalid control's
@@ -1292,19 +1321,16 @@ k_rov_resim(to_rov_args a, to_csc csc, int t0, int smem) {
                 if (last) {
                     r = now > 0.0f ? 0.0f : now;
                 } else {
-                    const float v = to_lsm_interp(to_rov_reg_block(a, u, c), R, S, st, prof);
-                    double ce = (double)(v / disc);
-                    if (ce > 0.0) ce = 0.0;
-                    r = (float)((double)now + ce);
+                    r = to_rovd::payoff(
+                        now, to_lsm_interp(to_rov_reg_block(a, u, c), R, S, st, prof) / disc);
                 }
             }
-            pay[c * kLanes + lane] = r;
+            pay[c * TP + lane] = r;
         }
-        float z[kResimHeld][4];
-        if (!last) {
-#pragma unroll
-            for (int i = 0; i < kResimHeld; ++i)
-                if (warp + i * W < S * NG) draw(u, warp + i * W, z[i]);
+        float z[4];
+        if (!last && own) {
+            to_stream_year(ps, (uint32_t)u, a.rk);
+            draw(spec, warp, z);
         }
         __syncthreads();
         // C
@@ -1312,7 +1338,7 @@ k_rov_resim(to_rov_args a, to_csc csc, int t0, int smem) {
         {
             float best = pay[lane];
             for (int c = 1; c < C; ++c) {
-                const float r = pay[c * kLanes + lane];
+                const float r = pay[c * TP + lane];
                 if (r < best) { best = r; cu = c; }
             }
         }
@@ -1322,29 +1348,27 @@ k_rov_resim(to_rov_args a, to_csc csc, int t0, int smem) {
             df = df / disc;
         }
         if (last) break;
-        auto grow = [&](int q, const float (&zz)[4]) {
-            const int s = q / NG, grp = q - s * NG;
+        auto grow = [&](int s, int q, const float (&zz)[4], float g) {
+            const int grp = q - s * NG;
             const float s7 = a.params[8 * s + 7];
-            const float g = live ? a.gmY[((size_t)u * S + s) * P + path] : 0.0f;
-            const float* mg = mig + (((size_t)s * C + cu) * NE + grp * 4) * kLanes + lane;
-            float* o = cur + ((size_t)s * NE + grp * 4) * kLanes + lane;
+            const float* mg = mig + (((size_t)s * C + cu) * NE + grp * 4) * TP + lane;
+            float* o = cur + ((size_t)s * NE + grp * 4) * TP + lane;
             float v[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                const float mv = mg[j * kLanes], cpk = capv[s * NE + grp * 4 + j];
+                const float mv = mg[j * TP], cpk = capv[s * NE + grp * 4 + j];
                 const float gr = fmaf(s7 * zz[j], g, g), x = gr * (cpk - mv);
                 const float d = sums ? to_div_rcp(x, cpk, rcap[s * NE + grp * 4 + j]) : x / cpk;
                 v[j] = fmaxf(mv * (1.0f + d), 0.0f);
-                o[j * kLanes] = v[j];
+                o[j * TP] = v[j];
             }
-            if (sums) tsum[q * kLanes + lane] = grouped4(v[0], v[1], v[2], v[3]);
+            if (sums) tsum[q * TP + lane] = grouped4(v[0], v[1], v[2], v[3]);
         };
-#pragma unroll
-        for (int i = 0; i < kResimHeld; ++i)
-            if (warp + i * W < S * NG) grow(warp + i * W, z[i]);
-        for (int q = warp + kResimHeld * W; q < S * NG; q += W) {
-            draw(u, q, z[0]);
-            grow(q, z[0]);
+        if (own) grow(spec, warp, z, gm);
+        for (int q = warp + W; q < S * NG; q += W) {
+            const int s = q / NG;
+            draw(s, q, z);
+            grow(s, q, z, live ? a.gmY[((size_t)u * S + s) * P + path] : 0.0f);
         }
         __syncthreads();
     }
@@ -1496,14 +1520,30 @@ to_status rov_forward_sparse(to_ctx ctx, const to_rov_args& a, to_csc csc) {
 
 
 to_status rov_resim_sparse(to_ctx ctx, const to_rov_args& a, to_csc csc, int t0) {
-    // the smallest layout has to fit; the kernel takes the best one that does
-    const size_t least = resim_bytes(a.ne, a.S, a.C, resim_lists(a.ne, a.S, a.C, csc.cap_smem), false);
+    // the smallest layout has to fit
+    const size_t least =
+        resim_bytes(a.ne, a.S, a.C, resim_lists(a.ne, a.S, a.C, csc.cap_smem), false, kLanes);
     const size_t limit = ctx->smem_optin;
     if (least > limit)
         return to_set_error(ctx, TO_ERR_UNSUPPORTED, "ALGO6 re-simulation needs %zu B", least);
-    const auto kern = a.S == 1 ? k_rov_resim<1> : a.S == 2 ? k_rov_resim<2> : a.S == 3 ? k_rov_resim<3>
-                                                                                       : k_rov_resim<4>;
-    const int blocks = (a.P + kLanes - 1) / kLanes;
+    // Tiles of 16 paths while the SMs take them all at once (2 species of 61 /
+    // 130 patches, 1,999 / 1,000 paths: 9.7 / 13.4 ms a valuation against
+    // 10.2 / 16.2 in tiles of 32; 2,500 paths fill the SMs either way)
+    const int tp = (a.P + 15) / 16 <= ctx->sm_count ? 16 : 32;
+    const size_t ulists = (size_t)a.S * ((size_t)csc.ucap_smem * 16 + (size_t)(a.ne + 1) * 4);
+    const bool uni = csc.uent && resim_bytes(a.ne, a.S, a.C, ulists, true, tp) + 16 +
+                                         sizeof(to_bm_tables) <= limit;
+    using kern_t = void (*)(to_rov_args, to_csc, int, int);
+    const auto pick = [&](kern_t u16, kern_t u32, kern_t c16, kern_t c32) {
+        return tp == 16 ? (uni ? u16 : c16) : (uni ? u32 : c32);
+    };
+#define TO_RESIM(S) \
+    pick(k_rov_resim<S, 16, true>, k_rov_resim<S, 32, true>, k_rov_resim<S, 16, false>, \
+         k_rov_resim<S, 32, false>)
+    const kern_t kern = a.S == 1 ? TO_RESIM(1) : a.S == 2 ? TO_RESIM(2) : a.S == 3 ? TO_RESIM(3)
+                                                                                   : TO_RESIM(4);
+#undef TO_RESIM
+    const int blocks = (a.P + tp - 1) / tp;
     to_prof_begin(ctx, "rov_resim");
     TO_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit));
     kern<<<blocks, 1024, limit, ctx->stream>>>(a, csc, t0, (int)limit);
