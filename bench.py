@@ -763,24 +763,21 @@ def main():
     return 0
 
 
-# Per unit of work, from one ncu capture of this bench's own replayed step at
-# 64 roads (640 ROV paths a road, 192,000 forward units, 6,180,003 fitted
-# queries over the step's 48 kNN launches):
+# Per unit of work, from one ncu capture of a generation of 24 random roads x
+# 3 species on this bench's scene and options (768 ROV paths a road, 86,400
+# forward units, 2,244,925 fitted queries over the five selection launches):
 #   ncu --metrics smsp__inst_executed.sum,dram__bytes_read.sum,
-#       dram__bytes_write.sum,gpu__time_duration.sum --clock-control none
-#       -k "regex:k_knn_rov|k_rov_forward_union" -s 98 -c 49 --csv
-#       python bench.py --profile-only --roads 64 --no-rov-leg
-#       --surrogate-samples 0 --no-cpu-baseline --warmup 1
+#       dram__bytes_write.sum --clock-control none
+#       -k "regex:k_knn_rov|k_rov_forward_union" --csv
 # warp instructions executed and DRAM bytes (read + write) divided by the
-# units that step processed.
+# units that generation processed.
 #   k_rov_forward_union: unit = one 32-path tile of a road, one species, one year
-#   k_knn_rov: unit = one fitted regression query (k nearest points and the
-#              local normal equations)
+#   k_knn_rov: unit = one fitted regression query (its k nearest points)
 ROOF = {
-    "rov_forward_sparse": {"kernel": "k_rov_forward_union", "inst_per_unit": 46845.0,
-                           "bytes_per_unit": 280.0,
+    "rov_forward_sparse": {"kernel": "k_rov_forward_union", "inst_per_unit": 34174.0,
+                           "bytes_per_unit": 223.0,
                            "unit": "(32-path tile, species, year)"},
-    "knn": {"kernel": "k_knn_rov", "inst_per_unit": 1588.3, "bytes_per_unit": 22.8,
+    "knn": {"kernel": "k_knn_rov", "inst_per_unit": 377.0, "bytes_per_unit": 45.0,
             "unit": "fitted regression query"},
 }
 SMS, SCHEDULERS = 152, 4
@@ -789,7 +786,7 @@ SMS, SCHEDULERS = 152, 4
 def roofline_line(top, split, units, clock_mhz, mte_flops, mte_useful, bf16_peak, hbm_peak,
                   peak_kind):
     """Roofline of the step's dominant kernel.  The ROV's forward pass and
-    its kNN + regression kernel are both bound by instruction issue: their
+    its kNN selection are given against instruction issue: their
     data stay in shared memory and L1/L2 (DRAM idle), and the migration
     matrices are 2.3-5% non-zero (a dense tensor-core contraction would do
     20-40x the work).  `achieved` is warp instructions per second (ncu's

@@ -462,7 +462,8 @@ to_status to_select_samples(to_ctx ctx, int n_current, const double* current, in
                             const double* candidates, int n_dims, int n, int* sample);
 
 /* The autotuner's record: one line per tuned shape, "kind ne paths rs ->
- * choice (sparse ms, simt ms, tc ms)", -1 where a kernel was not feasible.
+ * choice (sparse ms, simt ms, tc ms)", -1 where a kernel was not feasible or,
+ * the matrices being sparse, not timed.
  * Writes at most len bytes (NUL-terminated); returns the number of lines. */
 int to_ctx_tuning(to_ctx ctx, char* buf, int len);
 
