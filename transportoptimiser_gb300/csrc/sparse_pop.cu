@@ -582,7 +582,7 @@ k_rov_forward_union(to_rov_args a, to_csc csc, int smem) {
 // that there is one loop a group and eight gathers in flight.
 // 40,000 paths, 2 species of 115 patches, 50 years: 1.93 -> 1.50 ms (one CTA
 // an SM with the next year's values in registers and two barriers a year
-// before); 256 roads of 3 species, 64 paths: 2.86 -> 2.57 ms.
+// before); 256 roads of 3 species, 64 paths: 2.86 -> 2.53 ms.
 // The values do not depend on which warp computes a group.
 // ---------------------------------------------------------------------------
 // a lane's paths and the arithmetic on them: two (packed) or one
