@@ -656,7 +656,7 @@ to_status launch_select(to_ctx ctx, const to_rov_args& a, int years) {
 }
 
 template <int D, bool REF>
-to_status launch_fit(to_ctx ctx, const to_rov_args& a, int t) {
+to_status launch_fit(to_ctx ctx, const to_rov_args& a, int t, bool ahead) {
     const int sms = ctx->sm_count > 0 ? ctx->sm_count : TO_SM_TARGET;
     const int tiles = a.G * ((a.Q + kT - 1) / kT);
     // few queries: at most two tiles an SM even if every grid query is
@@ -669,7 +669,7 @@ to_status launch_fit(to_ctx ctx, const to_rov_args& a, int t) {
     TO_CUDA(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     to_prof_begin(ctx, "knn_solve");
     const int units = wide ? tiles * (kT / kW) : tiles;
-    TO_CUDA(ctx, to_pdl_launch(k, units < 16 * sms ? units : 16 * sms, wide ? kWide : kT, smem,
+    TO_CUDA(ctx, to_pdl_launch(ahead, k, units < 16 * sms ? units : 16 * sms, wide ? kWide : kT, smem,
                                ctx->stream, a, t));
     to_prof_end(ctx);
     TO_LAUNCHED(ctx);
@@ -698,17 +698,17 @@ to_status knn_rov_select(to_ctx ctx, const to_rov_args& a, int years) {
     return to_set_error(ctx, TO_ERR_UNSUPPORTED, "regression dimension %d", d);
 }
 
-to_status knn_rov_fit(to_ctx ctx, const to_rov_args& a, int t) {
+to_status knn_rov_fit(to_ctx ctx, const to_rov_args& a, int t, bool ahead) {
     const int d = a.S + 1;
     if (a.sem == 0) {                          // one species
         if (d != 2) return to_set_error(ctx, TO_ERR_UNSUPPORTED, "reference semantics, %d dimensions", d);
-        return launch_fit<2, true>(ctx, a, t);
+        return launch_fit<2, true>(ctx, a, t, ahead);
     }
     switch (d) {
-        case 2: return launch_fit<2, false>(ctx, a, t);
-        case 3: return launch_fit<3, false>(ctx, a, t);
-        case 4: return launch_fit<4, false>(ctx, a, t);
-        default: return launch_fit<5, false>(ctx, a, t);
+        case 2: return launch_fit<2, false>(ctx, a, t, ahead);
+        case 3: return launch_fit<3, false>(ctx, a, t, ahead);
+        case 4: return launch_fit<4, false>(ctx, a, t, ahead);
+        default: return launch_fit<5, false>(ctx, a, t, ahead);
     }
 }
 

@@ -33,6 +33,7 @@
 #include "to_lsm_math.h"
 #include "to_rov.cuh"
 #include "to_rov_dev.cuh"
+#include "to_rov_years.h"
 #include "to_sparse.cuh"
 
 namespace {
@@ -941,31 +942,30 @@ to_status rov_backward(to_ctx ctx, const to_rov_args& args, int pblocks, int tpb
     const size_t bits = (a.touched && !a.bmap) ? (size_t)a.C * ((a.Q + 31) / 32) * 4 : 0;
     TO_CUDA(ctx, cudaFuncSetAttribute(k_lsm_prepare, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       kPrepBitmap));
-    int low = a.Y - 1, sel = a.Y - 1;          // first prepared year, first with neighbours
-    for (int t = a.Y - 2; t > 0; --t) {
-        if (t < low) {
-            low = t - a.slots + 1 > 1 ? t - a.slots + 1 : 1;
-            a.slot0 = low;
+    to_rov_years y(a.Y, a.slots, a.sel_slots);
+    while (y.next()) {
+        const int t = y.t;
+        if (y.prepare) {
+            a.slot0 = y.low;
             to_prof_begin(ctx, "lsm_prepare");
             TO_CUDA(ctx, cudaMemsetAsync(a.ntiles, 0, 2 * (size_t)a.slots * sizeof(int), ctx->stream));
-            k_lsm_prepare<<<dim3(a.nr, t - low + 1), kPrepThreads, bits, ctx->stream>>>(a);
+            k_lsm_prepare<<<dim3(a.nr, y.prepare), kPrepThreads, bits, ctx->stream>>>(a);
             to_prof_end(ctx);
             TO_LAUNCHED(ctx);
         }
         if (scan) {
-            if (t < sel) {
-                sel = t - a.sel_slots + 1 > low ? t - a.sel_slots + 1 : low;
-                a.sel0 = sel - low;
-                TO_TRY(knn_rov_select(ctx, a, t - sel + 1));
+            if (y.select) {
+                a.sel0 = y.sel - y.low;
+                TO_TRY(knn_rov_select(ctx, a, y.select));
             }
-            TO_TRY(knn_rov_fit(ctx, a, t));
+            TO_TRY(knn_rov_fit(ctx, a, t, y.fit_ahead()));
         } else {
             k_lsm_values<<<dim3((a.P + 255) / 256, a.G), 256, 0, ctx->stream>>>(a, t, t - a.slot0);
             TO_LAUNCHED(ctx);
             TO_TRY(knn_rov_grid(ctx, a, t));
         }
         to_prof_begin(ctx, "rov_backward");
-        TO_CUDA(ctx, to_pdl_launch(a.sem == 0 ? k_rov_backward_ref
+        TO_CUDA(ctx, to_pdl_launch(true, a.sem == 0 ? k_rov_backward_ref
                                    : a.S == 1 ? k_rov_backward<1, 3>
                                    : a.S == 2 ? k_rov_backward<2, 3>
                                    : a.S == 3 ? k_rov_backward<3, 3>

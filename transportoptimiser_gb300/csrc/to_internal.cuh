@@ -92,11 +92,13 @@ to_status to_read_device_flags(to_ctx ctx, int* flag);
 // that ran out, TO_ERR_UNSUPPORTED for the other device checks
 to_status to_check_device_flags(to_ctx ctx);
 
-// Programmatic dependent launch: a kernel launched so starts once every CTA
-// of the kernel before it has called to_pdl_next (or is done); what it does
-// before to_pdl_wait must not touch anything that kernel writes or reads.
-// Every thread calls to_pdl_wait before it exits, so that a kernel is done
-// only after all before it.
+// Programmatic dependent launch (`ahead`; otherwise a plain launch): a kernel
+// launched so starts once every CTA of the kernel before it has called
+// to_pdl_next (or is done); what it does before to_pdl_wait must not touch
+// anything that kernel writes or reads.  A CTA that is done has not thereby
+// made its stores visible: only the wait, or a plain launch in between, does
+// that.  Every thread calls to_pdl_wait before it exits, so that a kernel is
+// done only after all before it.
 #ifdef __CUDACC__
 __device__ __forceinline__ void to_pdl_next() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -105,8 +107,8 @@ __device__ __forceinline__ void to_pdl_wait() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 template <class... A, class... B>
-static inline cudaError_t to_pdl_launch(void (*kern)(A...), dim3 grid, int threads, size_t smem,
-                                        cudaStream_t stream, B... args) {
+static inline cudaError_t to_pdl_launch(bool ahead, void (*kern)(A...), dim3 grid, int threads,
+                                        size_t smem, cudaStream_t stream, B... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(threads);
@@ -116,7 +118,7 @@ static inline cudaError_t to_pdl_launch(void (*kern)(A...), dim3 grid, int threa
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = ahead ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kern, A(args)...);
 }
 #endif

@@ -156,10 +156,11 @@ size_t rov_scratch(to_rov_args& a, int max_roads, char* base);
 // sets the years to prepare and to select neighbours for at a time
 void rov_plan(to_rov_args& a, int max_roads);
 // the k nearest points of every listed grid query of `years` prepared years,
-// from slot a.sel0; then the local linear regressions of one of them
+// from slot a.sel0; then the local linear regressions of one of them (ahead:
+// not the kernel after a selection, to_rov_years.h)
 size_t knn_select_bytes(const to_rov_args& a, int max_roads);
 to_status knn_rov_select(to_ctx ctx, const to_rov_args& a, int years);
-to_status knn_rov_fit(to_ctx ctx, const to_rov_args& a, int t);
+to_status knn_rov_fit(to_ctx ctx, const to_rov_args& a, int t, bool ahead);
 // both for year t by the cell-grid search (groups of very many points)
 to_status knn_rov_grid(to_ctx ctx, const to_rov_args& a, int t);
 // generic kNN: ref dim-major [dim][n], query dim-major [dim][Q]
