@@ -1174,7 +1174,7 @@ k_rov_resim(to_rov_args a, to_csc csc, int t0, int smem) {
                 cptr[s * (NE + 1) + k] = e0 + csc.uptr[(size_t)s * (NP + 1) + (k <= NP ? k : NP)];
             for (int e = tid; e < n; e += blockDim.x) {
                 int4 v = csc.uent[(size_t)s * csc.ucap + e];
-                if (v.x == kNoOrigin) v.x = 0;      // its values are zero
+                if (v.x == kNoOrigin) v.x = 0;      // its values are zero: no term
                 v.x *= TP * (int)sizeof(float);
                 ue[e0 + e] = v;
             }
@@ -1281,6 +1281,30 @@ k_rov_resim(to_rov_args a, to_csc csc, int t0, int smem) {
                     g0 = j ? g0 + q0 : q0;
                     g1 = j ? g1 + q1 : q1;
                     g2 = j ? g2 + q2 : q2;
+                }
+                const float any = g0 + g1 + g2;
+                if (any != any) {
+                    // an infinite population times a zero: a control's sum
+                    // is over its own entries, so without the zeros
+#pragma unroll 1
+                    for (int j = 0; j < 4; ++j) {
+                        float q0 = 0.0f, q1 = 0.0f, q2 = 0.0f;
+#pragma unroll 1
+                        for (int e = up[j]; e < up[j + 1]; ++e) {
+                            const int4 en = ue[e];
+                            const float x = *reinterpret_cast<const float*>(
+                                reinterpret_cast<const unsigned char*>(cs) + en.x);
+                            if (en.y) q0 = fmaf(x, __int_as_float(en.y), q0);
+                            if (en.z) q1 = fmaf(x, __int_as_float(en.z), q1);
+                            if (en.w) q2 = fmaf(x, __int_as_float(en.w), q2);
+                        }
+                        mg[j * TP] = q0;
+                        if (C > 1) mg[(size_t)(NE + j) * TP] = q1;
+                        if (C > 2) mg[(size_t)(2 * NE + j) * TP] = q2;
+                        g0 = j ? g0 + q0 : q0;
+                        g1 = j ? g1 + q1 : q1;
+                        g2 = j ? g2 + q2 : q2;
+                    }
                 }
                 float* o = msum + ((size_t)s * C * NG + grp) * TP + lane;
                 o[0] = g0;
