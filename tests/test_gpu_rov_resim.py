@@ -56,3 +56,7 @@ def _same_where_the_forward_pass_is_finite(ctx, others, own):
 @pytest.mark.parametrize("own", [False, True])
 def test_infinite_patch_leaves_the_others_alone(ctx, own):
     _same_where_the_forward_pass_is_finite(ctx, 5000, own)
+
+
+def test_infinite_patch_stays_infinite(ctx):
+    _same_where_the_forward_pass_is_finite(ctx, 20, False)

@@ -1384,7 +1384,7 @@ k_rov_resim(to_rov_args a, to_csc csc, int t0, int smem) {
             for (int j = 0; j < 4; ++j) {
                 const float mv = mg[j * TP], cpk = capv[s * NE + grp * 4 + j];
                 const float gr = fmaf(s7 * zz[j], g, g), x = gr * (cpk - mv);
-                const float d = sums ? to_div_rcp(x, cpk, rcap[s * NE + grp * 4 + j]) : x / cpk;
+                const float d = sums ? to_div_rcp_inf(x, cpk, rcap[s * NE + grp * 4 + j]) : x / cpk;
                 v[j] = fmaxf(mv * (1.0f + d), 0.0f);
                 o[j * TP] = v[j];
             }

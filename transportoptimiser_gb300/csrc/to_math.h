@@ -278,6 +278,12 @@ TO_HD float to_div_rcp(float a, float b, float rb) {
     const float r = fmaf(-q, b, a);
     return fmaf(r, rb, q);
 }
+/* the same where q may overflow: an infinite q is the quotient, but its
+ * remainder is not a number */
+TO_HD float to_div_rcp_inf(float a, float b, float rb) {
+    const float d = to_div_rcp(a, b, rb);
+    return d == d ? d : a * rb;
+}
 
 /* ------------------------------------------------------------------------ */
 /* Stream layout.  A stream value is addressed by (stream, path, year,        */
