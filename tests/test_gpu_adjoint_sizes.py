@@ -54,3 +54,27 @@ def test_sweeps_match_fp64(ctx, N, nnz, P, Y, C, S):
               po.adjoint_forward(pr, ctl, cross, hz, th - d)) / (2 * h)
         scale = np.abs(J).max(axis=1)
         assert np.all(np.abs(J[:, i] - fd) <= 2e-3 * np.abs(fd) + 1e-3 * scale), (i, J[:, i], fd)
+
+
+def _overflow_problem(M, ip, cap):
+    pr, _, _, _ = _problem(1, 1, 3, 2, 1, 1, 0)
+    M = np.asarray(M, np.float32)
+    C, N = M.shape[0], M.shape[1]
+    prm = np.array([-0.05, -0.05, 0, 0, 0.5, 0, 0, 0], np.float32)
+    pr.update(species=[dict(N=N, params=prm, init_pops=np.array(ip, np.float32),
+                            caps=np.array(cap, np.float32), mmm=M)],
+              flows=np.zeros(C, np.float32))
+    return pr, [np.zeros((N, N), np.int32)], np.zeros(C)
+
+
+def _end(ctx, pr, cross, hz, ctl):
+    ctl = np.repeat(np.array(ctl, np.int32)[:, None], pr["n_paths"], axis=1)
+    pr = dict(pr, n_years=ctl.shape[0])
+    out, tape = FrozenPolicy(pr, ctl, cross, hz, ctx).forward(theta_from_problem(pr, hz), False)
+    return out[1]
+
+
+def test_overflowing_population_stays_infinite(ctx):
+    # 1e20 (1 + 0.05 (1e20 - 1)) overflows; infinite from then on
+    pr, cross, hz = _overflow_problem([[[1.0]]], [1e20], [1.0])
+    assert _end(ctx, pr, cross, hz, [0, 0, 0]) == np.inf

@@ -307,7 +307,8 @@ __device__ __forceinline__ f2 adj_migrated(const AdjArgs& a, const AdjTile& q, i
 
 // minus x / c.  A capacity with a normal reciprocal: multiply by it and
 // correct once, which gives the division's bits for quotients in the normal
-// range; any other capacity: divide.
+// range, and an infinite quotient without the correction, whose remainder is
+// not a number; any other capacity: divide.
 struct AdjCap {
     f2 c, nr;
     float cap;
@@ -324,7 +325,10 @@ __device__ __forceinline__ AdjCap adj_cap(float cap) {
 __device__ __forceinline__ f2 adj_neg_div(f2 x, const AdjCap& c) {
     if (c.normal) {
         const f2 nq = mul2(x, c.nr);
-        return fma2(fma2(nq, c.c, x), c.nr, nq);
+        float d0, d1, q0, q1;
+        unpack2(fma2(fma2(nq, c.c, x), c.nr, nq), d0, d1);
+        unpack2(nq, q0, q1);
+        return pack2(d0 == d0 ? d0 : q0, d1 == d1 ? d1 : q1);
     }
     float x0, x1;
     unpack2(x, x0, x1);
