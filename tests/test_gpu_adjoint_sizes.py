@@ -78,3 +78,14 @@ def test_overflowing_population_stays_infinite(ctx):
     # 1e20 (1 + 0.05 (1e20 - 1)) overflows; infinite from then on
     pr, cross, hz = _overflow_problem([[[1.0]]], [1e20], [1.0])
     assert _end(ctx, pr, cross, hz, [0, 0, 0]) == np.inf
+
+
+def test_infinite_patch_leaves_the_others_alone(ctx):
+    # the first patch overflows under control 1 and is left behind under
+    # control 2; the second receives from it under control 0 only
+    M = [[[1, 0], [1e-30, 1]], [[1e25, 0], [0, 1]], [[0, 0], [0, 1]]]
+    pr, cross, hz = _overflow_problem(M, [1e6, 500], [1e6, 1000])
+    x = 500.0
+    for _ in range(3):
+        x *= 1 - 0.05 * (1000 - x) / 1000
+    np.testing.assert_allclose(_end(ctx, pr, cross, hz, [1, 2, 2]), x, rtol=1e-5)

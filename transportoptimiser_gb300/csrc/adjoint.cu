@@ -291,18 +291,37 @@ __device__ __forceinline__ void adj_normals(const AdjArgs& a, const AdjTile& q, 
     to_normal4x2(q.ps0, q.ps1, to_stream_group(q.group0 + grp, q.stream_road, a.rk), a.rk, *q.tab, z);
 }
 
-// migrated state of patch k: the values of the lane's controls times the
-// origins' rows
-__device__ __forceinline__ f2 adj_migrated(const AdjArgs& a, const AdjTile& q, int k,
-                                           const AdjYear& y, const f2* rows) {
-    const int W = a.C + 1, e1 = q.up[k + 1];
+// sum over entries [e0, e1) of a list: the values of the lane's controls
+// times the other patches' rows.  A value is zero where another control has
+// the pair, which is no term of this control's: that matters where the row is
+// infinite, and the sum is then made again without the zeros.
+__device__ __forceinline__ f2 adj_list_sum(const float* val, const int* other, int W, int e0, int e1,
+                                           int c0, int c1, const f2* rows) {
     f2 acc = 0ull;
 #pragma unroll 4
-    for (int e = q.up[k]; e < e1; ++e) {
-        const float* v = a.uval + (size_t)e * W;
-        acc = fma2(pack2(v[y.c0], v[y.c1]), rows[a.ul[e] * 32], acc);
+    for (int e = e0; e < e1; ++e) {
+        const float* v = val + (size_t)e * W;
+        acc = fma2(pack2(v[c0], v[c1]), rows[other[e] * 32], acc);
     }
-    return acc;
+    float s0, s1;
+    unpack2(acc, s0, s1);
+    if (s0 == s0 && s1 == s1) return acc;
+    s0 = s1 = 0.0f;
+#pragma unroll 1
+    for (int e = e0; e < e1; ++e) {
+        const float v0 = val[(size_t)e * W + c0], v1 = val[(size_t)e * W + c1];
+        float x0, x1;
+        unpack2(rows[other[e] * 32], x0, x1);
+        if (v0 != 0.0f) s0 = fmaf(v0, x0, s0);
+        if (v1 != 0.0f) s1 = fmaf(v1, x1, s1);
+    }
+    return pack2(s0, s1);
+}
+
+// migrated state of patch k
+__device__ __forceinline__ f2 adj_migrated(const AdjArgs& a, const AdjTile& q, int k,
+                                           const AdjYear& y, const f2* rows) {
+    return adj_list_sum(a.uval, a.ul, a.C + 1, q.up[k], q.up[k + 1], y.c0, y.c1, rows);
 }
 
 // minus x / c.  A capacity with a normal reciprocal: multiply by it and
@@ -420,7 +439,21 @@ __device__ __forceinline__ f2 adj_hazard_chain(const AdjArgs& a, const AdjTile& 
         const f2 v = mul2(both2(__int_as_float(u.z)), pack2(v0[(size_t)e * W], v1[(size_t)e * W]));
         acc = fma2(mul2(v, mu[u.y + lane]), xt[u.x + lane], acc);
     }
-    return acc;
+    float s0, s1;
+    unpack2(acc, s0, s1);
+    if (s0 == s0 && s1 == s1) return acc;
+    s0 = s1 = 0.0f;                            // without the zeros, as adj_list_sum
+#pragma unroll 1
+    for (int e = q.up[0]; e < e1; ++e) {
+        const int4 u = a.uchain[e];
+        const float x = __int_as_float(u.z), w0 = v0[(size_t)e * W], w1 = v1[(size_t)e * W];
+        float m0, m1, x0, x1;
+        unpack2(mu[u.y + lane], m0, m1);
+        unpack2(xt[u.x + lane], x0, x1);
+        if (w0 != 0.0f) s0 = fmaf(x * w0 * m0, x0, s0);
+        if (w1 != 0.0f) s1 = fmaf(x * w1 * m1, x1, s1);
+    }
+    return pack2(s0, s1);
 }
 
 // the rows a year wrote become the rows the next one reads
@@ -561,13 +594,7 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_adj_pop_bwd(AdjArgs a, int t
                 for (int j = 0; j < 4; ++j) {
                     const int k = grp * 4 + j;
                     if (k >= q.N) break;
-                    const float* v0 = a.tval + c0;
-                    const float* v1 = a.tval + c1;
-                    f2 l = 0ull;
-                    const int e1 = q.tp[k + 1];
-#pragma unroll 4
-                    for (int e = q.tp[k]; e < e1; ++e)
-                        l = fma2(pack2(v0[(size_t)e * W], v1[(size_t)e * W]), x[a.tk[e] * 32 + lane], l);
+                    const f2 l = adj_list_sum(a.tval, a.tk, W, q.tp[k], q.tp[k + 1], c0, c1, x + lane);
                     if (t > t0)
                         nx[k * 32 + lane] = mt[k * 32 + lane] =
                             adj_through(q, y, q.cap[k], z[j], mt[k * 32 + lane], l, tt[k * 32],
