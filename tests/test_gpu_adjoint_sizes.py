@@ -89,3 +89,20 @@ def test_infinite_patch_leaves_the_others_alone(ctx):
     for _ in range(3):
         x *= 1 - 0.05 * (1000 - x) / 1000
     np.testing.assert_allclose(_end(ctx, pr, cross, hz, [1, 2, 2]), x, rtol=1e-5)
+
+
+def test_most_parameters(ctx):
+    """Eight processes, species and controls: 40 sensitivities an output."""
+    pr, cross, hz, ctl = _problem(4, 2, 5, 3, 8, 8, 1)
+    pr["uncert"] = np.tile(np.array([1, 1, 0.1, 0.2, 0.1, 0.2], np.float32), 8)
+    th = theta_from_problem(pr, hz)
+    assert th.size == 40
+    out, J = FrozenPolicy(pr, ctl, cross, hz, ctx).jacobian(th)
+    np.testing.assert_allclose(out, po.adjoint_forward(pr, ctl, cross, hz, th), rtol=1e-4)
+    for i in range(th.size):
+        h = 1e-4 * max(abs(th[i]), 1.0)
+        d = np.eye(th.size)[i] * h
+        fd = (po.adjoint_forward(pr, ctl, cross, hz, th + d) -
+              po.adjoint_forward(pr, ctl, cross, hz, th - d)) / (2 * h)
+        scale = np.abs(J).max(axis=1)
+        assert np.all(np.abs(J[:, i] - fd) <= 2e-3 * np.abs(fd) + 1e-3 * scale), (i, J[:, i], fd)

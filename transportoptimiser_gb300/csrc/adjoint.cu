@@ -765,7 +765,7 @@ to_status to_adjoint_forward(to_ctx ctx, const to_adjoint_problem* pr, const dou
     acc(rowb); acc(rowb * 4);
     if (!two_f || !two_b) acc(rowb);
     acc((size_t)S * Y * P * 4); acc((size_t)S * Y * P * 4); acc((size_t)P * 8);
-    acc((size_t)S * P * 8); acc((size_t)P * ntheta * 8); acc(64); acc(256); acc(256);
+    acc((size_t)S * P * 8); acc((size_t)P * ntheta * 8); acc(64); acc(256); acc(ntheta * 8);
     to_tape t = new to_tape_s();
     t->ctx = ctx;
     cudaError_t e = cudaMalloc(&t->buf, bytes);
@@ -809,7 +809,7 @@ to_status to_adjoint_forward(to_ctx ctx, const to_adjoint_problem* pr, const dou
     float* d_gout = (float*)take(64);
     double* d_out = (double*)take(256);
     t->d_out = d_out;
-    t->d_grad = (double*)take(256);
+    t->d_grad = (double*)take(ntheta * 8);
     a.theta = d_th; a.uncert = d_unc; a.flows = d_fl; a.fuel_costs = d_fc; a.fuel_idx = d_fi;
     a.ore_content = d_oc; a.ore_sd = d_os; a.controls = d_ctl; a.n_patches = d_np;
     a.params = d_prm; a.init_pops = d_ip; a.caps = d_cp; a.uptr = d_up; a.tptr = d_tp;
