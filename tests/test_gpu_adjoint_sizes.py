@@ -8,6 +8,7 @@ import numpy as np
 import pytest
 
 from oracle import pyoracle as po
+from transportoptimiser_gb300._capi import TransOptError
 from transportoptimiser_gb300.adjoint import FrozenPolicy, theta_from_problem
 
 pytestmark = pytest.mark.gpu
@@ -106,3 +107,18 @@ def test_most_parameters(ctx):
               po.adjoint_forward(pr, ctl, cross, hz, th - d)) / (2 * h)
         scale = np.abs(J).max(axis=1)
         assert np.all(np.abs(J[:, i] - fd) <= 2e-3 * np.abs(fd) + 1e-3 * scale), (i, J[:, i], fd)
+
+
+def test_processes_and_controls_out_of_range(ctx):
+    """Profits of processes that do not exist are refused; under a control that
+    does not exist nothing earns or survives."""
+    pr, cross, hz, ctl = _problem(4, 2, 5, 3, 2, 1, 1)
+    th = theta_from_problem(pr, hz)
+    for bad in (dict(fuel_idx=np.array([2], np.int32)), dict(fuel_idx=np.array([-1], np.int32)),
+                dict(demand_idx=2), dict(fuel_costs=np.ones(2, np.float32),
+                                         fuel_idx=np.array([0, 1], np.int32))):
+        with pytest.raises(TransOptError) as e:
+            FrozenPolicy(dict(pr, **bad), ctl, cross, hz, ctx).forward(th, False)
+        assert e.value.status == 1
+    out, _ = FrozenPolicy(pr, np.full_like(ctl, 1 << 30), cross, hz, ctx).forward(th, False)
+    assert np.all(out == 0.0)

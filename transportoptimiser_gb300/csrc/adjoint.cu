@@ -68,7 +68,7 @@ struct AdjArgs {
     // uptr[s][k + 1]) are the patches it receives from, ascending; the
     // transposed lists those it sends to.  Entry e holds the values of all
     // controls at the current hazards (k_adj_values) and a zero, which a
-    // control outside 0 .. C - 1 reads: under it nothing migrates
+    // control outside 0 .. C - 1 reads: under it nothing migrates or earns
     const int *uptr, *tptr;             // [S][NP + 1]
     const int *ul, *tk;                 // [E] the other patch
     const int* tsrc;                    // [E] the transposed entry's place in the first lists
@@ -131,7 +131,7 @@ __device__ void exog_path(const AdjArgs& a, int p, bool tangents, double* pv_out
         const float dem = a.demand_idx >= 0 ? U[a.demand_idx] : 1.0f;
         const float pi = base * dem;
         const int ctl = a.controls[(size_t)t * a.P + p];
-        const float w = disc * a.flows[ctl];
+        const float w = (unsigned)ctl < (unsigned)a.C ? disc * a.flows[ctl] : 0.0f;
         pv += (double)(w * pi);
         if (tangents) {
             for (int f = 0; f < a.nF; ++f) dpi_du[a.fuel_idx[f]] += a.fuel_costs[f] * dem;
@@ -681,6 +681,12 @@ to_status to_adjoint_forward(to_ctx ctx, const to_adjoint_problem* pr, const dou
     if (S <= 0 || S > 8 || C <= 0 || C > 8 || U < 0 || U > 8 || P <= 0 || Y <= 0 ||
         rp->n_commodities > 8 || !pr->controls || !pr->crossings || !pr->hazard)
         return TO_ERR_INVALID;
+    // every process the profits read exists (as the ROV's entry checks)
+    if (rp->n_fuels < 0 || rp->n_commodities < 0 || rp->n_fuels + rp->n_commodities > U ||
+        rp->demand_idx >= U)
+        return TO_ERR_INVALID;
+    for (int f = 0; f < rp->n_fuels; ++f)
+        if (rp->fuel_idx[f] < 0 || rp->fuel_idx[f] >= U) return TO_ERR_INVALID;
     const int ntheta = 2 * U + 2 * S + C;
     for (int i = 0; i < ntheta; ++i)
         if (!std::isfinite(theta[i])) return to_set_error(ctx, TO_ERR_NONFINITE, "theta %d", i);
