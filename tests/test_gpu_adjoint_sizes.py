@@ -122,3 +122,34 @@ def test_processes_and_controls_out_of_range(ctx):
         assert e.value.status == 1
     out, _ = FrozenPolicy(pr, np.full_like(ctl, 1 << 30), cross, hz, ctx).forward(th, False)
     assert np.all(out == 0.0)
+
+
+def test_many_paths_tape(ctx):
+    """More (species, tile) pairs than CTAs at work at a time: the sweeps equal
+    those of a few paths, and the tape keeps checkpoints by path, not a
+    segment's scratch (the free memory before and while it is held)."""
+    torch = pytest.importorskip("torch")
+    pr, cross, hz, ctl = _problem(64, 2, 30000, 21, 2, 2, 5)
+    th = theta_from_problem(pr, hz)
+    model = FrozenPolicy(pr, ctl, cross, hz, ctx)
+    free = torch.cuda.mem_get_info()[0]
+    out, tape = model.forward(th)
+    held = free - torch.cuda.mem_get_info()[0]
+    S, P, Y = 2, 30000, 21
+    paths = 4 * (S * (Y // 10 + 1 + 10) * 64 + S * Y * 2 + Y) + 8 * (1 + S + th.size)
+    assert held <= paths * P + (8 << 20), held      # checkpoints and one segment; lists and rounding
+    g = model.backward(tape, [1.0, 2.0, -1.0])
+    model.free(tape)
+    parts = np.zeros_like(g)
+    few = np.zeros(3)
+    for p0 in range(0, P, 5000):                    # Philox streams are a path's own: masks, not slices
+        w = slice(p0, p0 + 5000)
+        sub = np.full_like(ctl, 2)                  # no control: nothing earns or migrates
+        sub[:, w] = ctl[:, w]
+        m = FrozenPolicy(pr, sub, cross, hz, ctx)
+        o, t = m.forward(th)
+        few += o
+        parts += m.backward(t, [1.0, 2.0, -1.0])
+        m.free(t)
+    np.testing.assert_allclose(out, few, rtol=1e-12)
+    np.testing.assert_allclose(g, parts, rtol=1e-9, atol=1e-12)

@@ -80,11 +80,14 @@ struct AdjArgs {
     to_round_keys rk;
     // tape
     float* ckpt;                        // [S][Y/K + 1][NP][P]
-    f2* segx;                           // [S][tiles][K][NP][32] a segment's states
-    f2* segm;                           // [S][tiles][K][NP][32] and migrated states
-    f2* terms;                          // [S][tiles][2][2][NP][32] a year's terms of mu_s and v_s
-    f2* lam;                            // [S][tiles][NP][32] adjoint of a segment's first state
-    f2* rows;                           // [S][tiles][NP][32] rows shared memory has no room for
+    // scratch of a sweep's CTAs, which take one (species, tile) after another:
+    // a tile's own would be 25 rows a path beside the 6 of its checkpoints
+    int slots;                          // of the scratch: the most CTAs at work
+    f2* segx;                           // [slots][K][NP][32] a segment's states
+    f2* segm;                           // [slots][K][NP][32] and migrated states
+    f2* terms;                          // [slots][2][2][NP][32] a year's terms of mu_s and v_s
+    f2* lam;                            // [slots][NP][32] adjoint of a segment's first state
+    f2* rows;                           // [slots][NP][32] rows shared memory has no room for
     float* gtab;                        // [S][Y][P] growth-rate mean used in year t
     float* gdot;                        // [S][Y][P] its derivative in mu_s
     double* pv;                         // [P]
@@ -244,12 +247,15 @@ struct AdjTile {
     const to_bm_tables* tab;
 };
 
-__device__ __forceinline__ AdjTile adj_tile(const AdjArgs& a, const to_bm_tables* tab) {
+__host__ __device__ inline int adj_tiles(const AdjArgs& a) { return (a.P + kAdjPaths - 1) / kAdjPaths; }
+// item: the (species, tile), tiles of a species in a row
+__device__ __forceinline__ AdjTile adj_tile(const AdjArgs& a, const to_bm_tables* tab, int item) {
     AdjTile q;
-    q.s = blockIdx.y;
+    const int tiles = adj_tiles(a);
+    q.s = item / tiles;
     q.N = a.n_patches[q.s];
     q.N4 = (q.N + 3) & ~3;
-    q.p0 = blockIdx.x * kAdjPaths + (threadIdx.x & 31);
+    q.p0 = (item - q.s * tiles) * kAdjPaths + (threadIdx.x & 31);
     q.p1 = q.p0 + 32;
     q.live0 = q.p0 < a.P;
     q.live1 = q.p1 < a.P;
@@ -471,16 +477,11 @@ __device__ __forceinline__ void adj_turn(f2*& x, f2*& nx, int n, int two) {
 
 // forward: end population per path and checkpoints.  `two`: shared memory
 // holds both years' rows, else the next year's go through global memory
-__global__ void __launch_bounds__(kAdjThreads, 2) k_adj_pop_fwd(AdjArgs a, int two) {
-    extern __shared__ __align__(16) unsigned char sm_adj[];
-    __shared__ to_bm_tables s_tab;
+__device__ __forceinline__ void adj_forward(const AdjArgs& a, AdjTile q, int two, unsigned char* sm) {
     const int tid = threadIdx.x, lane = tid & 31;
-    AdjTile q = adj_tile(a, &s_tab);
-    f2* x = reinterpret_cast<f2*>(sm_adj);                     // [N][32]
-    f2* nx = two ? x + (size_t)q.N * 32
-                 : a.rows + ((size_t)q.s * gridDim.x + blockIdx.x) * a.NP * 32;
+    f2* x = reinterpret_cast<f2*>(sm);                         // [N][32]
+    f2* nx = two ? x + (size_t)q.N * 32 : a.rows + (size_t)blockIdx.x * a.NP * 32;
     const float* ip = a.init_pops + (size_t)q.s * a.NP;
-    to_bm_load(s_tab);
     for (int i = tid; i < q.N * 32; i += kAdjThreads) x[i] = both2(ip[i >> 5]);
     __syncthreads();
     for (int t = 0; t < a.Y; ++t) {
@@ -510,36 +511,38 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_adj_pop_fwd(AdjArgs a, int t
     }
 }
 
+__global__ void __launch_bounds__(kAdjThreads, 2) k_adj_pop_fwd(AdjArgs a, int two) {
+    extern __shared__ __align__(16) unsigned char sm_adj[];
+    __shared__ to_bm_tables s_tab;
+    to_bm_load(s_tab);
+    for (int item = blockIdx.x; item < a.S * adj_tiles(a); item += gridDim.x) {
+        __syncthreads();                       // the one before is done with
+        adj_forward(a, adj_tile(a, &s_tab, item), two, sm_adj);
+    }
+}
+
 // backward: reverse sweep over the K-year segments.  The rows other patches
 // read are a segment's states while it is recomputed, then mu: a warp turns
 // year t's mu into lambda_t of four patches and that at once into their
 // year t - 1's mu, so a year takes one barrier either way.  In the reverse
 // years warps take groups from a counter, one of them after the growth sums.
-__global__ void __launch_bounds__(kAdjThreads, 2) k_adj_pop_bwd(AdjArgs a, int two, int ntheta) {
-    extern __shared__ __align__(16) unsigned char sm_adj[];
-    __shared__ to_bm_tables s_tab;
-    __shared__ int s_grab[2];
-    // the sweep is linear in the species' output weight: a zero weight
-    // contributes exactly zero (the per-path gradients start zeroed)
-    const float w = a.gout[1 + blockIdx.y];
-    if (w == 0.0f) return;
+__device__ __forceinline__ void adj_backward(const AdjArgs& a, AdjTile q, float w, int two, int ntheta,
+                                             unsigned char* sm, int* s_grab) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, W = a.C + 1;
-    AdjTile q = adj_tile(a, &s_tab);
     const int NG = q.N4 / 4;
-    const size_t tile = (size_t)q.s * gridDim.x + blockIdx.x, seg = (size_t)a.NP * 32;
-    f2* gsum = reinterpret_cast<f2*>(sm_adj);                      // [2][32] v_s, mu_s
+    const size_t slot = blockIdx.x, seg = (size_t)a.NP * 32;
+    f2* gsum = reinterpret_cast<f2*>(sm);                          // [2][32] v_s, mu_s
     float* gh = reinterpret_cast<float*>(gsum + 64);               // [W][64]
     float* gy = gh + (size_t)W * kAdjPaths;                        // [kCk][64] a year's
     f2* x = reinterpret_cast<f2*>(gy + kCk * kAdjPaths);           // [N][32]
-    f2* nx = two ? x + (size_t)q.N * 32 : a.rows + tile * seg;     // [N][32]
-    f2* lam = a.lam + tile * seg;
-    f2* segx = a.segx + tile * kCk * seg;
-    f2* segm = a.segm + tile * kCk * seg;      // in the reverse years mu takes a year's place
-    f2* terms = a.terms + tile * 4 * seg;                          // [t & 1][v_s, mu_s][NP][32]
+    f2* nx = two ? x + (size_t)q.N * 32 : a.rows + slot * seg;     // [N][32]
+    f2* lam = a.lam + slot * seg;
+    f2* segx = a.segx + slot * kCk * seg;
+    f2* segm = a.segm + slot * kCk * seg;      // in the reverse years mu takes a year's place
+    f2* terms = a.terms + slot * 4 * seg;                          // [t & 1][v_s, mu_s][NP][32]
     if (tid < 64) gsum[tid] = 0ull;
     for (int i = tid; i < W * kAdjPaths; i += kAdjThreads) gh[i] = 0.0f;
     if (tid < 2) s_grab[tid] = 0;
-    to_bm_load(s_tab);
     for (int i = tid; i < q.N * 32; i += kAdjThreads) lam[i] = both2(w);
     int turn = 0;                                                  // of the counters
     const int nseg = (a.Y + kCk - 1) / kCk;
@@ -626,12 +629,28 @@ __global__ void __launch_bounds__(kAdjThreads, 2) k_adj_pop_bwd(AdjArgs a, int t
     __syncthreads();
     const float* gs = reinterpret_cast<const float*>(gsum);
     for (int i = tid; i < (2 + a.C) * kAdjPaths; i += kAdjThreads) {
-        const int what = i / kAdjPaths, j = i - what * kAdjPaths, p = blockIdx.x * kAdjPaths + j;
+        const int what = i / kAdjPaths, j = i - what * kAdjPaths, p = q.p0 - lane + j;
         if (p >= a.P) continue;
         double* gp = a.gpath + (size_t)p * ntheta;
         // species blocks are disjoint, so each species writes its own entries
         if (what < 2) gp[2 * a.U + (1 - what) * a.S + q.s] = (double)gs[what * 64 + (j & 31) * 2 + (j >> 5)];
         else atomicAdd(&gp[2 * a.U + 2 * a.S + what - 2], (double)gh[(what - 2) * kAdjPaths + j]);
+    }
+}
+
+__global__ void __launch_bounds__(kAdjThreads, 2) k_adj_pop_bwd(AdjArgs a, int two, int ntheta) {
+    extern __shared__ __align__(16) unsigned char sm_adj[];
+    __shared__ to_bm_tables s_tab;
+    __shared__ int s_grab[2];
+    to_bm_load(s_tab);
+    for (int item = blockIdx.x; item < a.S * adj_tiles(a); item += gridDim.x) {
+        const AdjTile q = adj_tile(a, &s_tab, item);
+        // the sweep is linear in the species' output weight: a zero weight
+        // contributes exactly zero (the per-path gradients start zeroed)
+        const float w = a.gout[1 + q.s];
+        if (w == 0.0f) continue;
+        __syncthreads();                       // the one before is done with
+        adj_backward(a, q, w, two, ntheta, sm_adj, s_grab);
     }
 }
 
@@ -743,7 +762,10 @@ to_status to_adjoint_forward(to_ctx ctx, const to_adjoint_problem* pr, const dou
     }
     const size_t nE = ul.size() > 0 ? ul.size() : 1;
     const int tiles = (P + kAdjPaths - 1) / kAdjPaths;
-    const size_t rowb = (size_t)S * tiles * NP * 32 * 8;       // rows of every (species, tile)
+    // two CTAs an SM at most are at work (their registers)
+    const int sms = ctx->sm_count > 0 ? ctx->sm_count : TO_SM_TARGET;
+    const int slots = S * tiles < 2 * sms ? S * tiles : 2 * sms;
+    const size_t rowb = (size_t)slots * NP * 32 * 8;           // one row of each
     const bool two_f = adj_fwd_smem(maxN, true) + kAdjStatic <= ctx->smem_optin;
     const bool two_b = adj_bwd_smem(maxN, C, true) + kAdjStatic <= ctx->smem_optin;
     std::vector<int> np(S);
@@ -802,6 +824,7 @@ to_status to_adjoint_forward(to_ctx ctx, const to_adjoint_problem* pr, const dou
     a.uval = (float*)take(nE * (C + 1) * 4); a.tval = (float*)take(nE * (C + 1) * 4);
     float* d_bh = (float*)take(C * 4);
     a.ckpt = (float*)take((size_t)S * (Y / kCk + 1) * NP * P * 4);
+    a.slots = slots;
     a.segx = (f2*)take(rowb * kCk);
     a.segm = (f2*)take(rowb * kCk);
     a.lam = (f2*)take(rowb);
@@ -856,7 +879,7 @@ to_status to_adjoint_forward(to_ctx ctx, const to_adjoint_problem* pr, const dou
     if (a.E > 0) k_adj_values<<<(a.E + 255) / 256, 256, 0, ctx->stream>>>(a);
     k_adj_growth<<<dim3((P + 127) / 128, S), 128, 0, ctx->stream>>>(a);
     to_prof_begin(ctx, "adjoint_forward");
-    k_adj_pop_fwd<<<dim3(tiles, S), kAdjThreads, smf, ctx->stream>>>(a, two_f ? 1 : 0);
+    k_adj_pop_fwd<<<two_f ? S * tiles : slots, kAdjThreads, smf, ctx->stream>>>(a, two_f ? 1 : 0);
     to_prof_end(ctx);
     k_col_mean<<<1, 256, 0, ctx->stream>>>(P, 1, a.pv, d_out);
     for (int s = 0; s < S; ++s)
@@ -891,8 +914,7 @@ to_status to_adjoint_backward(to_ctx ctx, to_tape t, const double* grad_outputs,
     TO_CUDA(ctx, cudaFuncSetAttribute(k_adj_pop_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)(ctx->smem_optin - kAdjStatic)));
     to_prof_begin(ctx, "adjoint_backward");
-    k_adj_pop_bwd<<<dim3((P + kAdjPaths - 1) / kAdjPaths, S), kAdjThreads, smb, ctx->stream>>>(
-        a, t->two_b ? 1 : 0, ntheta);
+    k_adj_pop_bwd<<<a.slots, kAdjThreads, smb, ctx->stream>>>(a, t->two_b ? 1 : 0, ntheta);
     to_prof_end(ctx);
     TO_LAUNCHED(ctx);
     std::vector<double> g(ntheta);
