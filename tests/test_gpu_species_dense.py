@@ -35,3 +35,15 @@ def test_species_model_dense_outputs(ctx, side, tile, res, habitable, cap, sem):
     for k in ("trans", "surv"):
         np.testing.assert_allclose(got[k], ref[k], rtol=1e-12, atol=0)
     np.testing.assert_allclose(got["mmm"], ref["mmm"], rtol=1e-6, atol=1.1e-5)
+
+
+def test_species_model_holds_its_own_patches_only(ctx):
+    """The outputs own their memory: nothing of max_patches' size stays alive."""
+    sc = synth.mte_road(0)
+    sp, road = sc.species[0], sc.roads[0]
+    hab = sc.hab_map(road)
+    m = sg.createSpeciesModel(hab, sc.pop_map(sp, hab), sc.W, sc.H, sc.res, sp.habitats, road.colmajor(),
+                              road.G, sp.hazard, sp.lambda_mean, sem=1, max_patches=2000, ctx=ctx)
+    N, C = m["N"], len(sp.hazard)
+    for k, shape in (("crossings", (N, N)), ("trans", (N, N)), ("surv", (C, N, N)), ("mmm", (C, N, N))):
+        assert m[k].base is None and m[k].flags.owndata and m[k].shape == shape, k

@@ -124,10 +124,10 @@ def createSpeciesModel(hab_map, pop_map, W, H, res, habitats, road_colmajor, G, 
     res_ = {k: v[:N].copy() for k, v in b.items()}
     res_["N"] = N
     res_["n_transitions"] = out.n_transitions
-    res_["crossings"] = big["crossings"][:N * N].reshape(N, N)
-    res_["trans"] = big["trans"][:N * N].reshape(N, N)
-    res_["surv"] = big["surv"][:Cn * N * N].reshape(Cn, N, N)
-    res_["mmm"] = big["mmm"][:Cn * N * N].reshape(Cn, N, N)
+    for k, shape in (("crossings", (N, N)), ("trans", (N, N)), ("surv", (Cn, N, N)),
+                     ("mmm", (Cn, N, N))):
+        big[k].resize(shape, refcheck=False)    # in place: the rest goes back
+        res_[k] = big[k]
     res_["init_pops"] = res_["pop"].astype(np.float32)
     res_["caps"] = res_["cap"].astype(np.float32)
     res_["iar"] = iar
