@@ -605,11 +605,12 @@ to_status to_simulate_mte(to_ctx ctx, const to_mte_problem* prob,
     }
     TO_TRY(to_k::mte_stats(ctx, a, S, d_stats));
     std::vector<double> st((size_t)S * 5);
-    TO_TRY(to_download_parts(ctx, d_end, 1, 1, (size_t)S * P, [=](size_t) { return end_pops; }));
     TO_TRY(d2h(ctx, st.data(), d_stats, st.size()));
     TO_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    // a bounded wait that ran out (tensor-core kernel) or a plan check
+    // a bounded wait that ran out (tensor-core kernel) or a plan check: the
+    // caller's arrays stay as they are
     TO_TRY(to_check_device_flags(ctx));
+    TO_TRY(to_download_parts(ctx, d_end, 1, 1, (size_t)S * P, [=](size_t) { return end_pops; }));
     if (stats)
         for (int s = 0; s < S; ++s) {
             stats[s].mean = st[5 * s];
