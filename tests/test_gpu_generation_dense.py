@@ -26,3 +26,25 @@ def test_auto_on_dense_matrices(ctx, lam, trial):
     # end populations: FP32 sums in one order on both kernels (3xTF32: 1e-5)
     np.testing.assert_allclose(auto[:, :, 2:7], ref[:, :, 2:7], rtol=1e-4, atol=1e-6)
     gen.close()
+
+
+@pytest.mark.parametrize("lam", [0.075, 0.02])
+def test_tuned_shape_builds_its_models_once(ctx, lam):
+    """After the trial a generation's species models are built in one pass,
+    whichever kernel the record names, with the results of the first."""
+    sc = synth.generation(11, n_roads=2)
+    for sp in sc.species:
+        sp.lambda_mean = lam
+    gen = Generation(sc, max_roads=2, max_patches=512, ctx=ctx)
+    packed = pack_roads(sc, sc.roads)
+    opts = gen.opts(48 + int(1000 * lam), 5, seed=4, sem=1, migration=MIG_AUTO)
+    first = gen.evaluate(packed, opts)
+    for _ in range(2):
+        ctx.profile(True)
+        n0 = ctx.kernel_time("species_links")[1]
+        again = gen.evaluate(packed, opts)
+        n1 = ctx.kernel_time("species_links")[1]
+        ctx.profile(False)
+        assert n1 - n0 == 1
+        assert np.array_equal(again, first, equal_nan=True)      # no ROV, no penalty: NaN
+    gen.close()

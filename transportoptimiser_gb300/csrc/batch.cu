@@ -74,6 +74,7 @@ struct to_gen_s {
     // to_gen_end_pops): its shape and which migration-matrix forms it wrote
     int last_R = 0, last_paths = 0;
     bool last_dense = false, last_csc = false;
+    bool dense_first = false;            // the automatic choice was a dense kernel last time
     bool graph_dense = false, graph_csc = false;
     double* d_iar = nullptr;             // [RS][C] initial animals at risk
     // MTE penalty (to_scene_set_penalty): z = inverse normal CDF of
@@ -310,13 +311,19 @@ void tuned_record(to_ctx ctx, const to_mte_args& m, int RS, int NE) {
     ctx->tune.push_back(te);
 }
 
-to_status tuned_choice(to_ctx ctx, to_gen g, const to_mte_args& m, int RS, int NE,
-                       bool sparse_ok, bool tc_ok, int* choice) {
+// the choice of an earlier trial of the shape, or -1
+int tuned_known(to_ctx ctx, const to_mte_args& m, int RS, int NE, bool sparse_ok) {
     const uint64_t key = tune_key(m, RS, NE, sparse_ok);
     for (const auto& e : ctx->tune)
-        if (e.key == key && e.kind == 0) { *choice = e.choice; return TO_OK; }
+        if (e.key == key && e.kind == 0) return e.choice;
+    return -1;
+}
+
+to_status tuned_choice(to_ctx ctx, to_gen g, const to_mte_args& m, int RS, int NE,
+                       bool sparse_ok, bool tc_ok, int* choice) {
     to_ctx_s::tune_entry te;
-    te.key = key; te.kind = 0; te.ne = NE; te.paths = m.n_paths; te.n_rs = RS;
+    te.key = tune_key(m, RS, NE, sparse_ok);
+    te.kind = 0; te.ne = NE; te.paths = m.n_paths; te.n_rs = RS;
     te.ms[0] = te.ms[1] = te.ms[2] = -1.0f;
     cudaEvent_t e0, e1;
     TO_CUDA(ctx, cudaEventCreate(&e0));
@@ -360,14 +367,18 @@ to_status evaluate_direct(to_ctx ctx, to_gen g, int R, const int* cell_off,
     to_model_args a;
     model_args(g, R, cell_off, cells, seg_off, segs, o, ctx, a);
     // The model kernel writes the packed matrices itself wherever the sparse
-    // kernel may run.  The dense form is made only if a dense kernel is asked
-    // for or has to be timed (the ROV stage reads the packed matrices of
-    // every control, so a scene with a ROV always runs the sparse kernel).
+    // kernel may run (the ROV stage reads the packed matrices of every
+    // control, so a scene with a ROV always runs the sparse kernel).  The
+    // dense form is made if a dense kernel is asked for, was chosen for the
+    // scene's last generation - the packed form is then made from it - or
+    // turns out to be needed, by a second pass of the model.
     const bool try_sparse = (o->migration == TO_MIG_AUTO || o->migration == TO_MIG_SPARSE_FP32 ||
                              g->rov_on);
-    bool dense = !try_sparse;
-    if (try_sparse) csc_direct(g, a);
+    const bool trial = o->migration == TO_MIG_AUTO && !g->rov_on;
+    bool dense = !try_sparse || (trial && g->dense_first);
+    if (!dense) csc_direct(g, a);
     TO_TRY(to_k::species_model(ctx, a, RS));
+    if (try_sparse && dense) TO_TRY(to_k::pack_csc(ctx, g->d_mmm, NP, g->C, g->d_np, RS, g->csc));
     // the widest species model decides the tile shape of the path kernel
     int* d_max = reinterpret_cast<int*>(g->d_results + (size_t)g->max_roads * S * TO_RESULT_STRIDE);
     k_max_int<<<1, 1024, 0, ctx->stream>>>(RS, g->d_np, d_max);
@@ -396,22 +407,28 @@ to_status evaluate_direct(to_ctx ctx, to_gen g, int R, const int* cell_off,
     TO_TRY(grow_end(ctx, g, (size_t)RS * o->mte_paths));
     to_mte_args m = mte_args(ctx, g, o, NE);
     int choice;
-    if (o->migration == TO_MIG_SPARSE_FP32 || g->rov_on) choice = CH_SPARSE;
-    else if (o->migration == TO_MIG_TC_3XTF32) choice = CH_TC;
-    else if (o->migration == TO_MIG_SIMT_FP32) choice = CH_SIMT;
+    if (!trial)
+        choice = g->rov_on ? CH_SPARSE
+               : o->migration == TO_MIG_TC_3XTF32 ? CH_TC
+               : o->migration == TO_MIG_SIMT_FP32 ? CH_SIMT : CH_SPARSE;
     else if (sparse_ok && (long)mm[2] * 10 <= (long)NE * NE) {
-        // No trial where no matrix has a tenth of its entries: the sparse
-        // kernel's time grows with the entries, the dense kernels' does not
-        // (256 roads at 2.5%: 2.6 against 30.6 ms; they meet above 20%), and
-        // the trial would take a hundred milliseconds and the dense matrices.
+        // No trial where no matrix has more than a tenth of the NE x NE
+        // entries that the dense kernels work through for each of them: the
+        // sparse kernel's time grows with the entries, theirs does not (256
+        // roads at 2.5%: 2.6 against 30.6 ms; they meet above 20%), and the
+        // trial would take a hundred milliseconds and the dense matrices.
         choice = CH_SPARSE;
         tuned_record(ctx, m, RS, NE);
     } else {
-        a.csc_ptr = nullptr;
-        TO_TRY(to_k::species_model(ctx, a, RS));
-        dense = true;
-        TO_TRY(tuned_choice(ctx, g, m, RS, NE, sparse_ok, NE <= 512, &choice));
+        choice = tuned_known(ctx, m, RS, NE, sparse_ok);
+        if (choice != CH_SPARSE && !dense) {
+            a.csc_ptr = nullptr;
+            TO_TRY(to_k::species_model(ctx, a, RS));
+            dense = true;
+        }
+        if (choice < 0) TO_TRY(tuned_choice(ctx, g, m, RS, NE, sparse_ok, NE <= 512, &choice));
     }
+    if (trial) g->dense_first = choice != CH_SPARSE && NP <= 1024;     // pack_csc's limit
     TO_TRY(tail(ctx, g, m, RS, choice, d_results_out));
     if (plan) { plan[0] = NE; plan[1] = g->csc.cap_smem; plan[2] = choice; }
     g->last_R = R; g->last_paths = o->mte_paths;
