@@ -50,3 +50,9 @@ def test_epochs_match_host_adam(ctx, n, batch):
     # the steps differ by a rounding of the bias corrections at most
     np.testing.assert_allclose(got, p, rtol=1e-5, atol=1e-6)
     np.testing.assert_allclose(curve, losses, rtol=1e-6)
+
+
+def test_more_tiles_than_sms_match_host_adam(ctx):
+    """A batch of 154 tiles, which are not all at work at once: steps of three
+    launches in place of the epoch's one."""
+    test_epochs_match_host_adam(ctx, 20000, 19600)

@@ -5,10 +5,13 @@ number of species; both semantics and both algorithms, with and without the
 surfaces; ties (profits all equal: no distance is a number), states that
 take few values, species below their thresholds; the cell-grid search above
 32,768 paths; few queries and many (more than two tiles of 128 an SM)."""
+import ctypes
+
 import numpy as np
 import pytest
 
 from oracle import pyoracle as po
+from transportoptimiser_gb300 import _capi
 from transportoptimiser_gb300 import simulate_gpu as sg
 
 pytestmark = pytest.mark.gpu
@@ -69,3 +72,33 @@ def test_regressions_equal_oracle(ctx, S, R, P, Y, sem, algo, N, surf, kind):
     same(np.reshape(g["adj_pops"], (Y, S, P))[1:], np.reshape(o["adj_pops"], (Y, S, P))[1:])
     if surf:
         same(g["regression"], o["regression"])
+
+
+def test_year_zero_is_zero(ctx):
+    """No kernel writes year 0 of the profits and populations; the call returns
+    zeros there whatever an earlier one left in the scratch, also where one
+    road of a batch asks for them and the others do not."""
+    big = _problem(2, 8, 9000, 12, 1, 4, 40, "")
+    sg.simulateROVCUDA(big, ctx=ctx)
+    for sem, S in ((0, 1), (1, 2)):
+        g = sg.simulateROVCUDA(_problem(S, 6, 500, 5, sem, 4, 9, ""), ctx=ctx)
+        assert np.all(g["unit_profits"][:500] == 0.0) and np.all(g["adj_pops"][:S * 500] == 0.0)
+        assert np.all(g["adj_pops"][S * 500:] > 0.0)
+        sg.simulateROVCUDA(big, ctx=ctx)
+    prs, keep = zip(*[sg.rov_ctypes(dict(_problem(2, 6, 500, 5, 1, 4, 9, ""), road=r)) for r in range(3)])
+    pops, prof = np.full(5 * 2 * 500, -7.0), np.full(5 * 500, -7.0)
+    res = (_capi.RovResult * 3)()
+    res[1].adj_pops = _capi.ptr(pops, ctypes.c_double)
+    res[2].unit_profits = _capi.ptr(prof, ctypes.c_double)
+    assert ctx.lib.to_simulate_rov_batch(ctx.handle, 3, (_capi.RovProblem * 3)(*prs), res) == 0
+    assert np.all(pops[:1000] == 0.0) and np.all(pops[1000:] > 0.0)
+    assert np.all(prof[:500] == 0.0) and not np.any(prof[500:] == -7.0)
+    one = sg.simulateROVCUDA(dict(_problem(2, 6, 500, 5, 1, 4, 9, ""), road=1), ctx=ctx)
+    np.testing.assert_array_equal(pops, one["adj_pops"])
+
+
+@pytest.mark.parametrize("S,R,P,Y,sem,algo,N,surf,kind", [
+    (1, 120, 400, 4, 0, 4, 12, True, ""), (4, 11, 300, 3, 1, 4, 6, False, "")])
+def test_many_tiles_equal_oracle(ctx, S, R, P, Y, sem, algo, N, surf, kind):
+    """More than two tiles an SM for the fewest and the most dimensions."""
+    test_regressions_equal_oracle(ctx, S, R, P, Y, sem, algo, N, surf, kind)
