@@ -11,7 +11,8 @@
 // ever idles over a short list and the per-query bookkeeping - scans,
 // selections, solves - costs a thread what it used to cost a warp.  The
 // neighbours do not depend on the values of later years, so they are
-// selected (k_knn_rov) for as many years at once as fill the GPU:
+// selected (k_knn_rov) for as many years at once as half a gigabyte holds the
+// lists of, every grid query counted (a road: all; 256 roads: one):
 //   1 a histogram of a sample of the squared distances, 8 buckets an octave,
 //     estimates the k-th;
 //   2 a histogram of all of them, 32 buckets an octave around the estimate,
@@ -28,10 +29,11 @@
 // as the values; a distance that is not a number comes last).
 //
 // What bounds it: instruction issue and, at the few warps an SM that the
-// histograms (256 bytes a query) and the sums (registers) leave room for,
-// the latency of dependent instructions.  Two kernels instead of one for
-// that reason: selecting needs no registers to speak of, fitting no shared
-// memory.  256 roads, 24.7 M queries of about 256 points and k = 65 (a
+// histograms (256 bytes a query) and the sums (registers, up to three
+// species; four take 880 bytes a thread of local memory for the solve) leave
+// room for, the latency of dependent instructions.  Two kernels instead of
+// one for that reason: selecting needs no registers to speak of, fitting no
+// shared memory.  256 roads, 24.7 M queries of about 256 points and k = 65 (a
 // generation): kNN and solves 44.1 -> 19.9 ms (select 10.5, fit 9.4; 528 warp
 // instructions a query, 1,588 with a warp a query).  One road of 10,000
 // paths, 100,000 queries of about 3,300 points: 4.2 -> 1.2 ms.

@@ -597,7 +597,8 @@ namespace {
 // the regressions stay in L2): 47 -> 29 us a year of 196,608 paths of three
 // species, 21 -> 10 us of 10,000 paths of two.  A year's fit and decisions
 // follow one another 48 times, so each starts while the one before runs and
-// loads what does not depend on it (to_pdl_wait): 19 -> 14 us a year of those
+// loads what does not depend on it (to_pdl_wait; the fit after a selection
+// starts at its end): 19 -> 14 us a year of those
 // 10,000 paths, 25 -> 17 us of 2,000 under the reference's semantics.
 template <int S, int CU>
 __global__ void __launch_bounds__(128) k_rov_backward(to_rov_args a, int t) {

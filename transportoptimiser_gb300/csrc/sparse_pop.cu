@@ -8,13 +8,14 @@
 // ~8 per column on the benchmark grids), so a dense (paths x N)(N x N)
 // product would spend >95% of its work on zeros.  Here:
 //   * k_pack_csc packs every (road, species, control) matrix once;
-//   * a CTA owns 32 paths (lane = path) and keeps their populations
-//     ([patch][lane], conflict-free) and the CSC lists in shared memory for
-//     all years; its warps split the destination patches in groups of four,
-//     so one Philox call gives the four growth normals a lane needs;
+//   * a CTA works on a tile of 16, 32 or 64 paths (a lane is one path, or two
+//     on packed FP32) and keeps their populations ([patch][lane],
+//     conflict-free) and, where they fit, the lists in shared memory for all
+//     years; its warps take the destination patches in groups of four, so one
+//     Philox call gives the four growth normals a path needs;
 //   * each destination sums its non-zeros in ascending origin order with
-//     explicit FMAs - the same chain as the dense form (skipped terms are
-//     exact zeros), so results stay bit-identical to the oracle;
+//     explicit FMAs - the same chain as the dense form (skipped and padding
+//     terms are exact zeros), so results stay bit-identical to the oracle;
 //   * patch totals use the fixed grouped order ((v0+v1)+v2)+v3, groups
 //     ascending.
 #include <cstring>
@@ -1419,6 +1420,10 @@ to_status pack_csc(to_ctx ctx, const float* mmm, int NP, int C, const int* n_pat
     return TO_OK;
 }
 
+// What is admitted: models whose lists fit beside one path a lane (8 bytes an
+// entry) with their groups' sums, up to 512 patches.  The kernel lays a model
+// out by mte_bytes and can leave its lists in global memory, so this is a rule
+// of choice - longer lists go to the dense kernels - and not its limit.
 size_t mte_sparse_smem(int NE, int cap_smem) {
     if (NE > 32 * kMaxG * 4) return ~size_t(0);  // 32 warps of kMaxG groups of four
     const int NG = NE / 4;
@@ -1444,8 +1449,6 @@ to_status mte_sparse(to_ctx ctx, to_mte_args a, int n_rs, to_csc csc) {
     if (a.npe <= 0) a.npe = a.npad;
     if (!a.flags) a.flags = ctx->d_flags;
     const int NE = a.npe, NE4 = (NE + 3) & ~3;
-    if (csc.cap_smem & 1)       // the 8-byte entries must leave the column pointers 16-byte aligned
-        return to_set_error(ctx, TO_ERR_INVALID, "packed capacity %d is odd", csc.cap_smem);
     size_t smem = mte_sparse_smem(NE, csc.cap_smem);
     if (smem > ctx->smem_optin)
         return to_set_error(ctx, TO_ERR_UNSUPPORTED, "sparse MTE needs %zu B", smem);

@@ -84,8 +84,9 @@ __device__ __forceinline__ void decide_terminal(const to_rov_args& a, const floa
 
 // A control's payoff: this year's plus the discounted value, capped at zero.
 // Summed in FP32: the reference's sum in double rounded to float is the same
-// value, since 53 bits are two more than twice 24 (S. Figueroa, "When is
-// double rounding innocuous?", 1995), and FP64 is slow on this part.
+// value, since 53 bits are at least the 2 * 24 + 2 that a sum takes (S.
+// Figueroa, "When is double rounding innocuous?", 1995), and FP64 is slow on
+// this part.
 __device__ __forceinline__ float payoff(float now, float later) {
     return now + (later > 0.0f ? 0.0f : later);
 }
